@@ -1,0 +1,51 @@
+"""The pruned transforms of the long range (csrc/fourier.cu) over grid sizes: every radix and number of
+passes, rows that are odd or even in number, lines shorter and longer than one tile, periods of
+different lengths, and both fields from one transform.  The long-range fields at the nodes (with a weak
+filter, so that every kept mode counts) against the CPU restatement; FP64 to 1e-10 as everywhere, mixed to
+2e-6 (sixteen times the 1.2e-7 of the 32-bit grid sums and transforms; a wrong twiddle or row is above 1e-3)."""
+
+import math
+
+import numpy as np
+import pytest
+
+L = 2 * math.pi
+
+# (Ns, sigma): FFT sizes 8 .. 768 per dimension, with 2, 3 and 4 passes, radices 2 .. 32
+SIZES = [((6, 6, 6), 1.3), ((12, 17, 31), 1.5), ((32, 20, 18), 1.5), ((50, 30, 36), 1.5), ((33, 48, 40), 2.0),
+         ((54, 100, 25), 1.25), ((120, 16, 12), 2.0), ((16, 160, 14), 1.5), ((14, 12, 192), 1.5), ((256, 12, 10), 1.5),
+         ((12, 256, 12), 1.5), ((10, 14, 256), 1.5), ((20, 12, 512), 1.5), ((400, 10, 12), 1.25), ((12, 10, 500), 1.25)]
+
+
+def system(vp):
+    rng = np.random.default_rng(8)
+    return [vp.curves.ring(n, 0.7 + 0.5 * rng.random(), L * rng.random(3), vp.curves.random_rotation(rng)) for n in (9, 24, 31)]
+
+
+def params(vp, Ns, sigma, Ls=(L, 1.25 * L, 0.8 * L), **kw):
+    m = 3 if min(Ns) < 10 else 4
+    return vp.ParamsBiotSavart(Gamma=1.3, a=1e-8, splitting=vp.GaussianSplitting(Ls=Ls, alpha=12.0, rcut=L / 4, Ns=Ns),
+                               backend_long=vp.NonuniformFFTsBackend(sigma, m), **kw)
+
+
+def rel(a, b):
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Ns,sigma", SIZES)
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("mixed", 2e-6)])
+def test_long_range_over_grid_sizes(vp, oracle, Ns, sigma, precision, tol):
+    fs = system(vp)
+    p = params(vp, Ns, sigma, precision=precision)
+    v, s, _ = oracle.compute_on_nodes(p, fs, velocity=True, streamfunction=True, LIA=False, shortrange=False)
+    cache = vp.init_cache(p)
+    try:
+        for names in (("velocity", "streamfunction"), ("velocity",), ("streamfunction",)):
+            out = {n: [np.zeros((len(f), 3)) for f in fs] for n in names}
+            vp.compute_on_nodes_(out, cache, fs, LIA=False, shortrange=False)
+            for n, want in (("velocity", v), ("streamfunction", s)):
+                if n in out:
+                    assert rel(np.concatenate(out[n]), want) <= tol, (n, names)
+    finally:
+        cache.close()

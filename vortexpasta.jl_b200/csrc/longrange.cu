@@ -1125,8 +1125,6 @@ int longrange_init(vpbs_handle* h) {
     const bool mixed = P.precision == VPBS_PRECISION_MIXED;
     const size_t rsz = mixed ? sizeof(float) : sizeof(double);  // grid precision
     if ((rc = ensure(h, h->grid_r, rsz * 3 * S.ngrid, "real grid"))) return rc;
-    if ((rc = ensure(h, h->grid_c, 2 * rsz * 3 * S.ncgrid, "complex grid"))) return rc;
-    if ((rc = ensure(h, h->grid_c2, 2 * rsz * 3 * S.ncgrid, "complex grid (streamfunction)"))) return rc;
     if ((rc = ensure(h, h->uhat, sizeof(double2) * 3 * S.nmodes, "uhat"))) return rc;
     // separable deconvolution factors 1/psi_hat and 1/psi_hat * exp(-k^2 / 4 alpha^2) (the
     // Kaiser-Bessel filter is not separable: the Fourier kernel applies it per mode)
@@ -1154,6 +1152,11 @@ int longrange_init(vpbs_handle* h) {
     for (int d = 0; d < 6; ++d) all.insert(all.end(), tab[d].begin(), tab[d].end());
     if ((rc = check_cuda(h, cudaMemcpy(h->decx.p, all.data(), sizeof(double) * tot, cudaMemcpyHostToDevice), "copy tables")))
         return rc;
+    if ((rc = fourier_init(h))) return rc;
+    if (h->fplan) return 0;
+    // sizes the pruned transforms do not take (lines longer than a block can hold, or of one factor)
+    if ((rc = ensure(h, h->grid_c, 2 * rsz * 3 * S.ncgrid, "complex grid"))) return rc;
+    if ((rc = ensure(h, h->grid_c2, 2 * rsz * 3 * S.ncgrid, "complex grid (streamfunction)"))) return rc;
     int nrev[3] = {S.n[2], S.n[1], S.n[0]};
     if ((rc = check_fft(h, cufftPlanMany(&h->plan_r2c, 3, nrev, nullptr, 1, (int)S.ngrid, nullptr, 1, (int)S.ncgrid,
                                          mixed ? CUFFT_R2C : CUFFT_D2Z, 3), "plan r2c")))
@@ -1166,6 +1169,7 @@ int longrange_init(vpbs_handle* h) {
 }
 
 void longrange_free(vpbs_handle* h) {
+    fourier_free(h);
     if (h->have_plans) {
         cufftDestroy(h->plan_r2c);
         cufftDestroy(h->plan_c2r);
@@ -1299,40 +1303,59 @@ int longrange_compute_t(vpbs_handle* h, int fields) {
         h->launches++;
         if ((rc = check_cuda(h, cudaGetLastError(), "spread kernel"))) return rc;
     }
-    {
+    if (h->fplan) {
         StageScope st(h, ST_FFT_FORWARD);
-        if ((rc = check_fft(h, cufftSetStream(h->plan_r2c, h->stream), "set stream"))) return rc;
-        if ((rc = check_fft(h, exec_r2c(h->plan_r2c, grid, gc), "exec r2c"))) return rc;
+        if ((rc = fourier_forward(h, grid))) return rc;
+    } else {
+        {
+            StageScope st(h, ST_FFT_FORWARD);
+            if ((rc = check_fft(h, cufftSetStream(h->plan_r2c, h->stream), "set stream"))) return rc;
+            if ((rc = check_fft(h, exec_r2c(h->plan_r2c, grid, gc), "exec r2c"))) return rc;
+        }
+        double kmax = INFINITY;
+        for (int d = 0; d < 3; ++d) kmax = fmin(kmax, 2.0 * kPi * ((P.Ns[d] - 1) / 2) / P.L[d]);
+        const double pref = P.Gamma / (P.L[0] * P.L[1] * P.L[2]);
+        const bool kb = P.splitting == VPBS_SPLITTING_KAISER_BESSEL;
+        const double* t = (const double*)h->decx.p;
+        const double* dec0 = t;
+        const double* dec1 = dec0 + S.nkx;
+        const double* dec2 = dec1 + S.Ns[1];
+        const double* decE0 = dec2 + S.Ns[2];
+        const double* decE1 = decE0 + S.nkx;
+        const double* decE2 = decE1 + S.Ns[1];
+        {
+            StageScope st(h, ST_FOURIER);
+            fourier_kernel<C><<<grid_for(S.ncgrid, 256), 256, 0, h->stream>>>(
+                S, pref, sx[0], sx[1], sx[2], P.truncate_spherical, kmax * kmax, fields, kb ? P.kb_beta * P.kb_beta : 0.0,
+                P.rcut * P.rcut, kb ? P.kb_beta / std::sinh(P.kb_beta) : 0.0, dec0, dec1, dec2, decE0, decE1,
+                decE2, gc, gc2, (double2*)h->uhat.p, 1);
+            h->launches++;
+            h->have_uhat = true;
+            if ((rc = check_cuda(h, cudaGetLastError(), "fourier kernel"))) return rc;
+        }
+        if ((rc = check_fft(h, cufftSetStream(h->plan_c2r, h->stream), "set stream"))) return rc;
     }
-    double kmax = INFINITY;
-    for (int d = 0; d < 3; ++d) kmax = fmin(kmax, 2.0 * kPi * ((P.Ns[d] - 1) / 2) / P.L[d]);
-    const double pref = P.Gamma / (P.L[0] * P.L[1] * P.L[2]);
-    const bool kb = P.splitting == VPBS_SPLITTING_KAISER_BESSEL;
-    const double* t = (const double*)h->decx.p;
-    const double* dec0 = t;
-    const double* dec1 = dec0 + S.nkx;
-    const double* dec2 = dec1 + S.Ns[1];
-    const double* decE0 = dec2 + S.Ns[2];
-    const double* decE1 = decE0 + S.nkx;
-    const double* decE2 = decE1 + S.Ns[1];
-    {
-        StageScope st(h, ST_FOURIER);
-        fourier_kernel<C><<<grid_for(S.ncgrid, 256), 256, 0, h->stream>>>(
-            S, pref, sx[0], sx[1], sx[2], P.truncate_spherical, kmax * kmax, fields, kb ? P.kb_beta * P.kb_beta : 0.0,
-            P.rcut * P.rcut, kb ? P.kb_beta / std::sinh(P.kb_beta) : 0.0, dec0, dec1, dec2, decE0, decE1,
-            decE2, gc, gc2, (double2*)h->uhat.p, 1);
-        h->launches++;
-        h->have_uhat = true;
-        if ((rc = check_cuda(h, cudaGetLastError(), "fourier kernel"))) return rc;
-    }
-    if ((rc = check_fft(h, cufftSetStream(h->plan_c2r, h->stream), "set stream"))) return rc;
     const int32_t* order = (const int32_t*)h->dst_order.p;
     for (int f = 0; f < 2; ++f) {
         const int field = f == 0 ? VPBS_STREAMFUNCTION : VPBS_VELOCITY;
         if (!(fields & field)) continue;
         C* in = field == VPBS_VELOCITY ? gc : gc2;
         double* out = (double*)(field == VPBS_VELOCITY ? h->vel.p : h->psi.p);
-        {
+        if (h->fplan) {
+            // the first field takes the transform of the grid and keeps the coefficients (the second one
+            // starts from them: the grid's transform has been overwritten by then)
+            const bool both = fields == (VPBS_STREAMFUNCTION | VPBS_VELOCITY), first = !both || field == VPBS_STREAMFUNCTION;
+            const bool keep = both || !h->skip_uhat;
+            {
+                StageScope st(h, ST_FOURIER);
+                const FourierOp op = {first ? FourierOp::GRID : FourierOp::COEFFICIENTS,
+                                      field == VPBS_VELOCITY ? FourierOp::VELOCITY : FourierOp::STREAMFUNCTION, keep, 1};
+                if ((rc = fourier_operator(h, op))) return rc;
+                h->have_uhat = keep;
+            }
+            StageScope st(h, ST_FFT_INVERSE);
+            if ((rc = fourier_inverse(h, grid))) return rc;
+        } else {
             StageScope st(h, ST_FFT_INVERSE);
             if ((rc = check_fft(h, exec_c2r(h->plan_c2r, in, grid), "exec c2r"))) return rc;
         }
@@ -1423,12 +1446,17 @@ int longrange_interpolate_t(vpbs_handle* h, int quantity, double* out) {
     const double* dec0 = (const double*)h->decx.p;
     const double* dec1 = dec0 + S.nkx;
     const double* dec2 = dec1 + S.Ns[1];
-    field_grid_kernel<C><<<grid_for(S.ncgrid, 256), 256, 0, h->stream>>>(S, sx[0], sx[1], sx[2], quantity, dec0, dec1,
-                                                                         dec2, (const double2*)h->uhat.p, gc);
-    h->launches++;
-    if ((rc = check_cuda(h, cudaGetLastError(), "field grid kernel"))) return rc;
-    if ((rc = check_fft(h, cufftSetStream(h->plan_c2r, h->stream), "set stream"))) return rc;
-    if ((rc = check_fft(h, exec_c2r(h->plan_c2r, gc, grid), "exec c2r"))) return rc;
+    if (h->fplan) {
+        if ((rc = fourier_operator(h, FourierOp{FourierOp::COEFFICIENTS, quantity, 0, 0}))) return rc;
+        if ((rc = fourier_inverse(h, grid))) return rc;
+    } else {
+        field_grid_kernel<C><<<grid_for(S.ncgrid, 256), 256, 0, h->stream>>>(S, sx[0], sx[1], sx[2], quantity, dec0, dec1,
+                                                                             dec2, (const double2*)h->uhat.p, gc);
+        h->launches++;
+        if ((rc = check_cuda(h, cudaGetLastError(), "field grid kernel"))) return rc;
+        if ((rc = check_fft(h, cufftSetStream(h->plan_c2r, h->stream), "set stream"))) return rc;
+        if ((rc = check_fft(h, exec_c2r(h->plan_c2r, gc, grid), "exec c2r"))) return rc;
+    }
     if ((rc = check_cuda(h, cudaMemsetAsync(out, 0, sizeof(double) * 3 * h->Np, h->stream), "memset"))) return rc;
     const int32_t* order = (const int32_t*)h->dst_order.p;
     auto launch_interp = [&](auto kern) {

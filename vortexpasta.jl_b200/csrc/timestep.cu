@@ -60,7 +60,10 @@ extern "C" int vpbs_rk4_step(vpbs_handle* h, double* nodes, double dt) {
         if ((rc = geometry_from_filaments(h, h->nfil, offs, stage_nodes, h->nmax, s > 0))) return rc;
         h->li_valid = h->K.lia_fraction > 0;
         if ((rc = process_point_charges(h))) return rc;
-        if ((rc = vpbs_compute(h, VPBS_VELOCITY, VPBS_LIA_TRUE, 1, 1, 0.0))) return rc;
+        h->skip_uhat = s < 3;  // the last stage's long-range coefficients are the ones the step leaves behind
+        rc = vpbs_compute(h, VPBS_VELOCITY, VPBS_LIA_TRUE, 1, 1, 0.0);
+        h->skip_uhat = false;
+        if (rc) return rc;
         const int mode = s == 0 ? 0 : (s < 3 ? 1 : 2);
         rk_update_kernel<<<grid_for(3 * Np, 256), 256, 0, h->stream>>>(Np, mode, a[s], (const double*)h->vel.p, nodes,
                                                                       vs, tmp);

@@ -125,6 +125,16 @@ struct LRSizes {
     int kernel;      // VPBS_NUFFT_*
 };
 
+// What the Fourier-space pass does between the forward and the inverse z transforms (fourier.cu).
+struct FourierOp {
+    enum Source { GRID, COEFFICIENTS };  // the spread grid's transform, or the held coefficients
+    enum Quantity { VORTICITY = 1, STREAMFUNCTION = 2, VELOCITY = 3 };
+    int source, quantity;
+    int store;  // keep the vorticity coefficients (GRID only)
+    int ewald;  // apply the long-range filter
+};
+struct FourierPlan;
+
 // Host <-> device staging of flat node and output arrays goes in chunks of at least
 // kStageChunk bytes (at most kStageEvents of them), host copies overlapping the transfers.
 constexpr size_t kStageChunk = (size_t)4 << 20;
@@ -184,7 +194,10 @@ struct vpbs_handle {
     int nbrick[3] = {0, 0, 0};
     cufftHandle plan_r2c = 0, plan_c2r = 0, plan_c2r_6 = 0;
     bool have_plans = false;
+    vpbs::FourierPlan* fplan = nullptr;  // pruned transforms (null: cuFFT)
+    vpbs::DevBuf fft_tw;                 // their twiddle tables
     bool have_uhat = false;
+    bool skip_uhat = false;  // the coefficients of this evaluation are overwritten before anyone can read them
 
     // outputs (SoA, 3*Np each)
     vpbs::DevBuf vel, psi;
@@ -251,6 +264,13 @@ int add_local_integrals(vpbs_handle* h, int fields);
 int longrange_init(vpbs_handle* h);
 void longrange_free(vpbs_handle* h);
 int longrange_compute(vpbs_handle* h, int fields);  // adds into h->vel / h->psi
+
+// fourier.cu: pruned transforms (h->fplan set by fourier_init where the sizes allow them)
+int fourier_init(vpbs_handle* h);
+void fourier_free(vpbs_handle* h);
+int fourier_forward(vpbs_handle* h, const void* grid);
+int fourier_operator(vpbs_handle* h, const FourierOp& op);
+int fourier_inverse(vpbs_handle* h, void* grid);
 
 // stage timing
 enum Stage {
