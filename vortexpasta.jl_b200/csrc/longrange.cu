@@ -112,8 +112,6 @@ __device__ __forceinline__ double es_kernel_w(double u, double beta, double edge
     return exp(beta * (sqrt(s) - 1.0)) - edge;
 }
 
-constexpr int kSpreadBatch = 32;
-
 // Complex value of the grid precision T from double parts.
 template <typename C>
 __device__ __forceinline__ C mkc(double x, double y);
@@ -121,51 +119,6 @@ template <>
 __device__ __forceinline__ double2 mkc<double2>(double x, double y) { return make_double2(x, y); }
 template <>
 __device__ __forceinline__ float2 mkc<float2>(double x, double y) { return make_float2((float)x, (float)y); }
-
-// Type-1 spreading with global atomics (fallback when the grid cannot be tiled into bricks):
-// each block takes kSpreadBatch points; kernel values are tabulated in shared memory, then
-// every thread adds the charges along x-lines of the (2m)^3 footprint.
-template <typename T>
-__global__ void __launch_bounds__(256) spread_kernel_atomic(
-    LRSizes S, int64_t Nq, const double* __restrict__ src, double sx0, double sx1, double sx2,
-    T* __restrict__ grid) {
-    __shared__ double phi[kSpreadBatch][3][2 * kMaxHalfSupport];
-    __shared__ int i0s[kSpreadBatch][3];
-    __shared__ double qs[kSpreadBatch][3];
-    const int w = 2 * S.m;
-    const int64_t pbase = (int64_t)blockIdx.x * kSpreadBatch;
-    const int np = (int)((Nq - pbase) < kSpreadBatch ? (Nq - pbase) : kSpreadBatch);
-    const double scale[3] = {sx0, sx1, sx2};
-    for (int idx = threadIdx.x; idx < np * 3; idx += blockDim.x) {
-        const int p = idx / 3, d = idx % 3;
-        const int64_t j = pbase + p;
-        const double h = 2.0 * kPi / S.n[d];
-        const double xh = (src[d * Nq + j] * scale[d]) / h;
-        const int i0 = (int)floor(xh) - S.m + 1;
-        i0s[p][d] = i0;
-        for (int s = 0; s < w; ++s) phi[p][d][s] = es_kernel(xh - (i0 + s), S.m, S.beta, S.edge, S.kernel);
-        qs[p][d] = src[(3 + d) * Nq + j];
-    }
-    __syncthreads();
-    const int per = w * w;
-    const int64_t ng = S.ngrid;
-    for (int item = threadIdx.x; item < np * per; item += blockDim.x) {
-        const int p = item / per, l = item % per;
-        const int sy = l % w, sz = l / w;
-        const int iz = wrapi(i0s[p][2] + sz, S.n[2]);
-        const int iy = wrapi(i0s[p][1] + sy, S.n[1]);
-        const double fyz = phi[p][2][sz] * phi[p][1][sy];
-        const double q0 = qs[p][0] * fyz, q1 = qs[p][1] * fyz, q2 = qs[p][2] * fyz;
-        const int64_t row = ((int64_t)iz * S.n[1] + iy) * S.n[0];
-        for (int sx = 0; sx < w; ++sx) {
-            const int ix = wrapi(i0s[p][0] + sx, S.n[0]);
-            const double f = phi[p][0][sx];
-            atomicAdd(grid + row + ix, (T)(q0 * f));
-            atomicAdd(grid + ng + row + ix, (T)(q1 * f));
-            atomicAdd(grid + 2 * ng + row + ix, (T)(q2 * f));
-        }
-    }
-}
 
 // Fused Fourier-space kernel over the r2c grid [n2][n1][n0/2+1] (C: double2 or float2; the
 // arithmetic is FP64 in both forms, only the grids are stored in the grid precision).
@@ -299,82 +252,6 @@ __global__ void spread_bin_scatter_kernel(LRSizes S, int64_t Nq, const double* _
         const int i0 = (int)floor(xh) - S.m + 1;
         foot[3 * pos + d] = wrapi(i0, S.n[d]);
         for (int s = 0; s < w; ++s) out[3 + d * w + s] = (T)es_kernel(xh - (i0 + s), S.m, S.beta, S.edge, S.kernel);
-    }
-}
-
-// Shared-memory brick spreading: one CTA per brick keeps the brick's three components in
-// shared memory (x rows padded to B+1 against bank conflicts), adds the part of every nearby
-// footprint that falls inside the brick with shared-memory atomics (one warp per point, lanes
-// over the footprint's (y, z) lines), then writes the brick to the grid with plain stores.
-constexpr int kBrickThreads = 256;
-
-template <int B, typename T>
-__global__ void __launch_bounds__(kBrickThreads) spread_brick_kernel(
-    LRSizes S, int nb0, int nb1, int nb2, const int32_t* __restrict__ bin_start, const T* __restrict__ binned,
-    const int32_t* __restrict__ foot, T* __restrict__ grid) {
-    extern __shared__ __align__(16) unsigned char tile_raw[];
-    T* tile = reinterpret_cast<T*>(tile_raw);  // [3][B][PZ] with rows of RX values
-    __shared__ T phw[kBrickThreads / 32][3 + 6 * kMaxHalfSupport];
-    constexpr int RX = B + 1;        // x-row stride (bank spread along y)
-    constexpr int PZ = B * RX + 8;   // z-plane stride (16-word bank shift between planes)
-    constexpr int TC = B * PZ;       // doubles per component
-    const int w = 2 * S.m;
-    const int stride = 3 + 3 * w;
-    const int bx = blockIdx.x % nb0;
-    const int by = (blockIdx.x / nb0) % nb1;
-    const int bz = blockIdx.x / (nb0 * nb1);
-    const int bs[3] = {bx * B, by * B, bz * B};
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < 3 * TC; i += kBrickThreads) tile[i] = (T)0;
-    __syncthreads();
-    T* ph = phw[warp];  // [q0 q1 q2 | phi_x[w] | phi_y[w] | phi_z[w]]
-    for (int nbr = 0; nbr < 8; ++nbr) {
-        const int cx = (bx - (nbr & 1) + nb0) % nb0;
-        const int cy = (by - ((nbr >> 1) & 1) + nb1) % nb1;
-        const int cz = (bz - ((nbr >> 2) & 1) + nb2) % nb2;
-        const int b = (cz * nb1 + cy) * nb0 + cx;
-        const int64_t p1 = bin_start[b + 1];
-        for (int64_t j = bin_start[b] + warp; j < p1; j += kBrickThreads / 32) {
-            // footprint offset relative to the brick (periodic) and overlap range, per dimension
-            int o[3], lo[3], hi[3];
-            bool empty = false;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                o[d] = foot[3 * j + d] - bs[d];
-                if (o[d] >= B) o[d] -= S.n[d];
-                lo[d] = o[d] < 0 ? -o[d] : 0;
-                hi[d] = B - o[d] < w ? B - o[d] : w;
-                empty = empty || lo[d] >= hi[d];
-            }
-            if (empty) continue;  // warp-uniform
-            for (int it = lane; it < stride; it += 32) ph[it] = binned[j * stride + it];
-            __syncwarp();
-            const T q0 = ph[0], q1 = ph[1], q2 = ph[2];
-            const T* phx = ph + 3;
-            const T* phy = phx + w;
-            const T* phz = phy + w;
-            const int ny = hi[1] - lo[1], nz = hi[2] - lo[2];
-            for (int l = lane; l < ny * nz; l += 32) {
-                const int sy = lo[1] + l % ny, sz = lo[2] + l / ny;
-                const T f = phy[sy] * phz[sz];
-                T* row = tile + (o[2] + sz) * PZ + (o[1] + sy) * RX + o[0];
-                for (int sx = lo[0]; sx < hi[0]; ++sx) {
-                    const T g = f * phx[sx];
-                    atomicAdd(row + sx, q0 * g);
-                    atomicAdd(row + TC + sx, q1 * g);
-                    atomicAdd(row + 2 * TC + sx, q2 * g);
-                }
-            }
-            __syncwarp();
-        }
-    }
-    __syncthreads();
-    const int64_t ng = S.ngrid;
-    for (int i = threadIdx.x; i < 3 * B * B * B; i += kBrickThreads) {
-        const int c = i / (B * B * B), r = i % (B * B * B);
-        const int x = r % B, y = (r / B) % B, z = r / (B * B);
-        grid[c * ng + ((int64_t)(bs[2] + z) * S.n[1] + (bs[1] + y)) * S.n[0] + bs[0] + x] =
-            tile[c * TC + z * PZ + y * RX + x];
     }
 }
 
@@ -908,124 +785,237 @@ __global__ void __launch_bounds__(kTcThreads, 2) spread_tc_kernel(LRSizes S, int
     if (warp == 0) tc::tmem_dealloc(tmem, 128);
 }
 
-// Register-column brick spreading for 16^3 bricks (no atomics at all): the 256 threads of a CTA
-// are the 16 x 16 (x, y) columns of the brick and each keeps its column's 16 z values of the
-// three components in registers.  The points whose footprint meets the brick are staged in
-// batches in shared memory as brick-aligned, zero-padded kernel rows phi_x[16], phi_y[16],
-// phi_z[16], so every point is one unconditional rank-1 update per thread:
+// Register-column spreading for FP64 grids and wide kernels, any grid size, no atomics: one CTA of two
+// warps per 8^3 brick (the last brick of a dimension may be shorter), thread (x, y) keeping its
+// column's 8 z values of the three components in registers.  The points whose footprint can meet the
+// brick are those that start in its own bin or the few before it (periodic); they are tested one per
+// thread and the overlapping ones staged in shared memory, in batches, as brick-aligned zero-padded
+// kernel rows phi_x[8], phi_y[8], phi_z[8], so every point is one unconditional rank-1 update:
 //     acc_c[z] += q_c phi_x[x] phi_y[y] * phi_z[z].
-// A warp covers two y rows and skips the points whose footprint misses both.
-constexpr int kColB = 16;
-constexpr int kColThreads = 256;
+// A warp covers four y rows and skips the points whose footprint misses them.
+// Bound: the FP64 pipe (28 instructions per point, warp and brick met).  Bricks of 8 instead of 16
+// give 6.6 (m = 4) or 9.6 (m = 5) bricks met per point instead of 3.0 or 3.8, each of an eighth of the
+// cells: 2.5 to 3.2 times fewer updates with zero.
+constexpr int kColB = 8;
+constexpr int kColThreads = kColB * kColB;
 constexpr int kColBatch = 32;
+constexpr int kColRanges = 64;  // runs of bins a brick collects (at most 4 x 4 rows, split by the period)
 
 template <typename T>
-struct ColSlot {
-    T q[4];          // charges (q[3] unused)
-    T px[kColB];     // brick-aligned kernel rows, zero outside the footprint
-    T py[kColB];
-    T pz[kColB];
+struct __align__(16) ColSlot {
+    T q[4];                             // charges (q[3] unused)
+    T px[kColB], py[kColB], pz[kColB];  // brick-aligned kernel rows, zero outside the footprint
 };
 
+// A column's sums of one component: acc[z] += c pz[z].  FP32 takes two z per instruction (packed
+// multiply-add, each half rounded as the scalar one).
 template <typename T>
-__global__ void __launch_bounds__(kColThreads, 2) spread_column_kernel(
+struct ColAcc {
+    T a[kColB];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int z = 0; z < kColB; ++z) a[z] = (T)0;
+    }
+    __device__ __forceinline__ T get(int z) const { return a[z]; }
+};
+template <>
+struct ColAcc<float> {
+    unsigned long long a[kColB / 2];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int z = 0; z < kColB / 2; ++z) a[z] = 0ull;
+    }
+    __device__ __forceinline__ float get(int z) const {
+        return __uint_as_float((unsigned)(z & 1 ? a[z >> 1] >> 32 : a[z >> 1] & 0xffffffffull));
+    }
+};
+__device__ __forceinline__ void col_update(ColAcc<double>& x, ColAcc<double>& y, ColAcc<double>& w, const double* pz,
+                                           double c0, double c1, double c2) {
+#pragma unroll
+    for (int z = 0; z < kColB; ++z) {
+        const double f = pz[z];
+        x.a[z] = fma(c0, f, x.a[z]);
+        y.a[z] = fma(c1, f, y.a[z]);
+        w.a[z] = fma(c2, f, w.a[z]);
+    }
+}
+__device__ __forceinline__ unsigned long long dup2(float c) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(c));
+    return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long& a, unsigned long long b, unsigned long long c) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(b), "l"(c));
+}
+__device__ __forceinline__ void col_update(ColAcc<float>& x, ColAcc<float>& y, ColAcc<float>& w, const float* pz, float c0,
+                                           float c1, float c2) {
+    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(pz);  // 16-byte aligned (ColSlot)
+    const unsigned long long d0 = dup2(c0), d1 = dup2(c1), d2 = dup2(c2);
+#pragma unroll
+    for (int h = 0; h < kColB / 4; ++h) {
+        const ulonglong2 f = p[h];
+        fma2(x.a[2 * h], d0, f.x);
+        fma2(y.a[2 * h], d1, f.x);
+        fma2(w.a[2 * h], d2, f.x);
+        fma2(x.a[2 * h + 1], d0, f.y);
+        fma2(y.a[2 * h + 1], d1, f.y);
+        fma2(w.a[2 * h + 1], d2, f.y);
+    }
+}
+
+// Bins per dimension that can reach the brick starting at cell s0: from bin `first` on, `count` of them.
+__device__ __forceinline__ void col_bins(int s0, int b, int w, int n, int nb, int& first, int& count) {
+    int c = s0 - (w - 1);
+    if (c >= 0) {
+        first = c / kColB;
+        count = b - first + 1;
+    } else {
+        c += n;  // w <= n
+        first = c / kColB;
+        count = min(nb - first + b + 1, nb);
+        if (count == nb) first = 0;
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kColThreads) spread_column_kernel(
     LRSizes S, int nb0, int nb1, int nb2, const int32_t* __restrict__ bin_start, const T* __restrict__ binned,
     const int32_t* __restrict__ foot, T* __restrict__ grid) {
     __shared__ __align__(16) ColSlot<T> slot[kColBatch];
-    __shared__ int2 yrange[kColBatch];  // overlap rows [lo, hi) in y; (0, 0) when the overlap is empty
-    __shared__ int nbin_start[8], nbin_base[9];
+    __shared__ int yrows[kColBatch];    // bit y: the footprint meets row y of the brick
+    __shared__ int32_t pend[kColThreads];
+    __shared__ int32_t rstart[kColRanges], rbase[kColRanges + 1];
+    __shared__ int wcount[2];
     const int w = 2 * S.m;
     const int stride = 3 + 3 * w;
     const int bx = blockIdx.x % nb0;
     const int by = (blockIdx.x / nb0) % nb1;
     const int bz = blockIdx.x / (nb0 * nb1);
     const int bs[3] = {bx * kColB, by * kColB, bz * kColB};
-    const int tx = threadIdx.x & (kColB - 1), ty = threadIdx.x / kColB;
-    const int y0 = 2 * (threadIdx.x >> 5);  // the warp's rows: y0, y0 + 1
-    if (threadIdx.x < 8) {
-        const int nbr = threadIdx.x;
-        const int cx = (bx - (nbr & 1) + nb0) % nb0;
-        const int cy = (by - ((nbr >> 1) & 1) + nb1) % nb1;
-        const int cz = (bz - ((nbr >> 2) & 1) + nb2) % nb2;
-        const int b = (cz * nb1 + cy) * nb0 + cx;
-        nbin_start[nbr] = bin_start[b];
-        nbin_base[nbr + 1] = bin_start[b + 1] - bin_start[b];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tx = tid & (kColB - 1), ty = tid / kColB;
+    // ---- runs of bins: x runs (two where they wrap around the period) of the (y, z) rows ----
+    int fx, cx, fy, cy, fz, cz;
+    col_bins(bs[0], bx, w, S.n[0], nb0, fx, cx);
+    col_bins(bs[1], by, w, S.n[1], nb1, fy, cy);
+    col_bins(bs[2], bz, w, S.n[2], nb2, fz, cz);
+    const int nx1 = min(cx, nb0 - fx), halves = cx > nx1 ? 2 : 1;  // first run [fx, fx + nx1), second [0, cx - nx1)
+    const int nr = cy * cz * halves;
+    if (tid < nr) {
+        const int h = tid % halves, row = tid / halves;
+        int yy = fy + row % cy, zz = fz + row / cy;
+        yy = yy >= nb1 ? yy - nb1 : yy;
+        zz = zz >= nb2 ? zz - nb2 : zz;
+        const int32_t b0 = (zz * nb1 + yy) * nb0 + (h ? 0 : fx);
+        const int a = bin_start[b0];
+        rstart[tid] = a;
+        rbase[tid + 1] = bin_start[b0 + (h ? cx - nx1 : nx1)] - a;
+    }
+    if (tid == 0) rbase[0] = 0;
+    __syncthreads();
+    if (warp == 0) {  // counts -> offsets
+        int carry = 0;
+        for (int b = 0; b < nr; b += 32) {
+            int v = b + lane < nr ? rbase[b + lane + 1] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += t;
+            }
+            if (b + lane < nr) rbase[b + lane + 1] = carry + v;
+            carry += __shfl_sync(0xffffffffu, v, 31);
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        nbin_base[0] = 0;
-        for (int k = 1; k <= 8; ++k) nbin_base[k] += nbin_base[k - 1];
-    }
-    __syncthreads();
-    const int ntot = nbin_base[8];
-    T acc0[kColB], acc1[kColB], acc2[kColB];
+    const int ntot = rbase[nr];
+    ColAcc<T> acc0, acc1, acc2;
+    acc0.zero();
+    acc1.zero();
+    acc2.zero();
+    const int ymask = 0xf << (4 * warp);
+    for (int k0 = 0; k0 < ntot; k0 += kColThreads) {
+        // ---- the candidates of this chunk whose footprint meets the brick ----
+        const int k = k0 + tid;
+        bool meets = false;
+        int32_t j = 0;
+        if (k < ntot) {
+            int r = 0;
+            for (int step = kColRanges / 2; step >= 1; step >>= 1)  // last run with rbase <= k
+                if (r + step < nr && rbase[r + step] <= k) r += step;
+            j = rstart[r] + (k - rbase[r]);
+            meets = true;
 #pragma unroll
-    for (int z = 0; z < kColB; ++z) acc0[z] = acc1[z] = acc2[z] = (T)0;
-    for (int k0 = 0; k0 < ntot; k0 += kColBatch) {
-        // ---- stage: 8 threads per point slot ----
-        {
-            const int s = threadIdx.x >> 3, part = threadIdx.x & 7;
-            const int k = k0 + s;
-            ColSlot<T>& sl = slot[s];
-            if (k < ntot) {
-                int nb = 0;
-#pragma unroll
-                for (int i = 1; i < 8; ++i) nb += k >= nbin_base[i];
-                const int64_t j = nbin_start[nb] + (k - nbin_base[nb]);
-                int o[3];
-                bool empty = false;
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    o[d] = foot[3 * j + d] - bs[d];
-                    if (o[d] >= kColB) o[d] -= S.n[d];
-                    const int lo = o[d] < 0 ? 0 : o[d];
-                    const int hi = o[d] + w < kColB ? o[d] + w : kColB;
-                    empty = empty || lo >= hi;
-                }
-                const T* src = binned + j * stride;
-                for (int e = part; e < 3 * kColB; e += 8) {
-                    const int d = e / kColB, t = e % kColB, r = t - o[d];
-                    const T v = (r >= 0 && r < w) ? src[3 + d * w + r] : (T)0;
-                    (d == 0 ? sl.px : d == 1 ? sl.py : sl.pz)[t] = v;
-                }
-                if (part < 3) sl.q[part] = src[part];
-                if (part == 3) {
-                    const int lo = o[1] < 0 ? 0 : o[1];
-                    const int hi = o[1] + w < kColB ? o[1] + w : kColB;
-                    yrange[s] = empty ? make_int2(0, 0) : make_int2(lo, hi);
-                }
-            } else if (part == 0) {
-                yrange[s] = make_int2(0, 0);
+            for (int d = 0; d < 3; ++d) {
+                int o = foot[3 * (int64_t)j + d] - bs[d];  // in (-n, n): starts inside the brick, or reaches it
+                const int e = o < 0 ? o + S.n[d] : o;      // cells from the brick's start to the footprint's (mod n)
+                meets = meets && (e < min(kColB, S.n[d] - bs[d]) || e + w > S.n[d]);
             }
         }
+        const unsigned m = __ballot_sync(0xffffffffu, meets);
+        if (lane == 0) wcount[warp] = __popc(m);
         __syncthreads();
-        // ---- accumulate ----
-        const int nbatch = ntot - k0 < kColBatch ? ntot - k0 : kColBatch;
-        for (int s = 0; s < nbatch; ++s) {
-            const int2 yr = yrange[s];
-            if (y0 + 2 <= yr.x || y0 >= yr.y) continue;  // warp-uniform
-            const ColSlot<T>& sl = slot[s];
-            const T fxy = sl.px[tx] * sl.py[ty];
-            const T c0 = sl.q[0] * fxy, c1 = sl.q[1] * fxy, c2 = sl.q[2] * fxy;
+        if (meets) pend[(warp ? wcount[0] : 0) + __popc(m & ((1u << lane) - 1u))] = j;
+        const int np = wcount[0] + wcount[1];
+        __syncthreads();
+        for (int p0 = 0; p0 < np; p0 += kColBatch) {
+            const int nbatch = np - p0 < kColBatch ? np - p0 : kColBatch;
+            // ---- stage: two threads per slot ----
+            {
+                const int s = tid >> 1, part = tid & 1;
+                if (s < nbatch) {
+                    ColSlot<T>& sl = slot[s];
+                    const int64_t jj = pend[p0 + s];
+                    const T* src = binned + jj * stride;
 #pragma unroll
-            for (int z = 0; z < kColB; ++z) {
-                const T f = sl.pz[z];
-                acc0[z] = fma(c0, f, acc0[z]);
-                acc1[z] = fma(c1, f, acc1[z]);
-                acc2[z] = fma(c2, f, acc2[z]);
+                    for (int d = 0; d < 3; ++d) {
+                        T* row = d == 0 ? sl.px : d == 1 ? sl.py : sl.pz;
+                        const int i0 = foot[3 * jj + d];
+#pragma unroll
+                        for (int e = 0; e < kColB / 2; ++e) {
+                            const int t = part * (kColB / 2) + e;
+                            int r = bs[d] + t - i0;
+                            r = r < 0 ? r + S.n[d] : r;  // cells past a short brick are not stored
+                            row[t] = r < w ? src[3 + d * w + r] : (T)0;
+                        }
+                    }
+                    if (part) {
+                        const int i1 = foot[3 * jj + 1];
+                        int bits = 0;
+#pragma unroll
+                        for (int t = 0; t < kColB; ++t) {
+                            int r = bs[1] + t - i1;
+                            r = r < 0 ? r + S.n[1] : r;
+                            if (r < w) bits |= 1 << t;
+                        }
+                        yrows[s] = bits;
+                    }
+                    if (part) sl.q[0] = src[0];
+                    else { sl.q[1] = src[1]; sl.q[2] = src[2]; }
+                }
             }
+            __syncthreads();
+            // ---- accumulate ----
+            for (int s = 0; s < nbatch; ++s) {
+                if (!(yrows[s] & ymask)) continue;  // warp-uniform
+                const ColSlot<T>& sl = slot[s];
+                const T fxy = sl.px[tx] * sl.py[ty];
+                col_update(acc0, acc1, acc2, sl.pz, sl.q[0] * fxy, sl.q[1] * fxy, sl.q[2] * fxy);
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
+    if (bs[0] + tx >= S.n[0] || bs[1] + ty >= S.n[1]) return;
     const int64_t ng = S.ngrid;
     const int64_t plane = (int64_t)S.n[1] * S.n[0];
     T* g = grid + ((int64_t)bs[2] * S.n[1] + bs[1] + ty) * S.n[0] + bs[0] + tx;
+    const int nz = min(kColB, S.n[2] - bs[2]);
 #pragma unroll
-    for (int z = 0; z < kColB; ++z) {
-        g[z * plane] = acc0[z];
-        g[ng + z * plane] = acc1[z];
-        g[2 * ng + z * plane] = acc2[z];
-    }
+    for (int z = 0; z < kColB; ++z)
+        if (z < nz) {
+            g[z * plane] = acc0.get(z);
+            g[ng + z * plane] = acc1.get(z);
+            g[2 * ng + z * plane] = acc2.get(z);
+        }
 }
 
 // Type-2 interpolation, one warp per node (cell order when available).  The node's 3 x W
@@ -1110,17 +1100,13 @@ int longrange_init(vpbs_handle* h) {
         S.beta = 0.97 * kPi * (1.0 - 1.0 / (2.0 * P.sigma)) * (2.0 * P.m);
         S.edge = std::exp(-S.beta);
     }
-    // brick edge for atomic-free spreading: divides every grid size, >= kernel width, >= 2 bricks
-    h->gatherB = 0;
-    for (int B : {16, 12, 10, 8}) {
-        bool ok = B >= 2 * S.m;
-        for (int d = 0; d < 3; ++d) ok = ok && S.n[d] % B == 0 && S.n[d] / B >= 2;
-        if (ok) {
-            h->gatherB = B;
-            for (int d = 0; d < 3; ++d) h->nbrick[d] = S.n[d] / B;
-            break;
-        }
-    }
+    // bricks of 16^3 (tensor-core and plane-owner spreading) where they divide an FP32 grid and the kernel is
+    // narrow; else bricks of 8^3, of which the last in a dimension may be shorter
+    h->brick = 16;
+    if (P.precision != VPBS_PRECISION_MIXED || S.m > 4) h->brick = kColB;
+    for (int d = 0; d < 3; ++d)
+        if (S.n[d] % 16 != 0 || S.n[d] < 32) h->brick = kColB;
+    for (int d = 0; d < 3; ++d) h->nbrick[d] = (S.n[d] + h->brick - 1) / h->brick;
     int rc;
     const bool mixed = P.precision == VPBS_PRECISION_MIXED;
     const size_t rsz = mixed ? sizeof(float) : sizeof(double);  // grid precision
@@ -1201,107 +1187,76 @@ int longrange_compute_t(vpbs_handle* h, int fields) {
     C* gc2 = (C*)h->grid_c2.p;
     // sources: cell-sorted copy (SoA x,y,z,qx,qy,qz), built by build_cell_lists
     const double* src = (const double*)h->src_sorted.p;
-    if (h->gatherB) {
+    {
         StageScope st(h, ST_SPREAD);
-        const int B = h->gatherB, nb0 = h->nbrick[0], nb1 = h->nbrick[1], nb2 = h->nbrick[2];
+        const int nb0 = h->nbrick[0], nb1 = h->nbrick[1], nb2 = h->nbrick[2];
         const int64_t nbins = (int64_t)nb0 * nb1 * nb2, Nq = h->Nq;
-        // FP32 grids with narrow kernels (m <= 4) on 16^3 bricks: tensor cores, with their own per-brick
-        // records instead of the bins below
-        const bool use_tc = std::is_same<T, float>::value && B == kColB && S.m <= 4 && h->spread_mode == 0;
-        if ((rc = ensure(h, h->spread_bin, sizeof(int32_t) * 2 * Nq, "spread bins"))) return rc;
-        if ((rc = ensure(h, h->spread_counts, sizeof(int32_t) * nbins, "spread bin counts"))) return rc;
-        if ((rc = ensure(h, h->spread_start, sizeof(int32_t) * (nbins + 1), "spread bin starts"))) return rc;
-        const int stride = 3 + 6 * S.m;  // values per binned point
-        if ((rc = ensure(h, h->binned, sizeof(T) * stride * Nq, "binned points"))) return rc;
-        if ((rc = ensure(h, h->spread_foot, sizeof(int32_t) * 3 * Nq, "footprints"))) return rc;
-        int32_t* bin = (int32_t*)h->spread_bin.p;
-        int32_t* rank = bin + Nq;
-        int32_t* counts = (int32_t*)h->spread_counts.p;
-        int32_t* start = (int32_t*)h->spread_start.p;
-        int32_t* foot = (int32_t*)h->spread_foot.p;
-        if (!use_tc) {
-            if ((rc = check_cuda(h, cudaMemsetAsync(counts, 0, sizeof(int32_t) * nbins, h->stream), "memset"))) return rc;
-            spread_bin_count_kernel<<<grid_for(Nq, 256), 256, 0, h->stream>>>(S, B, nb0, nb1, nb2, Nq, src, sx[0],
-                                                                               sx[1], sx[2], bin, rank, counts);
-            h->launches++;
-            if ((rc = exclusive_scan(h, counts, start, nbins, h->scan_tmp_lr))) return rc;
-            spread_bin_scatter_kernel<T><<<grid_for(Nq, 128), 128, 0, h->stream>>>(S, Nq, src, sx[0], sx[1], sx[2],
-                                                                                    bin, rank, start, (T*)h->binned.p,
-                                                                                    foot);
-            h->launches++;
-        }
         const unsigned nblk = (unsigned)nbins;
-        const T* bsrc = (const T*)h->binned.p;
-        const size_t smem = sizeof(T) * 3 * B * (B * (B + 1) + 8);
-        auto launch = [&](auto kern) {
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<nblk, kBrickThreads, smem, h->stream>>>(S, nb0, nb1, nb2, start, bsrc, foot, grid);
-        };
-        // plane-owner kernel (FP32 grids only; the branch that calls it is never taken for T = double)
-        auto launch_plane = [&](void (*kern)(LRSizes, int, int, int, const int32_t*, const float*, const int32_t*,
-                                             float*), int P) {
-            const size_t psmem = sizeof(float) * 3 * kPlaneB * kPlaneB * (P == 8 ? PlaneLayout<8>::RX : PlaneLayout<4>::RX);
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
-            kern<<<nblk, kPlaneThreads, psmem, h->stream>>>(S, nb0, nb1, nb2, start, (const float*)bsrc, foot,
-                                                           (float*)grid);
-        };
-        switch (B) {
-            case kColB:
-                // FP32 grids with narrow kernels (m <= 4): the plane-owner kernel (the 16-deep
-                // register columns mostly multiply zeros there); wider kernels and FP64 grids use
-                // the columns
-                if (use_tc) {
-                    // tensor cores: per-brick records, then the brick product in 3xTF32
-                    if ((rc = ensure_status(h))) return rc;
-                    const int R = tc_record_floats(2 * S.m);
-                    if ((rc = ensure(h, h->tc_counts, sizeof(int32_t) * 2 * nbins, "record counts"))) return rc;
-                    if ((rc = ensure(h, h->tc_start, sizeof(int32_t) * (nbins + 1), "record starts"))) return rc;
-                    if ((rc = ensure(h, h->tc_rec, sizeof(float) * R * 8 * (size_t)Nq, "brick records"))) return rc;
-                    int32_t* tcount = (int32_t*)h->tc_counts.p;
-                    int32_t* tfill = tcount + nbins;
-                    if ((rc = check_cuda(h, cudaMemsetAsync(tcount, 0, sizeof(int32_t) * 2 * nbins, h->stream), "memset")))
-                        return rc;
-                    tc_rec_count_kernel<<<grid_for(Nq, 256), 256, 0, h->stream>>>(S, nb0, nb1, nb2, Nq, src, sx[0], sx[1],
-                                                                                   sx[2], tcount);
-                    if ((rc = exclusive_scan(h, tcount, (int32_t*)h->tc_start.p, nbins, h->scan_tmp_lr))) return rc;
-                    auto launch_tc = [&](auto wtag) {
-                        constexpr int W = decltype(wtag)::value;
-                        tc_rec_scatter_kernel<W><<<grid_for(Nq, 128), 128, 0, h->stream>>>(
-                            S, nb0, nb1, nb2, Nq, src, sx[0], sx[1], sx[2], (const int32_t*)h->tc_start.p, tfill,
-                            (float*)h->tc_rec.p);
-                        const size_t tsmem = sizeof(TcSpreadSmem);
-                        cudaFuncSetAttribute(spread_tc_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem);
-                        spread_tc_kernel<W><<<nblk, kTcThreads, tsmem, h->stream>>>(
-                            S, nb0, nb1, (const int32_t*)h->tc_start.p, (const float*)h->tc_rec.p, (float*)grid,
-                            h->status_dev);
-                    };
-                    switch (S.m) {
-                        case 1: launch_tc(std::integral_constant<int, 2>()); break;
-                        case 2: launch_tc(std::integral_constant<int, 4>()); break;
-                        case 3: launch_tc(std::integral_constant<int, 6>()); break;
-                        default: launch_tc(std::integral_constant<int, 8>()); break;
-                    }
-                    h->launches += 2;
-                } else if (std::is_same<T, float>::value && S.m <= 4)
-                    launch_plane(S.m <= 2 ? spread_plane_kernel<4> : spread_plane_kernel<8>, S.m <= 2 ? 4 : 8);
-                else
-                    spread_column_kernel<T><<<nblk, kColThreads, 0, h->stream>>>(S, nb0, nb1, nb2, start, bsrc, foot,
-                                                                                 grid);
-                break;
-            case 12: launch(spread_brick_kernel<12, T>); break;
-            case 10: launch(spread_brick_kernel<10, T>); break;
-            default: launch(spread_brick_kernel<8, T>); break;
+        if (h->brick == 16 && h->spread_mode == 0) {
+            // tensor cores: per-brick records, then the brick product in 3xTF32
+            if ((rc = ensure_status(h))) return rc;
+            const int R = tc_record_floats(2 * S.m);
+            if ((rc = ensure(h, h->tc_counts, sizeof(int32_t) * 2 * nbins, "record counts"))) return rc;
+            if ((rc = ensure(h, h->tc_start, sizeof(int32_t) * (nbins + 1), "record starts"))) return rc;
+            if ((rc = ensure(h, h->tc_rec, sizeof(float) * R * 8 * (size_t)Nq, "brick records"))) return rc;
+            int32_t* tcount = (int32_t*)h->tc_counts.p;
+            int32_t* tfill = tcount + nbins;
+            if ((rc = check_cuda(h, cudaMemsetAsync(tcount, 0, sizeof(int32_t) * 2 * nbins, h->stream), "memset"))) return rc;
+            tc_rec_count_kernel<<<grid_for(Nq, 256), 256, 0, h->stream>>>(S, nb0, nb1, nb2, Nq, src, sx[0], sx[1], sx[2],
+                                                                           tcount);
+            if ((rc = exclusive_scan(h, tcount, (int32_t*)h->tc_start.p, nbins, h->scan_tmp_lr))) return rc;
+            auto launch_tc = [&](auto wtag) {
+                constexpr int W = decltype(wtag)::value;
+                tc_rec_scatter_kernel<W><<<grid_for(Nq, 128), 128, 0, h->stream>>>(
+                    S, nb0, nb1, nb2, Nq, src, sx[0], sx[1], sx[2], (const int32_t*)h->tc_start.p, tfill,
+                    (float*)h->tc_rec.p);
+                const size_t tsmem = sizeof(TcSpreadSmem);
+                cudaFuncSetAttribute(spread_tc_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem);
+                spread_tc_kernel<W><<<nblk, kTcThreads, tsmem, h->stream>>>(
+                    S, nb0, nb1, (const int32_t*)h->tc_start.p, (const float*)h->tc_rec.p, (float*)grid, h->status_dev);
+            };
+            switch (S.m) {
+                case 1: launch_tc(std::integral_constant<int, 2>()); break;
+                case 2: launch_tc(std::integral_constant<int, 4>()); break;
+                case 3: launch_tc(std::integral_constant<int, 6>()); break;
+                default: launch_tc(std::integral_constant<int, 8>()); break;
+            }
+            h->launches += 3;
+        } else {
+            const int stride = 3 + 6 * S.m;  // values per binned point
+            if ((rc = ensure(h, h->spread_bin, sizeof(int32_t) * 2 * Nq, "spread bins"))) return rc;
+            if ((rc = ensure(h, h->spread_counts, sizeof(int32_t) * nbins, "spread bin counts"))) return rc;
+            if ((rc = ensure(h, h->spread_start, sizeof(int32_t) * (nbins + 1), "spread bin starts"))) return rc;
+            if ((rc = ensure(h, h->binned, sizeof(T) * stride * Nq, "binned points"))) return rc;
+            if ((rc = ensure(h, h->spread_foot, sizeof(int32_t) * 3 * Nq, "footprints"))) return rc;
+            int32_t* bin = (int32_t*)h->spread_bin.p;
+            int32_t* rank = bin + Nq;
+            int32_t* counts = (int32_t*)h->spread_counts.p;
+            int32_t* start = (int32_t*)h->spread_start.p;
+            int32_t* foot = (int32_t*)h->spread_foot.p;
+            const T* bsrc = (const T*)h->binned.p;
+            if ((rc = check_cuda(h, cudaMemsetAsync(counts, 0, sizeof(int32_t) * nbins, h->stream), "memset"))) return rc;
+            spread_bin_count_kernel<<<grid_for(Nq, 256), 256, 0, h->stream>>>(S, h->brick, nb0, nb1, nb2, Nq, src, sx[0],
+                                                                               sx[1], sx[2], bin, rank, counts);
+            if ((rc = exclusive_scan(h, counts, start, nbins, h->scan_tmp_lr))) return rc;
+            spread_bin_scatter_kernel<T><<<grid_for(Nq, 128), 128, 0, h->stream>>>(S, Nq, src, sx[0], sx[1], sx[2], bin, rank,
+                                                                                    start, (T*)h->binned.p, foot);
+            if (h->brick == 16) {
+                // plane-owner kernel (FP32 grids only)
+                auto launch_plane = [&](void (*kern)(LRSizes, int, int, int, const int32_t*, const float*, const int32_t*,
+                                                     float*), int P) {
+                    const size_t psmem = sizeof(float) * 3 * kPlaneB * kPlaneB * (P == 8 ? PlaneLayout<8>::RX : PlaneLayout<4>::RX);
+                    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
+                    kern<<<nblk, kPlaneThreads, psmem, h->stream>>>(S, nb0, nb1, nb2, start, (const float*)bsrc, foot,
+                                                                   (float*)grid);
+                };
+                launch_plane(S.m <= 2 ? spread_plane_kernel<4> : spread_plane_kernel<8>, S.m <= 2 ? 4 : 8);
+            } else {
+                spread_column_kernel<T><<<nblk, kColThreads, 0, h->stream>>>(S, nb0, nb1, nb2, start, bsrc, foot, grid);
+            }
+            h->launches += 3;
         }
-        h->launches++;
-        if ((rc = check_cuda(h, cudaGetLastError(), "spread gather kernels"))) return rc;
-    } else {
-        StageScope st(h, ST_SPREAD);
-        if ((rc = check_cuda(h, cudaMemsetAsync(grid, 0, sizeof(T) * 3 * S.ngrid, h->stream), "memset grid")))
-            return rc;
-        spread_kernel_atomic<T><<<grid_for(h->Nq, kSpreadBatch), 256, 0, h->stream>>>(S, h->Nq, src, sx[0], sx[1], sx[2],
-                                                                                      grid);
-        h->launches++;
-        if ((rc = check_cuda(h, cudaGetLastError(), "spread kernel"))) return rc;
+        if ((rc = check_cuda(h, cudaGetLastError(), "spread kernels"))) return rc;
     }
     if (h->fplan) {
         StageScope st(h, ST_FFT_FORWARD);

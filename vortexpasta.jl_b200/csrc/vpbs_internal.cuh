@@ -187,7 +187,7 @@ struct vpbs_handle {
     vpbs::DevBuf tc_counts, tc_start, tc_rec;  // tensor-core spreading: per-brick (point, brick) records
     vpbs::DevBuf peer_in;                       // vpbs_add_field: a field copied from another GPU
     cudaEvent_t xfer_done = nullptr;            // vpbs_add_field: this handle's fields are complete
-    int gatherB = 0;   // brick edge of the atomic-free spreading (0: atomic fallback)
+    int brick = 0;     // brick edge of the spreading (longrange_init)
     int spread_mode = 0;  // 0: tensor-core spreading where it applies; 1: CUDA-core kernels only
     int* status_host = nullptr;  // mapped pinned word: device-side faults of bounded waits (0: none)
     int* status_dev = nullptr;
