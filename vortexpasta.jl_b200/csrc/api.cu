@@ -297,7 +297,15 @@ int vpbs_create(const vpbs_params* params, vpbs_handle** out) {
         f32_table_host(tab.data(), ntab, xmax_c, tabc.data());
         const size_t bytes_d = sizeof(double) * tab.size(), bytes_f = sizeof(float) * tabf.size();
         const size_t off_c = (2 * bytes_d + bytes_f + 15) / 16 * 16, bytes_c = sizeof(float4) * tabc.size();
-        if (!rc) rc = ensure(h, h->ewald_tab, off_c + bytes_c, "Ewald tables");
+        // FP64 tables of the cell-tiled pair kernel, stored after the FP32 cubic ones (16-byte multiples)
+        const int ntab_s = tab_s_size(xmax_c);
+        std::vector<double> tabs((size_t)2 * ntab_s * kTabSNC);
+        tab_s_host(tab.data(), ntab, xmax_c, tabs.data());
+        const size_t off_s = off_c + bytes_c, bytes_s = sizeof(double) * tabs.size();
+        if (!rc) rc = ensure(h, h->ewald_tab, off_s + bytes_s, "Ewald tables");
+        if (!rc)
+            rc = check_cuda(h, cudaMemcpy((char*)h->ewald_tab.p + off_s, tabs.data(), bytes_s, cudaMemcpyHostToDevice),
+                            "copy Ewald tables");
         if (!rc)
             rc = check_cuda(h, cudaMemcpy((char*)h->ewald_tab.p + off_c, tabc.data(), bytes_c, cudaMemcpyHostToDevice),
                             "copy Ewald tables");
@@ -315,6 +323,8 @@ int vpbs_create(const vpbs_params* params, vpbs_handle** out) {
         h->K.ewald_ntab = ntab;
         h->K.tab_c = (const float4*)((const char*)h->ewald_tab.p + off_c);
         h->K.ntab_c = ntab_c;
+        h->K.tab_s = (const double*)((const char*)h->ewald_tab.p + off_s);
+        h->K.ntab_s = ntab_s;
         // streamfunction factor of a uniform background vorticity (BiotSavart.jl:255-286): 1 / (4 alpha^2)
         // for the Gaussian splitting (gaussian.jl:241); int_0^rcut r^2 f(r) dr / 2 for the Kaiser-Bessel one
         // (kaiser_bessel.jl:160-165, 280), with f(r) = beta / (rcut sinh beta) I0(beta sqrt(1 - r^2 / rcut^2)),

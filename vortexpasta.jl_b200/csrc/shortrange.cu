@@ -8,6 +8,7 @@
 //    weights of splitting/gaussian.jl:273-279): one warp per destination node, lanes
 //    stride over the contiguous cell-sorted source ranges of the (2M+1)^2 neighbour rows,
 //    warp-shuffle reduction at the end.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -390,20 +391,21 @@ __global__ void __launch_bounds__(256) pair_kernel(
 // dependency chains overlap.  Destinations are handled in passes of up to kPassDst nodes;
 // warps take (destination, row-part) items and add each item's warp-reduced sum to the
 // destination's shared-memory accumulator.
-constexpr int kTile = 2560;
-constexpr int kTilePad = kTile + 32;  // a chunk of 32 lanes may read past the tile end (masked)
 constexpr int kPassDst = 64;
-constexpr int kMaxNbCells = 2048;  // neighbour slabs of a block: rows x slabs per row
+constexpr int kMaxNbCells = 1024;  // neighbour slabs of a block: rows x slabs per row
 constexpr int kMaxBlockRows = 16;  // (y, z) cell rows of a block (destination ranges)
 constexpr int kMaxRows = 81;      // (2M+1)^2
 constexpr int kTileQueue = 128;   // screened pairs are evaluated 64 at a time (two per lane)
 constexpr double kScreenMargin = 2e-5;
 
+// TILE sources: one field 1024, both fields 640 (two weight tables), so that two CTAs share an SM.
+template <int TILE>
 struct TileSmem {
-    // relative source position split as hi + lo FP32 parts (|lo| <= ulp(hi) / 2, together ~48
-    // significant bits); hi.w holds the cell-sorted index, lo.w the segment (int bits)
-    float4 hi[kTilePad];
-    float4 lo[kTilePad];
+    static constexpr int kPad = TILE + 32;  // a chunk of 32 lanes may read past the tile end (masked)
+    float4 hi[kPad];    // FP32 position relative to the block corner, segment (int bits): the screen
+    double2 pxy[kPad];  // the FP64 position and the charge: the evaluation
+    double2 pzq[kPad];
+    double2 qyz[kPad];
     int32_t queue[kPairThreads / 32][kTileQueue];  // per warp: tile indices of screened pairs
     double acc[kPassDst][6];  // per destination: velocity, streamfunction
     double dx[kPassDst][3];   // destination positions
@@ -412,7 +414,10 @@ struct TileSmem {
     int32_t off[kMaxNbCells + 1];  // concatenated offsets of the neighbour slabs
     int32_t cstart[kMaxNbCells];   // first cell-sorted source of each neighbour slab
     int2 rng[kPairThreads / 32][kMaxRows];  // per warp: candidate range of every row
+    alignas(16) double tab[2];  // the weight tables follow: [weight][interval][kTabSNC]
 };
+constexpr size_t kPairSmemMost = 226 * 1024;
+__host__ __device__ constexpr int tile_sources(bool vel, bool psi) { return vel && psi ? 640 : 1024; }
 
 // 1/sqrt(s) in FP64: FP32 hardware estimate refined by two Newton-Raphson steps
 // y <- y (3 - s y^2) / 2 (quadratic convergence: ~1e-7 -> ~1e-14 -> rounding level).
@@ -442,19 +447,8 @@ __device__ __forceinline__ void ewald_weights2(const KParams& K, double x, doubl
     }
 }
 
-// One of the Ewald weights (erfc for the streamfunction, g for the velocity).
-__device__ __forceinline__ double ewald_weight1(const KParams& K, double x, int which) {
-    int k = (int)(x * kEwaldInvH);
-    k = k < K.ewald_ntab ? k : K.ewald_ntab - 1;
-    const double t = x - (k + 0.5) * kEwaldH;
-    const double* c = K.ewald_tab + (which * K.ewald_ntab + k) * kEwaldNC;
-    double a = __ldg(c + kEwaldNC - 1);
-#pragma unroll
-    for (int n = kEwaldNC - 2; n >= 0; --n) a = fma(a, t, __ldg(c + n));
-    return a;
-}
-
-static_assert(sizeof(TileSmem) <= 113 * 1024, "two pair-kernel CTAs must fit in one SM's shared memory");
+static_assert(sizeof(TileSmem<1024>) <= 92 * 1024 && sizeof(TileSmem<640>) <= 68 * 1024,
+              "two pair-kernel CTAs (with the tables of x <= 4) must fit in one SM's shared memory");
 
 // Largest row r in [0, n] whose first concatenated index off[r W] is <= T (off[0] = 0 <= T).
 __device__ __forceinline__ int last_row_le(const int32_t* off, int W, int n, int T) {
@@ -474,78 +468,76 @@ __device__ __forceinline__ double box_gap(double x, double lo, double h) {
     return fmax(g - 1e-9 * h, 0.0);
 }
 
-// Two queued pairs per lane (tile indices t0, t1; v0, v1 mark valid entries): the separation
-// formed in FP64 from the hi + lo parts, the r^2 <= r_cut^2 decision, and the pair integrand
-// (short_range_integrand, integrands.jl:2-18) in precision R.  Entries that are invalid or out
-// of range are evaluated at a harmless separation (r_cut, 0, 0) with zero charge, so both
-// chains run straight through.  Called by all lanes of the warp.
-template <bool VEL, bool PSI, typename R>
-__device__ __forceinline__ void tile_eval2(const KParams& K, const double xd[3], const TileSmem& S,
-                                           const double* __restrict__ src, int64_t Ns, int t0, bool v0, int t1,
-                                           bool v1, PairAcc<double>& acc, unsigned long long& ninr) {
+// Interval and local coordinate of x in the shared-memory tables (intervals centred at k / 96):
+// k = round(96 x) by the 1.5 * 2^52 trick, t = 96 x - k in [-1/2, 1/2].
+__device__ __forceinline__ double tab_s_pos(double x, int ntab, int* k) {
+    const double y = fma(x, kTabSInvH, 6755399441055744.0);
+    const unsigned kk = (unsigned)__double2loint(y), top = (unsigned)(ntab - 1);
+    *k = (int)(kk < top ? kk : top);
+    return fma(x, kTabSInvH, -(y - 6755399441055744.0));
+}
+
+__device__ __forceinline__ double tab_s_poly(const double* c, double t) {
+    const double2* v = reinterpret_cast<const double2*>(c);
+    const double2 c0 = v[0], c1 = v[1], c2 = v[2];
+    return fma(fma(fma(fma(fma(c2.y, t, c2.x), t, c1.y), t, c1.x), t, c0.y), t, c0.x);
+}
+
+// Two queued pairs per lane (tile indices t0, t1; v0, v1 mark valid entries): the FP64 separation, the
+// r^2 <= r_cut^2 decision, and the pair integrand (short_range_integrand, integrands.jl:2-18).  Entries
+// that are invalid or out of range are evaluated at r = r_cut and add zero, so both chains run straight
+// through.  Called by all lanes of the warp.
+template <bool VEL, bool PSI, int TILE>
+__device__ __forceinline__ void tile_eval2(const KParams& K, const double xd[3], const TileSmem<TILE>& S, int t0,
+                                           bool v0, int t1, bool v1, double (&av)[3], double (&ap)[3],
+                                           unsigned long long& ninr) {
     const int tt[2] = {t0, t1};
     const bool vv[2] = {v0, v1};
     double d[2][3], q[2][3], s2[2];
+    bool ok[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-        const float4 h = S.hi[tt[u]], l = S.lo[tt[u]];
-        const int64_t j = __float_as_int(h.w);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) q[u][c] = vv[u] ? src[(3 + c) * Ns + j] : 0.0;
-        d[u][0] = xd[0] - ((double)h.x + (double)l.x);
-        d[u][1] = xd[1] - ((double)h.y + (double)l.y);
-        d[u][2] = xd[2] - ((double)h.z + (double)l.z);
+        const double2 a = S.pxy[tt[u]], b = S.pzq[tt[u]], c = S.qyz[tt[u]];
+        d[u][0] = xd[0] - a.x;
+        d[u][1] = xd[1] - a.y;
+        d[u][2] = xd[2] - b.x;
+        q[u][0] = b.y;
+        q[u][1] = c.x;
+        q[u][2] = c.y;
         s2[u] = d[u][0] * d[u][0] + d[u][1] * d[u][1] + d[u][2] * d[u][2];
+        ok[u] = vv[u] && s2[u] <= K.rcut2;
+        ninr += __popc(__ballot_sync(0xffffffffu, ok[u]));
+        if (!ok[u]) s2[u] = K.rcut2;
     }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-        const bool ok = vv[u] && s2[u] <= K.rcut2;
-        ninr += __popc(__ballot_sync(0xffffffffu, ok));
-        if (!ok) {
-            d[u][0] = K.rcut;
-            d[u][1] = d[u][2] = 0.0;
-            s2[u] = K.rcut2;
-            q[u][0] = q[u][1] = q[u][2] = 0.0;
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const R r0 = (R)d[u][0], r1 = (R)d[u][1], r2 = (R)d[u][2];
-        R rinv, wa = 1, wg = 1;
-        if constexpr (std::is_same<R, float>::value) {
-            rinv = rsqrtf((float)s2[u]);
-            ewald_weights_f(K, (float)K.alpha / rinv, wa, wg);
-        } else {
-            rinv = rsqrt_nr(s2[u]);
-            const double xa = K.alpha * (s2[u] * rinv);
-            if (VEL && PSI) ewald_weights2(K, xa, wa, wg);
-            else if (VEL) wg = ewald_weight1(K, xa, 1);
-            else wa = ewald_weight1(K, xa, 0);
-        }
-        // each pair's contribution is formed in R and accumulated in FP64
-        const R q0 = (R)q[u][0], q1 = (R)q[u][1], q2 = (R)q[u][2];
+        const double rinv = rsqrt_nr(s2[u]);
+        int k;
+        const double t = tab_s_pos(K.alpha * (s2[u] * rinv), K.ntab_s, &k);
         if (VEL) {
-            const R f = wg * rinv * rinv * rinv;
-            acc.v[0] += (double)(f * (q1 * r2 - q2 * r1));
-            acc.v[1] += (double)(f * (q2 * r0 - q0 * r2));
-            acc.v[2] += (double)(f * (q0 * r1 - q1 * r0));
+            const double w = tab_s_poly(S.tab + (PSI ? K.ntab_s + k : k) * kTabSNC, t);
+            const double f = ok[u] ? w * rinv * rinv * rinv : 0.0;
+            av[0] += f * (q[u][1] * d[u][2] - q[u][2] * d[u][1]);
+            av[1] += f * (q[u][2] * d[u][0] - q[u][0] * d[u][2]);
+            av[2] += f * (q[u][0] * d[u][1] - q[u][1] * d[u][0]);
         }
         if (PSI) {
-            const R f = wa * rinv;
-            acc.p[0] += (double)(f * q0);
-            acc.p[1] += (double)(f * q1);
-            acc.p[2] += (double)(f * q2);
+            const double w = tab_s_poly(S.tab + k * kTabSNC, t);
+            const double f = ok[u] ? w * rinv : 0.0;
+            ap[0] += f * q[u][0];
+            ap[1] += f * q[u][1];
+            ap[2] += f * q[u][2];
         }
     }
 }
 
-// Candidates [a, b) of the tile against the destination (cell-relative position xd in FP64,
-// xr in FP32; node i, previous node iprev): FP32 screen on the hi parts, compaction of the
-// survivors into the warp's queue, evaluation 64 at a time.
-template <bool VEL, bool PSI, bool SKIP, typename R>
+// Candidates [a, b) of the tile against the destination (block-relative position xd in FP64, xr in
+// FP32; node i, previous node iprev): FP32 screen on the hi parts, compaction of the survivors into
+// the warp's queue, evaluation 64 at a time.
+template <bool VEL, bool PSI, bool SKIP, int TILE>
 __device__ __forceinline__ void tile_range_q(const KParams& K, const double xd[3], float3 xr, float rc2s, int i,
-                                             int iprev, const TileSmem& S, const double* __restrict__ src, int64_t Ns,
-                                             int a, int b, int lane, PairAcc<double>& acc, int32_t* Q, int& qcount,
+                                             int iprev, const TileSmem<TILE>& S, int a, int b, int lane,
+                                             double (&av)[3], double (&ap)[3], int32_t* Q, int& qcount,
                                              unsigned long long& ninr) {
     for (int base = a; base < b; base += 32) {
         const int t = base + lane;
@@ -553,7 +545,7 @@ __device__ __forceinline__ void tile_range_q(const KParams& K, const double xd[3
         const float e0 = xr.x - p.x, e1 = xr.y - p.y, e2 = xr.z - p.z;
         bool inr = t < b && fmaf(e0, e0, fmaf(e1, e1, e2 * e2)) <= rc2s;
         if (SKIP) {
-            const int sg = __float_as_int(S.lo[t].w);
+            const int sg = __float_as_int(p.w);
             inr = inr && sg != i && sg != iprev;
         }
         const unsigned m = __ballot_sync(0xffffffffu, inr);
@@ -561,7 +553,7 @@ __device__ __forceinline__ void tile_range_q(const KParams& K, const double xd[3
         qcount += __popc(m);
         __syncwarp();
         if (qcount >= 64) {
-            tile_eval2<VEL, PSI, R>(K, xd, S, src, Ns, Q[lane], true, Q[32 + lane], true, acc, ninr);
+            tile_eval2<VEL, PSI, TILE>(K, xd, S, Q[lane], true, Q[32 + lane], true, av, ap, ninr);
             __syncwarp();
             if (lane < qcount - 64) Q[lane] = Q[64 + lane];
             __syncwarp();
@@ -570,7 +562,7 @@ __device__ __forceinline__ void tile_range_q(const KParams& K, const double xd[3
     }
 }
 
-template <bool VEL, bool PSI, bool SKIP, typename R>
+template <bool VEL, bool PSI, bool SKIP>
 __global__ void __launch_bounds__(kPairThreads, 2) pair_cell_kernel(
     KParams K, CellGrid cg, int64_t Np, int64_t Ns, const int32_t* __restrict__ dst_start,
     const int32_t* __restrict__ dst_order, const double* __restrict__ nodes, const int32_t* __restrict__ idx_prev,
@@ -578,7 +570,8 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_cell_kernel(
     double* __restrict__ vel, double* __restrict__ psi, unsigned long long* __restrict__ counters, int3 bk,
     int3 nb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    TileSmem& S = *reinterpret_cast<TileSmem*>(smem_raw);
+    constexpr int kTile = tile_sources(VEL, PSI);
+    TileSmem<kTile>& S = *reinterpret_cast<TileSmem<kTile>*>(smem_raw);
     const int M = cg.M, G = cg.G;
     const int nc0 = cg.nc[0], nc1 = cg.nc[1], nc2 = cg.nc[2];
     const int ncc = nc0 / G;  // cells in x (each made of G slabs)
@@ -601,8 +594,16 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_cell_kernel(
         S.dr_base[ndr] = acc;
     }
     __syncthreads();
-    const int nd = S.dr_base[ndr];
-    if (nd == 0) return;  // uniform over the CTA
+    // this CTA's share of the block's nodes
+    const int nall = S.dr_base[ndr];
+    const int n0 = (int)((int64_t)nall * blockIdx.y / gridDim.y), nd = (int)((int64_t)nall * (blockIdx.y + 1) / gridDim.y);
+    if (n0 == nd) return;  // uniform over the CTA
+    {
+        constexpr int first = VEL && !PSI ? 1 : 0, nw = VEL && PSI ? 2 : 1;
+        const double2* src_tab = reinterpret_cast<const double2*>(K.tab_s + (size_t)first * K.ntab_s * kTabSNC);
+        double2* dst_tab = reinterpret_cast<double2*>(S.tab);
+        for (int k = threadIdx.x; k < nw * K.ntab_s * kTabSNC / 2; k += kPairThreads) dst_tab[k] = src_tab[k];
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const double hx = K.L[0] / nc0, h1 = K.L[1] / nc1, h2 = K.L[2] / nc2, inv_hx = nc0 / K.L[0];
     // neighbourhood: rows (y, z) of the block widened by M cells, slabs in x widened by M G
@@ -643,7 +644,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_cell_kernel(
     const int ntot = S.off[ncb];
     const double pref = K.Gamma / (4.0 * kPi);
     unsigned long long ninr = 0, ncand = 0;  // warp-uniform
-    for (int p0 = 0; p0 < nd; p0 += kPassDst) {
+    for (int p0 = n0; p0 < nd; p0 += kPassDst) {
         const int np = nd - p0 < kPassDst ? nd - p0 : kPassDst;
         __syncthreads();  // the previous pass has written its results
         for (int t = threadIdx.x; t < np; t += kPairThreads) {
@@ -688,9 +689,10 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_cell_kernel(
                     const double sx = inA ? sxA : sxB;
                     const double u0 = src[j] + sx - o0, u1 = src[Ns + j] + sy - o1, u2 = src[2 * Ns + j] + sz - o2;
                     const float f0 = (float)u0, f1 = (float)u1, f2 = (float)u2;
-                    S.hi[t - T0] = make_float4(f0, f1, f2, __int_as_float(j));
-                    S.lo[t - T0] = make_float4((float)(u0 - f0), (float)(u1 - f1), (float)(u2 - f2),
-                                               __int_as_float(SKIP ? seg[j] : 0));
+                    S.hi[t - T0] = make_float4(f0, f1, f2, __int_as_float(SKIP ? seg[j] : 0));
+                    S.pxy[t - T0] = make_double2(u0, u1);
+                    S.pzq[t - T0] = make_double2(u2, src[3 * Ns + j]);
+                    S.qyz[t - T0] = make_double2(src[4 * Ns + j], src[5 * Ns + j]);
                 }
             }
             __syncthreads();
@@ -717,7 +719,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_cell_kernel(
                     S.rng[warp][r] = make_int2(a, b);
                 }
                 __syncwarp();
-                PairAcc<double> acc = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}, 0ull, 0ull};
+                double av[3] = {0, 0, 0}, ap[3] = {0, 0, 0};
                 int qcount = 0;
                 int32_t* Q = S.queue[warp];
                 const double xd[3] = {x[0] - o0, x[1] - o1, x[2] - o2};
@@ -728,20 +730,20 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_cell_kernel(
                     const int a = ab.x > T0 ? ab.x : T0, b = ab.y < T1 ? ab.y : T1;
                     if (a < b) {
                         ncand += b - a;
-                        tile_range_q<VEL, PSI, SKIP, R>(K, xd, xr, rc2s, i, iprev, S, src, Ns, a - T0, b - T0, lane, acc, Q,
-                                                        qcount, ninr);
+                        tile_range_q<VEL, PSI, SKIP, kTile>(K, xd, xr, rc2s, i, iprev, S, a - T0, b - T0, lane, av, ap, Q,
+                                                            qcount, ninr);
                     }
                 }
                 if (qcount > 0)  // warp-uniform
-                    tile_eval2<VEL, PSI, R>(K, xd, S, src, Ns, lane < qcount ? Q[lane] : 0, lane < qcount,
-                                            32 + lane < qcount ? Q[32 + lane] : 0, 32 + lane < qcount, acc, ninr);
+                    tile_eval2<VEL, PSI, kTile>(K, xd, S, lane < qcount ? Q[lane] : 0, lane < qcount,
+                                                32 + lane < qcount ? Q[32 + lane] : 0, 32 + lane < qcount, av, ap, ninr);
                 double s[6] = {0, 0, 0, 0, 0, 0};
                 if (VEL)
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) s[c] = warp_sum(acc.v[c]);
+                    for (int c = 0; c < 3; ++c) s[c] = warp_sum(av[c]);
                 if (PSI)
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) s[3 + c] = warp_sum(acc.p[c]);
+                    for (int c = 0; c < 3; ++c) s[3 + c] = warp_sum(ap[c]);
                 if (lane == 0) {
                     if (VEL)
                         for (int c = 0; c < 3; ++c) atomicAdd(&S.acc[dl][c], s[c]);
@@ -1366,6 +1368,43 @@ void table_eval_host(const double* tab, int ntab, double x, double* a, double* g
     *g = vg;
 }
 
+int tab_s_size(double xmax) { return (int)std::floor(xmax * kTabSInvH) + 2; }
+
+// Degree-5 interpolants of both weights on every interval centred at k / 96, through the values of the
+// FP64 table at the 6 Chebyshev points of the interval, in powers of t = 96 x - k (error below 2e-16 for
+// the Gaussian weights).
+void tab_s_host(const double* tab, int ntab, double xmax, double* out) {
+    constexpr int NC = kTabSNC;
+    const int nf = tab_s_size(xmax);
+    long double T[NC], A[NC][NC];
+    for (int j = 0; j < NC; ++j) T[j] = 0.5L * std::cos((2 * j + 1) * 3.14159265358979323846L / (2 * NC));
+    // rows of the inverse of the Vandermonde matrix: the Lagrange polynomials in powers of t
+    for (int j = 0; j < NC; ++j) {
+        long double c[NC] = {1.0L}, den = 1.0L;
+        int deg = 0;
+        for (int i = 0; i < NC; ++i) {
+            if (i == j) continue;
+            den *= T[j] - T[i];
+            for (int n = ++deg; n > 0; --n) c[n] = c[n - 1] - T[i] * c[n];
+            c[0] *= -T[i];
+        }
+        for (int n = 0; n < NC; ++n) A[j][n] = c[n] / den;
+    }
+    for (int k = 0; k < nf; ++k) {
+        long double cf[2][NC] = {};
+        for (int j = 0; j < NC; ++j) {
+            double a, g;
+            table_eval_host(tab, ntab, (double)((k + T[j]) / (long double)kTabSInvH), &a, &g);
+            for (int n = 0; n < NC; ++n) {
+                cf[0][n] += A[j][n] * a;
+                cf[1][n] += A[j][n] * g;
+            }
+        }
+        for (int w = 0; w < 2; ++w)
+            for (int n = 0; n < NC; ++n) out[((size_t)w * nf + k) * NC + n] = (double)cf[w][n];
+    }
+}
+
 int f32_table_size(double xmax) { return (int)std::floor(xmax * kTabCInvH) + 2; }
 
 // Cubic interpolants of both weights on every interval [k/32, (k+1)/32], through the values of
@@ -1435,11 +1474,6 @@ int exclusive_scan(vpbs_handle* h, const int32_t* counts, int32_t* start, int64_
     return check_cuda(h, cudaGetLastError(), "scan kernels");
 }
 
-template <typename T>
-struct PrecTag {
-    using type = T;
-};
-
 int pair_interactions(vpbs_handle* h, int fields) {
     const int64_t Np = h->Np, Nq = h->Nq;
     const bool open = h->K.open_domain;
@@ -1465,7 +1499,8 @@ int pair_interactions(vpbs_handle* h, int fields) {
     const bool v = fields & VPBS_VELOCITY, p = fields & VPBS_STREAMFUNCTION;
     const CellGrid& cg = h->cg;
     const int Wc = 2 * cg.M + 1;
-    if (!open && cg.M > 0 && Wc * Wc <= kMaxRows && Wc * Wc * Wc * cg.G <= kMaxNbCells) {
+    if (!open && cg.M > 0 && Wc * Wc <= kMaxRows && Wc * Wc * Wc * cg.G <= kMaxNbCells &&
+        sizeof(TileSmem<1024>) + 2 * sizeof(double) * kTabSNC * h->K.ntab_s <= kPairSmemMost) {
         // blocks of Bc^3 cells per CTA, grown while a block holds fewer than ~24 nodes on average,
         // at least 16 CTAs per SM remain, and the neighbourhood fits the shared-memory tables and
         // stays inside one period
@@ -1533,30 +1568,29 @@ int pair_interactions(vpbs_handle* h, int fields) {
         }
         const int3 bk = make_int3(Bc, Bc, Bc);
         const int3 nb = make_int3((ncc + Bc - 1) / Bc, (cg.nc[1] + Bc - 1) / Bc, (cg.nc[2] + Bc - 1) / Bc);
-        const size_t smem = sizeof(TileSmem);
         const unsigned nblocks = (unsigned)((int64_t)nb.x * nb.y * nb.z);
-        auto launch_tiled = [&](auto kern) {
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<nblocks, kPairThreads, smem, h->stream>>>(
+        // several CTAs share a block's nodes where there are few blocks (two CTAs run on an SM at a time)
+        const double per_block = per_cell * Bc * Bc * Bc;
+        const unsigned nparts = (unsigned)std::max(1.0, std::min({std::ceil(8.0 * nsm / nblocks), std::ceil(per_block / 8.0), 64.0}));
+        auto launch_tiled = [&](auto kern, bool vel, bool psi) {
+            const size_t smem = (vel && psi ? sizeof(TileSmem<tile_sources(true, true)>) : sizeof(TileSmem<tile_sources(true, false)>)) +
+                                sizeof(double) * kTabSNC * h->K.ntab_s * (vel && psi ? 2 : 1);
+            // the most a table can need, not this handle's: the attribute belongs to the function
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemMost);
+            kern<<<dim3(nblocks, nparts), kPairThreads, smem, h->stream>>>(
                 h->K, h->cg, Np, Nq, (const int32_t*)h->dst_start.p, (const int32_t*)h->dst_order.p,
                 (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p, (const double*)h->src_sorted.p,
                 (const int32_t*)h->src_start.p, (const int32_t*)h->src_seg.p, (double*)h->vel.p, (double*)h->psi.p,
                 (unsigned long long*)h->counters.p, bk, nb);
         };
-        auto by_fields = [&](auto skip, auto prec) {
+        auto by_fields = [&](auto skip) {
             constexpr bool SK = decltype(skip)::value;
-            using R = typename decltype(prec)::type;
-            if (v && p) launch_tiled(pair_cell_kernel<true, true, SK, R>);
-            else if (v) launch_tiled(pair_cell_kernel<true, false, SK, R>);
-            else launch_tiled(pair_cell_kernel<false, true, SK, R>);
+            if (v && p) launch_tiled(pair_cell_kernel<true, true, SK>, true, true);
+            else if (v) launch_tiled(pair_cell_kernel<true, false, SK>, true, false);
+            else launch_tiled(pair_cell_kernel<false, true, SK>, false, true);
         };
-        if (skip_local) {
-            if (mixed) by_fields(std::true_type{}, PrecTag<float>{});
-            else by_fields(std::true_type{}, PrecTag<double>{});
-        } else {
-            if (mixed) by_fields(std::false_type{}, PrecTag<float>{});
-            else by_fields(std::false_type{}, PrecTag<double>{});
-        }
+        if (skip_local) by_fields(std::true_type{});
+        else by_fields(std::false_type{});
         h->launches++;
         return check_cuda(h, cudaGetLastError(), "pair kernel");
     }

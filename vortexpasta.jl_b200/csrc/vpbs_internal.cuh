@@ -37,6 +37,10 @@ struct KParams {
     // (c0, c1, c2, c3) in powers of t = 32 x - k per interval k; weight a then weight g
     const float4* tab_c;
     int ntab_c;
+    // FP64 tables of the cell-tiled pair kernel, read from shared memory: intervals centred at k / 96 in
+    // x, kTabSNC coefficients in powers of t = 96 x - k; weight a then weight g
+    const double* tab_s;
+    int ntab_s;
 };
 
 // Ewald weight tables: intervals of width 1/16 in x = alpha r, degree-9 Taylor polynomials
@@ -55,6 +59,12 @@ int f32_table_size(double xmax);
 void f32_table_host(const double* tab, int ntab, double xmax, float4* out);  // out: 2 * f32_table_size(xmax)
 // Device-identical host evaluation of the FP32 cubic tables (same float operations).
 void f32_table_eval_host(const float4* tabc, int nf, float x, float* a, float* g);
+
+// FP64 tables of KParams::tab_s fitted to an FP64 table over [0, xmax]: 2 tab_s_size(xmax) kTabSNC values.
+constexpr double kTabSInvH = 96.0;
+constexpr int kTabSNC = 6;
+int tab_s_size(double xmax);
+void tab_s_host(const double* tab, int ntab, double xmax, double* out);
 
 // Gauss-Legendre rule on [-1, 1] (host; longrange.cu).
 void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w);
