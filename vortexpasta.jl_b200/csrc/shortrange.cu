@@ -206,6 +206,7 @@ __device__ __forceinline__ void ewald_weights_f(const KParams& K, float x, float
     }
 }
 
+// ---- naive pair kernel (periodic, without cell lists) ----
 // Per-warp queue of in-range pairs: the separations and source indices of candidates that
 // passed the r^2 <= r_cut^2 test are compacted here (ballot + prefix popcount), so that the
 // erfc/exp evaluation always runs on 32 live lanes instead of on the ~30% of lanes whose
@@ -301,6 +302,75 @@ __device__ __forceinline__ unsigned long long warp_sum_u(unsigned long long v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// All pairs of an open domain (no splitting: the full Biot-Savart integrand, no cut-off).  A thread
+// per node, sources broadcast from shared memory in tiles; blockIdx.y takes its share of the sources
+// and adds its sums to the output with one atomic per component, so that few nodes still fill the
+// device.  Bound: the FP64 pipe (about 30 instructions per pair).
+constexpr int kOpenThreads = 128;
+constexpr int kOpenTile = 128;
+
+template <bool VEL, bool PSI>
+__global__ void __launch_bounds__(kOpenThreads) pair_open_kernel(int64_t Np, int64_t Ns, int per, double pref,
+                                                                 const double* __restrict__ nodes,
+                                                                 const double* __restrict__ points,
+                                                                 const double* __restrict__ charges, double* __restrict__ vel,
+                                                                 double* __restrict__ psi,
+                                                                 unsigned long long* __restrict__ counters) {
+    __shared__ double2 pxy[kOpenTile], pzq[kOpenTile], qyz[kOpenTile];
+    const int64_t i = (int64_t)blockIdx.x * kOpenThreads + threadIdx.x;
+    const int64_t ic = i < Np ? i : Np - 1;
+    const double x0 = nodes[ic], x1 = nodes[Np + ic], x2 = nodes[2 * Np + ic];
+    const int64_t j0 = (int64_t)blockIdx.y * per, j1 = j0 + per < Ns ? j0 + per : Ns;
+    double v0 = 0, v1 = 0, v2 = 0, p0 = 0, p1 = 0, p2 = 0;
+    for (int64_t jt = j0; jt < j1; jt += kOpenTile) {
+        const int n = j1 - jt < kOpenTile ? (int)(j1 - jt) : kOpenTile;
+        __syncthreads();
+        for (int t = threadIdx.x; t < n; t += kOpenThreads) {
+            const int64_t j = jt + t;
+            double s0 = points[j], s1 = points[Ns + j], s2 = points[2 * Ns + j];
+            double q0 = charges[j], q1 = charges[Ns + j], q2 = charges[2 * Ns + j];
+            if (!(s0 == s0 && s1 == s1 && s2 == s2)) {  // a NaN position takes part in no pair
+                s0 = s1 = s2 = 1e100;
+                q0 = q1 = q2 = 0.0;
+            }
+            pxy[t] = make_double2(s0, s1);
+            pzq[t] = make_double2(s2, q0);
+            qyz[t] = make_double2(q1, q2);
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int t = 0; t < n; ++t) {
+            const double2 a = pxy[t], b = pzq[t], c = qyz[t];
+            const double r0 = x0 - a.x, r1 = x1 - a.y, r2 = x2 - b.x;
+            const double rinv = rsqrt(r0 * r0 + r1 * r1 + r2 * r2);
+            if (VEL) {
+                const double f = rinv * rinv * rinv;
+                v0 += f * (c.x * r2 - c.y * r1);
+                v1 += f * (c.y * r0 - b.y * r2);
+                v2 += f * (b.y * r1 - c.x * r0);
+            }
+            if (PSI) {
+                p0 += rinv * b.y;
+                p1 += rinv * c.x;
+                p2 += rinv * c.y;
+            }
+        }
+    }
+    if (i < Np && j0 < j1) {
+        if (VEL) {
+            atomicAdd(&vel[i], pref * v0);
+            atomicAdd(&vel[Np + i], pref * v1);
+            atomicAdd(&vel[2 * Np + i], pref * v2);
+        }
+        if (PSI) {
+            atomicAdd(&psi[i], pref * p0);
+            atomicAdd(&psi[Np + i], pref * p1);
+            atomicAdd(&psi[2 * Np + i], pref * p2);
+        }
+    }
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) counters[threadIdx.x] = (unsigned long long)Np * (unsigned long long)Ns;
 }
 
 // One warp per destination node (visited in cell order when cell lists are used).  R = double
@@ -1481,25 +1551,33 @@ int pair_interactions(vpbs_handle* h, int fields) {
     if ((rc = ensure(h, h->counters, sizeof(unsigned long long) * 2, "counters"))) return rc;
     if ((rc = check_cuda(h, cudaMemsetAsync(h->counters.p, 0, sizeof(unsigned long long) * 2, h->stream), "memset")))
         return rc;
-    if (open) {
-        // naive pair loop over the unsorted point data; the segment of point j is j / nquad
-        if ((rc = ensure(h, h->src_sorted, sizeof(double) * 6 * Nq, "src"))) return rc;
-        if ((rc = ensure(h, h->src_seg, sizeof(int32_t) * Nq, "src_seg"))) return rc;
-        for (int d = 0; d < 3; ++d) {
-            cudaMemcpyAsync((double*)h->src_sorted.p + d * Nq, (double*)h->points.p + d * Nq, sizeof(double) * Nq,
-                            cudaMemcpyDeviceToDevice, h->stream);
-            cudaMemcpyAsync((double*)h->src_sorted.p + (3 + d) * Nq, (double*)h->charges.p + d * Nq,
-                            sizeof(double) * Nq, cudaMemcpyDeviceToDevice, h->stream);
-        }
-    }
     const int skip_local = (!h->K.avoid_explicit_erf && h->K.alpha > 0) ? 1 : 0;
     if (skip_local && open) return set_error(h, VPBS_ERR_PARAMS, "avoid_explicit_erf=false requires Ewald splitting");
     StageScope st(h, ST_PAIRS);
     const unsigned grid = grid_for(Np, 8);
     const bool v = fields & VPBS_VELOCITY, p = fields & VPBS_STREAMFUNCTION;
+    if (open) {
+        // about eight CTAs per SM, each with at least one tile of sources
+        const unsigned gx = grid_for(Np, kOpenThreads);
+        int nsm = 148;
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
+        const int64_t want = std::min<int64_t>((8 * (int64_t)nsm + gx - 1) / gx, (Nq + kOpenTile - 1) / kOpenTile);
+        const int64_t parts = std::max<int64_t>(1, std::min<int64_t>(want, 65535));
+        const int per = (int)((Nq + parts - 1) / parts);
+        auto launch_open = [&](auto kern) {
+            kern<<<dim3(gx, (unsigned)parts), kOpenThreads, 0, h->stream>>>(
+                Np, Nq, per, h->K.Gamma / (4.0 * kPi), (const double*)h->nodes.p, (const double*)h->points.p,
+                (const double*)h->charges.p, (double*)h->vel.p, (double*)h->psi.p, (unsigned long long*)h->counters.p);
+        };
+        if (v && p) launch_open(pair_open_kernel<true, true>);
+        else if (v) launch_open(pair_open_kernel<true, false>);
+        else launch_open(pair_open_kernel<false, true>);
+        h->launches++;
+        return check_cuda(h, cudaGetLastError(), "open-domain pair kernel");
+    }
     const CellGrid& cg = h->cg;
     const int Wc = 2 * cg.M + 1;
-    if (!open && cg.M > 0 && Wc * Wc <= kMaxRows && Wc * Wc * Wc * cg.G <= kMaxNbCells &&
+    if ( cg.M > 0 && Wc * Wc <= kMaxRows && Wc * Wc * Wc * cg.G <= kMaxNbCells &&
         sizeof(TileSmem<1024>) + 2 * sizeof(double) * kTabSNC * h->K.ntab_s <= kPairSmemMost) {
         // blocks of Bc^3 cells per CTA, grown while a block holds fewer than ~24 nodes on average,
         // at least 16 CTAs per SM remain, and the neighbourhood fits the shared-memory tables and
@@ -1597,7 +1675,7 @@ int pair_interactions(vpbs_handle* h, int fields) {
     auto launch = [&](auto kern) {
         kern<<<grid, 256, 0, h->stream>>>(h->K, h->cg, Np, Nq, (const int32_t*)h->dst_order.p, (const double*)h->nodes.p,
                                           (const int32_t*)h->idx_prev.p, (const double*)h->src_sorted.p,
-                                          (const int32_t*)h->src_start.p, (const int32_t*)h->src_seg.p, (open || h->cg.M == 0) ? 0 : 1,
+                                          (const int32_t*)h->src_start.p, (const int32_t*)h->src_seg.p, h->cg.M == 0 ? 0 : 1,
                                           skip_local, (double*)h->vel.p, (double*)h->psi.p,
                                           (unsigned long long*)h->counters.p);
     };
