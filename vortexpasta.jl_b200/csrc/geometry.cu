@@ -2,10 +2,9 @@
 // the point data of add_point_charges! (src/BiotSavart/pointdata_impl.jl:41-108).
 //
 // One warp per filament solves the cyclic pentadiagonal B-spline collocation system
-// (src/Filaments/spline/quintic.jl:9-100 solves the same system): the band part is
-// factorised by elimination without pivoting (collocation matrices of B-splines are totally
-// positive), the seven right-hand sides (x, y, z and the four wrap-around columns) are swept
-// by seven lanes in parallel, and the corners are folded back with the Woodbury identity.
+// (src/Filaments/spline/quintic.jl:9-100 solves the same system): cut into one block per lane, eliminated
+// in parallel and joined by cyclic reduction between the lanes (short filaments and extreme node spacings:
+// banded elimination and the Woodbury identity).
 // A second kernel evaluates the splines at the nodes and quadrature points, one thread per node.
 #include "vpbs_internal.cuh"
 #include "periodic.cuh"
@@ -189,6 +188,298 @@ __device__ void solve4(double H[4][4], double r[4][3]) {
         }
 }
 
+// The cyclic pentadiagonal system of one filament by the lanes of a warp together.  The n rows are cut
+// into P blocks (P a power of two, at least 4 rows each, one lane per block).  Every lane eliminates its
+// block for 7 right-hand sides: the three coordinates and the 2 + 2 columns that couple it to the last two
+// unknowns of the block before and the first two of the block after, which leaves
+//     y_l + A_l b_{l-1} + C_l t_{l+1} = g_l,   y_l = (t_l, b_l): first two and last two unknowns of block l.
+// log2 P steps of cyclic reduction double the distance of the coupling (shuffles between lanes l and l +- s,
+// a 4 x 4 system each) until every block is coupled to itself alone.  Solution in Y[.][0..2].
+// Elimination goes without pivoting: false if a pivot is below 1/16 of the unit diagonal (node spacings that
+// differ by orders of magnitude from one to the next), and the caller solves serially.
+// Bound: a chain of about n / P + 5 * 4 dependent divisions instead of n (200 nodes: 75 us serially).
+__device__ __noinline__ bool solve_partitioned(const FilView& f, const double* t, double T, const double* Xf, int n,
+                                               double o0, double o1, double o2, double* band, double* Y, int lane) {
+    const int P = n >= 128 ? 32 : n >= 64 ? 16 : n >= 32 ? 8 : 4;
+    const unsigned full = 0xffffffffu;
+    // collocation rows (cyclic): band[5 i + s] multiplies u_{i + s - 2}
+    for (int i = lane; i < n; i += 32) {
+        double N[6];
+        bsplvb<6>(f, i, knot_at(f, i), N);
+#pragma unroll
+        for (int s = 0; s < 5; ++s) band[5 * i + s] = N[s];
+        const double r = t[i] / T;
+        Y[7 * i + 0] = Xf[3 * i + 0] - r * o0;
+        Y[7 * i + 1] = Xf[3 * i + 1] - r * o1;
+        Y[7 * i + 2] = Xf[3 * i + 2] - r * o2;
+#pragma unroll
+        for (int q = 3; q < 7; ++q) Y[7 * i + q] = 0.0;
+    }
+    __syncwarp();
+    const int l = lane & (P - 1);  // lanes past P repeat a block (and write nothing)
+    const bool own = lane < P;
+    const int s0 = (int)((int64_t)l * n / P), s1 = (int)((int64_t)(l + 1) * n / P), p = s1 - s0;
+    if (own) {
+        Y[7 * s0 + 3] = band[5 * s0];
+        Y[7 * s0 + 4] = band[5 * s0 + 1];
+        Y[7 * (s0 + 1) + 4] = band[5 * (s0 + 1)];
+        Y[7 * (s1 - 1) + 5] = band[5 * (s1 - 1) + 3];
+        Y[7 * (s1 - 1) + 6] = band[5 * (s1 - 1) + 4];
+        Y[7 * (s1 - 2) + 5] = band[5 * (s1 - 2) + 4];
+        double iu_2 = 0.0, u1_2 = 0.0, u2_2 = 0.0, iu_1 = 0.0, u1_1 = 0.0, u2_1 = 0.0, z1[7], z2[7];
+#pragma unroll
+        for (int q = 0; q < 7; ++q) z1[q] = z2[q] = 0.0;
+        for (int r = 0; r < p; ++r) {
+            double* w = band + 5 * (s0 + r);
+            double* y = Y + 7 * (s0 + r);
+            const double e = r >= 2 ? w[0] : 0.0, d = r >= 1 ? w[1] : 0.0, c = w[2], b = r + 1 < p ? w[3] : 0.0,
+                         a = r + 2 < p ? w[4] : 0.0;
+            const double l2 = e * iu_2, l1 = (d - l2 * u1_2) * iu_1;
+            const double iu = 1.0 / (c - l2 * u2_2 - l1 * u1_1), u1 = b - l1 * u2_1;
+#pragma unroll
+            for (int q = 0; q < 7; ++q) {
+                const double z = y[q] - l1 * z1[q] - l2 * z2[q];
+                y[q] = z;
+                z2[q] = z1[q];
+                z1[q] = z;
+            }
+            w[2] = iu;
+            w[3] = u1;
+            w[4] = a;
+            iu_2 = iu_1; u1_2 = u1_1; u2_2 = u2_1;
+            iu_1 = iu; u1_1 = u1; u2_1 = a;
+        }
+#pragma unroll
+        for (int q = 0; q < 7; ++q) z1[q] = z2[q] = 0.0;
+        for (int r = p - 1; r >= 0; --r) {
+            const double* w = band + 5 * (s0 + r);
+            double* y = Y + 7 * (s0 + r);
+#pragma unroll
+            for (int q = 0; q < 7; ++q) {
+                const double x = (y[q] - w[3] * z1[q] - w[4] * z2[q]) * w[2];
+                y[q] = x;
+                z2[q] = z1[q];
+                z1[q] = x;
+            }
+        }
+    }
+    __syncwarp();
+    double g[4][3], A[4][2], C[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const double* y = Y + 7 * (r < 2 ? s0 + r : s1 - 4 + r);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) g[r][q] = y[q];
+        A[r][0] = y[3];
+        A[r][1] = y[4];
+        C[r][0] = y[5];
+        C[r][1] = y[6];
+    }
+    bool fine = true;
+    for (int s = 1; s < P; s <<= 1) {
+        const int lm = (l - s) & (P - 1), lp = (l + s) & (P - 1);
+        double gm[2][3], Am[2][2], Cm[2][2], gp[2][3], Ap[2][2], Cp[2][2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                gm[r][q] = __shfl_sync(full, g[2 + r][q], lm);
+                gp[r][q] = __shfl_sync(full, g[r][q], lp);
+            }
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                Am[r][q] = __shfl_sync(full, A[2 + r][q], lm);
+                Cm[r][q] = __shfl_sync(full, C[2 + r][q], lm);
+                Ap[r][q] = __shfl_sync(full, A[r][q], lp);
+                Cp[r][q] = __shfl_sync(full, C[r][q], lp);
+            }
+        }
+        double M[4][4], R[4][7];  // M y = R: columns 0-2 the new g, 3-4 minus the new A, 5-6 minus the new C
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                M[r][q] = (r == q ? 1.0 : 0.0) - (A[r][0] * Cm[0][q] + A[r][1] * Cm[1][q]);
+                M[r][2 + q] = (r == 2 + q ? 1.0 : 0.0) - (C[r][0] * Ap[0][q] + C[r][1] * Ap[1][q]);
+                R[r][3 + q] = -(A[r][0] * Am[0][q] + A[r][1] * Am[1][q]);
+                R[r][5 + q] = -(C[r][0] * Cp[0][q] + C[r][1] * Cp[1][q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                R[r][q] = g[r][q] - (A[r][0] * gm[0][q] + A[r][1] * gm[1][q]) - (C[r][0] * gp[0][q] + C[r][1] * gp[1][q]);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            fine = fine && fabs(M[c][c]) >= 0.0625;
+            const double inv = 1.0 / M[c][c];
+#pragma unroll
+            for (int k = c + 1; k < 4; ++k) M[c][k] *= inv;
+#pragma unroll
+            for (int k = 0; k < 7; ++k) R[c][k] *= inv;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                if (r == c) continue;
+                const double m = M[r][c];
+#pragma unroll
+                for (int k = c + 1; k < 4; ++k) M[r][k] -= m * M[c][k];
+#pragma unroll
+                for (int k = 0; k < 7; ++k) R[r][k] -= m * R[c][k];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) g[r][q] = R[r][q];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                A[r][q] = R[r][3 + q];
+                C[r][q] = R[r][5 + q];
+            }
+        }
+    }
+    if (!__all_sync(full, fine)) return false;
+    // every block by itself: y + A b + C t = g
+    {
+        double H[4][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                H[r][q] = (r == q ? 1.0 : 0.0) + C[r][q];
+                H[r][2 + q] = (r == 2 + q ? 1.0 : 0.0) + A[r][q];
+            }
+        solve4(H, g);
+    }
+    // back substitution with the neighbours' unknowns
+    double bm[2][3], tp[2][3];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            bm[r][q] = __shfl_sync(full, g[2 + r][q], (l - 1) & (P - 1));
+            tp[r][q] = __shfl_sync(full, g[r][q], (l + 1) & (P - 1));
+        }
+    if (own)
+        for (int r = 0; r < p; ++r) {
+            double* y = Y + 7 * (s0 + r);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) y[q] -= y[3] * bm[0][q] + y[4] * bm[1][q] + y[5] * tp[0][q] + y[6] * tp[1][q];
+        }
+    __syncwarp();
+    return true;
+}
+
+// The same system by banded elimination (one lane, no pivoting: collocation matrices of B-splines are
+// totally positive) and the Woodbury identity for the wrap-around corners.  Solution in Y[.][0..2].
+__device__ __noinline__ void solve_serial(const FilView& f, const double* t, double T, const double* Xf, int n, double o0,
+                                          double o1, double o2, double* band, double* Y, int lane) {
+    // collocation rows, band part only (corners handled below)
+    for (int i = lane; i < n; i += 32) {
+        double N[6];
+        bsplvb<6>(f, i, knot_at(f, i), N);
+#pragma unroll
+        for (int s = 0; s < 5; ++s) {
+            int col = i + s - 2;
+            band[5 * i + s] = (col >= 0 && col < n) ? N[s] : 0.0;
+        }
+        const double r = t[i] / T;
+        Y[7 * i + 0] = Xf[3 * i + 0] - r * o0;
+        Y[7 * i + 1] = Xf[3 * i + 1] - r * o1;
+        Y[7 * i + 2] = Xf[3 * i + 2] - r * o2;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            int ur = (q == 0) ? 0 : (q == 1) ? 1 : (q == 2) ? n - 2 : n - 1;
+            Y[7 * i + 3 + q] = (i == ur) ? 1.0 : 0.0;
+        }
+    }
+    __syncwarp();
+
+    // pentadiagonal LU without pivoting (serial, lane 0), as a register recurrence: row i of
+    //    the band (e, d, c, b, a at columns i-2..i+2) becomes (l2, l1, 1/u0, u1, u2):
+    //    l2 = e/u0[i-2], l1 = (d - l2 u1[i-2])/u0[i-1], u0 = c - l2 u2[i-2] - l1 u1[i-1],
+    //    u1 = b - l1 u2[i-1], u2 = a.
+    if (lane == 0) {
+        double iu0_m2 = 0.0, u1_m2 = 0.0, u2_m2 = 0.0;  // row i-2
+        double iu0_m1 = 0.0, u1_m1 = 0.0, u2_m1 = 0.0;  // row i-1
+        for (int i = 0; i < n; ++i) {
+            double* r = band + 5 * i;
+            const double e = r[0], d = r[1], c = r[2], b = r[3], a = r[4];
+            const double l2 = e * iu0_m2;
+            const double l1 = (d - l2 * u1_m2) * iu0_m1;
+            const double u0 = c - l2 * u2_m2 - l1 * u1_m1;
+            const double u1 = b - l1 * u2_m1;
+            const double iu0 = 1.0 / u0;
+            r[0] = l2;
+            r[1] = l1;
+            r[2] = iu0;
+            r[3] = u1;
+            r[4] = a;
+            iu0_m2 = iu0_m1; u1_m2 = u1_m1; u2_m2 = u2_m1;
+            iu0_m1 = iu0; u1_m1 = u1; u2_m1 = a;
+        }
+    }
+    __syncwarp();
+
+    // forward / backward sweeps, one right-hand side per lane (register recurrences)
+    if (lane < 7) {
+        const int q = lane;
+        double z1 = 0.0, z2 = 0.0;  // z[i-1], z[i-2]
+        for (int i = 0; i < n; ++i) {
+            const double* r = band + 5 * i;
+            const double z = Y[7 * i + q] - r[1] * z1 - r[0] * z2;
+            Y[7 * i + q] = z;
+            z2 = z1;
+            z1 = z;
+        }
+        double x1 = 0.0, x2 = 0.0;  // x[i+1], x[i+2]
+        for (int i = n - 1; i >= 0; --i) {
+            const double* r = band + 5 * i;
+            const double x = (Y[7 * i + q] - r[3] * x1 - r[4] * x2) * r[2];
+            Y[7 * i + q] = x;
+            x2 = x1;
+            x1 = x;
+        }
+    }
+    __syncwarp();
+
+    // Woodbury correction: corners W of rows 0, 1, n-2, n-1
+    __shared__ double sh_s[4][4][3];
+    double (*s4)[3] = sh_s[threadIdx.x >> 5];
+    if (lane == 0) {
+        double H[4][4], rh[4][3];
+        const int rows[4] = {0, 1, n - 2, n - 1};
+        for (int r = 0; r < 4; ++r) {
+            for (int q = 0; q < 4; ++q) H[r][q] = (r == q) ? 1.0 : 0.0;
+            for (int d = 0; d < 3; ++d) rh[r][d] = 0.0;
+            int i = rows[r];
+            double N[6];
+            bsplvb<6>(f, i, knot_at(f, i), N);
+            for (int s = 0; s < 5; ++s) {
+                int col = i + s - 2;
+                if (col >= 0 && col < n) continue;
+                int cw = (int)pmodl(col, n);
+                for (int q = 0; q < 4; ++q) H[r][q] += N[s] * Y[7 * cw + 3 + q];
+                for (int d = 0; d < 3; ++d) rh[r][d] += N[s] * Y[7 * cw + d];
+            }
+        }
+        solve4(H, rh);
+        for (int r = 0; r < 4; ++r)
+            for (int d = 0; d < 3; ++d) s4[r][d] = rh[r][d];
+    }
+    __syncwarp();
+
+    // u = y - Z s
+    for (int i = lane; i < n; i += 32)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            double u = Y[7 * i + d];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) u -= Y[7 * i + 3 + q] * s4[q][d];
+            Y[7 * i + d] = u;
+        }
+    __syncwarp();
+}
+
 // One warp per filament.  Work space: 12 doubles per node (5 band + 7 right-hand sides), in
 // dynamic shared memory (smem_n doubles x 12 per warp) when smem_n > 0, else in `scratch`.
 // keep_knots: reuse the knots and periods already in `knots` / `periods` (the knots frozen
@@ -251,114 +542,16 @@ __global__ void __launch_bounds__(128) spline_solve_kernel(
     const double o0 = foff ? foff[3 * fidx] : 0.0, o1 = foff ? foff[3 * fidx + 1] : 0.0,
                  o2 = foff ? foff[3 * fidx + 2] : 0.0;
 
-    // 2. collocation rows, band part only (corners handled below)
+    // 2. spline coefficients: cyclic pentadiagonal collocation system
+    const bool solved = n >= 16 && solve_partitioned(f, t, T, Xf, n, o0, o1, o2, band, Y, lane);
+    if (!solved) solve_serial(f, t, T, Xf, n, o0, o1, o2, band, Y, lane);
     for (int i = lane; i < n; i += 32) {
-        double N[6];
-        bsplvb<6>(f, i, knot_at(f, i), N);
+        const int j = (int)pmodl(i - 3, n);  // u_i = c_{i-3}
 #pragma unroll
-        for (int s = 0; s < 5; ++s) {
-            int col = i + s - 2;
-            band[5 * i + s] = (col >= 0 && col < n) ? N[s] : 0.0;
-        }
-        const double r = t[i] / T;
-        Y[7 * i + 0] = Xf[3 * i + 0] - r * o0;
-        Y[7 * i + 1] = Xf[3 * i + 1] - r * o1;
-        Y[7 * i + 2] = Xf[3 * i + 2] - r * o2;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int ur = (q == 0) ? 0 : (q == 1) ? 1 : (q == 2) ? n - 2 : n - 1;
-            Y[7 * i + 3 + q] = (i == ur) ? 1.0 : 0.0;
-        }
+        for (int d = 0; d < 3; ++d) c[3 * j + d] = Y[7 * i + d];
     }
     __syncwarp();
-
-    // 3. pentadiagonal LU without pivoting (serial, lane 0), as a register recurrence: row i of
-    //    the band (e, d, c, b, a at columns i-2..i+2) becomes (l2, l1, 1/u0, u1, u2):
-    //    l2 = e/u0[i-2], l1 = (d - l2 u1[i-2])/u0[i-1], u0 = c - l2 u2[i-2] - l1 u1[i-1],
-    //    u1 = b - l1 u2[i-1], u2 = a.
-    if (lane == 0) {
-        double iu0_m2 = 0.0, u1_m2 = 0.0, u2_m2 = 0.0;  // row i-2
-        double iu0_m1 = 0.0, u1_m1 = 0.0, u2_m1 = 0.0;  // row i-1
-        for (int i = 0; i < n; ++i) {
-            double* r = band + 5 * i;
-            const double e = r[0], d = r[1], c = r[2], b = r[3], a = r[4];
-            const double l2 = e * iu0_m2;
-            const double l1 = (d - l2 * u1_m2) * iu0_m1;
-            const double u0 = c - l2 * u2_m2 - l1 * u1_m1;
-            const double u1 = b - l1 * u2_m1;
-            const double iu0 = 1.0 / u0;
-            r[0] = l2;
-            r[1] = l1;
-            r[2] = iu0;
-            r[3] = u1;
-            r[4] = a;
-            iu0_m2 = iu0_m1; u1_m2 = u1_m1; u2_m2 = u2_m1;
-            iu0_m1 = iu0; u1_m1 = u1; u2_m1 = a;
-        }
-    }
-    __syncwarp();
-
-    // 4. forward / backward sweeps, one right-hand side per lane (register recurrences)
-    if (lane < 7) {
-        const int q = lane;
-        double z1 = 0.0, z2 = 0.0;  // z[i-1], z[i-2]
-        for (int i = 0; i < n; ++i) {
-            const double* r = band + 5 * i;
-            const double z = Y[7 * i + q] - r[1] * z1 - r[0] * z2;
-            Y[7 * i + q] = z;
-            z2 = z1;
-            z1 = z;
-        }
-        double x1 = 0.0, x2 = 0.0;  // x[i+1], x[i+2]
-        for (int i = n - 1; i >= 0; --i) {
-            const double* r = band + 5 * i;
-            const double x = (Y[7 * i + q] - r[3] * x1 - r[4] * x2) * r[2];
-            Y[7 * i + q] = x;
-            x2 = x1;
-            x1 = x;
-        }
-    }
-    __syncwarp();
-
-    // 5. Woodbury correction: corners W of rows 0, 1, n-2, n-1
-    __shared__ double sh_s[4][4][3];
-    double (*s4)[3] = sh_s[threadIdx.x >> 5];
-    if (lane == 0) {
-        double H[4][4], rh[4][3];
-        const int rows[4] = {0, 1, n - 2, n - 1};
-        for (int r = 0; r < 4; ++r) {
-            for (int q = 0; q < 4; ++q) H[r][q] = (r == q) ? 1.0 : 0.0;
-            for (int d = 0; d < 3; ++d) rh[r][d] = 0.0;
-            int i = rows[r];
-            double N[6];
-            bsplvb<6>(f, i, knot_at(f, i), N);
-            for (int s = 0; s < 5; ++s) {
-                int col = i + s - 2;
-                if (col >= 0 && col < n) continue;
-                int cw = (int)pmodl(col, n);
-                for (int q = 0; q < 4; ++q) H[r][q] += N[s] * Y[7 * cw + 3 + q];
-                for (int d = 0; d < 3; ++d) rh[r][d] += N[s] * Y[7 * cw + d];
-            }
-        }
-        solve4(H, rh);
-        for (int r = 0; r < 4; ++r)
-            for (int d = 0; d < 3; ++d) s4[r][d] = rh[r][d];
-    }
-    __syncwarp();
-
-    // 6. coefficients c_j = u_{j+3}, u = y - Z s
-    for (int i = lane; i < n; i += 32) {
-        int j = (int)pmodl(i - 3, n);  // u_i = c_{i-3}
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            double u = Y[7 * i + d];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) u -= Y[7 * i + 3 + q] * s4[q][d];
-            c[3 * j + d] = u;
-        }
-    }
-    __syncwarp();
-    // 7. derivative coefficients (spline derivative recurrence, spline.jl:301-319)
+    // 3. derivative coefficients (spline derivative recurrence, spline.jl:301-319)
     for (int j = lane; j < n; j += 32) {
         int jm = (j == 0) ? n - 1 : j - 1;
         double den = knot_at(f, j + 5) - knot_at(f, j);
