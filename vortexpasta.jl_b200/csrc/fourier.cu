@@ -150,6 +150,22 @@ __global__ void __launch_bounds__(kFftThreads, sizeof(T) == 4 && !W ? 2 : 1) fft
     }
 }
 
+// Value pos of the packed transform of a line X of half-spectrum modes:
+// Z_k = (X_k + conj X_{H-k}) + i e^{2 pi i k / n} (X_k - conj X_{H-k}); X_k = 0 for k >= kx (kx <= H); the
+// imaginary part of X_0 does not enter a real field.
+template <typename C>
+__device__ __forceinline__ C x_inverse_input(const C* __restrict__ X, int pos, int H, int kx, const C* __restrict__ twr) {
+    using T = decltype(C::x);
+    C a = fft::mk((T)0, (T)0), b = a;
+    if (pos < kx) a = X[pos];
+    if (pos == 0) a.y = (T)0;
+    const int q = H - pos;
+    if (q < kx) b = X[q];
+    const C s = fft::mk(a.x + b.x, a.y - b.y), d = fft::mk(a.x - b.x, a.y + b.y);
+    const C t = fft::mul_tw<1>(d, __ldg(twr + pos));
+    return fft::mk(s.x - t.y, s.y + t.x);
+}
+
 template <typename T, bool W>
 __global__ void __launch_bounds__(kFftThreads, sizeof(T) == 4 && !W ? 2 : 1) fft_x_inverse(Plan P, int64_t nl, int LY, int kx, int kxp,
                                                              const typename Cplx<T>::type* __restrict__ in,
@@ -165,22 +181,41 @@ __global__ void __launch_bounds__(kFftThreads, sizeof(T) == 4 && !W ? 2 : 1) fft
     const LinesX lay{P.len};
     in += l0 * kxp;
     out += l0 * H;
-    // Z_k = (X_k + conj X_{H-k}) + i e^{2 pi i k / n} (X_k - conj X_{H-k}); X_k = 0 for k >= kx (kx <= H);
-    // the imaginary part of X_0 does not enter a real field
     fft::run_in<1, W>(S, lay, P.p[0], nlines, [&](int line, int pos) {
-        const C* X = in + (int64_t)line * kxp;
-        C a = fft::mk((T)0, (T)0), b = a;
-        if (pos < kx) a = X[pos];
-        if (pos == 0) a.y = (T)0;
-        const int q = H - pos;
-        if (q < kx) b = X[q];
-        const C s = fft::mk(a.x + b.x, a.y - b.y), d = fft::mk(a.x - b.x, a.y + b.y);
-        const C t = fft::mul_tw<1>(d, __ldg(twr + pos));
-        return fft::mk(s.x - t.y, s.y + t.x);
+        return x_inverse_input(in + (int64_t)line * kxp, pos, H, kx, twr);
     });
     for (int i = 1; i + 1 < P.np; ++i) fft::run_mid<1, W>(S, lay, P.p[i], nlines, tw);
     fft::run_out<1, W>(S, lay, P.p[P.np - 1], nlines, tw,
                     [&](int line, int pos, C v) { out[(int64_t)line * H + pos] = v; });
+}
+
+// fft_x_inverse with the three components of a grid point side by side, out[row][x] = (c0, c1, c2, 0), the
+// layout the interpolation of many nodes reads: a block takes whole rows of all components, the last pass
+// stays in shared memory and the rows are written from there, 32 bytes a thread.  FP32 grids only.
+template <bool W>
+__global__ void __launch_bounds__(kFftThreads, W ? 1 : 2) fft_x_inverse_quad(Plan P, int64_t rows, int LY, int kx, int kxp,
+                                                                             const float2* __restrict__ in,
+                                                                             float4* __restrict__ out,
+                                                                             const float2* __restrict__ tw,
+                                                                             const float2* __restrict__ twr) {
+    extern __shared__ __align__(16) unsigned char fft_raw[];
+    float2* S = reinterpret_cast<float2*>(fft_raw);
+    const int H = P.n;
+    const int64_t r0 = (int64_t)blockIdx.x * LY;
+    const int nr = rows - r0 < LY ? (int)(rows - r0) : LY;
+    const LinesX lay{P.len};
+    fft::run_in<1, W>(S, lay, P.p[0], 3 * nr, [&](int line, int pos) {
+        const int c = line >= 2 * nr ? 2 : line >= nr ? 1 : 0;
+        return x_inverse_input(in + (c * rows + r0 + (line - c * nr)) * kxp, pos, H, kx, twr);
+    });
+    for (int i = 1; i < P.np; ++i) fft::run_mid<1, W>(S, lay, P.p[i], 3 * nr, tw);
+    out += r0 * 2 * H;
+    for (int idx = threadIdx.x; idx < nr * H; idx += blockDim.x) {
+        const int row = idx / H, pos = idx - row * H;
+        const float2 a = S[lay.at(row, pos)], b = S[lay.at(nr + row, pos)], c = S[lay.at(2 * nr + row, pos)];
+        out[2 * idx] = make_float4(a.x, b.x, c.x, 0.0f);
+        out[2 * idx + 1] = make_float4(a.y, b.y, c.y, 0.0f);
+    }
 }
 
 // ---- y: n1 rows <-> the Ns1 kept ones (row = k_y mod Ns1, k_y = -(Ns1/2) .. (Ns1-1)/2) ----
@@ -334,8 +369,8 @@ struct Shape {
 
 struct FourierPlan {
     Plan px, py, pz;
-    int LY = 1, ltxy = 0, ltxz = 0, kx = 0, kxp = 0;
-    Shape sx, sy, sz;
+    int LY = 1, LYq = 1, ltxy = 0, ltxz = 0, kx = 0, kxp = 0;
+    Shape sx, sq, sy, sz;
     size_t twr = 0;  // offset (in complex values) of e^{-2 pi i k / n0} in the tables
 };
 
@@ -365,7 +400,8 @@ template <typename T>
 int set_attributes(vpbs_handle* h, const FourierPlan& F) {
     const void* k[] = {(const void*)VPBS_FFT_KERNEL(fft_x_forward, T, F.px), (const void*)VPBS_FFT_KERNEL(fft_x_inverse, T, F.px),
                        (const void*)VPBS_FFT_KERNEL(fft_y_forward, T, F.py), (const void*)VPBS_FFT_KERNEL(fft_y_inverse, T, F.py),
-                       (const void*)VPBS_FFT_KERNEL(fft_z_operator, T, F.pz)};
+                       (const void*)VPBS_FFT_KERNEL(fft_z_operator, T, F.pz),
+                       F.px.wide ? (const void*)fft_x_inverse_quad<true> : (const void*)fft_x_inverse_quad<false>};
     for (const void* f : k) {
         // the limit, not this plan's size: the attribute belongs to the function, not to the handle
         int rc = check_cuda(h, cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFftSmemMost),
@@ -430,7 +466,7 @@ int run_operator_t(vpbs_handle* h, const FourierOp& op) {
 }
 
 template <typename T>
-int run_inverse_t(vpbs_handle* h, void* grid) {
+int run_inverse_t(vpbs_handle* h, void* grid, bool quad) {
     using C = typename Cplx<T>::type;
     const FourierPlan& F = *h->fplan;
     const LRSizes& S = h->lr;
@@ -439,6 +475,16 @@ int run_inverse_t(vpbs_handle* h, void* grid) {
     const int64_t nl = (int64_t)3 * S.n[2] * S.n[1];
     VPBS_FFT_KERNEL(fft_y_inverse, T, F.py)<<<dim3(F.kxp >> F.ltxy, 3 * S.n[2]), F.sy.threads, F.sy.smem, h->stream>>>(F.py, F.ltxy, S.Ns[1], F.kxp,
                                                                                               g, tw);
+    if constexpr (sizeof(T) == 4) {
+        if (quad) {
+            const int64_t rows = (int64_t)S.n[2] * S.n[1];
+            auto* kern = F.px.wide ? fft_x_inverse_quad<true> : fft_x_inverse_quad<false>;
+            kern<<<(unsigned)((rows + F.LYq - 1) / F.LYq), F.sq.threads, F.sq.smem, h->stream>>>(
+                F.px, rows, F.LYq, F.kx, F.kxp, g, (float4*)grid, tw, tw + F.twr);
+            h->launches += 2;
+            return check_cuda(h, cudaGetLastError(), "inverse FFT kernels");
+        }
+    }
     VPBS_FFT_KERNEL(fft_x_inverse, T, F.px)<<<(unsigned)((nl + F.LY - 1) / F.LY), F.sx.threads, F.sx.smem, h->stream>>>(
         F.px, nl, F.LY, F.kx, F.kxp, g, (C*)grid, tw, tw + F.twr);
     h->launches += 2;
@@ -484,7 +530,10 @@ int fourier_init(vpbs_handle* h) {
     F.LY = std::max(1, 256 / tpl);
     F.sx.threads = round32(F.LY * tpl);
     F.sx.smem = csize * F.LY * F.px.len;
-    if (F.sx.smem > kFftSmemMost) return 0;
+    F.LYq = std::max(1, F.LY / 3);
+    F.sq.threads = round32(3 * F.LYq * tpl);
+    F.sq.smem = csize * 3 * F.LYq * F.px.len;
+    if (F.sx.smem > kFftSmemMost || F.sq.threads > kFftThreads || F.sq.smem > kFftSmemMost) return 0;
     if (!tile_shape(F.py, 1, csize, F.kx, &F.ltxy, &F.sy) || !tile_shape(F.pz, 3, csize, F.kx, &F.ltxz, &F.sz)) return 0;
     const int tile = 1 << std::max(F.ltxy, F.ltxz);
     F.kxp = (F.kx + tile - 1) / tile * tile;
@@ -511,8 +560,8 @@ int fourier_forward(vpbs_handle* h, const void* grid) {
 int fourier_operator(vpbs_handle* h, const FourierOp& op) {
     return h->P.precision == VPBS_PRECISION_MIXED ? run_operator_t<float>(h, op) : run_operator_t<double>(h, op);
 }
-int fourier_inverse(vpbs_handle* h, void* grid) {
-    return h->P.precision == VPBS_PRECISION_MIXED ? run_inverse_t<float>(h, grid) : run_inverse_t<double>(h, grid);
+int fourier_inverse(vpbs_handle* h, void* grid, bool quad) {
+    return h->P.precision == VPBS_PRECISION_MIXED ? run_inverse_t<float>(h, grid, quad) : run_inverse_t<double>(h, grid, false);
 }
 
 }  // namespace vpbs

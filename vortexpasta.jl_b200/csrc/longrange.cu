@@ -1071,6 +1071,76 @@ __global__ void __launch_bounds__(256) interp_warp_kernel(
     }
 }
 
+// Type-2 interpolation from an FP32 grid of (c0, c1, c2, 0) values: 8 lanes per node, each with its share
+// of the footprint's (x, y) points (weight and offset kept in registers) for all z, one 16-byte load a point
+// for the three components.  A z-slab's few products are added in FP32, the slabs and the lanes in FP64.
+// Bound: issue slots and the cache lines of the gathers (36 rows of 96 bytes at m = 3, a third of the lines
+// that three separate components touch).
+template <int W>
+__global__ void __launch_bounds__(256) interp_quad_kernel(LRSizes S, int64_t Np, const int32_t* __restrict__ order,
+                                                          const double* __restrict__ nodes, double sx0, double sx1,
+                                                          double sx2, const float4* __restrict__ grid,
+                                                          double* __restrict__ out) {
+    constexpr int G = 8, NB = 256 / G, NP = (W * W + G - 1) / G;
+    __shared__ float phs[NB][3][W];
+    __shared__ int ixs[NB][3][W];
+    const int l8 = threadIdx.x % G, nd = threadIdx.x / G;
+    const int64_t t = (int64_t)blockIdx.x * NB + nd;
+    const bool have = t < Np;
+    const int64_t i = have ? (order ? order[t] : t) : 0;
+    for (int e = l8; e < 3 * W; e += G) {
+        const int d = e / W, s = e % W;
+        const double scale = d == 0 ? sx0 : (d == 1 ? sx1 : sx2);
+        const double xh = (nodes[d * Np + i] * scale) / (2.0 * kPi / S.n[d]);
+        const int i0 = (int)floor(xh) - S.m + 1;
+        phs[nd][d][s] = (float)es_kernel_w<W>(xh - (i0 + s), S.beta, S.edge, S.kernel);
+        // the start folded once by a modulo (any i0, also from a non-finite node), then i0w + s < 2n
+        ixs[nd][d][s] = wrap1(wrapi(i0, S.n[d]) + s, S.n[d]);
+    }
+    __syncwarp();
+    const int n0 = S.n[0];
+    const int64_t plane = (int64_t)S.n[1] * n0;
+    float w[NP];
+    int o[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        const int q = l8 + G * p;
+        const bool in = q < W * W;
+        const int sx = in ? q % W : 0, sy = in ? q / W : 0;
+        w[p] = in ? phs[nd][0][sx] * phs[nd][1][sy] : 0.0f;
+        o[p] = ixs[nd][1][sy] * n0 + ixs[nd][0][sx];
+    }
+    double b0 = 0.0, b1 = 0.0, b2 = 0.0;
+#pragma unroll 2
+    for (int z = 0; z < W; ++z) {
+        const float fz = phs[nd][2][z];
+        const float4* g = grid + ixs[nd][2][z] * plane;
+        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+            const float4 v = g[o[p]];
+            const float f = w[p] * fz;
+            a0 = fmaf(f, v.x, a0);
+            a1 = fmaf(f, v.y, a1);
+            a2 = fmaf(f, v.z, a2);
+        }
+        b0 += a0;
+        b1 += a1;
+        b2 += a2;
+    }
+#pragma unroll
+    for (int s = G / 2; s > 0; s >>= 1) {
+        b0 += __shfl_xor_sync(0xffffffffu, b0, s);
+        b1 += __shfl_xor_sync(0xffffffffu, b1, s);
+        b2 += __shfl_xor_sync(0xffffffffu, b2, s);
+    }
+    if (l8 == 0 && have) {
+        out[i] += b0;
+        out[Np + i] += b1;
+        out[2 * Np + i] += b2;
+    }
+}
+
 int check_fft(vpbs_handle* h, cufftResult r, const char* what) {
     if (r == CUFFT_SUCCESS) return 0;
     return set_error(h, VPBS_ERR_CUDA, std::string("cuFFT error in ") + what + " (code " + std::to_string((int)r) + ")");
@@ -1182,6 +1252,11 @@ int longrange_compute_t(vpbs_handle* h, int fields) {
     const vpbs_params& P = h->P;
     int rc;
     const double sx[3] = {2.0 * kPi / P.L[0], 2.0 * kPi / P.L[1], 2.0 * kPi / P.L[2]};
+    // interleaved components for the interpolation: the inverse transform writes a third more, the gathers of
+    // a node cost a third (1M nodes, m = 3, 288^3: +0.05 ms against -0.5 ms)
+    const double footprints = (double)h->Np * 8.0 * S.m * S.m * S.m;
+    const bool quad = std::is_same<T, float>::value && h->fplan && S.m <= 4 && footprints >= 4.0 * (double)S.ngrid;
+    if (quad && (rc = ensure(h, h->grid_r, sizeof(float4) * (size_t)S.ngrid, "real grid"))) return rc;
     T* grid = (T*)h->grid_r.p;
     C* gc = (C*)h->grid_c.p;
     C* gc2 = (C*)h->grid_c2.p;
@@ -1309,7 +1384,7 @@ int longrange_compute_t(vpbs_handle* h, int fields) {
                 h->have_uhat = keep;
             }
             StageScope st(h, ST_FFT_INVERSE);
-            if ((rc = fourier_inverse(h, grid))) return rc;
+            if ((rc = fourier_inverse(h, grid, quad))) return rc;
         } else {
             StageScope st(h, ST_FFT_INVERSE);
             if ((rc = check_fft(h, exec_c2r(h->plan_c2r, in, grid), "exec c2r"))) return rc;
@@ -1318,6 +1393,21 @@ int longrange_compute_t(vpbs_handle* h, int fields) {
             if ((rc = check_cuda(h, cudaStreamWaitEvent(h->stream, h->interp_wait, 0), "wait short range"))) return rc;
         }
         StageScope st(h, ST_INTERP);
+        if (quad) {
+            auto launch_quad = [&](auto kern) {
+                kern<<<grid_for(h->Np, 32), 256, 0, h->stream>>>(S, h->Np, order, (const double*)h->nodes.p, sx[0], sx[1],
+                                                                 sx[2], (const float4*)grid, out);
+            };
+            switch (S.m) {
+                case 1: launch_quad(interp_quad_kernel<2>); break;
+                case 2: launch_quad(interp_quad_kernel<4>); break;
+                case 3: launch_quad(interp_quad_kernel<6>); break;
+                default: launch_quad(interp_quad_kernel<8>); break;
+            }
+            h->launches++;
+            if ((rc = check_cuda(h, cudaGetLastError(), "interp kernel"))) return rc;
+            continue;
+        }
         auto launch_interp = [&](auto kern) {
             kern<<<grid_for(h->Np, 8), 256, 0, h->stream>>>(S, h->Np, order, (const double*)h->nodes.p, sx[0], sx[1],
                                                             sx[2], grid, out);

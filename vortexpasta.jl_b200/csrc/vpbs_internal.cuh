@@ -280,7 +280,7 @@ int fourier_init(vpbs_handle* h);
 void fourier_free(vpbs_handle* h);
 int fourier_forward(vpbs_handle* h, const void* grid);
 int fourier_operator(vpbs_handle* h, const FourierOp& op);
-int fourier_inverse(vpbs_handle* h, void* grid);
+int fourier_inverse(vpbs_handle* h, void* grid, bool quad = false);  // quad: [z][y][x] of (c0, c1, c2, 0), FP32
 
 // stage timing
 enum Stage {
