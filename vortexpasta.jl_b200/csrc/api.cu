@@ -361,7 +361,7 @@ int vpbs_destroy(vpbs_handle* h) {
     DevBuf* bufs[] = {&h->nodes_in, &h->offsets, &h->fil_of_node, &h->knots, &h->coefs, &h->dcoef1, &h->dcoef2,
                       &h->spline_scratch, &h->nodes, &h->idx_prev, &h->d1, &h->d2, &h->dm, &h->dp, &h->points,
                       &h->charges, &h->li_vel, &h->li_psi, &h->src_cell, &h->src_start, &h->src_fill, &h->src_sorted,
-                      &h->src_seg, &h->dst_cell, &h->dst_start, &h->dst_fill, &h->dst_order, &h->counters,
+                      &h->src_seg, &h->src_f32, &h->dst_cell, &h->dst_start, &h->dst_fill, &h->dst_order, &h->counters,
                       &h->grid_r, &h->grid_c, &h->grid_c2, &h->uhat, &h->decx, &h->decy, &h->decz, &h->nodes_lr,
                       &h->vel, &h->psi, &h->spread_bin, &h->spread_counts, &h->spread_start, &h->binned,
                       &h->spread_foot, &h->tc_counts, &h->tc_start, &h->tc_rec, &h->peer_in, &h->ewald_tab, &h->scan_tmp, &h->scan_tmp_lr, &h->rk_vs, &h->rk_tmp,

@@ -151,16 +151,27 @@ __global__ void __launch_bounds__(kScanThreads) scan_chunks_kernel(const int32_t
 __global__ void scatter_sources_kernel(int64_t Nq, int nquad, const double* __restrict__ points,
                                        const double* __restrict__ charges, const int32_t* __restrict__ cell,
                                        const int32_t* __restrict__ rank, const int32_t* __restrict__ start,
-                                       double* __restrict__ sorted, int32_t* __restrict__ seg) {
+                                       double* __restrict__ sorted, int32_t* __restrict__ seg,
+                                       float4* __restrict__ f32) {
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= Nq) return;
     int64_t pos = (int64_t)start[cell[j]] + rank[j];
+    double x[3], q[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-        sorted[d * Nq + pos] = points[d * Nq + j];
-        sorted[(3 + d) * Nq + pos] = charges[d * Nq + j];
+        x[d] = points[d * Nq + j];
+        q[d] = charges[d * Nq + j];
+        sorted[d * Nq + pos] = x[d];
+        sorted[(3 + d) * Nq + pos] = q[d];
     }
-    seg[pos] = (int32_t)(j / nquad);
+    const int32_t sg = (int32_t)(j / nquad);
+    seg[pos] = sg;
+    if (f32) {  // hi parts and segment | lo parts and charge x | charge y, z
+        const float h0 = (float)x[0], h1 = (float)x[1], h2 = (float)x[2];
+        f32[pos] = make_float4(h0, h1, h2, __int_as_float(sg));
+        f32[Nq + pos] = make_float4((float)(x[0] - h0), (float)(x[1] - h1), (float)(x[2] - h2), (float)q[0]);
+        reinterpret_cast<float2*>(f32 + 2 * Nq)[pos] = make_float2((float)q[1], (float)q[2]);
+    }
 }
 
 __global__ void scatter_nodes_kernel(int64_t Np, const int32_t* __restrict__ cell, const int32_t* __restrict__ rank,
@@ -845,399 +856,329 @@ __global__ void __launch_bounds__(kPairThreads, 2) pair_cell_kernel(
 }
 
 // ---- FP32 pair kernel of the mixed form ----
-// Same decomposition as pair_cell_kernel (CTA per block of cells, the block's neighbour slabs
-// concatenated in (row, slab) order and streamed through shared memory in row-aligned tiles,
-// per-node candidate ranges trimmed to the slabs within r_cut), with every per-pair operation in
-// FP32 and every operand in shared memory:
-//  * staging: source position relative to the block corner split into FP32 hi + lo parts (from
-//    the FP64 position), FP32 charge, segment index; 32-source units spread over all warps;
-//  * per node, only the (2M+1)^2 rows around its own cell are examined (a lane each), and only
-//    the non-empty ones are walked;
-//  * screen: hi parts only, against r_cut^2 (1 + 2e-5) (their rounding is below 1e-6 r_cut^2);
-//  * separation of a queued pair: (x_hi - s_hi) + (x_lo - s_lo) -- the FP64 separation rounded
-//    to FP32 within ~2 ulps (the hi difference is rounded relative to the separation itself);
-//  * decision r^2 <= r_cut^2 in FP32, redone in FP64 from the hi + lo parts when r^2 lies within
-//    4e-6 r_cut^2 of the cut-off, so the pair set equals the FP64 one; local segments (avoid
-//    explicit erf off) are left out here;
-//  * weights from cubic tables on 1/32-wide intervals in x = alpha r (FP32, ~3e-8 absolute),
-//    interval index without a conversion instruction;
-//  * per-lane FP32 sums (a few pairs per lane and node), FP32 warp reduction, FP64 output sums.
-constexpr int kF32Tile = 1280;
-constexpr int kF32TilePad = kF32Tile + 32;  // a chunk of 32 lanes may read past the tile end (masked)
-constexpr int kF32MaxDst = 128;
-constexpr int kF32MaxNb = 576;    // neighbour slabs of a block: rows x slabs per row
-constexpr int kF32MaxRows = 36;   // (y, z) rows of a block's neighbourhood
-constexpr int kF32EvalU = 1;      // screened pairs per lane and evaluation (2: interleaved; measured slower)
-constexpr int kF32Queue = 32 * kF32EvalU + 32;  // screened pairs, evaluated 32 kF32EvalU at a time
+// Every per-pair operation in FP32.  A warp works on its own, without tiles or barriers: it takes D nodes
+// that follow one another in cell order, finds the runs of cell-sorted sources within r_cut of their
+// bounding box (a lane per row of cells) and reads them, as FP32 hi + lo parts that the cell sort wrote,
+// through the L1 cache (neighbouring warps read the same rows).
+//  * Each 32 sources are loaded once and screened against the D nodes in turn, two nodes per packed
+//    instruction, on the hi parts against r_cut^2 (1 + margin).
+//  * The survivors (one in six) go to the warp's queue of that node and are evaluated 32 at a time:
+//    separation (x_hi - s_hi) + (x_lo - s_lo) -- the FP64 separation rounded to FP32 within ~2 ulps;
+//    periodic images shift the node (its hi + lo parts at x - L, x, x + L are tabulated, each from FP64).
+//  * Decision r^2 <= r_cut^2 in FP32, redone in FP64 from the hi + lo parts when r^2 lies within
+//    4e-6 r_cut^2 of the cut-off, so the pair set equals the FP64 one; the node's own two segments are
+//    left out (the mixed form always takes their long-range part out explicitly).
+//  * Weights from cubic tables on 1/32-wide intervals in x = alpha r (FP32, ~3e-8 absolute),
+//    interval index without a conversion instruction.
+//  * Per-lane FP32 sums, FP32 warp reduction (the D x 3 sums halved from lane half to lane half), FP64
+//    output sums.
+// blockIdx.y: the rows are dealt to gridDim.y warps where a system has too few nodes to fill the device.
+// Bound: issue slots (81 % busy, 10 warp instructions per pair in range; 1M nodes, 155 M pairs: 1.76 ms).
+// CTAs that stage tiles of a block's neighbourhood and take a node per warp at a time: 14 instructions per
+// pair, a fifth of the time at barriers, 2.89 ms.  D = 4 at 64 registers (32 warps per SM) against D = 8 at
+// 80: 2.09 ms, at 128: 2.48, D = 2: 2.18; evaluating a chunk as soon as one lane is in range, unqueued: 2.89.
 constexpr int kF32TabMax = 192;   // intervals per weight table (x = alpha r_cut <= 5.9)
 constexpr float kF32Band = 4e-6f; // relative band around r_cut^2 decided in FP64
-constexpr int kF32StageUnroll = 1;
+constexpr float kF32Far = 1e18f;  // coordinate of an absent node or source (its square is finite)
+constexpr int kF32Warps = 4;
+constexpr int kF32Blocks = 8;  // CTAs per SM (64 registers)
+constexpr int kF32IndexBits = 26;  // of a queue entry: the source; 2 bits for its image in x, y and z above them
 
-struct F32Smem {
-    float4 P[kF32TilePad];  // hi parts of the position, segment (int bits)
-    float4 Q[kF32TilePad];  // lo parts of the position, charge x
-    float2 R[kF32TilePad];  // charge y, z
-    float4 tab[2][kF32TabMax];
-    int32_t queue[kPairThreads / 32][kF32Queue];
-    double dx[kF32MaxDst][3];
-    float acc[kF32MaxDst][6];
-    int32_t di[kF32MaxDst], dprev[kF32MaxDst], drow[kF32MaxDst];  // drow: the node's own row, y | z << 8
-    int32_t dr_start[kMaxBlockRows], dr_cnt[kMaxBlockRows], dr_base[kMaxBlockRows + 1];
-    int32_t off[kF32MaxNb + 1];
-    int32_t cstart[kF32MaxNb];
-    int32_t row_gA[kF32MaxRows], row_gB[kF32MaxRows];  // first cell-sorted source of the row's two runs
-    int32_t row_code[kF32MaxRows];  // periodic image of the row: bits 0-1 / 2-3 = -L, 0, +L in y / z
-    double dc[9];  // block constants: corner o0, o1, o2; x images sxA, sxB; cell sizes hx, h1, h2; 1 / hx
+
+__device__ __forceinline__ float rsqrt_fast(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Two FP32 values in one register pair, and the packed operations on them (each half rounded as the
+// scalar operation).
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 dup2(float a) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float half2f(f32x2 a, int u) { return __uint_as_float((unsigned)(u ? a >> 32 : a)); }
+
+struct F32Warp {
+    float2 x[8][3][3];       // node, dimension, image (-L, 0, +L): hi and lo parts of the node's place
+    int2 id[8];              // node and previous node
+    ulonglong2 xy2[4];       // hi parts of two nodes in the images of the current row: x, x | y, y
+    f32x2 z2[4];
+    uint32_t queue[8][64];   // per node: screened sources, cell-sorted index and image (kF32IndexBits)
 };
-static_assert(sizeof(F32Smem) <= 74 * 1024, "three FP32 pair-kernel CTAs must fit in one SM's shared memory");
 
-// U queued pairs per lane (tile indices t[u]; `valid[u]` false for the entries past the queue's end,
-// which evaluate a valid entry and add nothing); the U evaluations are interleaved.
-template <bool VEL, bool PSI, bool SKIP, int U>
-__device__ __forceinline__ void f32_eval(const KParams& K, const F32Smem& S, float3 xh, float3 xl, float rc2,
-                                         float alpha, int nf, int i, int iprev, const int (&t)[U],
-                                         const bool (&valid_in)[U], float acc[6], unsigned& ninr) {
-    float d0[U], d1[U], d2[U], s2[U], q0[U], q1[U], q2[U];
-    bool ok[U], near[U], anynear = false;
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const float4 p = S.P[t[u]];
-        const float4 q = S.Q[t[u]];
-        const float2 qr = S.R[t[u]];
-        d0[u] = (xh.x - p.x) + (xl.x - q.x);
-        d1[u] = (xh.y - p.y) + (xl.y - q.y);
-        d2[u] = (xh.z - p.z) + (xl.z - q.z);
-        q0[u] = q.w;
-        q1[u] = qr.x;
-        q2[u] = qr.y;
-        s2[u] = fmaf(d0[u], d0[u], fmaf(d1[u], d1[u], d2[u] * d2[u]));
-        bool valid = valid_in[u];
-        if (SKIP) {
-            const int sg = __float_as_int(p.w);
-            valid = valid && sg != i && sg != iprev;
+// 32 queued pairs (one a lane; `live` false for lanes past the queue's end) of one node.
+template <bool VEL, bool PSI>
+__device__ __forceinline__ void f32_eval(const F32Warp& S, int d, int e, bool live, const float4* __restrict__ srcP,
+                                         const float4* __restrict__ srcQ, const float2* __restrict__ srcR,
+                                         const float4* __restrict__ tab, float rc2lo, float rc2hi, double rcut2, float alpha,
+                                         int nf, float (&v)[3], float (&w)[3], int& ninr) {
+    const uint32_t entry = S.queue[d][e], j = entry & ((1u << kF32IndexBits) - 1u);
+    const float4 p = __ldg(srcP + j), q = __ldg(srcQ + j);
+    const float2 qr = __ldg(srcR + j);
+    const float2 x0 = S.x[d][0][entry >> kF32IndexBits & 3u], x1 = S.x[d][1][entry >> (kF32IndexBits + 2) & 3u],
+                 x2 = S.x[d][2][entry >> (kF32IndexBits + 4)];
+    const int2 id = S.id[d];
+    const float d0 = (x0.x - p.x) + (x0.y - q.x), d1 = (x1.x - p.y) + (x1.y - q.y), d2 = (x2.x - p.z) + (x2.y - q.z);
+    const float s2 = fmaf(d0, d0, fmaf(d1, d1, d2 * d2));
+    live = live && __float_as_int(p.w) != id.x && __float_as_int(p.w) != id.y;
+    bool ok = live && s2 <= rc2lo;
+    const bool near = live && !ok && s2 <= rc2hi;
+    if (__any_sync(0xffffffffu, near)) {
+        if (near) {  // the FP64 decision on the hi + lo separation (rare)
+            const double f0 = ((double)x0.x + (double)x0.y) - ((double)p.x + (double)q.x);
+            const double f1 = ((double)x1.x + (double)x1.y) - ((double)p.y + (double)q.y);
+            const double f2 = ((double)x2.x + (double)x2.y) - ((double)p.z + (double)q.z);
+            ok = f0 * f0 + f1 * f1 + f2 * f2 <= rcut2;
         }
-        ok[u] = valid && s2[u] <= rc2;
-        near[u] = valid && fabsf(s2[u] - rc2) <= kF32Band * rc2;
-        anynear = anynear || near[u];
     }
-    if (__any_sync(0xffffffffu, anynear)) {
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (near[u]) {  // the FP64 decision on the hi + lo separation (rare)
-                const float4 p = S.P[t[u]];
-                const float4 q = S.Q[t[u]];
-                const double e0 = ((double)xh.x + (double)xl.x) - ((double)p.x + (double)q.x);
-                const double e1 = ((double)xh.y + (double)xl.y) - ((double)p.y + (double)q.y);
-                const double e2 = ((double)xh.z + (double)xl.z) - ((double)p.z + (double)q.z);
-                ok[u] = e0 * e0 + e1 * e1 + e2 * e2 <= K.rcut2;
-            }
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        ninr += __popc(__ballot_sync(0xffffffffu, ok[u]));
-        const float rinv = rsqrtf(s2[u]);
-        int k;
-        float tt;
-        f32_table_pos(s2[u] * rinv * alpha, nf, &k, &tt);
-        if (VEL) {
-            const float wg = f32_cubic(S.tab[1][k], tt);
-            const float f = ok[u] ? wg * (rinv * rinv * rinv) : 0.0f;
-            acc[0] = fmaf(f, fmaf(q1[u], d2[u], -q2[u] * d1[u]), acc[0]);
-            acc[1] = fmaf(f, fmaf(q2[u], d0[u], -q0[u] * d2[u]), acc[1]);
-            acc[2] = fmaf(f, fmaf(q0[u], d1[u], -q1[u] * d0[u]), acc[2]);
+    const float rinv = rsqrt_fast(s2);
+    int k;
+    float tt;
+    f32_table_pos(s2 * rinv * alpha, nf, &k, &tt);
+    if (ok) ++ninr;
+    if (VEL) {
+        const float f = f32_cubic(tab[(PSI ? nf : 0) + k], tt) * (rinv * rinv * rinv);
+        const float c0 = fmaf(qr.x, d2, -qr.y * d1), c1 = fmaf(qr.y, d0, -q.w * d2), c2 = fmaf(q.w, d1, -qr.x * d0);
+        if (ok) {
+            v[0] = fmaf(f, c0, v[0]);
+            v[1] = fmaf(f, c1, v[1]);
+            v[2] = fmaf(f, c2, v[2]);
         }
-        if (PSI) {
-            const float wa = f32_cubic(S.tab[0][k], tt);
-            const float f = ok[u] ? wa * rinv : 0.0f;
-            acc[3] = fmaf(f, q0[u], acc[3]);
-            acc[4] = fmaf(f, q1[u], acc[4]);
-            acc[5] = fmaf(f, q2[u], acc[5]);
+    }
+    if (PSI) {
+        const float f = f32_cubic(tab[k], tt) * rinv;
+        if (ok) {
+            w[0] = fmaf(f, q.w, w[0]);
+            w[1] = fmaf(f, qr.x, w[1]);
+            w[2] = fmaf(f, qr.y, w[2]);
         }
     }
 }
 
-template <bool VEL, bool PSI, bool SKIP>
-__global__ void __launch_bounds__(kPairThreads, 3) pair_f32_kernel(
-    KParams K, CellGrid cg, int64_t Np, int64_t Ns, const int32_t* __restrict__ dst_start,
+// Sums of v[n][3] over the warp's lanes, n = D a power of two: lane halves exchange halves of the n
+// until a lane holds one of them (number lane / (32 / D)); every lane of its 32 / D has the total.
+template <int D>
+__device__ __forceinline__ void f32_reduce(float (&v)[D][3], int lane, float (&out)[3]) {
+#pragma unroll
+    for (int h = D / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < h; ++i)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float keep = up ? v[h + i][c] : v[i][c], give = up ? v[i][c] : v[h + i][c];
+                v[i][c] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        float x = v[0][c];
+#pragma unroll
+        for (int o = 16 / D; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        out[c] = x;
+    }
+}
+
+template <bool VEL, bool PSI, int D>
+__global__ void __launch_bounds__(32 * kF32Warps, kF32Blocks) pair_f32_kernel(
+    KParams K, CellGrid cg, int64_t Np, float rc2s, const int32_t* __restrict__ dst_start,
     const int32_t* __restrict__ dst_order, const double* __restrict__ nodes, const int32_t* __restrict__ idx_prev,
-    const double* __restrict__ src, const int32_t* __restrict__ src_start, const int32_t* __restrict__ seg,
-    double* __restrict__ vel, double* __restrict__ psi, unsigned long long* __restrict__ counters, int3 bk,
-    int3 nb) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    F32Smem& S = *reinterpret_cast<F32Smem*>(smem_raw);
-    const int M = cg.M, G = cg.G;
-    const int nc0 = cg.nc[0], nc1 = cg.nc[1], nc2 = cg.nc[2];
-    const int ncc = nc0 / G;
-    const int bxi = blockIdx.x % nb.x, byi = (blockIdx.x / nb.x) % nb.y, bzi = blockIdx.x / (nb.x * nb.y);
-    const int cx0 = bxi * bk.x, cx1 = min(cx0 + bk.x, ncc);
-    const int cy0 = byi * bk.y, cy1 = min(cy0 + bk.y, nc1);
-    const int cz0 = bzi * bk.z, cz1 = min(cz0 + bk.z, nc2);
-    const int ndr = (cy1 - cy0) * (cz1 - cz0);
+    const float4* __restrict__ srcP, const float4* __restrict__ srcQ, const float2* __restrict__ srcR,
+    const int32_t* __restrict__ src_start, double* __restrict__ vel, double* __restrict__ psi,
+    unsigned long long* __restrict__ counters) {
+    __shared__ F32Warp warps[kF32Warps];
+    __shared__ float4 tab[(VEL && PSI ? 2 : 1) * kF32TabMax];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int WY = cy1 - cy0 + 2 * M, WZ = cz1 - cz0 + 2 * M, WX = (cx1 - cx0 + 2 * M) * G;
-    const int nrow = WY * WZ, ncb = nrow * WX;
-    const int ry0 = cy0 - M, rz0 = cz0 - M, xs0 = cx0 * G - M * G;
-    // ---- prologue: destination rows, weight tables, neighbour slabs (independent loads) ----
-    if (threadIdx.x < ndr) {
-        const int k = threadIdx.x;
-        const int yy = cy0 + k % (cy1 - cy0), zz = cz0 + k / (cy1 - cy0);
-        const int64_t s0 = ((int64_t)zz * nc1 + yy) * nc0 + (int64_t)cx0 * G;
-        const int a = dst_start[s0], b = dst_start[s0 + (int64_t)(cx1 - cx0) * G];
-        S.dr_start[k] = a;
-        S.dr_cnt[k] = b - a;
-    }
     const int nf = K.ntab_c;
-    for (int k = threadIdx.x; k < 2 * nf; k += kPairThreads) S.tab[k / nf][k % nf] = K.tab_c[k];
-    for (int ci = threadIdx.x; ci < ncb; ci += kPairThreads) {
-        const int r = ci / WX, k = ci % WX;
-        int xx = xs0 + k, yy = ry0 + r % WY, zz = rz0 + r / WY;
-        xx = xx < 0 ? xx + nc0 : (xx >= nc0 ? xx - nc0 : xx);
-        yy = yy < 0 ? yy + nc1 : (yy >= nc1 ? yy - nc1 : yy);
-        zz = zz < 0 ? zz + nc2 : (zz >= nc2 ? zz - nc2 : zz);
-        const int64_t c = ((int64_t)zz * nc1 + yy) * nc0 + xx;
-        const int s0 = src_start[c];
-        S.cstart[ci] = s0;
-        S.off[ci + 1] = src_start[c + 1] - s0;
-    }
+    for (int k = threadIdx.x; k < (VEL && PSI ? 2 : 1) * nf; k += 32 * kF32Warps) tab[k] = K.tab_c[(VEL && !PSI ? nf : 0) + k];
     __syncthreads();
-    if (warp == 0) {  // slab counts -> concatenated offsets
-        int carry = 0;
-        for (int base = 0; base < ncb; base += 32) {
-            const int ci = base + lane;
-            int v = ci < ncb ? S.off[ci + 1] : 0;
+    F32Warp& S = warps[warp];
+    const int64_t first = ((int64_t)blockIdx.x * kF32Warps + warp) * D;
+    const int64_t nvalid = dst_start[cg.ncell];  // nodes of the sentinel cell (non-finite) come after these
+    if (first >= nvalid) return;
+    const int nd = nvalid - first < D ? (int)(nvalid - first) : D;
+    const int M = cg.M, nc0 = cg.nc[0], nc1 = cg.nc[1], nc2 = cg.nc[2], W = 2 * M + 1;
+    double x[3] = {0.0, 0.0, 0.0};
+    int i = -1, cy = 0, cz = 0;
+    if (lane < nd) {
+        i = dst_order[first + lane];
+        S.id[lane] = make_int2(i, idx_prev[i]);
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += t;
+        for (int d = 0; d < 3; ++d) {
+            x[d] = nodes[d * Np + i];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) {  // a source image at p + s meets the node at x - s
+                const double y = x[d] - (double)(m - 1) * K.L[d];
+                const float hi = (float)y;
+                S.x[lane][d][m] = make_float2(hi, (float)(y - hi));
             }
-            if (ci < ncb) S.off[ci + 1] = carry + v;
-            carry += __shfl_sync(0xffffffffu, v, 31);
         }
-        if (lane == 0) S.off[0] = 0;
-    } else if (warp == 1) {  // destination rows -> concatenated destination offsets
-        int v = lane < ndr ? S.dr_cnt[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= o) v += t;
-        }
-        if (lane < ndr) S.dr_base[lane + 1] = v;
-        if (lane == 0) S.dr_base[0] = 0;
+        cy = cell_coord(x[1], K.L[1], nc1);
+        cz = cell_coord(x[2], K.L[2], nc2);
     }
-    // the two runs of every row in the cell-sorted arrays: slabs before / after the wrap in x
-    const int kw = xs0 < 0 ? -xs0 : (xs0 + WX > nc0 ? nc0 - xs0 : WX);  // first slab past the wrap
-    for (int r = threadIdx.x; r < nrow; r += kPairThreads) {
-        S.row_gA[r] = S.cstart[r * WX];
-        S.row_gB[r] = kw < WX ? S.cstart[r * WX + kw] : 0;
-        const int yu = ry0 + r % WY, zu = rz0 + r / WY;
-        S.row_code[r] = (yu < 0 ? 0 : (yu >= nc1 ? 2 : 1)) | ((zu < 0 ? 0 : (zu >= nc2 ? 2 : 1)) << 2);
-    }
-    if (threadIdx.x == 0) {
-        const double hx = K.L[0] / nc0, h1 = K.L[1] / nc1, h2 = K.L[2] / nc2;
-        S.dc[0] = cx0 * G * hx;
-        S.dc[1] = cy0 * h1;
-        S.dc[2] = cz0 * h2;
-        S.dc[3] = xs0 < 0 ? -K.L[0] : 0.0;
-        S.dc[4] = xs0 < 0 ? 0.0 : K.L[0];
-        S.dc[5] = hx;
-        S.dc[6] = h1;
-        S.dc[7] = h2;
-        S.dc[8] = nc0 / K.L[0];
-    }
-    __syncthreads();
-    const int nd = S.dr_base[ndr];
-    if (nd == 0) return;  // uniform over the CTA
-    const float rc2s = (float)(K.rcut2 * (1.0 + kScreenMargin));
-    const float rc2 = (float)K.rcut2;
+    const float h1 = (float)(K.L[1] / nc1), h2 = (float)(K.L[2] / nc2);
+    const double inv_hx = nc0 / K.L[0];
+    const float rc = (float)K.rcut, rc2w = rc * rc * 1.0001f;
+    // slack of the row and slab ranges, far above the FP32 rounding of places in the box
+    const float slack = 1e-5f * rc + 1e-6f * (float)fmax(K.L[0], fmax(K.L[1], K.L[2]));
+    const float rc2lo = (float)(K.rcut2 * (1.0 - (double)kF32Band)), rc2hi = (float)(K.rcut2 * (1.0 + (double)kF32Band));
     const float alpha = (float)K.alpha;
-    const int ntot = S.off[ncb];
-    const int W = 2 * M + 1;  // rows around a node's own cell in y and in z
-    const int ldy = lane % W - M, ldz = lane / W - M;  // the row offset lane l examines (l < W^2)
-    const double pref = K.Gamma / (4.0 * kPi);
-    unsigned ninr = 0, ncand = 0;  // warp-uniform (a CTA sees far fewer than 2^32 candidates)
-    for (int p0 = 0; p0 < nd; p0 += kF32MaxDst) {
-        const int np = nd - p0 < kF32MaxDst ? nd - p0 : kF32MaxDst;
-        // row parts per destination: at least 16 items per CTA where the block has few nodes
-        const int P = np >= 16 ? 1 : (16 + np - 1) / np;
-        const int nitems = np * P;
-        for (int T0 = 0, T1 = 0; T0 < ntot; T0 = T1) {
-            const int ra = min(last_row_le(S.off, WX, nrow, T0), nrow - 1);
-            const int rf = last_row_le(S.off, WX, nrow, T0 + kF32Tile);
-            T1 = S.off[rf * WX] > T0 ? S.off[rf * WX] : min(T0 + kF32Tile, ntot);
-            const int rb = min(last_row_le(S.off, WX, nrow, T1 - 1) + 1, nrow);
-            __syncthreads();  // previous tile consumed; previous pass written out
-            if (T0 == 0) {
-                for (int t = threadIdx.x; t < np; t += kPairThreads) {
-                    const int tt = p0 + t;
-                    int k = 0;
-                    while (k + 1 < ndr && S.dr_base[k + 1] <= tt) ++k;
-                    const int i = dst_order[S.dr_start[k] + tt - S.dr_base[k]];
-                    S.di[t] = i;
-                    const int by = cy1 - cy0;
-                    S.drow[t] = ((M + k / by) << 8) | (M + k % by);  // (z, y) row coordinates, 8 bits each
-                    S.dprev[t] = idx_prev[i];
+    const unsigned lanelt = (1u << lane) - 1u;
+    int ninr = 0;
+    unsigned ncand = 0;
+    float v[D][3], w[D][3];
+    int cnt[D];  // queued pairs per node (warp-uniform)
 #pragma unroll
-                    for (int d = 0; d < 3; ++d) S.dx[t][d] = nodes[d * Np + i];
+    for (int d = 0; d < D; ++d) {
+        cnt[d] = 0;
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) S.acc[t][c] = 0.0f;
-                }
-            }
-            // staging in units of 32 consecutive sources, kF32StageUnroll units per warp at a time
-            // (their loads in flight together)
-            const int nunits = (T1 - T0 + 31) >> 5;
-            for (int u0 = warp; u0 < nunits; u0 += (kPairThreads / 32) * kF32StageUnroll) {
-                int jj[kF32StageUnroll], tt[kF32StageUnroll], code[kF32StageUnroll];
+        for (int c = 0; c < 3; ++c) v[d][c] = w[d][c] = 0.0f;
+    }
+    int turn = 0;  // rows seen so far: dealt to the gridDim.y warps of the group in turn
+    // the nodes of one (y, z) row of cells within r_cut in x at a time (nearly always all of them)
+    for (unsigned todo = __ballot_sync(0xffffffffu, lane < nd); todo;) {
+        const int lead = __ffs(todo) - 1;
+        const int gy_ = __shfl_sync(0xffffffffu, cy, lead), gz_ = __shfl_sync(0xffffffffu, cz, lead);
+        const double xlead = __shfl_sync(0xffffffffu, x[0], lead);
+        const bool mine = (todo >> lane & 1) && cy == gy_ && cz == gz_ && fabs(x[0] - xlead) <= K.rcut;
+        todo &= ~__ballot_sync(0xffffffffu, mine);
+        float lo[3], hi[3];
 #pragma unroll
-                for (int q = 0; q < kF32StageUnroll; ++q) {
-                    const int u = u0 + q * (kPairThreads / 32);
-                    const int t = T0 + (u << 5) + lane;
-                    tt[q] = -1;
-                    jj[q] = 0;
-                    code[q] = 0;
-                    if (u < nunits && t < T1) {
-                        int r = last_row_le(S.off, WX, nrow, T0 + (u << 5));
-                        while (r + 1 < nrow && S.off[(r + 1) * WX] <= t) ++r;
-                        const int rowA = S.off[r * WX], offB = S.off[r * WX + kw];
-                        const bool inA = t < offB;
-                        jj[q] = inA ? S.row_gA[r] + (t - rowA) : S.row_gB[r] + (t - offB);
-                        tt[q] = t - T0;
-                        // periodic image codes: bit 0 segment B in x; bits 1-2 / 3-4: -L, 0, +L in y / z
-                        code[q] = (inA ? 0 : 1) | (S.row_code[r] << 1);
-                    }
-                }
-                double v[kF32StageUnroll][6];
-                int sgv[kF32StageUnroll];
-#pragma unroll
-                for (int q = 0; q < kF32StageUnroll; ++q) {
-                    const int j = jj[q];
-                    if (tt[q] >= 0) {
-#pragma unroll
-                        for (int c = 0; c < 6; ++c) v[q][c] = src[c * Ns + j];
-                        sgv[q] = SKIP ? seg[j] : 0;
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < kF32StageUnroll; ++q) {
-                    if (tt[q] >= 0) {
-                        const int cd = code[q];
-                        const double u0d = v[q][0] + S.dc[3 + (cd & 1)] - S.dc[0];
-                        const double u1d = v[q][1] + (double)(((cd >> 1) & 3) - 1) * K.L[1] - S.dc[1];
-                        const double u2d = v[q][2] + (double)(((cd >> 3) & 3) - 1) * K.L[2] - S.dc[2];
-                        const float f0 = (float)u0d, f1 = (float)u1d, f2 = (float)u2d;
-                        S.P[tt[q]] = make_float4(f0, f1, f2, __int_as_float(sgv[q]));
-                        S.Q[tt[q]] = make_float4((float)(u0d - f0), (float)(u1d - f1), (float)(u2d - f2), (float)v[q][3]);
-                        S.R[tt[q]] = make_float2((float)v[q][4], (float)v[q][5]);
-                    }
-                }
-            }
-            __syncthreads();
-            for (int it = warp; it < nitems; it += kPairThreads / 32) {
-                const int dl = it % np, part = it / np;
-                const double x[3] = {S.dx[dl][0], S.dx[dl][1], S.dx[dl][2]};
-                // lane l examines the row (dy, dz) = (l % W - M, l / W - M) around the node's own cell
-                int a = 0, b = 0;
-                if (lane < W * W) {
-                    const int own = S.drow[dl];
-                    const int yr = (own & 255) + ldy, zr = (own >> 8) + ldz;
-                    if (yr >= 0 && yr < WY && zr >= 0 && zr < WZ) {
-                        const int r = zr * WY + yr;
-                        if (r >= ra && r < rb) {
-                            const double h1 = S.dc[6], h2 = S.dc[7], hx = S.dc[5], inv_hx = S.dc[8];
-                            const double gy = box_gap(x[1], (ry0 + yr) * h1, h1);
-                            const double gz = box_gap(x[2], (rz0 + zr) * h2, h2);
-                            const double gyz = gy * gy + gz * gz;
-                            if (gyz <= K.rcut2) {
-                                const double w = (double)sqrtf((float)(K.rcut2 - gyz)) * (1.0 + 1e-6) + 1e-9 * hx;
-                                int klo = (int)floor((x[0] - w) * inv_hx) - xs0;
-                                int khi = (int)floor((x[0] + w) * inv_hx) - xs0;
-                                klo = klo < 0 ? 0 : klo;
-                                khi = khi > WX - 1 ? WX - 1 : khi;
-                                if (klo <= khi) {
-                                    a = max(S.off[r * WX + klo], T0) - T0;
-                                    b = min(S.off[r * WX + khi + 1], T1) - T0;
-                                }
-                            }
-                        }
-                    }
-                }
-                unsigned rows = __ballot_sync(0xffffffffu, a < b);
-                float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                int qcount = 0;
-                int32_t* Qu = S.queue[warp];
-                const double xd0 = x[0] - S.dc[0], xd1 = x[1] - S.dc[1], xd2 = x[2] - S.dc[2];
-                const float3 xh = make_float3((float)xd0, (float)xd1, (float)xd2);
-                const float3 xl = make_float3((float)(xd0 - xh.x), (float)(xd1 - xh.y), (float)(xd2 - xh.z));
-                const int i = S.di[dl], iprev = S.dprev[dl];
-                for (int nrw = 0, next = part; rows; ++nrw, rows &= rows - 1) {
-                    if (nrw != next) continue;  // warp-uniform: rows are dealt to the parts in turn
-                    next += P;
-                    const int src_lane = __ffs(rows) - 1;
-                    const int ra_ = __shfl_sync(0xffffffffu, a, src_lane);
-                    const int rb_ = __shfl_sync(0xffffffffu, b, src_lane);
-                    ncand += rb_ - ra_;
-                    for (int base = ra_; base < rb_; base += 32) {
-                        const int t = base + lane;
-                        const float4 p = S.P[t];
-                        const float e0 = xh.x - p.x, e1 = xh.y - p.y, e2 = xh.z - p.z;
-                        const bool inr = t < rb_ && fmaf(e0, e0, fmaf(e1, e1, e2 * e2)) <= rc2s;
-                        const unsigned m = __ballot_sync(0xffffffffu, inr);
-                        if (inr) Qu[qcount + __popc(m & ((1u << lane) - 1u))] = t;
-                        qcount += __popc(m);
-                        __syncwarp();
-                        if (qcount >= 32 * kF32EvalU) {
-                            int tq[kF32EvalU];
-                            bool vq[kF32EvalU];
-#pragma unroll
-                            for (int u = 0; u < kF32EvalU; ++u) {
-                                tq[u] = Qu[32 * u + lane];
-                                vq[u] = true;
-                            }
-                            f32_eval<VEL, PSI, SKIP, kF32EvalU>(K, S, xh, xl, rc2, alpha, nf, i, iprev, tq, vq, acc, ninr);
-                            __syncwarp();
-                            if (lane < qcount - 32 * kF32EvalU) Qu[lane] = Qu[32 * kF32EvalU + lane];
-                            __syncwarp();
-                            qcount -= 32 * kF32EvalU;
-                        }
-                    }
-                }
-                for (int q0 = 0; q0 < qcount; q0 += 32) {  // warp-uniform remainder, one pair per lane
-                    const int tq[1] = {q0 + lane < qcount ? Qu[q0 + lane] : Qu[0]};
-                    const bool vq[1] = {q0 + lane < qcount};
-                    f32_eval<VEL, PSI, SKIP, 1>(K, S, xh, xl, rc2, alpha, nf, i, iprev, tq, vq, acc, ninr);
-                }
-                __syncwarp();  // the queue is reused by the warp's next item
-#pragma unroll
-                for (int c = 0; c < 6; ++c) {
-                    if ((c < 3 && !VEL) || (c >= 3 && !PSI)) continue;
-                    float v = acc[c];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                    acc[c] = v;
-                }
-                if (lane == 0) {
-#pragma unroll
-                    for (int c = 0; c < 6; ++c)
-                        if ((c < 3 && VEL) || (c >= 3 && PSI)) atomicAdd(&S.acc[dl][c], acc[c]);
-                }
-            }
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = mine ? (float)x[d] : kF32Far;
+            hi[d] = mine ? (float)x[d] : -kF32Far;
         }
-        __syncthreads();
-        for (int t = threadIdx.x; t < np; t += kPairThreads) {
-            const int64_t i = S.di[t];
-            if (VEL) {
-                vel[i] += pref * (double)S.acc[t][0];
-                vel[Np + i] += pref * (double)S.acc[t][1];
-                vel[2 * Np + i] += pref * (double)S.acc[t][2];
+#pragma unroll
+        for (int o = 1; o < D; o <<= 1)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+                hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
             }
-            if (PSI) {
-                psi[i] += pref * (double)S.acc[t][3];
-                psi[Np + i] += pref * (double)S.acc[t][4];
-                psi[2 * Np + i] += pref * (double)S.acc[t][5];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = __shfl_sync(0xffffffffu, lo[d], 0) - slack;
+            hi[d] = __shfl_sync(0xffffffffu, hi[d], 0) + slack;
+        }
+        // lane l takes the row (dy, dz) = (l % W - M, l / W - M) around the nodes' own row
+        int klo = 0, khi = -1, row = 0, iyz = 0;
+        if (lane < W * W) {
+            const int yu = gy_ + lane % W - M, zu = gz_ + lane / W - M;
+            const float ylo = (float)yu * h1, zlo = (float)zu * h2;
+            const float gy = fmaxf(fmaxf(ylo - hi[1], lo[1] - (ylo + h1)), 0.0f);
+            const float gz = fmaxf(fmaxf(zlo - hi[2], lo[2] - (zlo + h2)), 0.0f);
+            const float rest = rc2w - gy * gy - gz * gz;
+            if (rest >= 0.0f) {
+                const float r = sqrtf(rest) + slack;
+                klo = (int)floor((double)(lo[0] - r) * inv_hx);
+                khi = (int)floor((double)(hi[0] + r) * inv_hx);
+            }
+            const int my = yu < 0 ? 0 : (yu >= nc1 ? 2 : 1), mz = zu < 0 ? 0 : (zu >= nc2 ? 2 : 1);
+            row = ((zu + (1 - mz) * nc2) * nc1 + yu + (1 - my) * nc1) * nc0;
+            iyz = my + 3 * mz;
+        }
+        for (int mx = 0; mx < 3; ++mx) {  // images in x: -L, 0, +L
+            const int s0 = max(klo - (mx - 1) * nc0, 0), s1 = min(khi - (mx - 1) * nc0, nc0 - 1);
+            int a = 0, b = 0;
+            if (s0 <= s1) {
+                a = src_start[row + s0];
+                b = src_start[row + s1 + 1];
+            }
+            for (unsigned rows = __ballot_sync(0xffffffffu, a < b); rows; rows &= rows - 1) {
+                const bool skip = turn % (int)gridDim.y != (int)blockIdx.y;  // warp-uniform
+                ++turn;
+                if (skip) continue;
+                const int sl = __ffs(rows) - 1;
+                const int ra = __shfl_sync(0xffffffffu, a, sl), rb = __shfl_sync(0xffffffffu, b, sl);
+                const int im = __shfl_sync(0xffffffffu, iyz, sl), my = im % 3, mz = im / 3;
+                __syncwarp();
+                if (lane < D) {
+                    const float px = mine ? S.x[lane][0][mx].x : kF32Far;
+                    float* xy = reinterpret_cast<float*>(S.xy2) + 4 * (lane >> 1) + (lane & 1);
+                    xy[0] = px;
+                    xy[2] = mine ? S.x[lane][1][my].x : kF32Far;
+                    reinterpret_cast<float*>(S.z2)[lane] = mine ? S.x[lane][2][mz].x : kF32Far;
+                }
+                __syncwarp();
+                ncand += (unsigned)(rb - ra) * D;
+                const uint32_t code = (uint32_t)(mx | my << 2 | mz << 4) << kF32IndexBits;
+                float4 pn = __ldg(srcP + min(ra + lane, rb - 1));
+                for (int base = ra; base < rb; base += 32) {
+                    const int t = base + lane;
+                    float4 p = pn;
+                    pn = __ldg(srcP + min(t + 32, rb - 1));
+                    if (t >= rb) p.x = -kF32Far;
+                    const f32x2 px = dup2(-p.x), py = dup2(-p.y), pz = dup2(-p.z);
+                    const uint32_t entry = (uint32_t)t | code;
+#pragma unroll
+                    for (int h = 0; h < D / 2; ++h) {
+                        const ulonglong2 xy = S.xy2[h];
+                        const f32x2 e0 = add2(xy.x, px), e1 = add2(xy.y, py), e2 = add2(S.z2[h], pz);
+                        const f32x2 r2 = fma2(e0, e0, fma2(e1, e1, mul2(e2, e2)));
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int d = 2 * h + u;
+                            const bool in = half2f(r2, u) <= rc2s;
+                            const unsigned m = __ballot_sync(0xffffffffu, in);
+                            if (m == 0) continue;  // warp-uniform
+                            if (in) S.queue[d][cnt[d] + __popc(m & lanelt)] = entry;
+                            cnt[d] += __popc(m);
+                            if (cnt[d] >= 32) {
+                                __syncwarp();
+                                f32_eval<VEL, PSI>(S, d, lane, true, srcP, srcQ, srcR, tab, rc2lo, rc2hi, K.rcut2, alpha, nf, v[d],
+                                                   w[d], ninr);
+                                cnt[d] -= 32;
+                                __syncwarp();
+                                if (lane < cnt[d]) S.queue[d][lane] = S.queue[d][32 + lane];
+                                __syncwarp();
+                            }
+                        }
+                    }
+                }
             }
         }
     }
+    __syncwarp();
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        if (cnt[d] > 0)  // warp-uniform
+            f32_eval<VEL, PSI>(S, d, lane < cnt[d] ? lane : 0, lane < cnt[d], srcP, srcQ, srcR, tab, rc2lo, rc2hi, K.rcut2, alpha, nf,
+                               v[d], w[d], ninr);
+    const double pref = K.Gamma / (4.0 * kPi);
+    const int slot = lane / (32 / D);
+    const int is = __shfl_sync(0xffffffffu, i, slot);
+    float out[3];
+    if (VEL) {
+        f32_reduce<D>(v, lane, out);
+        if (lane % (32 / D) == 0 && is >= 0)
+            for (int c = 0; c < 3; ++c) atomicAdd(&vel[c * Np + is], pref * (double)out[c]);
+    }
+    if (PSI) {
+        f32_reduce<D>(w, lane, out);
+        if (lane % (32 / D) == 0 && is >= 0)
+            for (int c = 0; c < 3; ++c) atomicAdd(&psi[c * Np + is], pref * (double)out[c]);
+    }
+    const unsigned long long total = warp_sum_u((unsigned long long)ninr);
     if (lane == 0) {
-        atomicAdd(&counters[0], (unsigned long long)ninr);
+        atomicAdd(&counters[0], total);
         atomicAdd(&counters[1], (unsigned long long)ncand);
     }
 }
@@ -1337,6 +1278,8 @@ __global__ void __launch_bounds__(128) local_self_kernel(
 
 }  // namespace
 
+static bool use_f32_pairs(const vpbs_handle* h);
+
 int build_cell_lists(vpbs_handle* h) {
     if (h->K.open_domain) return 0;
     // Cell size (internal: the pair set does not depend on it).  Where cells r_cut/2 wide would
@@ -1366,6 +1309,8 @@ int build_cell_lists(vpbs_handle* h) {
     if ((rc = ensure(h, h->dst_start, sizeof(int32_t) * (ncell + 2), "dst_start"))) return rc;
     if ((rc = ensure(h, h->dst_fill, sizeof(int32_t) * (ncell + 1), "dst_counts"))) return rc;
     if ((rc = ensure(h, h->dst_order, sizeof(int32_t) * Np, "dst_order"))) return rc;
+    const bool f32 = use_f32_pairs(h);
+    if (f32 && (rc = ensure(h, h->src_f32, (2 * sizeof(float4) + sizeof(float2)) * Nq, "FP32 sources"))) return rc;
     int32_t* scell = (int32_t*)h->src_cell.p;
     int32_t* srank = scell + Nq;
     int32_t* dcell = (int32_t*)h->dst_cell.p;
@@ -1385,7 +1330,8 @@ int build_cell_lists(vpbs_handle* h) {
         return rc;
     scatter_sources_kernel<<<grid_for(Nq, 256), 256, 0, h->stream>>>(
         Nq, h->K.nquad, (const double*)h->points.p, (const double*)h->charges.p, scell, srank,
-        (const int32_t*)h->src_start.p, (double*)h->src_sorted.p, (int32_t*)h->src_seg.p);
+        (const int32_t*)h->src_start.p, (double*)h->src_sorted.p, (int32_t*)h->src_seg.p,
+        f32 ? (float4*)h->src_f32.p : nullptr);
     scatter_nodes_kernel<<<grid_for(Np, 256), 256, 0, h->stream>>>(Np, dcell, drank, (const int32_t*)h->dst_start.p,
                                                                    (int32_t*)h->dst_order.p);
     h->launches += 4;  // plus the scans, counted by exclusive_scan
@@ -1544,6 +1490,15 @@ int exclusive_scan(vpbs_handle* h, const int32_t* counts, int32_t* start, int64_
     return check_cuda(h, cudaGetLastError(), "scan kernels");
 }
 
+// The FP32 pair kernel serves the mixed form with cell lists of M <= 2 (a lane per row) and weight tables
+// that fit; it reads FP32 copies of the sources that the cell sort writes.
+static bool use_f32_pairs(const vpbs_handle* h) {
+    const int W = 2 * h->cg.M + 1;
+    return h->P.precision == VPBS_PRECISION_MIXED && !h->K.open_domain && !h->K.avoid_explicit_erf && h->K.alpha > 0 &&
+           h->cg.M > 0 && W * W <= 32 && h->K.ewald_ntab > 0 && h->K.ntab_c > 0 && h->K.ntab_c <= kF32TabMax &&
+           h->Nq < (int64_t)1 << kF32IndexBits;
+}
+
 int pair_interactions(vpbs_handle* h, int fields) {
     const int64_t Np = h->Np, Nq = h->Nq;
     const bool open = h->K.open_domain;
@@ -1577,6 +1532,30 @@ int pair_interactions(vpbs_handle* h, int fields) {
     }
     const CellGrid& cg = h->cg;
     const int Wc = 2 * cg.M + 1;
+    if (use_f32_pairs(h)) {
+        int nsm = 148;
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
+        const int D = v && p ? 2 : 4;
+        const unsigned nblk = grid_for(Np, D * kF32Warps);
+        // a group's rows are shared out where the groups are fewer than the 32 warps an SM holds (1400 nodes:
+        // 25 us with 9 parts)
+        const unsigned nparts = (unsigned)std::max(1, std::min(Wc * Wc, (int)((32 * nsm + nblk - 1) / nblk / kF32Warps)));
+        // screen margin: the hi parts of places in the box are rounded to 2^-25 of its size
+        const double Lmax = std::fmax(h->K.L[0], std::fmax(h->K.L[1], h->K.L[2]));
+        const float rc2s = (float)(h->K.rcut2 * (1.0 + kScreenMargin + 1e-6 * Lmax / h->K.rcut));
+        auto launch_f32 = [&](auto kern) {
+            kern<<<dim3(nblk, nparts), 32 * kF32Warps, 0, h->stream>>>(
+                h->K, h->cg, Np, rc2s, (const int32_t*)h->dst_start.p, (const int32_t*)h->dst_order.p,
+                (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p, (const float4*)h->src_f32.p,
+                (const float4*)h->src_f32.p + Nq, (const float2*)((const float4*)h->src_f32.p + 2 * Nq),
+                (const int32_t*)h->src_start.p, (double*)h->vel.p, (double*)h->psi.p, (unsigned long long*)h->counters.p);
+        };
+        if (v && p) launch_f32(pair_f32_kernel<true, true, 2>);
+        else if (v) launch_f32(pair_f32_kernel<true, false, 4>);
+        else launch_f32(pair_f32_kernel<false, true, 4>);
+        h->launches++;
+        return check_cuda(h, cudaGetLastError(), "FP32 pair kernel");
+    }
     if ( cg.M > 0 && Wc * Wc <= kMaxRows && Wc * Wc * Wc * cg.G <= kMaxNbCells &&
         sizeof(TileSmem<1024>) + 2 * sizeof(double) * kTabSNC * h->K.ntab_s <= kPairSmemMost) {
         // blocks of Bc^3 cells per CTA, grown while a block holds fewer than ~24 nodes on average,
@@ -1592,50 +1571,6 @@ int pair_interactions(vpbs_handle* h, int fields) {
             return w <= ncc && w <= cg.nc[1] && w <= cg.nc[2] && w * w <= kMaxRows && w * w * w * cg.G <= kMaxNbCells &&
                    nb * nb <= kMaxBlockRows;
         };
-        const bool mixed = h->P.precision == VPBS_PRECISION_MIXED;
-        const int nrow_max = kF32MaxRows, ncb_max = kF32MaxNb;
-        auto fits_f32 = [&](int b) {
-            const int w = b + 2 * cg.M;
-            return fits(b) && w * w <= nrow_max && w * w * w * cg.G <= ncb_max;
-        };
-        if (mixed && h->K.ewald_ntab > 0 && h->K.ntab_c > 0 && h->K.ntab_c <= kF32TabMax && fits_f32(1)) {
-            // FP32 kernel: blocks grown while they hold at most ~96 nodes on average (one pass of
-            // destinations) and at least 2 CTAs per SM remain; a neighbourhood of two tiles costs less
-            // than a block of few nodes (1M-node tangle at r_cut = L/45: 2 x 2 x 2 cells per CTA, two
-            // tiles, 2.8 ms; one cell, one tile, 4.2 ms)
-            int Bc = 1;
-            if (h->pair_block > 0 && fits_f32(h->pair_block)) {
-                Bc = h->pair_block;  // chosen by vpbs_autotune
-            } else {
-                while (fits_f32(Bc + 1) && (Bc + 1) * (Bc + 1) * (Bc + 1) * per_cell <= 96.0 &&
-                       ncoarse / ((double)(Bc + 1) * (Bc + 1) * (Bc + 1)) >= 2.0 * nsm)
-                    ++Bc;
-            }
-            const int3 bk = make_int3(Bc, Bc, Bc);
-            const int3 nb = make_int3((ncc + Bc - 1) / Bc, (cg.nc[1] + Bc - 1) / Bc, (cg.nc[2] + Bc - 1) / Bc);
-            const size_t smem = sizeof(F32Smem);
-            const unsigned nblocks = (unsigned)((int64_t)nb.x * nb.y * nb.z);
-            auto launch_f32 = [&](auto kern) {
-                cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-                kern<<<nblocks, kPairThreads, smem, h->stream>>>(
-                    h->K, h->cg, Np, Nq, (const int32_t*)h->dst_start.p, (const int32_t*)h->dst_order.p,
-                    (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p, (const double*)h->src_sorted.p,
-                    (const int32_t*)h->src_start.p, (const int32_t*)h->src_seg.p, (double*)h->vel.p, (double*)h->psi.p,
-                    (unsigned long long*)h->counters.p, bk, nb);
-            };
-            if (skip_local) {
-                if (v && p) launch_f32(pair_f32_kernel<true, true, true>);
-                else if (v) launch_f32(pair_f32_kernel<true, false, true>);
-                else launch_f32(pair_f32_kernel<false, true, true>);
-            } else {
-                if (v && p) launch_f32(pair_f32_kernel<true, true, false>);
-                else if (v) launch_f32(pair_f32_kernel<true, false, false>);
-                else launch_f32(pair_f32_kernel<false, true, false>);
-            }
-            h->launches++;
-            return check_cuda(h, cudaGetLastError(), "FP32 pair kernel");
-        }
         int Bc = 1;
         if (h->pair_block > 0 && fits(h->pair_block)) {
             Bc = h->pair_block;  // chosen by vpbs_autotune

@@ -185,7 +185,7 @@ struct vpbs_handle {
 
     // cell lists
     vpbs::CellGrid cg{};
-    vpbs::DevBuf src_cell, src_start, src_fill, src_sorted, src_seg, dst_cell, dst_start, dst_fill, dst_order;
+    vpbs::DevBuf src_cell, src_start, src_fill, src_sorted, src_seg, src_f32, dst_cell, dst_start, dst_fill, dst_order;
     vpbs::DevBuf counters;  // [0] in-range pairs, [1] candidates (unsigned long long)
     vpbs::DevBuf scan_tmp, scan_tmp_lr;  // multi-CTA scan scratch (cell lists; spreading bins)
     vpbs::DevBuf ewald_tab;  // Taylor tables of the Ewald weights (KParams::ewald_tab)
