@@ -54,7 +54,7 @@ void plan_search(int n, bool wide, std::vector<int>& cur, std::vector<int>& best
     }
     if ((int)cur.size() >= fft::kMaxPasses) return;
     for (int R : radices)
-        if (n % R == 0 && R <= fft::pass_values(wide)) {
+        if (n % R == 0 && R <= fft::pass_values(wide) && (cur.empty() || R <= cur.back())) {  // largest first
             cur.push_back(R);
             plan_search(n / R, wide, cur, best, cost, n_all);
             cur.pop_back();

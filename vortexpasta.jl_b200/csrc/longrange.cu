@@ -1180,7 +1180,9 @@ int longrange_init(vpbs_handle* h) {
     int rc;
     const bool mixed = P.precision == VPBS_PRECISION_MIXED;
     const size_t rsz = mixed ? sizeof(float) : sizeof(double);  // grid precision
-    if ((rc = ensure(h, h->grid_r, rsz * 3 * S.ngrid, "real grid"))) return rc;
+    // room for the interleaved layout (longrange_compute_t) where a later evaluation may take it
+    const size_t per_point = mixed && S.m <= 4 ? sizeof(float4) : 3 * rsz;
+    if ((rc = ensure(h, h->grid_r, per_point * S.ngrid, "real grid"))) return rc;
     if ((rc = ensure(h, h->uhat, sizeof(double2) * 3 * S.nmodes, "uhat"))) return rc;
     // separable deconvolution factors 1/psi_hat and 1/psi_hat * exp(-k^2 / 4 alpha^2) (the
     // Kaiser-Bessel filter is not separable: the Fourier kernel applies it per mode)
@@ -1256,7 +1258,6 @@ int longrange_compute_t(vpbs_handle* h, int fields) {
     // a node cost a third (1M nodes, m = 3, 288^3: +0.05 ms against -0.5 ms)
     const double footprints = (double)h->Np * 8.0 * S.m * S.m * S.m;
     const bool quad = std::is_same<T, float>::value && h->fplan && S.m <= 4 && footprints >= 4.0 * (double)S.ngrid;
-    if (quad && (rc = ensure(h, h->grid_r, sizeof(float4) * (size_t)S.ngrid, "real grid"))) return rc;
     T* grid = (T*)h->grid_r.p;
     C* gc = (C*)h->grid_c.p;
     C* gc2 = (C*)h->grid_c2.p;
