@@ -358,10 +358,8 @@ void* vpbs_ensemble_stream(vpbs_ensemble* e);
 int vpbs_ensemble_destroy(vpbs_ensemble* e);
 const char* vpbs_ensemble_last_error(void);
 
-/* Autotuner: times the pair kernel on the handle's current point data for each candidate
- * number of cells per CTA edge (1-4, and the built-in rule) and keeps the fastest for later
- * evaluations (`chosen`: 0 = the rule, else the edge).  Overwrites the handle's output fields.
- * Synchronous. */
+/* Autotuner of the pair kernel's blocks.  The pair kernels work per group of nodes and have no block size
+ * left to choose: `chosen` is 0, the built-in rule. */
 int vpbs_autotune(vpbs_handle* h, int32_t* chosen);
 
 /* Autotuner of the long range: times one long-range evaluation (spreading, FFTs, Fourier operators,
@@ -375,9 +373,8 @@ int vpbs_autotune_spread(vpbs_handle* h, int32_t* chosen);
  * cores only (plane-owner kernel).  Tuning and testing support; no counterpart in the reference. */
 int vpbs_spread_mode(vpbs_handle* h, int32_t mode);
 
-/* Sets the pair kernel's cells per CTA edge for later evaluations (0: the built-in rule; an edge
- * whose neighbourhood does not fit the kernel's tables falls back to the rule), as vpbs_autotune
- * does with its choice.  Tuning support; no counterpart in the reference. */
+/* A block edge for the pair kernel (0: the built-in rule).  Accepted and without effect, as in
+ * vpbs_autotune.  Tuning support; no counterpart in the reference. */
 int vpbs_pair_block(vpbs_handle* h, int32_t cells);
 
 /* ---- Learned parameter predictor (no counterpart in the reference, which removed its alpha

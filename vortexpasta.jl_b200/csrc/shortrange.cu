@@ -4,10 +4,10 @@
 //  * cell lists as a counting sort of the quadrature points (and of the nodes) by cell
 //    (replaces the linked lists of src/CellLists/gpu.jl:28-61 and the destination sort of
 //    gpu.jl:183-231);
-//  * the pair kernel (src/BiotSavart/shortrange/shortrange.jl:216-273 with the Gaussian
-//    weights of splitting/gaussian.jl:273-279): one warp per destination node, lanes
-//    stride over the contiguous cell-sorted source ranges of the (2M+1)^2 neighbour rows,
-//    warp-shuffle reduction at the end.
+//  * the pair kernels (src/BiotSavart/shortrange/shortrange.jl:216-273 with the Gaussian
+//    weights of splitting/gaussian.jl:273-279): a warp per few nodes that follow one another in
+//    cell order, lanes over the contiguous cell-sorted source ranges of the (2M+1)^2
+//    neighbour rows, warp-shuffle reduction at the end.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -152,7 +152,7 @@ __global__ void scatter_sources_kernel(int64_t Nq, int nquad, const double* __re
                                        const double* __restrict__ charges, const int32_t* __restrict__ cell,
                                        const int32_t* __restrict__ rank, const int32_t* __restrict__ start,
                                        double* __restrict__ sorted, int32_t* __restrict__ seg,
-                                       float4* __restrict__ f32) {
+                                       float4* __restrict__ f32, int f32_parts) {
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= Nq) return;
     int64_t pos = (int64_t)start[cell[j]] + rank[j];
@@ -166,9 +166,11 @@ __global__ void scatter_sources_kernel(int64_t Nq, int nquad, const double* __re
     }
     const int32_t sg = (int32_t)(j / nquad);
     seg[pos] = sg;
-    if (f32) {  // hi parts and segment | lo parts and charge x | charge y, z
-        const float h0 = (float)x[0], h1 = (float)x[1], h2 = (float)x[2];
-        f32[pos] = make_float4(h0, h1, h2, __int_as_float(sg));
+    if (f32_parts == 0) return;
+    // hi parts and segment | lo parts and charge x | charge y, z
+    const float h0 = (float)x[0], h1 = (float)x[1], h2 = (float)x[2];
+    f32[pos] = make_float4(h0, h1, h2, __int_as_float(sg));
+    if (f32_parts == 2) {
         f32[Nq + pos] = make_float4((float)(x[0] - h0), (float)(x[1] - h1), (float)(x[2] - h2), (float)q[0]);
         reinterpret_cast<float2*>(f32 + 2 * Nq)[pos] = make_float2((float)q[1], (float)q[2]);
     }
@@ -459,46 +461,9 @@ __global__ void __launch_bounds__(256) pair_kernel(
     }
 }
 
-// ---- cell-tiled pair kernel ----
-// One CTA per destination cell.  The sources of the (2M+1)^3 neighbour cells (in x: the G
-// slabs of each) are concatenated in (row (dy, dz), slab) order and streamed through shared
-// memory in tiles of kTile sources, as coordinates relative to the cell corner (already
-// shifted to the periodic image next to the cell) split into FP32 hi + lo parts.  Per
-// destination and row the candidate range is trimmed to the slabs within r_cut of the node.
-// Candidates are screened on the hi parts in FP32 against r_cut^2 (1 + 2e-5) -- the FP32
-// rounding of r^2 stays below 1e-6 r_cut^2 here, so no pair in range is lost -- and queued; the
-// queued pairs are decided (r^2 <= r_cut^2) and evaluated with the separation formed in FP64
-// from the hi + lo parts (relative error ~1e-15), two pairs per lane at a time so that their
-// dependency chains overlap.  Destinations are handled in passes of up to kPassDst nodes;
-// warps take (destination, row-part) items and add each item's warp-reduced sum to the
-// destination's shared-memory accumulator.
-constexpr int kPassDst = 64;
-constexpr int kMaxNbCells = 1024;  // neighbour slabs of a block: rows x slabs per row
-constexpr int kMaxBlockRows = 16;  // (y, z) cell rows of a block (destination ranges)
-constexpr int kMaxRows = 81;      // (2M+1)^2
-constexpr int kTileQueue = 128;   // screened pairs are evaluated 64 at a time (two per lane)
-constexpr double kScreenMargin = 2e-5;
-
-// TILE sources: one field 1024, both fields 640 (two weight tables), so that two CTAs share an SM.
-template <int TILE>
-struct TileSmem {
-    static constexpr int kPad = TILE + 32;  // a chunk of 32 lanes may read past the tile end (masked)
-    float4 hi[kPad];    // FP32 position relative to the block corner, segment (int bits): the screen
-    double2 pxy[kPad];  // the FP64 position and the charge: the evaluation
-    double2 pzq[kPad];
-    double2 qyz[kPad];
-    int32_t queue[kPairThreads / 32][kTileQueue];  // per warp: tile indices of screened pairs
-    double acc[kPassDst][6];  // per destination: velocity, streamfunction
-    double dx[kPassDst][3];   // destination positions
-    int32_t di[kPassDst], dprev[kPassDst];
-    int32_t dr_start[kMaxBlockRows], dr_base[kMaxBlockRows + 1];  // destination ranges of the block
-    int32_t off[kMaxNbCells + 1];  // concatenated offsets of the neighbour slabs
-    int32_t cstart[kMaxNbCells];   // first cell-sorted source of each neighbour slab
-    int2 rng[kPairThreads / 32][kMaxRows];  // per warp: candidate range of every row
-    alignas(16) double tab[2];  // the weight tables follow: [weight][interval][kTabSNC]
-};
-constexpr size_t kPairSmemMost = 226 * 1024;
-__host__ __device__ constexpr int tile_sources(bool vel, bool psi) { return vel && psi ? 640 : 1024; }
+// ---- pair kernels over cell lists: common parts ----
+constexpr double kScreenMargin = 2e-5;  // of r_cut^2, on top of the rounding of the FP32 places
+constexpr size_t kPairSmemMost = 200 * 1024;  // tables of an FP64 pair-kernel CTA
 
 // 1/sqrt(s) in FP64: FP32 hardware estimate refined by two Newton-Raphson steps
 // y <- y (3 - s y^2) / 2 (quadratic convergence: ~1e-7 -> ~1e-14 -> rounding level).
@@ -528,27 +493,6 @@ __device__ __forceinline__ void ewald_weights2(const KParams& K, double x, doubl
     }
 }
 
-static_assert(sizeof(TileSmem<1024>) <= 92 * 1024 && sizeof(TileSmem<640>) <= 68 * 1024,
-              "two pair-kernel CTAs (with the tables of x <= 4) must fit in one SM's shared memory");
-
-// Largest row r in [0, n] whose first concatenated index off[r W] is <= T (off[0] = 0 <= T).
-__device__ __forceinline__ int last_row_le(const int32_t* off, int W, int n, int T) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (off[mid * W] <= T) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// Distance from x to the cell [lo, lo + h], less a margin of 1e-9 h so that rounding in the
-// binning can never cull a source that is in range.
-__device__ __forceinline__ double box_gap(double x, double lo, double h) {
-    const double g = fmax(fmax(lo - x, x - (lo + h)), 0.0);
-    return fmax(g - 1e-9 * h, 0.0);
-}
-
 // Interval and local coordinate of x in the shared-memory tables (intervals centred at k / 96):
 // k = round(96 x) by the 1.5 * 2^52 trick, t = 96 x - k in [-1/2, 1/2].
 __device__ __forceinline__ double tab_s_pos(double x, int ntab, int* k) {
@@ -562,297 +506,6 @@ __device__ __forceinline__ double tab_s_poly(const double* c, double t) {
     const double2* v = reinterpret_cast<const double2*>(c);
     const double2 c0 = v[0], c1 = v[1], c2 = v[2];
     return fma(fma(fma(fma(fma(c2.y, t, c2.x), t, c1.y), t, c1.x), t, c0.y), t, c0.x);
-}
-
-// Two queued pairs per lane (tile indices t0, t1; v0, v1 mark valid entries): the FP64 separation, the
-// r^2 <= r_cut^2 decision, and the pair integrand (short_range_integrand, integrands.jl:2-18).  Entries
-// that are invalid or out of range are evaluated at r = r_cut and add zero, so both chains run straight
-// through.  Called by all lanes of the warp.
-template <bool VEL, bool PSI, int TILE>
-__device__ __forceinline__ void tile_eval2(const KParams& K, const double xd[3], const TileSmem<TILE>& S, int t0,
-                                           bool v0, int t1, bool v1, double (&av)[3], double (&ap)[3],
-                                           unsigned long long& ninr) {
-    const int tt[2] = {t0, t1};
-    const bool vv[2] = {v0, v1};
-    double d[2][3], q[2][3], s2[2];
-    bool ok[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const double2 a = S.pxy[tt[u]], b = S.pzq[tt[u]], c = S.qyz[tt[u]];
-        d[u][0] = xd[0] - a.x;
-        d[u][1] = xd[1] - a.y;
-        d[u][2] = xd[2] - b.x;
-        q[u][0] = b.y;
-        q[u][1] = c.x;
-        q[u][2] = c.y;
-        s2[u] = d[u][0] * d[u][0] + d[u][1] * d[u][1] + d[u][2] * d[u][2];
-        ok[u] = vv[u] && s2[u] <= K.rcut2;
-        ninr += __popc(__ballot_sync(0xffffffffu, ok[u]));
-        if (!ok[u]) s2[u] = K.rcut2;
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const double rinv = rsqrt_nr(s2[u]);
-        int k;
-        const double t = tab_s_pos(K.alpha * (s2[u] * rinv), K.ntab_s, &k);
-        if (VEL) {
-            const double w = tab_s_poly(S.tab + (PSI ? K.ntab_s + k : k) * kTabSNC, t);
-            const double f = ok[u] ? w * rinv * rinv * rinv : 0.0;
-            av[0] += f * (q[u][1] * d[u][2] - q[u][2] * d[u][1]);
-            av[1] += f * (q[u][2] * d[u][0] - q[u][0] * d[u][2]);
-            av[2] += f * (q[u][0] * d[u][1] - q[u][1] * d[u][0]);
-        }
-        if (PSI) {
-            const double w = tab_s_poly(S.tab + k * kTabSNC, t);
-            const double f = ok[u] ? w * rinv : 0.0;
-            ap[0] += f * q[u][0];
-            ap[1] += f * q[u][1];
-            ap[2] += f * q[u][2];
-        }
-    }
-}
-
-// Candidates [a, b) of the tile against the destination (block-relative position xd in FP64, xr in
-// FP32; node i, previous node iprev): FP32 screen on the hi parts, compaction of the survivors into
-// the warp's queue, evaluation 64 at a time.
-template <bool VEL, bool PSI, bool SKIP, int TILE>
-__device__ __forceinline__ void tile_range_q(const KParams& K, const double xd[3], float3 xr, float rc2s, int i,
-                                             int iprev, const TileSmem<TILE>& S, int a, int b, int lane,
-                                             double (&av)[3], double (&ap)[3], int32_t* Q, int& qcount,
-                                             unsigned long long& ninr) {
-    for (int base = a; base < b; base += 32) {
-        const int t = base + lane;
-        const float4 p = S.hi[t];
-        const float e0 = xr.x - p.x, e1 = xr.y - p.y, e2 = xr.z - p.z;
-        bool inr = t < b && fmaf(e0, e0, fmaf(e1, e1, e2 * e2)) <= rc2s;
-        if (SKIP) {
-            const int sg = __float_as_int(p.w);
-            inr = inr && sg != i && sg != iprev;
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, inr);
-        if (inr) Q[qcount + __popc(m & ((1u << lane) - 1u))] = t;
-        qcount += __popc(m);
-        __syncwarp();
-        if (qcount >= 64) {
-            tile_eval2<VEL, PSI, TILE>(K, xd, S, Q[lane], true, Q[32 + lane], true, av, ap, ninr);
-            __syncwarp();
-            if (lane < qcount - 64) Q[lane] = Q[64 + lane];
-            __syncwarp();
-            qcount -= 64;
-        }
-    }
-}
-
-template <bool VEL, bool PSI, bool SKIP>
-__global__ void __launch_bounds__(kPairThreads, 2) pair_cell_kernel(
-    KParams K, CellGrid cg, int64_t Np, int64_t Ns, const int32_t* __restrict__ dst_start,
-    const int32_t* __restrict__ dst_order, const double* __restrict__ nodes, const int32_t* __restrict__ idx_prev,
-    const double* __restrict__ src, const int32_t* __restrict__ src_start, const int32_t* __restrict__ seg,
-    double* __restrict__ vel, double* __restrict__ psi, unsigned long long* __restrict__ counters, int3 bk,
-    int3 nb) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int kTile = tile_sources(VEL, PSI);
-    TileSmem<kTile>& S = *reinterpret_cast<TileSmem<kTile>*>(smem_raw);
-    const int M = cg.M, G = cg.G;
-    const int nc0 = cg.nc[0], nc1 = cg.nc[1], nc2 = cg.nc[2];
-    const int ncc = nc0 / G;  // cells in x (each made of G slabs)
-    // this CTA's block of cells [cx0, cx1) x [cy0, cy1) x [cz0, cz1)
-    const int bxi = blockIdx.x % nb.x, byi = (blockIdx.x / nb.x) % nb.y, bzi = blockIdx.x / (nb.x * nb.y);
-    const int cx0 = bxi * bk.x, cx1 = min(cx0 + bk.x, ncc);
-    const int cy0 = byi * bk.y, cy1 = min(cy0 + bk.y, nc1);
-    const int cz0 = bzi * bk.z, cz1 = min(cz0 + bk.z, nc2);
-    const int ndr = (cy1 - cy0) * (cz1 - cz0);  // destination ranges: one per (y, z) cell row
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int k = 0; k < ndr; ++k) {
-            const int yy = cy0 + k % (cy1 - cy0), zz = cz0 + k / (cy1 - cy0);
-            const int64_t s0 = ((int64_t)zz * nc1 + yy) * nc0 + (int64_t)cx0 * G;
-            const int a = dst_start[s0], b = dst_start[s0 + (int64_t)(cx1 - cx0) * G];
-            S.dr_start[k] = a;
-            S.dr_base[k] = acc;
-            acc += b - a;
-        }
-        S.dr_base[ndr] = acc;
-    }
-    __syncthreads();
-    // this CTA's share of the block's nodes
-    const int nall = S.dr_base[ndr];
-    const int n0 = (int)((int64_t)nall * blockIdx.y / gridDim.y), nd = (int)((int64_t)nall * (blockIdx.y + 1) / gridDim.y);
-    if (n0 == nd) return;  // uniform over the CTA
-    {
-        constexpr int first = VEL && !PSI ? 1 : 0, nw = VEL && PSI ? 2 : 1;
-        const double2* src_tab = reinterpret_cast<const double2*>(K.tab_s + (size_t)first * K.ntab_s * kTabSNC);
-        double2* dst_tab = reinterpret_cast<double2*>(S.tab);
-        for (int k = threadIdx.x; k < nw * K.ntab_s * kTabSNC / 2; k += kPairThreads) dst_tab[k] = src_tab[k];
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double hx = K.L[0] / nc0, h1 = K.L[1] / nc1, h2 = K.L[2] / nc2, inv_hx = nc0 / K.L[0];
-    // neighbourhood: rows (y, z) of the block widened by M cells, slabs in x widened by M G
-    const int WY = cy1 - cy0 + 2 * M, WZ = cz1 - cz0 + 2 * M, WX = (cx1 - cx0 + 2 * M) * G;
-    const int nrow = WY * WZ, ncb = nrow * WX;
-    const int ry0 = cy0 - M, rz0 = cz0 - M, xs0 = cx0 * G - M * G;  // unwrapped first row / slab
-    const double o0 = cx0 * G * hx, o1 = cy0 * h1, o2 = cz0 * h2;  // block corner: origin of the FP32 coordinates
-    const float rc2s = (float)(K.rcut2 * (1.0 + kScreenMargin));
-    // neighbour slabs in (row, slab) order: first cell-sorted source and count
-    for (int ci = threadIdx.x; ci < ncb; ci += kPairThreads) {
-        const int r = ci / WX, k = ci % WX;
-        int xx = xs0 + k, yy = ry0 + r % WY, zz = rz0 + r / WY;
-        xx = xx < 0 ? xx + nc0 : (xx >= nc0 ? xx - nc0 : xx);
-        yy = yy < 0 ? yy + nc1 : (yy >= nc1 ? yy - nc1 : yy);
-        zz = zz < 0 ? zz + nc2 : (zz >= nc2 ? zz - nc2 : zz);
-        const int64_t c = ((int64_t)zz * nc1 + yy) * nc0 + xx;
-        const int s0 = src_start[c];
-        S.cstart[ci] = s0;
-        S.off[ci + 1] = src_start[c + 1] - s0;
-    }
-    __syncthreads();
-    if (warp == 0) {  // counts -> concatenated offsets
-        int carry = 0;
-        for (int base = 0; base < ncb; base += 32) {
-            const int ci = base + lane;
-            int v = ci < ncb ? S.off[ci + 1] : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, v, o);
-                if (lane >= o) v += t;
-            }
-            if (ci < ncb) S.off[ci + 1] = carry + v;
-            carry += __shfl_sync(0xffffffffu, v, 31);
-        }
-        if (lane == 0) S.off[0] = 0;
-    }
-    __syncthreads();
-    const int ntot = S.off[ncb];
-    const double pref = K.Gamma / (4.0 * kPi);
-    unsigned long long ninr = 0, ncand = 0;  // warp-uniform
-    for (int p0 = n0; p0 < nd; p0 += kPassDst) {
-        const int np = nd - p0 < kPassDst ? nd - p0 : kPassDst;
-        __syncthreads();  // the previous pass has written its results
-        for (int t = threadIdx.x; t < np; t += kPairThreads) {
-            const int tt = p0 + t;
-            int k = 0;
-            while (k + 1 < ndr && S.dr_base[k + 1] <= tt) ++k;
-            const int i = dst_order[S.dr_start[k] + tt - S.dr_base[k]];
-            S.di[t] = i;
-            S.dprev[t] = idx_prev[i];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) S.dx[t][d] = nodes[d * Np + i];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) S.acc[t][c] = 0.0;
-        }
-        const int P = np >= kPairThreads / 32 ? 1 : (kPairThreads / 32) / np;  // row parts per destination
-        const int nitems = np * P;
-        for (int T0 = 0, T1 = 0; T0 < ntot; T0 = T1) {
-            // tile [T0, T1): whole rows [ra, rb) while they fit, else a kTile piece of one row
-            const int ra = min(last_row_le(S.off, WX, nrow, T0), nrow - 1);
-            const int rf = last_row_le(S.off, WX, nrow, T0 + kTile);
-            T1 = S.off[rf * WX] > T0 ? S.off[rf * WX] : min(T0 + kTile, ntot);
-            const int rb = min(last_row_le(S.off, WX, nrow, T1 - 1) + 1, nrow);
-            __syncthreads();  // previous tile consumed, destinations loaded
-            // staging, a warp per row (periodic image of each slab next to the destination block): the
-            // slabs of a row are consecutive cells, so its sources are one contiguous range of the
-            // cell-sorted arrays, or two where the row wraps around the period in x
-            const int kw = xs0 < 0 ? -xs0 : (xs0 + WX > nc0 ? nc0 - xs0 : WX);  // first slab past the wrap
-            const double sxA = xs0 < 0 ? -K.L[0] : 0.0, sxB = xs0 < 0 ? 0.0 : K.L[0];
-            for (int r = ra + warp; r < rb; r += kPairThreads / 32) {
-                const int rowA = S.off[r * WX], rowE = S.off[(r + 1) * WX];
-                const int a = rowA > T0 ? rowA : T0, b = rowE < T1 ? rowE : T1;
-                if (a >= b) continue;  // warp-uniform
-                const int yu = ry0 + r % WY, zu = rz0 + r / WY;
-                const double sy = yu < 0 ? -K.L[1] : (yu >= nc1 ? K.L[1] : 0.0);
-                const double sz = zu < 0 ? -K.L[2] : (zu >= nc2 ? K.L[2] : 0.0);
-                const int offB = S.off[r * WX + kw];
-                const int gA = S.cstart[r * WX];
-                const int gB = kw < WX ? S.cstart[r * WX + kw] : 0;
-                for (int t = a + lane; t < b; t += 32) {
-                    const bool inA = t < offB;
-                    const int j = inA ? gA + (t - rowA) : gB + (t - offB);
-                    const double sx = inA ? sxA : sxB;
-                    const double u0 = src[j] + sx - o0, u1 = src[Ns + j] + sy - o1, u2 = src[2 * Ns + j] + sz - o2;
-                    const float f0 = (float)u0, f1 = (float)u1, f2 = (float)u2;
-                    S.hi[t - T0] = make_float4(f0, f1, f2, __int_as_float(SKIP ? seg[j] : 0));
-                    S.pxy[t - T0] = make_double2(u0, u1);
-                    S.pzq[t - T0] = make_double2(u2, src[3 * Ns + j]);
-                    S.qyz[t - T0] = make_double2(src[4 * Ns + j], src[5 * Ns + j]);
-                }
-            }
-            __syncthreads();
-            for (int it = warp; it < nitems; it += kPairThreads / 32) {
-                const int dl = it % np, part = it / np;
-                const double x[3] = {S.dx[dl][0], S.dx[dl][1], S.dx[dl][2]};
-                // candidate range of every row, trimmed to the slabs within r_cut of the node
-                for (int r = ra + lane; r < rb; r += 32) {
-                    const double gy = box_gap(x[1], (ry0 + r % WY) * h1, h1);
-                    const double gz = box_gap(x[2], (rz0 + r / WY) * h2, h2);
-                    const double gyz = gy * gy + gz * gz;
-                    int a = 0, b = 0;
-                    if (gyz <= K.rcut2) {
-                        const double w = (double)sqrtf((float)(K.rcut2 - gyz)) * (1.0 + 1e-6) + 1e-9 * hx;
-                        int klo = (int)floor((x[0] - w) * inv_hx) - xs0;
-                        int khi = (int)floor((x[0] + w) * inv_hx) - xs0;
-                        klo = klo < 0 ? 0 : klo;
-                        khi = khi > WX - 1 ? WX - 1 : khi;
-                        if (klo <= khi) {
-                            a = S.off[r * WX + klo];
-                            b = S.off[r * WX + khi + 1];
-                        }
-                    }
-                    S.rng[warp][r] = make_int2(a, b);
-                }
-                __syncwarp();
-                double av[3] = {0, 0, 0}, ap[3] = {0, 0, 0};
-                int qcount = 0;
-                int32_t* Q = S.queue[warp];
-                const double xd[3] = {x[0] - o0, x[1] - o1, x[2] - o2};
-                const float3 xr = make_float3((float)xd[0], (float)xd[1], (float)xd[2]);
-                const int i = S.di[dl], iprev = S.dprev[dl];
-                for (int r = ra + part; r < rb; r += P) {
-                    const int2 ab = S.rng[warp][r];
-                    const int a = ab.x > T0 ? ab.x : T0, b = ab.y < T1 ? ab.y : T1;
-                    if (a < b) {
-                        ncand += b - a;
-                        tile_range_q<VEL, PSI, SKIP, kTile>(K, xd, xr, rc2s, i, iprev, S, a - T0, b - T0, lane, av, ap, Q,
-                                                            qcount, ninr);
-                    }
-                }
-                if (qcount > 0)  // warp-uniform
-                    tile_eval2<VEL, PSI, kTile>(K, xd, S, lane < qcount ? Q[lane] : 0, lane < qcount,
-                                                32 + lane < qcount ? Q[32 + lane] : 0, 32 + lane < qcount, av, ap, ninr);
-                double s[6] = {0, 0, 0, 0, 0, 0};
-                if (VEL)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) s[c] = warp_sum(av[c]);
-                if (PSI)
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) s[3 + c] = warp_sum(ap[c]);
-                if (lane == 0) {
-                    if (VEL)
-                        for (int c = 0; c < 3; ++c) atomicAdd(&S.acc[dl][c], s[c]);
-                    if (PSI)
-                        for (int c = 0; c < 3; ++c) atomicAdd(&S.acc[dl][3 + c], s[3 + c]);
-                }
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        for (int t = threadIdx.x; t < np; t += kPairThreads) {
-            const int64_t i = S.di[t];
-            if (VEL) {
-                vel[i] += pref * S.acc[t][0];
-                vel[Np + i] += pref * S.acc[t][1];
-                vel[2 * Np + i] += pref * S.acc[t][2];
-            }
-            if (PSI) {
-                psi[i] += pref * S.acc[t][3];
-                psi[Np + i] += pref * S.acc[t][4];
-                psi[2 * Np + i] += pref * S.acc[t][5];
-            }
-        }
-    }
-    if (lane == 0) {
-        atomicAdd(&counters[0], ninr);
-        atomicAdd(&counters[1], ncand);
-    }
 }
 
 // ---- FP32 pair kernel of the mixed form ----
@@ -882,7 +535,14 @@ constexpr float kF32Band = 4e-6f; // relative band around r_cut^2 decided in FP6
 constexpr float kF32Far = 1e18f;  // coordinate of an absent node or source (its square is finite)
 constexpr int kF32Warps = 4;
 constexpr int kF32Blocks = 8;  // CTAs per SM (64 registers)
-constexpr int kF32IndexBits = 26;  // of a queue entry: the source; 2 bits for its image in x, y and z above them
+// A queue entry: the source's cell-sorted index and above it 2 bits each for its image in x, y and z (0, 1,
+// 2: -L, 0, +L).  32-bit entries hold 2^26 sources, larger systems take 64-bit ones.
+template <typename E>
+constexpr int kIndexBits = sizeof(E) == 4 ? 26 : 32;
+template <typename E>
+__device__ __forceinline__ uint32_t entry_source(E e) { return (uint32_t)(e & (((E)1 << kIndexBits<E>) - 1)); }
+template <typename E>
+__device__ __forceinline__ int entry_image(E e, int dim) { return (int)(e >> (kIndexBits<E> + 2 * dim)) & 3; }
 
 
 __device__ __forceinline__ float rsqrt_fast(float x) {
@@ -916,25 +576,27 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 }
 __device__ __forceinline__ float half2f(f32x2 a, int u) { return __uint_as_float((unsigned)(u ? a >> 32 : a)); }
 
+template <typename E>
 struct F32Warp {
-    float2 x[8][3][3];       // node, dimension, image (-L, 0, +L): hi and lo parts of the node's place
-    int2 id[8];              // node and previous node
-    ulonglong2 xy2[4];       // hi parts of two nodes in the images of the current row: x, x | y, y
-    f32x2 z2[4];
-    uint32_t queue[8][64];   // per node: screened sources, cell-sorted index and image (kF32IndexBits)
+    float2 x[4][3][3];       // node, dimension, image (-L, 0, +L): hi and lo parts of the node's place
+    int2 id[4];              // node and previous node
+    ulonglong2 xy2[2];       // hi parts of two nodes in the images of the current row: x, x | y, y
+    f32x2 z2[2];
+    E queue[4][64];          // per node: screened sources
 };
 
 // 32 queued pairs (one a lane; `live` false for lanes past the queue's end) of one node.
-template <bool VEL, bool PSI>
-__device__ __forceinline__ void f32_eval(const F32Warp& S, int d, int e, bool live, const float4* __restrict__ srcP,
+template <bool VEL, bool PSI, typename E>
+__device__ __forceinline__ void f32_eval(const F32Warp<E>& S, int d, int e, bool live, const float4* __restrict__ srcP,
                                          const float4* __restrict__ srcQ, const float2* __restrict__ srcR,
                                          const float4* __restrict__ tab, float rc2lo, float rc2hi, double rcut2, float alpha,
                                          int nf, float (&v)[3], float (&w)[3], int& ninr) {
-    const uint32_t entry = S.queue[d][e], j = entry & ((1u << kF32IndexBits) - 1u);
+    const E entry = S.queue[d][e];
+    const uint32_t j = entry_source(entry);
     const float4 p = __ldg(srcP + j), q = __ldg(srcQ + j);
     const float2 qr = __ldg(srcR + j);
-    const float2 x0 = S.x[d][0][entry >> kF32IndexBits & 3u], x1 = S.x[d][1][entry >> (kF32IndexBits + 2) & 3u],
-                 x2 = S.x[d][2][entry >> (kF32IndexBits + 4)];
+    const float2 x0 = S.x[d][0][entry_image(entry, 0)], x1 = S.x[d][1][entry_image(entry, 1)],
+                 x2 = S.x[d][2][entry_image(entry, 2)];
     const int2 id = S.id[d];
     const float d0 = (x0.x - p.x) + (x0.y - q.x), d1 = (x1.x - p.y) + (x1.y - q.y), d2 = (x2.x - p.z) + (x2.y - q.z);
     const float s2 = fmaf(d0, d0, fmaf(d1, d1, d2 * d2));
@@ -975,8 +637,8 @@ __device__ __forceinline__ void f32_eval(const F32Warp& S, int d, int e, bool li
 
 // Sums of v[n][3] over the warp's lanes, n = D a power of two: lane halves exchange halves of the n
 // until a lane holds one of them (number lane / (32 / D)); every lane of its 32 / D has the total.
-template <int D>
-__device__ __forceinline__ void f32_reduce(float (&v)[D][3], int lane, float (&out)[3]) {
+template <int D, typename T>
+__device__ __forceinline__ void group_reduce(T (&v)[D][3], int lane, T (&out)[3]) {
 #pragma unroll
     for (int h = D / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
         const bool up = lane & o;
@@ -984,33 +646,84 @@ __device__ __forceinline__ void f32_reduce(float (&v)[D][3], int lane, float (&o
         for (int i = 0; i < h; ++i)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const float keep = up ? v[h + i][c] : v[i][c], give = up ? v[i][c] : v[h + i][c];
+                const T keep = up ? v[h + i][c] : v[i][c], give = up ? v[i][c] : v[h + i][c];
                 v[i][c] = keep + __shfl_xor_sync(0xffffffffu, give, o);
             }
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        float x = v[0][c];
+        T x = v[0][c];
 #pragma unroll
         for (int o = 16 / D; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
         out[c] = x;
     }
 }
 
-template <bool VEL, bool PSI, int D>
-__global__ void __launch_bounds__(32 * kF32Warps, kF32Blocks) pair_f32_kernel(
+// Sources near a group of nodes of one (y, z) row of cells: row r (of the W^2 around it) as the unwrapped
+// slab range [klo, khi] within r_cut of the group's bounding box [lo, hi], the index of its first slab, and
+// its periodic image in y and z (0, 1, 2: -L, 0, +L; y + 3 z).
+struct RowRange {
+    int klo, khi, row, iyz;
+};
+__device__ __forceinline__ RowRange near_row(const CellGrid& cg, const KParams& K, int r, int gy, int gz,
+                                             const float (&lo)[3], const float (&hi)[3], float slack) {
+    const int M = cg.M, W = 2 * M + 1, nc0 = cg.nc[0], nc1 = cg.nc[1], nc2 = cg.nc[2];
+    RowRange R{0, -1, 0, 0};
+    if (r >= W * W) return R;
+    const int yu = gy + r % W - M, zu = gz + r / W - M;
+    const float h1 = (float)(K.L[1] / nc1), h2 = (float)(K.L[2] / nc2), rc = (float)K.rcut;
+    const float ylo = (float)yu * h1, zlo = (float)zu * h2;
+    const float ey = fmaxf(fmaxf(ylo - hi[1], lo[1] - (ylo + h1)), 0.0f);
+    const float ez = fmaxf(fmaxf(zlo - hi[2], lo[2] - (zlo + h2)), 0.0f);
+    const float rest = rc * rc * 1.0001f - ey * ey - ez * ez;
+    if (rest >= 0.0f) {
+        const float w = sqrtf(rest) + slack;
+        const double inv_hx = nc0 / K.L[0];
+        R.klo = (int)floor((double)(lo[0] - w) * inv_hx);
+        R.khi = (int)floor((double)(hi[0] + w) * inv_hx);
+    }
+    const int my = yu < 0 ? 0 : (yu >= nc1 ? 2 : 1), mz = zu < 0 ? 0 : (zu >= nc2 ? 2 : 1);
+    R.row = ((zu + (1 - mz) * nc2) * nc1 + yu + (1 - my) * nc1) * nc0;
+    R.iyz = my + 3 * mz;
+    return R;
+}
+
+// Bounding box of the lanes with `mine` among the first D, widened by `slack`, on every lane.
+template <int D>
+__device__ __forceinline__ void group_box(bool mine, const double (&x)[3], float slack, float (&lo)[3], float (&hi)[3]) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = mine ? (float)x[d] : kF32Far;
+        hi[d] = mine ? (float)x[d] : -kF32Far;
+    }
+#pragma unroll
+    for (int o = 1; o < D; o <<= 1)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+            hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+        }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        lo[d] = __shfl_sync(0xffffffffu, lo[d], 0) - slack;
+        hi[d] = __shfl_sync(0xffffffffu, hi[d], 0) + slack;
+    }
+}
+
+template <bool VEL, bool PSI, int D, typename E>
+__global__ void __launch_bounds__(32 * kF32Warps, sizeof(E) == 4 ? kF32Blocks : 6) pair_f32_kernel(
     KParams K, CellGrid cg, int64_t Np, float rc2s, const int32_t* __restrict__ dst_start,
     const int32_t* __restrict__ dst_order, const double* __restrict__ nodes, const int32_t* __restrict__ idx_prev,
     const float4* __restrict__ srcP, const float4* __restrict__ srcQ, const float2* __restrict__ srcR,
     const int32_t* __restrict__ src_start, double* __restrict__ vel, double* __restrict__ psi,
     unsigned long long* __restrict__ counters) {
-    __shared__ F32Warp warps[kF32Warps];
+    __shared__ F32Warp<E> warps[kF32Warps];
     __shared__ float4 tab[(VEL && PSI ? 2 : 1) * kF32TabMax];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nf = K.ntab_c;
     for (int k = threadIdx.x; k < (VEL && PSI ? 2 : 1) * nf; k += 32 * kF32Warps) tab[k] = K.tab_c[(VEL && !PSI ? nf : 0) + k];
     __syncthreads();
-    F32Warp& S = warps[warp];
+    F32Warp<E>& S = warps[warp];
     const int64_t first = ((int64_t)blockIdx.x * kF32Warps + warp) * D;
     const int64_t nvalid = dst_start[cg.ncell];  // nodes of the sentinel cell (non-finite) come after these
     if (first >= nvalid) return;
@@ -1034,9 +747,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, kF32Blocks) pair_f32_kernel(
         cy = cell_coord(x[1], K.L[1], nc1);
         cz = cell_coord(x[2], K.L[2], nc2);
     }
-    const float h1 = (float)(K.L[1] / nc1), h2 = (float)(K.L[2] / nc2);
-    const double inv_hx = nc0 / K.L[0];
-    const float rc = (float)K.rcut, rc2w = rc * rc * 1.0001f;
+    const float rc = (float)K.rcut;
     // slack of the row and slab ranges, far above the FP32 rounding of places in the box
     const float slack = 1e-5f * rc + 1e-6f * (float)fmax(K.L[0], fmax(K.L[1], K.L[2]));
     const float rc2lo = (float)(K.rcut2 * (1.0 - (double)kF32Band)), rc2hi = (float)(K.rcut2 * (1.0 + (double)kF32Band));
@@ -1061,46 +772,15 @@ __global__ void __launch_bounds__(32 * kF32Warps, kF32Blocks) pair_f32_kernel(
         const bool mine = (todo >> lane & 1) && cy == gy_ && cz == gz_ && fabs(x[0] - xlead) <= K.rcut;
         todo &= ~__ballot_sync(0xffffffffu, mine);
         float lo[3], hi[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = mine ? (float)x[d] : kF32Far;
-            hi[d] = mine ? (float)x[d] : -kF32Far;
-        }
-#pragma unroll
-        for (int o = 1; o < D; o <<= 1)
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-                hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-            }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            lo[d] = __shfl_sync(0xffffffffu, lo[d], 0) - slack;
-            hi[d] = __shfl_sync(0xffffffffu, hi[d], 0) + slack;
-        }
-        // lane l takes the row (dy, dz) = (l % W - M, l / W - M) around the nodes' own row
-        int klo = 0, khi = -1, row = 0, iyz = 0;
-        if (lane < W * W) {
-            const int yu = gy_ + lane % W - M, zu = gz_ + lane / W - M;
-            const float ylo = (float)yu * h1, zlo = (float)zu * h2;
-            const float gy = fmaxf(fmaxf(ylo - hi[1], lo[1] - (ylo + h1)), 0.0f);
-            const float gz = fmaxf(fmaxf(zlo - hi[2], lo[2] - (zlo + h2)), 0.0f);
-            const float rest = rc2w - gy * gy - gz * gz;
-            if (rest >= 0.0f) {
-                const float r = sqrtf(rest) + slack;
-                klo = (int)floor((double)(lo[0] - r) * inv_hx);
-                khi = (int)floor((double)(hi[0] + r) * inv_hx);
-            }
-            const int my = yu < 0 ? 0 : (yu >= nc1 ? 2 : 1), mz = zu < 0 ? 0 : (zu >= nc2 ? 2 : 1);
-            row = ((zu + (1 - mz) * nc2) * nc1 + yu + (1 - my) * nc1) * nc0;
-            iyz = my + 3 * mz;
-        }
+        group_box<D>(mine, x, slack, lo, hi);
+        for (int r0 = 0; r0 < W * W; r0 += 32) {  // a lane per row of cells around the nodes' own
+        const RowRange R = near_row(cg, K, r0 + lane, gy_, gz_, lo, hi, slack);
         for (int mx = 0; mx < 3; ++mx) {  // images in x: -L, 0, +L
-            const int s0 = max(klo - (mx - 1) * nc0, 0), s1 = min(khi - (mx - 1) * nc0, nc0 - 1);
+            const int s0 = max(R.klo - (mx - 1) * nc0, 0), s1 = min(R.khi - (mx - 1) * nc0, nc0 - 1);
             int a = 0, b = 0;
             if (s0 <= s1) {
-                a = src_start[row + s0];
-                b = src_start[row + s1 + 1];
+                a = src_start[R.row + s0];
+                b = src_start[R.row + s1 + 1];
             }
             for (unsigned rows = __ballot_sync(0xffffffffu, a < b); rows; rows &= rows - 1) {
                 const bool skip = turn % (int)gridDim.y != (int)blockIdx.y;  // warp-uniform
@@ -1108,7 +788,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, kF32Blocks) pair_f32_kernel(
                 if (skip) continue;
                 const int sl = __ffs(rows) - 1;
                 const int ra = __shfl_sync(0xffffffffu, a, sl), rb = __shfl_sync(0xffffffffu, b, sl);
-                const int im = __shfl_sync(0xffffffffu, iyz, sl), my = im % 3, mz = im / 3;
+                const int im = __shfl_sync(0xffffffffu, R.iyz, sl), my = im % 3, mz = im / 3;
                 __syncwarp();
                 if (lane < D) {
                     const float px = mine ? S.x[lane][0][mx].x : kF32Far;
@@ -1119,7 +799,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, kF32Blocks) pair_f32_kernel(
                 }
                 __syncwarp();
                 ncand += (unsigned)(rb - ra) * D;
-                const uint32_t code = (uint32_t)(mx | my << 2 | mz << 4) << kF32IndexBits;
+                const E code = (E)(mx | my << 2 | mz << 4) << kIndexBits<E>;
                 float4 pn = __ldg(srcP + min(ra + lane, rb - 1));
                 for (int base = ra; base < rb; base += 32) {
                     const int t = base + lane;
@@ -1127,7 +807,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, kF32Blocks) pair_f32_kernel(
                     pn = __ldg(srcP + min(t + 32, rb - 1));
                     if (t >= rb) p.x = -kF32Far;
                     const f32x2 px = dup2(-p.x), py = dup2(-p.y), pz = dup2(-p.z);
-                    const uint32_t entry = (uint32_t)t | code;
+                    const E entry = (E)t | code;
 #pragma unroll
                     for (int h = 0; h < D / 2; ++h) {
                         const ulonglong2 xy = S.xy2[h];
@@ -1143,7 +823,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, kF32Blocks) pair_f32_kernel(
                             cnt[d] += __popc(m);
                             if (cnt[d] >= 32) {
                                 __syncwarp();
-                                f32_eval<VEL, PSI>(S, d, lane, true, srcP, srcQ, srcR, tab, rc2lo, rc2hi, K.rcut2, alpha, nf, v[d],
+                                f32_eval<VEL, PSI, E>(S, d, lane, true, srcP, srcQ, srcR, tab, rc2lo, rc2hi, K.rcut2, alpha, nf, v[d],
                                                    w[d], ninr);
                                 cnt[d] -= 32;
                                 __syncwarp();
@@ -1155,26 +835,237 @@ __global__ void __launch_bounds__(32 * kF32Warps, kF32Blocks) pair_f32_kernel(
                 }
             }
         }
+        }
     }
     __syncwarp();
 #pragma unroll
     for (int d = 0; d < D; ++d)
         if (cnt[d] > 0)  // warp-uniform
-            f32_eval<VEL, PSI>(S, d, lane < cnt[d] ? lane : 0, lane < cnt[d], srcP, srcQ, srcR, tab, rc2lo, rc2hi, K.rcut2, alpha, nf,
+            f32_eval<VEL, PSI, E>(S, d, lane < cnt[d] ? lane : 0, lane < cnt[d], srcP, srcQ, srcR, tab, rc2lo, rc2hi, K.rcut2, alpha, nf,
                                v[d], w[d], ninr);
     const double pref = K.Gamma / (4.0 * kPi);
     const int slot = lane / (32 / D);
     const int is = __shfl_sync(0xffffffffu, i, slot);
     float out[3];
     if (VEL) {
-        f32_reduce<D>(v, lane, out);
+        group_reduce<D>(v, lane, out);
         if (lane % (32 / D) == 0 && is >= 0)
             for (int c = 0; c < 3; ++c) atomicAdd(&vel[c * Np + is], pref * (double)out[c]);
     }
     if (PSI) {
-        f32_reduce<D>(w, lane, out);
+        group_reduce<D>(w, lane, out);
         if (lane % (32 / D) == 0 && is >= 0)
             for (int c = 0; c < 3; ++c) atomicAdd(&psi[c * Np + is], pref * (double)out[c]);
+    }
+    const unsigned long long total = warp_sum_u((unsigned long long)ninr);
+    if (lane == 0) {
+        atomicAdd(&counters[0], total);
+        atomicAdd(&counters[1], (unsigned long long)ncand);
+    }
+}
+
+// ---- FP64 pair kernel ----
+// The same groups, rows, FP32 screen and queues; the evaluation reads the sources' FP64 positions and charges
+// (cell-sorted arrays), decides r^2 <= r_cut^2 and evaluates in FP64 (Newton-refined reciprocal square root,
+// weights from degree-5 tables in shared memory, one copy per CTA).  SKIP: the node's own two segments left
+// out.  Bound: shared-memory and L1 wavefronts of the gathers (per 32 pairs about 30 for the weights' three
+// 16-byte loads and 30 for the sources), then the FP64 pipe (17 cycles).  1M nodes, 3.13 G pairs: 28.7 ms (CTAs
+// that stage tiles of a block's neighbourhood: 39.5); 20k nodes, both fields: 0.205 (0.517).  Two CTAs of 128
+// registers instead of three of 80: 30.6.
+constexpr int kF64Warps = 8;
+constexpr int kF64Blocks = 3;  // CTAs per SM (80 registers)
+
+template <int D, typename E>
+struct F64Warp {
+    double x[D][3][3];      // node, dimension, image (-L, 0, +L)
+    int2 id[D];             // node and previous node
+    ulonglong2 xy2[D / 2];  // FP32 places of two nodes in the images of the current row: x, x | y, y
+    f32x2 z2[D / 2];
+    E queue[D][64];
+};
+
+template <bool VEL, bool PSI, bool SKIP, int D, typename E>
+__device__ __forceinline__ void f64_eval(const KParams& K, const F64Warp<D, E>& S, int d, int e, bool live,
+                                         const float4* __restrict__ srcP, const double* __restrict__ src, int64_t Ns,
+                                         const double* __restrict__ tab, double (&v)[3], double (&w)[3], int& ninr) {
+    const E entry = S.queue[d][e];
+    const uint32_t j = entry_source(entry);
+    const double* s = src + j;
+    const double d0 = S.x[d][0][entry_image(entry, 0)] - __ldg(s);
+    const double d1 = S.x[d][1][entry_image(entry, 1)] - __ldg(s + Ns);
+    const double d2 = S.x[d][2][entry_image(entry, 2)] - __ldg(s + 2 * Ns);
+    const double q0 = __ldg(s + 3 * Ns), q1 = __ldg(s + 4 * Ns), q2 = __ldg(s + 5 * Ns);
+    double s2 = d0 * d0 + d1 * d1 + d2 * d2;
+    bool ok = live && s2 <= K.rcut2;
+    if (SKIP) {
+        const int sg = __float_as_int(__ldg(&srcP[j].w));
+        const int2 id = S.id[d];
+        ok = ok && sg != id.x && sg != id.y;
+    }
+    if (!ok) s2 = K.rcut2;
+    if (ok) ++ninr;
+    const double rinv = rsqrt_nr(s2);
+    int k;
+    const double t = tab_s_pos(K.alpha * (s2 * rinv), K.ntab_s, &k);
+    if (VEL) {
+        const double f = tab_s_poly(tab + (PSI ? K.ntab_s + k : k) * kTabSNC, t) * rinv * rinv * rinv;
+        if (ok) {
+            v[0] += f * (q1 * d2 - q2 * d1);
+            v[1] += f * (q2 * d0 - q0 * d2);
+            v[2] += f * (q0 * d1 - q1 * d0);
+        }
+    }
+    if (PSI) {
+        const double f = tab_s_poly(tab + k * kTabSNC, t) * rinv;
+        if (ok) {
+            w[0] += f * q0;
+            w[1] += f * q1;
+            w[2] += f * q2;
+        }
+    }
+}
+
+template <bool VEL, bool PSI, bool SKIP, int D, typename E>
+__global__ void __launch_bounds__(32 * kF64Warps, kF64Blocks) pair_f64_kernel(
+    KParams K, CellGrid cg, int64_t Np, float rc2s, const int32_t* __restrict__ dst_start,
+    const int32_t* __restrict__ dst_order, const double* __restrict__ nodes, const int32_t* __restrict__ idx_prev,
+    const float4* __restrict__ srcP, const double* __restrict__ src, int64_t Ns, const int32_t* __restrict__ src_start,
+    double* __restrict__ vel, double* __restrict__ psi,
+    unsigned long long* __restrict__ counters) {
+    extern __shared__ __align__(16) double tab[];  // weight tables: [weight][interval][kTabSNC]
+    __shared__ F64Warp<D, E> warps[kF64Warps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    {
+        constexpr int from = VEL && !PSI ? 1 : 0, nw = VEL && PSI ? 2 : 1;
+        const double2* s = reinterpret_cast<const double2*>(K.tab_s + (size_t)from * K.ntab_s * kTabSNC);
+        for (int k = threadIdx.x; k < nw * K.ntab_s * kTabSNC / 2; k += 32 * kF64Warps) reinterpret_cast<double2*>(tab)[k] = s[k];
+    }
+    __syncthreads();
+    F64Warp<D, E>& S = warps[warp];
+    const int64_t first = ((int64_t)blockIdx.x * kF64Warps + warp) * D;
+    const int64_t nvalid = dst_start[cg.ncell];  // nodes of the sentinel cell (non-finite) come after these
+    if (first >= nvalid) return;
+    const int nd = nvalid - first < D ? (int)(nvalid - first) : D;
+    const int M = cg.M, nc0 = cg.nc[0], nc1 = cg.nc[1], nc2 = cg.nc[2], W = 2 * M + 1;
+    double x[3] = {0.0, 0.0, 0.0};
+    int i = -1, cy = 0, cz = 0;
+    if (lane < nd) {
+        i = dst_order[first + lane];
+        S.id[lane] = make_int2(i, idx_prev[i]);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            x[d] = nodes[d * Np + i];
+#pragma unroll
+            for (int m = 0; m < 3; ++m) S.x[lane][d][m] = x[d] - (double)(m - 1) * K.L[d];
+        }
+        cy = cell_coord(x[1], K.L[1], nc1);
+        cz = cell_coord(x[2], K.L[2], nc2);
+    }
+    const float rc = (float)K.rcut;
+    // slack of the row and slab ranges, far above the FP32 rounding of places in the box
+    const float slack = 1e-5f * rc + 1e-6f * (float)fmax(K.L[0], fmax(K.L[1], K.L[2]));
+    const unsigned lanelt = (1u << lane) - 1u;
+    int ninr = 0;
+    unsigned ncand = 0;
+    double v[D][3], w[D][3];
+    int cnt[D];  // queued pairs per node (warp-uniform)
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        cnt[d] = 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[d][c] = w[d][c] = 0.0;
+    }
+    int turn = 0;  // rows seen so far: dealt to the gridDim.y warps of the group in turn
+    // the nodes of one (y, z) row of cells within r_cut in x at a time (nearly always all of them)
+    for (unsigned todo = __ballot_sync(0xffffffffu, lane < nd); todo;) {
+        const int lead = __ffs(todo) - 1;
+        const int gy_ = __shfl_sync(0xffffffffu, cy, lead), gz_ = __shfl_sync(0xffffffffu, cz, lead);
+        const double xlead = __shfl_sync(0xffffffffu, x[0], lead);
+        const bool mine = (todo >> lane & 1) && cy == gy_ && cz == gz_ && fabs(x[0] - xlead) <= K.rcut;
+        todo &= ~__ballot_sync(0xffffffffu, mine);
+        float lo[3], hi[3];
+        group_box<D>(mine, x, slack, lo, hi);
+        for (int r0 = 0; r0 < W * W; r0 += 32) {  // a lane per row of cells around the nodes' own
+        const RowRange R = near_row(cg, K, r0 + lane, gy_, gz_, lo, hi, slack);
+        for (int mx = 0; mx < 3; ++mx) {  // images in x: -L, 0, +L
+            const int s0 = max(R.klo - (mx - 1) * nc0, 0), s1 = min(R.khi - (mx - 1) * nc0, nc0 - 1);
+            int a = 0, b = 0;
+            if (s0 <= s1) {
+                a = src_start[R.row + s0];
+                b = src_start[R.row + s1 + 1];
+            }
+            for (unsigned rows = __ballot_sync(0xffffffffu, a < b); rows; rows &= rows - 1) {
+                const bool skip = turn % (int)gridDim.y != (int)blockIdx.y;  // warp-uniform
+                ++turn;
+                if (skip) continue;
+                const int sl = __ffs(rows) - 1;
+                const int ra = __shfl_sync(0xffffffffu, a, sl), rb = __shfl_sync(0xffffffffu, b, sl);
+                const int im = __shfl_sync(0xffffffffu, R.iyz, sl), my = im % 3, mz = im / 3;
+                __syncwarp();
+                if (lane < D) {
+                    const float px = mine ? (float)S.x[lane][0][mx] : kF32Far;
+                    float* xy = reinterpret_cast<float*>(S.xy2) + 4 * (lane >> 1) + (lane & 1);
+                    xy[0] = px;
+                    xy[2] = mine ? (float)S.x[lane][1][my] : kF32Far;
+                    reinterpret_cast<float*>(S.z2)[lane] = mine ? (float)S.x[lane][2][mz] : kF32Far;
+                }
+                __syncwarp();
+                ncand += (unsigned)(rb - ra) * D;
+                const E code = (E)(mx | my << 2 | mz << 4) << kIndexBits<E>;
+                float4 pn = __ldg(srcP + min(ra + lane, rb - 1));
+                for (int base = ra; base < rb; base += 32) {
+                    const int t = base + lane;
+                    float4 p = pn;
+                    pn = __ldg(srcP + min(t + 32, rb - 1));
+                    if (t >= rb) p.x = -kF32Far;
+                    const f32x2 px = dup2(-p.x), py = dup2(-p.y), pz = dup2(-p.z);
+                    const E entry = (E)t | code;
+#pragma unroll
+                    for (int h = 0; h < D / 2; ++h) {
+                        const ulonglong2 xy = S.xy2[h];
+                        const f32x2 e0 = add2(xy.x, px), e1 = add2(xy.y, py), e2 = add2(S.z2[h], pz);
+                        const f32x2 r2 = fma2(e0, e0, fma2(e1, e1, mul2(e2, e2)));
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int d = 2 * h + u;
+                            const bool in = half2f(r2, u) <= rc2s;
+                            const unsigned m = __ballot_sync(0xffffffffu, in);
+                            if (m == 0) continue;  // warp-uniform
+                            if (in) S.queue[d][cnt[d] + __popc(m & lanelt)] = entry;
+                            cnt[d] += __popc(m);
+                            if (cnt[d] >= 32) {
+                                __syncwarp();
+                                f64_eval<VEL, PSI, SKIP, D, E>(K, S, d, lane, true, srcP, src, Ns, tab, v[d], w[d], ninr);
+                                cnt[d] -= 32;
+                                __syncwarp();
+                                if (lane < cnt[d]) S.queue[d][lane] = S.queue[d][32 + lane];
+                                __syncwarp();
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        if (cnt[d] > 0)  // warp-uniform
+            f64_eval<VEL, PSI, SKIP, D, E>(K, S, d, lane < cnt[d] ? lane : 0, lane < cnt[d], srcP, src, Ns, tab, v[d], w[d], ninr);
+    const double pref = K.Gamma / (4.0 * kPi);
+    const int slot = lane / (32 / D);
+    const int is = __shfl_sync(0xffffffffu, i, slot);
+    double out[3];
+    if (VEL) {
+        group_reduce<D>(v, lane, out);
+        if (lane % (32 / D) == 0 && is >= 0)
+            for (int c = 0; c < 3; ++c) atomicAdd(&vel[c * Np + is], pref * out[c]);
+    }
+    if (PSI) {
+        group_reduce<D>(w, lane, out);
+        if (lane % (32 / D) == 0 && is >= 0)
+            for (int c = 0; c < 3; ++c) atomicAdd(&psi[c * Np + is], pref * out[c]);
     }
     const unsigned long long total = warp_sum_u((unsigned long long)ninr);
     if (lane == 0) {
@@ -1309,8 +1200,10 @@ int build_cell_lists(vpbs_handle* h) {
     if ((rc = ensure(h, h->dst_start, sizeof(int32_t) * (ncell + 2), "dst_start"))) return rc;
     if ((rc = ensure(h, h->dst_fill, sizeof(int32_t) * (ncell + 1), "dst_counts"))) return rc;
     if ((rc = ensure(h, h->dst_order, sizeof(int32_t) * Np, "dst_order"))) return rc;
-    const bool f32 = use_f32_pairs(h);
-    if (f32 && (rc = ensure(h, h->src_f32, (2 * sizeof(float4) + sizeof(float2)) * Nq, "FP32 sources"))) return rc;
+    // FP32 sources of the pair kernels: the places (screen), and for the mixed form all of them
+    const int f32 = use_f32_pairs(h) ? 2 : h->cg.M > 0 ? 1 : 0;
+    const size_t f32_size = f32 == 2 ? 2 * sizeof(float4) + sizeof(float2) : f32 ? sizeof(float4) : 0;
+    if (f32 && (rc = ensure(h, h->src_f32, f32_size * Nq, "FP32 sources"))) return rc;
     int32_t* scell = (int32_t*)h->src_cell.p;
     int32_t* srank = scell + Nq;
     int32_t* dcell = (int32_t*)h->dst_cell.p;
@@ -1331,7 +1224,7 @@ int build_cell_lists(vpbs_handle* h) {
     scatter_sources_kernel<<<grid_for(Nq, 256), 256, 0, h->stream>>>(
         Nq, h->K.nquad, (const double*)h->points.p, (const double*)h->charges.p, scell, srank,
         (const int32_t*)h->src_start.p, (double*)h->src_sorted.p, (int32_t*)h->src_seg.p,
-        f32 ? (float4*)h->src_f32.p : nullptr);
+        (float4*)h->src_f32.p, f32);
     scatter_nodes_kernel<<<grid_for(Np, 256), 256, 0, h->stream>>>(Np, dcell, drank, (const int32_t*)h->dst_start.p,
                                                                    (int32_t*)h->dst_order.p);
     h->launches += 4;  // plus the scans, counted by exclusive_scan
@@ -1490,13 +1383,10 @@ int exclusive_scan(vpbs_handle* h, const int32_t* counts, int32_t* start, int64_
     return check_cuda(h, cudaGetLastError(), "scan kernels");
 }
 
-// The FP32 pair kernel serves the mixed form with cell lists of M <= 2 (a lane per row) and weight tables
-// that fit; it reads FP32 copies of the sources that the cell sort writes.
+// The FP32 pair kernel serves the mixed form with cell lists and weight tables that fit.
 static bool use_f32_pairs(const vpbs_handle* h) {
-    const int W = 2 * h->cg.M + 1;
     return h->P.precision == VPBS_PRECISION_MIXED && !h->K.open_domain && !h->K.avoid_explicit_erf && h->K.alpha > 0 &&
-           h->cg.M > 0 && W * W <= 32 && h->K.ewald_ntab > 0 && h->K.ntab_c > 0 && h->K.ntab_c <= kF32TabMax &&
-           h->Nq < (int64_t)1 << kF32IndexBits;
+           h->cg.M > 0 && h->K.ntab_c > 0 && h->K.ntab_c <= kF32TabMax;
 }
 
 int pair_interactions(vpbs_handle* h, int fields) {
@@ -1530,80 +1420,51 @@ int pair_interactions(vpbs_handle* h, int fields) {
         h->launches++;
         return check_cuda(h, cudaGetLastError(), "open-domain pair kernel");
     }
-    const CellGrid& cg = h->cg;
-    const int Wc = 2 * cg.M + 1;
-    if (use_f32_pairs(h)) {
+    const size_t tab_bytes = sizeof(double) * kTabSNC * h->K.ntab_s * (v && p ? 2 : 1);
+    if (h->cg.M > 0 && (use_f32_pairs(h) || tab_bytes <= kPairSmemMost)) {
         int nsm = 148;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-        const int D = v && p ? 2 : 4;
-        const unsigned nblk = grid_for(Np, D * kF32Warps);
-        // a group's rows are shared out where the groups are fewer than the 32 warps an SM holds (1400 nodes:
-        // 25 us with 9 parts)
-        const unsigned nparts = (unsigned)std::max(1, std::min(Wc * Wc, (int)((32 * nsm + nblk - 1) / nblk / kF32Warps)));
-        // screen margin: the hi parts of places in the box are rounded to 2^-25 of its size
+        const bool f32 = use_f32_pairs(h), big = Nq >= (int64_t)1 << kIndexBits<uint32_t>;
+        const int Wc = 2 * h->cg.M + 1, D = v && p ? 2 : 4, warps = f32 ? kF32Warps : kF64Warps;
+        const unsigned nblk = grid_for(Np, D * warps);
+        // a group's rows are shared out where the groups are fewer than the 32 warps an SM holds (1400 nodes,
+        // mixed: 25 us with 9 parts)
+        const unsigned nparts = (unsigned)std::max(1, std::min(Wc * Wc, (int)((32 * nsm + nblk - 1) / nblk / warps)));
+        // screen margin: the FP32 places in the box are rounded to 2^-25 of its size
         const double Lmax = std::fmax(h->K.L[0], std::fmax(h->K.L[1], h->K.L[2]));
         const float rc2s = (float)(h->K.rcut2 * (1.0 + kScreenMargin + 1e-6 * Lmax / h->K.rcut));
+        const float4* srcP = (const float4*)h->src_f32.p;
         auto launch_f32 = [&](auto kern) {
             kern<<<dim3(nblk, nparts), 32 * kF32Warps, 0, h->stream>>>(
                 h->K, h->cg, Np, rc2s, (const int32_t*)h->dst_start.p, (const int32_t*)h->dst_order.p,
-                (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p, (const float4*)h->src_f32.p,
-                (const float4*)h->src_f32.p + Nq, (const float2*)((const float4*)h->src_f32.p + 2 * Nq),
+                (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p, srcP, srcP + Nq, (const float2*)(srcP + 2 * Nq),
                 (const int32_t*)h->src_start.p, (double*)h->vel.p, (double*)h->psi.p, (unsigned long long*)h->counters.p);
         };
-        if (v && p) launch_f32(pair_f32_kernel<true, true, 2>);
-        else if (v) launch_f32(pair_f32_kernel<true, false, 4>);
-        else launch_f32(pair_f32_kernel<false, true, 4>);
-        h->launches++;
-        return check_cuda(h, cudaGetLastError(), "FP32 pair kernel");
-    }
-    if ( cg.M > 0 && Wc * Wc <= kMaxRows && Wc * Wc * Wc * cg.G <= kMaxNbCells &&
-        sizeof(TileSmem<1024>) + 2 * sizeof(double) * kTabSNC * h->K.ntab_s <= kPairSmemMost) {
-        // blocks of Bc^3 cells per CTA, grown while a block holds fewer than ~24 nodes on average,
-        // at least 16 CTAs per SM remain, and the neighbourhood fits the shared-memory tables and
-        // stays inside one period
-        const int ncc = cg.nc[0] / cg.G;
-        const double ncoarse = (double)ncc * cg.nc[1] * cg.nc[2];
-        const double per_cell = (double)Np / ncoarse;
-        int nsm = 148;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-        auto fits = [&](int nb) {
-            const int w = nb + 2 * cg.M;
-            return w <= ncc && w <= cg.nc[1] && w <= cg.nc[2] && w * w <= kMaxRows && w * w * w * cg.G <= kMaxNbCells &&
-                   nb * nb <= kMaxBlockRows;
-        };
-        int Bc = 1;
-        if (h->pair_block > 0 && fits(h->pair_block)) {
-            Bc = h->pair_block;  // chosen by vpbs_autotune
-        } else {
-            while (Bc * Bc * Bc * per_cell < 24.0 && fits(Bc + 1) &&
-                   ncoarse / ((double)(Bc + 1) * (Bc + 1) * (Bc + 1)) >= 16.0 * nsm)
-                ++Bc;
-        }
-        const int3 bk = make_int3(Bc, Bc, Bc);
-        const int3 nb = make_int3((ncc + Bc - 1) / Bc, (cg.nc[1] + Bc - 1) / Bc, (cg.nc[2] + Bc - 1) / Bc);
-        const unsigned nblocks = (unsigned)((int64_t)nb.x * nb.y * nb.z);
-        // several CTAs share a block's nodes where there are few blocks (two CTAs run on an SM at a time)
-        const double per_block = per_cell * Bc * Bc * Bc;
-        const unsigned nparts = (unsigned)std::max(1.0, std::min({std::ceil(8.0 * nsm / nblocks), std::ceil(per_block / 8.0), 64.0}));
-        auto launch_tiled = [&](auto kern, bool vel, bool psi) {
-            const size_t smem = (vel && psi ? sizeof(TileSmem<tile_sources(true, true)>) : sizeof(TileSmem<tile_sources(true, false)>)) +
-                                sizeof(double) * kTabSNC * h->K.ntab_s * (vel && psi ? 2 : 1);
+        auto launch_f64 = [&](auto kern) {
             // the most a table can need, not this handle's: the attribute belongs to the function
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemMost);
-            kern<<<dim3(nblocks, nparts), kPairThreads, smem, h->stream>>>(
-                h->K, h->cg, Np, Nq, (const int32_t*)h->dst_start.p, (const int32_t*)h->dst_order.p,
-                (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p, (const double*)h->src_sorted.p,
-                (const int32_t*)h->src_start.p, (const int32_t*)h->src_seg.p, (double*)h->vel.p, (double*)h->psi.p,
-                (unsigned long long*)h->counters.p, bk, nb);
+            kern<<<dim3(nblk, nparts), 32 * kF64Warps, tab_bytes, h->stream>>>(
+                h->K, h->cg, Np, rc2s, (const int32_t*)h->dst_start.p, (const int32_t*)h->dst_order.p,
+                (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p, srcP, (const double*)h->src_sorted.p, Nq,
+                (const int32_t*)h->src_start.p, (double*)h->vel.p, (double*)h->psi.p, (unsigned long long*)h->counters.p);
         };
-        auto by_fields = [&](auto skip) {
+        auto by_fields = [&](auto entry, auto skip) {
+            using E = decltype(entry);
             constexpr bool SK = decltype(skip)::value;
-            if (v && p) launch_tiled(pair_cell_kernel<true, true, SK>, true, true);
-            else if (v) launch_tiled(pair_cell_kernel<true, false, SK>, true, false);
-            else launch_tiled(pair_cell_kernel<false, true, SK>, false, true);
+            if (f32) {
+                if (v && p) launch_f32(pair_f32_kernel<true, true, 2, E>);
+                else if (v) launch_f32(pair_f32_kernel<true, false, 4, E>);
+                else launch_f32(pair_f32_kernel<false, true, 4, E>);
+            } else {
+                if (v && p) launch_f64(pair_f64_kernel<true, true, SK, 2, E>);
+                else if (v) launch_f64(pair_f64_kernel<true, false, SK, 4, E>);
+                else launch_f64(pair_f64_kernel<false, true, SK, 4, E>);
+            }
         };
-        if (skip_local) by_fields(std::true_type{});
-        else by_fields(std::false_type{});
+        if (big && skip_local) by_fields(uint64_t(), std::true_type{});
+        else if (big) by_fields(uint64_t(), std::false_type{});
+        else if (skip_local) by_fields(uint32_t(), std::true_type{});
+        else by_fields(uint32_t(), std::false_type{});
         h->launches++;
         return check_cuda(h, cudaGetLastError(), "pair kernel");
     }

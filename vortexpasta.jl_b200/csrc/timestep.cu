@@ -6,7 +6,7 @@
 //    synchronisation or allocation after the first call, so a step can be captured in a graph;
 //  * vpbs_ensemble_*: independent systems advanced together, each on its own stream; one RK4
 //    step of every system is captured in one CUDA graph and replayed with one launch per step;
-//  * vpbs_autotune: picks the pair kernel's cells per CTA edge by timing the candidates.
+//  * vpbs_autotune_spread: picks the spreading mode by timing the candidates.
 #include <string>
 #include <vector>
 
@@ -189,42 +189,8 @@ void* vpbs_ensemble_stream(vpbs_ensemble* e) { return e ? (void*)e->origin : nul
 int vpbs_autotune(vpbs_handle* h, int32_t* chosen) {
     if (!h) return VPBS_ERR_ARG;
     if (!h->have_points) return set_error(h, VPBS_ERR_STATE, "vpbs_autotune needs point data");
-    if (h->K.open_domain || h->cg.M < 1) {
-        if (chosen) *chosen = 0;
-        return 0;  // no cell lists: nothing to tune
-    }
-    int rc;
-    if ((rc = check_cuda(h, cudaSetDevice(h->device), "cudaSetDevice"))) return rc;
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    const bool timing = h->timing;
-    h->timing = false;
-    float best = 1e30f;
-    int best_b = 0;
-    for (int b = 0; b <= 4 && !rc; ++b) {  // b = 0: the built-in rule
-        h->pair_block = b;
-        float tmin = 1e30f;
-        for (int rep = 0; rep < 3 && !rc; ++rep) {
-            cudaEventRecord(e0, h->stream);
-            rc = pair_interactions(h, VPBS_VELOCITY);
-            cudaEventRecord(e1, h->stream);
-            if (!rc) rc = check_cuda(h, cudaEventSynchronize(e1), "autotune sync");
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            if (rep > 0) tmin = fminf(tmin, ms);
-        }
-        if (!rc && tmin < best * 0.97f) {  // keep the simpler choice unless clearly faster
-            best = tmin;
-            best_b = b;
-        }
-    }
-    h->pair_block = best_b;
-    h->timing = timing;
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    if (chosen) *chosen = best_b;
-    return rc;
+    if (chosen) *chosen = 0;  // the pair kernels work per group of nodes: no block size to choose
+    return 0;
 }
 
 int vpbs_autotune_spread(vpbs_handle* h, int32_t* chosen) {
@@ -270,9 +236,7 @@ int vpbs_autotune_spread(vpbs_handle* h, int32_t* chosen) {
 }
 
 int vpbs_pair_block(vpbs_handle* h, int32_t cells) {
-    if (!h || cells < 0 || cells > 8) return VPBS_ERR_ARG;
-    h->pair_block = cells;
-    return 0;
+    return !h || cells < 0 || cells > 8 ? VPBS_ERR_ARG : 0;
 }
 
 }  // extern "C"

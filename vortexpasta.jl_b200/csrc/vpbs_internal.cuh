@@ -234,8 +234,6 @@ struct vpbs_handle {
     int64_t nmax = 0;
     bool have_filaments = false;
     vpbs::DevBuf rk_vs, rk_tmp;
-    // pair-kernel cells per CTA edge chosen by vpbs_autotune (0: the built-in rule)
-    int pair_block = 0;
 
     // optional per-stage CUDA-event timing (vpbs_stage_timing)
     bool timing = false;

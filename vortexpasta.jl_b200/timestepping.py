@@ -53,7 +53,7 @@ def rk4_step(cache: BiotSavartCache, nodes_ptr: int, dt: float) -> None:
 
 
 def autotune(cache: BiotSavartCache) -> int:
-    """Pick the pair kernel's cells per CTA edge for the loaded point data (0: built-in rule)."""
+    """Pair-kernel block choice for the loaded point data (0: the built-in rule, the only one)."""
     b = ct.c_int32()
     _lib.check(cache._lib.vpbs_autotune(cache.handle, ct.byref(b)), cache.handle, "autotune")
     return int(b.value)
