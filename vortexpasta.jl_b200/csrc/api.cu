@@ -360,8 +360,8 @@ int vpbs_destroy(vpbs_handle* h) {
     longrange_free(h);
     DevBuf* bufs[] = {&h->nodes_in, &h->offsets, &h->fil_of_node, &h->knots, &h->coefs, &h->dcoef1, &h->dcoef2,
                       &h->spline_scratch, &h->nodes, &h->idx_prev, &h->d1, &h->d2, &h->dm, &h->dp, &h->points,
-                      &h->charges, &h->li_vel, &h->li_psi, &h->src_cell, &h->src_start, &h->src_fill, &h->src_sorted,
-                      &h->src_seg, &h->src_f32, &h->dst_cell, &h->dst_start, &h->dst_fill, &h->dst_order, &h->counters,
+                      &h->charges, &h->li_vel, &h->li_psi, &h->src_cell, &h->cell_start, &h->cell_counts, &h->src_sorted,
+                      &h->src_seg, &h->src_f32, &h->dst_order, &h->counters,
                       &h->grid_r, &h->grid_c, &h->grid_c2, &h->uhat, &h->decx, &h->decy, &h->decz, &h->nodes_lr,
                       &h->vel, &h->psi, &h->spread_bin, &h->spread_counts, &h->spread_start, &h->binned,
                       &h->spread_foot, &h->tc_counts, &h->tc_start, &h->tc_rec, &h->peer_in, &h->ewald_tab, &h->scan_tmp, &h->scan_tmp_lr, &h->rk_vs, &h->rk_tmp,
@@ -718,9 +718,10 @@ int vpbs_compute(vpbs_handle* h, int32_t fields, int32_t lia_mode, int32_t short
     int rc;
     if ((rc = activate(h))) return rc;
     const int64_t Np = h->Np;
-    if (fields & VPBS_VELOCITY)
+    // the local term is the first to write the outputs; without the short range they start from zero
+    if ((fields & VPBS_VELOCITY) && !shortrange)
         if ((rc = check_cuda(h, cudaMemsetAsync(h->vel.p, 0, sizeof(double) * 3 * Np, h->stream), "memset"))) return rc;
-    if (fields & VPBS_STREAMFUNCTION)
+    if ((fields & VPBS_STREAMFUNCTION) && !shortrange)
         if ((rc = check_cuda(h, cudaMemsetAsync(h->psi.p, 0, sizeof(double) * 3 * Np, h->stream), "memset"))) return rc;
     const bool with_long = longrange && lia_mode != VPBS_LIA_ONLY && !h->K.open_domain;
     // The long range (spread, FFTs, Fourier operators) runs on the auxiliary stream while the

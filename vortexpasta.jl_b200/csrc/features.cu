@@ -144,7 +144,7 @@ extern "C" int vpbs_features(vpbs_handle* h, float* out, int32_t n) {
     const int64_t nsample = (Np + stride - 1) / stride;
     nearest_hist_kernel<<<grid_for(nsample, 8), 256, 0, h->stream>>>(
         h->K, h->cg, Np, stride, (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p,
-        (const double*)h->src_sorted.p, h->Nq, (const int32_t*)h->src_start.p, (const int32_t*)h->src_seg.p, hist);
+        (const double*)h->src_sorted.p, h->Nq, h->src_start, (const int32_t*)h->src_seg.p, hist);
     h->launches += 2;
     double hsum = 0;
     unsigned int hmin = 0, hh[kHistBins];

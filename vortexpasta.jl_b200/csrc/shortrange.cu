@@ -50,20 +50,26 @@ __device__ __forceinline__ int64_t cell_of(const CellGrid& cg, const KParams& K,
     return cell_index(cg.nc, K.L, x, y, z);
 }
 
-// Cell of every element and its rank within the cell (atomic counter).
-__global__ void cell_count_kernel(KParams K, CellGrid cg, int64_t n, const double* __restrict__ xyz,
-                                  int32_t* __restrict__ cell, int32_t* __restrict__ rank,
+// Cell of every quadrature point and node and its rank within the cell (atomic counters).  The nodes'
+// entries follow the points' in every array; their threads start at a whole warp, so that no warp counts
+// both.
+__global__ void cell_count_kernel(KParams K, CellGrid cg, int64_t Nq, int64_t Np, const double* __restrict__ points,
+                                  const double* __restrict__ nodes, int32_t* __restrict__ cell, int32_t* __restrict__ rank,
                                   int32_t* __restrict__ counts) {
-    int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    int64_t c = cell_of(cg, K, xyz[j], xyz[n + j], xyz[2 * n + j]);
-    cell[j] = (int32_t)c;
-    rank[j] = warp_aggregated_rank(counts, (int32_t)c);
+    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, j0 = (Nq + 31) & ~(int64_t)31;
+    if ((j >= Nq && j < j0) || j >= j0 + Np) return;
+    const bool node = j >= j0;
+    const int64_t k = node ? j - j0 : j, n = node ? Np : Nq, e = node ? Nq + k : k;
+    const double* xyz = node ? nodes : points;
+    const int32_t c = (int32_t)cell_of(cg, K, xyz[k], xyz[n + k], xyz[2 * n + k]);
+    cell[e] = c;
+    rank[e] = warp_aggregated_rank(node ? counts + cg.ncell + 1 : counts, c);
 }
 
-// Exclusive scan of counts[0..n) into start[0..n] with one CTA of 1024 threads.
+// Exclusive scan of counts[0..n) into start[0..n] with one CTA of 1024 threads; `sub` is subtracted from
+// start[split] on (two arrays scanned as one).
 __global__ void __launch_bounds__(1024) scan_kernel(const int32_t* __restrict__ counts, int32_t* __restrict__ start,
-                                                    int64_t n) {
+                                                    int64_t n, int64_t split, int32_t sub) {
     __shared__ int32_t part[1024];
     const int tid = threadIdx.x;
     const int64_t chunk = (n + 1023) / 1024;
@@ -81,10 +87,10 @@ __global__ void __launch_bounds__(1024) scan_kernel(const int32_t* __restrict__ 
     }
     int32_t acc = part[tid] - s;  // exclusive prefix of this chunk
     for (int64_t i = lo; i < hi; ++i) {
-        start[i] = acc;
+        start[i] = acc - (i >= split ? sub : 0);
         acc += counts[i];
     }
-    if (tid == 1023) start[n] = part[1023];
+    if (tid == 1023) start[n] = part[1023] - (n >= split ? sub : 0);
 }
 
 // Multi-CTA exclusive scan for long count arrays: per-chunk sums, a scan of the sums (with
@@ -123,7 +129,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_partials_kernel(const int32
 
 __global__ void __launch_bounds__(kScanThreads) scan_chunks_kernel(const int32_t* __restrict__ counts, int64_t n,
                                                                   const int32_t* __restrict__ part_start,
-                                                                  int32_t* __restrict__ start) {
+                                                                  int32_t* __restrict__ start, int64_t split, int32_t sub) {
     __shared__ int wt[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t base = (int64_t)blockIdx.x * kScanChunk + (int64_t)threadIdx.x * kScanPer;
@@ -141,21 +147,27 @@ __global__ void __launch_bounds__(kScanThreads) scan_chunks_kernel(const int32_t
     int acc = part_start[blockIdx.x] + (warp > 0 ? wt[warp - 1] : 0) + x - s;
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
-        if (base + k < n) start[base + k] = acc;
+        if (base + k < n) start[base + k] = acc - (base + k >= split ? sub : 0);
         acc += c[k];
     }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) start[n] = part_start[gridDim.x];
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) start[n] = part_start[gridDim.x] - (n >= split ? sub : 0);
 }
 
-// Scatter the sources into cell order (SoA: x, y, z, qx, qy, qz) and record their segment.
-__global__ void scatter_sources_kernel(int64_t Nq, int nquad, const double* __restrict__ points,
+// Scatter the sources into cell order (SoA: x, y, z, qx, qy, qz) and record their segment; list the nodes in
+// cell order.
+__global__ void scatter_kernel(int64_t Nq, int64_t Np, int nquad, const double* __restrict__ points,
                                        const double* __restrict__ charges, const int32_t* __restrict__ cell,
                                        const int32_t* __restrict__ rank, const int32_t* __restrict__ start,
                                        double* __restrict__ sorted, int32_t* __restrict__ seg,
-                                       float4* __restrict__ f32, int f32_parts) {
+                                       float4* __restrict__ f32, int f32_parts, const int32_t* __restrict__ dst_start,
+                               int32_t* __restrict__ order) {
     int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= Nq) return;
-    int64_t pos = (int64_t)start[cell[j]] + rank[j];
+    if (j >= Nq + Np) return;
+    if (j >= Nq) {
+        order[(int64_t)dst_start[cell[j]] + rank[j]] = (int32_t)(j - Nq);
+        return;
+    }
+    const int64_t pos = (int64_t)start[cell[j]] + rank[j];
     double x[3], q[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -174,13 +186,6 @@ __global__ void scatter_sources_kernel(int64_t Nq, int nquad, const double* __re
         f32[Nq + pos] = make_float4((float)(x[0] - h0), (float)(x[1] - h1), (float)(x[2] - h2), (float)q[0]);
         reinterpret_cast<float2*>(f32 + 2 * Nq)[pos] = make_float2((float)q[1], (float)q[2]);
     }
-}
-
-__global__ void scatter_nodes_kernel(int64_t Np, const int32_t* __restrict__ cell, const int32_t* __restrict__ rank,
-                                     const int32_t* __restrict__ start, int32_t* __restrict__ order) {
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= Np) return;
-    order[(int64_t)start[cell[i]] + rank[i]] = (int32_t)i;
 }
 
 // Per-lane accumulators in the evaluation precision R; in FP32 they are Kahan-compensated
@@ -1074,7 +1079,7 @@ __global__ void __launch_bounds__(32 * kF64Warps, kF64Blocks) pair_f64_kernel(
     }
 }
 
-// Local term (overwrites nothing: adds into the zeroed outputs), self-interaction removal
+// Local term (the first to write the outputs), self-interaction removal
 // and, when lia_segment_fraction is set, the local integrals over the excluded sub-segments.
 __global__ void __launch_bounds__(128) local_self_kernel(
     KParams K, int64_t Np, int fields, int do_local, int do_self, int do_li, double rv, double rpsi,
@@ -1157,13 +1162,13 @@ __global__ void __launch_bounds__(128) local_self_kernel(
         }
     }
     if (want_v)
-        for (int d = 0; d < 3; ++d) vel[d * Np + i] += v[d];
+        for (int d = 0; d < 3; ++d) vel[d * Np + i] = v[d];
     if (want_p) {
         // streamfunction of the uniform background vorticity of unclosed filaments (zero otherwise)
         p[0] += psi_bg.x;
         p[1] += psi_bg.y;
         p[2] += psi_bg.z;
-        for (int d = 0; d < 3; ++d) psi[d * Np + i] += p[d];
+        for (int d = 0; d < 3; ++d) psi[d * Np + i] = p[d];
     }
 }
 
@@ -1190,44 +1195,34 @@ int build_cell_lists(vpbs_handle* h) {
     }
     const int64_t Np = h->Np, Nq = h->Nq, ncell = h->cg.ncell;
     int rc;
-    if ((rc = ensure(h, h->src_cell, sizeof(int32_t) * 2 * Nq, "src_cell"))) return rc;
-    // ncell + 1 cells: the last one is the sentinel of points with non-finite coordinates
-    if ((rc = ensure(h, h->src_start, sizeof(int32_t) * (ncell + 2), "src_start"))) return rc;
-    if ((rc = ensure(h, h->src_fill, sizeof(int32_t) * (ncell + 1), "src_counts"))) return rc;
+    // the nodes' cells, counts and starts follow the points' in the same arrays: one pass and one scan for both
+    const int64_t n = Nq + Np, nscan = 2 * (ncell + 1);
+    if ((rc = ensure(h, h->src_cell, sizeof(int32_t) * 2 * n, "cells"))) return rc;
+    // ncell + 1 cells each: the last one is the sentinel of points with non-finite coordinates
+    if ((rc = ensure(h, h->cell_start, sizeof(int32_t) * (nscan + 1), "cell starts"))) return rc;
+    if ((rc = ensure(h, h->cell_counts, sizeof(int32_t) * nscan, "cell counts"))) return rc;
     if ((rc = ensure(h, h->src_sorted, sizeof(double) * 6 * Nq, "src_sorted"))) return rc;
     if ((rc = ensure(h, h->src_seg, sizeof(int32_t) * Nq, "src_seg"))) return rc;
-    if ((rc = ensure(h, h->dst_cell, sizeof(int32_t) * 2 * Np, "dst_cell"))) return rc;
-    if ((rc = ensure(h, h->dst_start, sizeof(int32_t) * (ncell + 2), "dst_start"))) return rc;
-    if ((rc = ensure(h, h->dst_fill, sizeof(int32_t) * (ncell + 1), "dst_counts"))) return rc;
     if ((rc = ensure(h, h->dst_order, sizeof(int32_t) * Np, "dst_order"))) return rc;
     // FP32 sources of the pair kernels: the places (screen), and for the mixed form all of them
     const int f32 = use_f32_pairs(h) ? 2 : h->cg.M > 0 ? 1 : 0;
     const size_t f32_size = f32 == 2 ? 2 * sizeof(float4) + sizeof(float2) : f32 ? sizeof(float4) : 0;
     if (f32 && (rc = ensure(h, h->src_f32, f32_size * Nq, "FP32 sources"))) return rc;
-    int32_t* scell = (int32_t*)h->src_cell.p;
-    int32_t* srank = scell + Nq;
-    int32_t* dcell = (int32_t*)h->dst_cell.p;
-    int32_t* drank = dcell + Np;
+    int32_t* cell = (int32_t*)h->src_cell.p;
+    int32_t* rank = cell + n;
+    int32_t* counts = (int32_t*)h->cell_counts.p;
+    h->src_start = (int32_t*)h->cell_start.p;
+    h->dst_start = h->src_start + ncell + 1;
     StageScope st(h, ST_CELL_LISTS);
-    if ((rc = check_cuda(h, cudaMemsetAsync(h->src_fill.p, 0, sizeof(int32_t) * (ncell + 1), h->stream), "memset")))
-        return rc;
-    if ((rc = check_cuda(h, cudaMemsetAsync(h->dst_fill.p, 0, sizeof(int32_t) * (ncell + 1), h->stream), "memset")))
-        return rc;
-    cell_count_kernel<<<grid_for(Nq, 256), 256, 0, h->stream>>>(h->K, h->cg, Nq, (const double*)h->points.p, scell, srank,
-                                                                (int32_t*)h->src_fill.p);
-    cell_count_kernel<<<grid_for(Np, 256), 256, 0, h->stream>>>(h->K, h->cg, Np, (const double*)h->nodes.p, dcell, drank,
-                                                                (int32_t*)h->dst_fill.p);
-    if ((rc = exclusive_scan(h, (const int32_t*)h->src_fill.p, (int32_t*)h->src_start.p, ncell + 1, h->scan_tmp)))
-        return rc;
-    if ((rc = exclusive_scan(h, (const int32_t*)h->dst_fill.p, (int32_t*)h->dst_start.p, ncell + 1, h->scan_tmp)))
-        return rc;
-    scatter_sources_kernel<<<grid_for(Nq, 256), 256, 0, h->stream>>>(
-        Nq, h->K.nquad, (const double*)h->points.p, (const double*)h->charges.p, scell, srank,
-        (const int32_t*)h->src_start.p, (double*)h->src_sorted.p, (int32_t*)h->src_seg.p,
-        (float4*)h->src_f32.p, f32);
-    scatter_nodes_kernel<<<grid_for(Np, 256), 256, 0, h->stream>>>(Np, dcell, drank, (const int32_t*)h->dst_start.p,
-                                                                   (int32_t*)h->dst_order.p);
-    h->launches += 4;  // plus the scans, counted by exclusive_scan
+    if ((rc = check_cuda(h, cudaMemsetAsync(counts, 0, sizeof(int32_t) * nscan, h->stream), "memset"))) return rc;
+    cell_count_kernel<<<grid_for(n + 32, 256), 256, 0, h->stream>>>(h->K, h->cg, Nq, Np, (const double*)h->points.p,
+                                                               (const double*)h->nodes.p, cell, rank, counts);
+    if ((rc = exclusive_scan(h, counts, h->src_start, nscan, h->scan_tmp, ncell + 1, (int32_t)Nq))) return rc;
+    scatter_kernel<<<grid_for(n, 256), 256, 0, h->stream>>>(
+        Nq, Np, h->K.nquad, (const double*)h->points.p, (const double*)h->charges.p, cell, rank, h->src_start,
+        (double*)h->src_sorted.p, (int32_t*)h->src_seg.p, (float4*)h->src_f32.p, f32, h->dst_start,
+        (int32_t*)h->dst_order.p);
+    h->launches += 2;  // plus the scan, counted by exclusive_scan
     return check_cuda(h, cudaGetLastError(), "cell list kernels");
 }
 
@@ -1365,10 +1360,10 @@ void f32_table_eval_host(const float4* tabc, int nf, float x, float* a, float* g
     *g = f32_cubic(tabc[nf + k], t);
 }
 
-int exclusive_scan(vpbs_handle* h, const int32_t* counts, int32_t* start, int64_t n, DevBuf& tmp) {
+int exclusive_scan(vpbs_handle* h, const int32_t* counts, int32_t* start, int64_t n, DevBuf& tmp, int64_t split, int32_t sub) {
     const int64_t nblk = (n + kScanChunk - 1) / kScanChunk;
     if (nblk <= 1) {
-        scan_kernel<<<1, 1024, 0, h->stream>>>(counts, start, n);
+        scan_kernel<<<1, 1024, 0, h->stream>>>(counts, start, n, split, sub);
         h->launches++;
         return check_cuda(h, cudaGetLastError(), "scan kernel");
     }
@@ -1377,8 +1372,8 @@ int exclusive_scan(vpbs_handle* h, const int32_t* counts, int32_t* start, int64_
     int32_t* part = (int32_t*)tmp.p;
     int32_t* part_start = part + nblk;
     scan_partials_kernel<<<(unsigned)nblk, kScanThreads, 0, h->stream>>>(counts, n, part);
-    scan_kernel<<<1, 1024, 0, h->stream>>>(part, part_start, nblk);
-    scan_chunks_kernel<<<(unsigned)nblk, kScanThreads, 0, h->stream>>>(counts, n, part_start, start);
+    scan_kernel<<<1, 1024, 0, h->stream>>>(part, part_start, nblk, INT64_MAX, 0);
+    scan_chunks_kernel<<<(unsigned)nblk, kScanThreads, 0, h->stream>>>(counts, n, part_start, start, split, sub);
     h->launches += 3;
     return check_cuda(h, cudaGetLastError(), "scan kernels");
 }
@@ -1436,17 +1431,17 @@ int pair_interactions(vpbs_handle* h, int fields) {
         const float4* srcP = (const float4*)h->src_f32.p;
         auto launch_f32 = [&](auto kern) {
             kern<<<dim3(nblk, nparts), 32 * kF32Warps, 0, h->stream>>>(
-                h->K, h->cg, Np, rc2s, (const int32_t*)h->dst_start.p, (const int32_t*)h->dst_order.p,
+                h->K, h->cg, Np, rc2s, h->dst_start, (const int32_t*)h->dst_order.p,
                 (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p, srcP, srcP + Nq, (const float2*)(srcP + 2 * Nq),
-                (const int32_t*)h->src_start.p, (double*)h->vel.p, (double*)h->psi.p, (unsigned long long*)h->counters.p);
+                h->src_start, (double*)h->vel.p, (double*)h->psi.p, (unsigned long long*)h->counters.p);
         };
         auto launch_f64 = [&](auto kern) {
             // the most a table can need, not this handle's: the attribute belongs to the function
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemMost);
             kern<<<dim3(nblk, nparts), 32 * kF64Warps, tab_bytes, h->stream>>>(
-                h->K, h->cg, Np, rc2s, (const int32_t*)h->dst_start.p, (const int32_t*)h->dst_order.p,
+                h->K, h->cg, Np, rc2s, h->dst_start, (const int32_t*)h->dst_order.p,
                 (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p, srcP, (const double*)h->src_sorted.p, Nq,
-                (const int32_t*)h->src_start.p, (double*)h->vel.p, (double*)h->psi.p, (unsigned long long*)h->counters.p);
+                h->src_start, (double*)h->vel.p, (double*)h->psi.p, (unsigned long long*)h->counters.p);
         };
         auto by_fields = [&](auto entry, auto skip) {
             using E = decltype(entry);
@@ -1471,7 +1466,7 @@ int pair_interactions(vpbs_handle* h, int fields) {
     auto launch = [&](auto kern) {
         kern<<<grid, 256, 0, h->stream>>>(h->K, h->cg, Np, Nq, (const int32_t*)h->dst_order.p, (const double*)h->nodes.p,
                                           (const int32_t*)h->idx_prev.p, (const double*)h->src_sorted.p,
-                                          (const int32_t*)h->src_start.p, (const int32_t*)h->src_seg.p, h->cg.M == 0 ? 0 : 1,
+                                          h->src_start, (const int32_t*)h->src_seg.p, h->cg.M == 0 ? 0 : 1,
                                           skip_local, (double*)h->vel.p, (double*)h->psi.p,
                                           (unsigned long long*)h->counters.p);
     };

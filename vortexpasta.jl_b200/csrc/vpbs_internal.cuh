@@ -185,7 +185,8 @@ struct vpbs_handle {
 
     // cell lists
     vpbs::CellGrid cg{};
-    vpbs::DevBuf src_cell, src_start, src_fill, src_sorted, src_seg, src_f32, dst_cell, dst_start, dst_fill, dst_order;
+    vpbs::DevBuf src_cell, cell_start, cell_counts, src_sorted, src_seg, src_f32, dst_order;
+    int32_t *src_start = nullptr, *dst_start = nullptr;  // of the points' and the nodes' cells, in cell_start
     vpbs::DevBuf counters;  // [0] in-range pairs, [1] candidates (unsigned long long)
     vpbs::DevBuf scan_tmp, scan_tmp_lr;  // multi-CTA scan scratch (cell lists; spreading bins)
     vpbs::DevBuf ewald_tab;  // Taylor tables of the Ewald weights (KParams::ewald_tab)
@@ -262,8 +263,9 @@ CellGrid make_cell_grid(const double L[3], double rcut, int M);
 
 // shortrange.cu
 int build_cell_lists(vpbs_handle* h);
-int exclusive_scan(vpbs_handle* h, const int32_t* counts, int32_t* start, int64_t n,
-                   DevBuf& tmp);  // start[0..n]; tmp: scratch of the multi-CTA scan
+// start[0..n]; tmp: scratch of the multi-CTA scan; `sub` is subtracted from start[split] on
+int exclusive_scan(vpbs_handle* h, const int32_t* counts, int32_t* start, int64_t n, DevBuf& tmp,
+                   int64_t split = INT64_MAX, int32_t sub = 0);
 int local_and_self(vpbs_handle* h, int fields, int lia_mode, int with_pairs_self, double integration_cutoff);
 int pair_interactions(vpbs_handle* h, int fields);
 int add_local_integrals(vpbs_handle* h, int fields);
