@@ -204,8 +204,10 @@ __device__ __noinline__ bool solve_partitioned(const FilView& f, const double* t
     const unsigned full = 0xffffffffu;
     // collocation rows (cyclic): band[5 i + s] multiplies u_{i + s - 2}
     for (int i = lane; i < n; i += 32) {
+        SegBasis B;  // independent divisions, instead of five dependent levels of them
+        seg_basis_init(f, i, B);
         double N[6];
-        bsplvb<6>(f, i, knot_at(f, i), N);
+        bsplvb_seg<6>(B, B.t[4], N);
 #pragma unroll
         for (int s = 0; s < 5; ++s) band[5 * i + s] = N[s];
         const double r = t[i] / T;
@@ -508,34 +510,42 @@ __global__ void __launch_bounds__(128) spline_solve_kernel(
     double* c1 = dcoef1 + 3 * off;
     double* c2 = dcoef2 + 3 * off;
 
-    // 1. chordal knots: warp-wide inclusive scan of segment lengths (parametrisations.jl:43-44)
-    double carry = keep_knots ? periods[fidx] : 0.0;
-    for (int base = 0; base < n && !keep_knots; base += 32) {
-        int i = base + lane;
-        double len = 0.0;
-        if (i < n) {
-            int j = (i + 1 == n) ? 0 : i + 1;
+    // 1. chordal knots (parametrisations.jl:43-44): segment lengths into the work space, a run of them summed
+    // per lane, one warp-wide scan of the sums
+    double T = keep_knots ? periods[fidx] : 0.0;
+    if (!keep_knots) {
+#pragma unroll 4
+        for (int i = lane; i < n; i += 32) {
+            const int j = (i + 1 == n) ? 0 : i + 1;
             double dx = Xf[3 * j] - Xf[3 * i], dy = Xf[3 * j + 1] - Xf[3 * i + 1], dz = Xf[3 * j + 2] - Xf[3 * i + 2];
             if (j == 0 && foff) {  // closing segment of an unclosed filament: to X_0 + offset
                 dx += foff[3 * fidx];
                 dy += foff[3 * fidx + 1];
                 dz += foff[3 * fidx + 2];
             }
-            len = sqrt(dx * dx + dy * dy + dz * dz);
+            band[i] = sqrt(dx * dx + dy * dy + dz * dz);
             fil_of_node[off + i] = (int32_t)fidx;
         }
-        double incl = len;
+        __syncwarp();
+        const int a = (int)((int64_t)lane * n / 32), b = (int)((int64_t)(lane + 1) * n / 32);
+        double sum = 0.0;
+        for (int i = a; i < b; ++i) sum += band[i];
+        double incl = sum;
 #pragma unroll
         for (int s = 1; s < 32; s <<= 1) {
-            double v = __shfl_up_sync(0xffffffffu, incl, s);
+            const double v = __shfl_up_sync(0xffffffffu, incl, s);
             if (lane >= s) incl += v;
         }
-        if (i < n) t[i] = carry + (incl - len);  // exclusive prefix: t_i
-        carry += __shfl_sync(0xffffffffu, incl, 31);
+        T = __shfl_sync(0xffffffffu, incl, 31);
+        double acc = incl - sum;
+        if (lane == 0) acc = 0.0;
+        for (int i = a; i < b; ++i) {
+            t[i] = acc;
+            acc += band[i];
+        }
+        if (lane == 0) periods[fidx] = T;
+        __syncwarp();
     }
-    const double T = carry;
-    if (lane == 0 && !keep_knots) periods[fidx] = T;
-    __syncwarp();
     FilView f{t, T, n, {0.0, 0.0, 0.0}};
     // an unclosed filament is interpolated as the periodic y_i = X_i - (t_i / T) offset
     // (spline.jl:163-182, quintic.jl:9-17)
@@ -554,16 +564,16 @@ __global__ void __launch_bounds__(128) spline_solve_kernel(
     // 3. derivative coefficients (spline derivative recurrence, spline.jl:301-319)
     for (int j = lane; j < n; j += 32) {
         int jm = (j == 0) ? n - 1 : j - 1;
-        double den = knot_at(f, j + 5) - knot_at(f, j);
+        const double inv = 5.0 / (knot_at(f, j + 5) - knot_at(f, j));
 #pragma unroll
-        for (int d = 0; d < 3; ++d) c1[3 * j + d] = 5.0 * (c[3 * j + d] - c[3 * jm + d]) / den;
+        for (int d = 0; d < 3; ++d) c1[3 * j + d] = (c[3 * j + d] - c[3 * jm + d]) * inv;
     }
     __syncwarp();
     for (int j = lane; j < n; j += 32) {
         int jm = (j == 0) ? n - 1 : j - 1;
-        double den = knot_at(f, j + 4) - knot_at(f, j);
+        const double inv = 4.0 / (knot_at(f, j + 4) - knot_at(f, j));
 #pragma unroll
-        for (int d = 0; d < 3; ++d) c2[3 * j + d] = 4.0 * (c1[3 * j + d] - c1[3 * jm + d]) / den;
+        for (int d = 0; d < 3; ++d) c2[3 * j + d] = (c1[3 * j + d] - c1[3 * jm + d]) * inv;
     }
 }
 
