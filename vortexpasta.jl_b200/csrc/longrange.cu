@@ -1254,8 +1254,9 @@ int longrange_compute_t(vpbs_handle* h, int fields) {
     const vpbs_params& P = h->P;
     int rc;
     const double sx[3] = {2.0 * kPi / P.L[0], 2.0 * kPi / P.L[1], 2.0 * kPi / P.L[2]};
-    // interleaved components for the interpolation: the inverse transform writes a third more, the gathers of
-    // a node cost a third (1M nodes, m = 3, 288^3: +0.05 ms against -0.5 ms)
+    // interleaved components for the interpolation where many nodes share the grid's lines: the inverse transform
+    // writes a third more, the gathers of a node cost less (1M nodes, m = 3, 288^3, 9 footprint points per grid
+    // point: +0.02 ms against -0.38; 200k nodes, m = 4, 384^3, 1.8 per grid point: +0.10 against +0.03)
     const double footprints = (double)h->Np * 8.0 * S.m * S.m * S.m;
     const bool quad = std::is_same<T, float>::value && h->fplan && S.m <= 4 && footprints >= 4.0 * (double)S.ngrid;
     T* grid = (T*)h->grid_r.p;

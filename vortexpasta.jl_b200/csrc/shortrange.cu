@@ -874,11 +874,12 @@ __global__ void __launch_bounds__(32 * kF32Warps, sizeof(E) == 4 ? kF32Blocks : 
 // (cell-sorted arrays), decides r^2 <= r_cut^2 and evaluates in FP64 (Newton-refined reciprocal square root,
 // weights from degree-5 tables in shared memory, one copy per CTA).  SKIP: the node's own two segments left
 // out.  Bound: shared-memory and L1 wavefronts of the gathers (per 32 pairs about 30 for the weights' three
-// 16-byte loads and 30 for the sources), then the FP64 pipe (17 cycles).  1M nodes, 3.13 G pairs: 28.7 ms (CTAs
-// that stage tiles of a block's neighbourhood: 39.5); 20k nodes, both fields: 0.205 (0.517).  Two CTAs of 128
-// registers instead of three of 80: 30.6.
+// 16-byte loads and 30 for the sources), then the FP64 pipe (17 cycles).  1M nodes, 3.13 G pairs: 26.8 ms (CTAs
+// that stage tiles of a block's neighbourhood: 39.5); 20k nodes, both fields: 0.205 (0.517).  Three CTAs per SM of
+// 80 registers: 28.7, two of 128: 30.6; both fields in four of 64: 0.217.
 constexpr int kF64Warps = 8;
-constexpr int kF64Blocks = 3;  // CTAs per SM (80 registers)
+// CTAs per SM: 64 registers for one field (some spilled outside the loops), 80 for both
+__host__ __device__ constexpr int f64_blocks(bool both) { return both ? 3 : 4; }
 
 template <int D, typename E>
 struct F64Warp {
@@ -931,7 +932,7 @@ __device__ __forceinline__ void f64_eval(const KParams& K, const F64Warp<D, E>& 
 }
 
 template <bool VEL, bool PSI, bool SKIP, int D, typename E>
-__global__ void __launch_bounds__(32 * kF64Warps, kF64Blocks) pair_f64_kernel(
+__global__ void __launch_bounds__(32 * kF64Warps, f64_blocks(VEL && PSI)) pair_f64_kernel(
     KParams K, CellGrid cg, int64_t Np, float rc2s, const int32_t* __restrict__ dst_start,
     const int32_t* __restrict__ dst_order, const double* __restrict__ nodes, const int32_t* __restrict__ idx_prev,
     const float4* __restrict__ srcP, const double* __restrict__ src, int64_t Ns, const int32_t* __restrict__ src_start,
