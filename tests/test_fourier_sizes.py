@@ -11,10 +11,12 @@ import pytest
 
 L = 2 * math.pi
 
-# (Ns, sigma): FFT sizes 8 .. 768 per dimension, with 2, 3 and 4 passes, radices 2 .. 32
+# (Ns, sigma): FFT sizes 8 .. 2250 per dimension, with 2, 3 and 4 passes, radices 2 .. 32
 SIZES = [((6, 6, 6), 1.3), ((12, 17, 31), 1.5), ((32, 20, 18), 1.5), ((50, 30, 36), 1.5), ((33, 48, 40), 2.0),
          ((54, 100, 25), 1.25), ((120, 16, 12), 2.0), ((16, 160, 14), 1.5), ((14, 12, 192), 1.5), ((256, 12, 10), 1.5),
-         ((12, 256, 12), 1.5), ((10, 14, 256), 1.5), ((20, 12, 512), 1.5), ((400, 10, 12), 1.25), ((12, 10, 500), 1.25)]
+         ((12, 256, 12), 1.5), ((10, 14, 256), 1.5), ((20, 12, 512), 1.5), ((400, 10, 12), 1.25), ((12, 10, 500), 1.25),
+         # tiles of one line; lines too long for a block and a packed length of one factor (cuFFT)
+         ((12, 10, 1360), 1.5), ((12, 10, 1500), 1.5), ((6, 12, 10), 1.5)]
 
 
 def system(vp):
