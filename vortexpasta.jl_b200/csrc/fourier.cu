@@ -15,6 +15,8 @@
 //
 // Bound: HBM traffic of the passes (sigma = 1.5: 4.3 grids of real values in all, against 8 for the
 // unpruned transforms plus 1.3 for a separate operator pass), then shared-memory and issue rate.
+// Against cuFFT and the separate operator kernel: 768^3 FP64 59.0 -> 29.3 ms when first measured, 25 since;
+// 384^3 FP32, four evaluations, 13.1 -> 5.8 ms; 288^3 FP32 1.39 -> 0.73 ms.
 #include <algorithm>
 #include <cmath>
 #include <vector>

@@ -2,14 +2,14 @@
 // longrange/backends/nonuniformffts.jl):
 //  1. type-1 NUFFT of the quadrature charges: exponential-of-semicircle (ES) kernel spreading
 //     onto the oversampled grid (Barnett, Magland & af Klinteberg, SIAM J. Sci. Comput. 2019),
-//     then a batched 3-D real-to-complex FFT (cuFFT);
-//  2. one fused Fourier-space kernel: deconvolution, Gamma/V prefactor, Hermitian-symmetry
+//     then the pruned transforms of fourier.cu (cuFFT for the sizes that those have no plan for);
+//  2. the Fourier-space operators, inside the z transform (one kernel beside cuFFT): deconvolution, Gamma/V prefactor, Hermitian-symmetry
 //     zeroing (longrange.jl:556-583), optional spherical truncation (longrange.jl:497-532),
 //     the vorticity coefficients kept for get_longrange_field_fourier, and the
 //     streamfunction (longrange.jl:102-125) / Biot-Savart (longrange.jl:128-142) operators
 //     times the Ewald Gaussian exp(-k^2/4 alpha^2) (cache_common.jl:64-76) and the type-2
-//     deconvolution, written straight into the complex-to-real FFT input;
-//  3. batched complex-to-real FFT and ES-kernel interpolation at the nodes (type 2).
+//     deconvolution, left where the inverse transforms read them;
+//  3. complex-to-real transforms and ES-kernel interpolation at the nodes (type 2).
 #include <cmath>
 #include <type_traits>
 #include <vector>
@@ -795,7 +795,9 @@ __global__ void __launch_bounds__(kTcThreads, 2) spread_tc_kernel(LRSizes S, int
 // A warp covers four y rows and skips the points whose footprint misses them.
 // Bound: the FP64 pipe (28 instructions per point, warp and brick met).  Bricks of 8 instead of 16
 // give 6.6 (m = 4) or 9.6 (m = 5) bricks met per point instead of 3.0 or 3.8, each of an eighth of the
-// cells: 2.5 to 3.2 times fewer updates with zero.
+// cells: 2.5 to 3.2 times fewer updates with zero.  1M nodes, FP64, 768^3, m = 5: 7.25 ms (16^3 bricks: 13.96);
+// 100k nodes, 288^3, m = 4: 0.43 ms (1.18).  A warp per brick, without barriers, waits for every staging load in
+// turn: 2.4 times slower.  Batches of 32 slots are as fast as of 64.
 constexpr int kColB = 8;
 constexpr int kColThreads = kColB * kColB;
 constexpr int kColBatch = 32;
