@@ -704,6 +704,7 @@ int vpbs_set_points(vpbs_handle* h, int64_t Np, vpbs_cvec3 nodes, const int32_t*
         if ((rc = check_cuda(h, cudaMemcpyAsync(c.dst, c.src, c.n, cudaMemcpyHostToDevice, h->stream), "H2D point data")))
             return rc;
     if ((rc = check_cuda(h, cudaEventRecord(h->h2d_done, h->stream), "event record"))) return rc;
+    h->dm_pending = false;
     h->li_valid = false;  // add_local_integrals! stays with the caller in the point-data contract
     h->have_filaments = false;  // point data without a filament layout: no time stepping
     return process_point_charges(h);

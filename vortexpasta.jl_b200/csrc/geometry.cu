@@ -768,7 +768,6 @@ int geometry_from_filaments(vpbs_handle* h, int64_t nfil, const int64_t* d_offse
     int32_t* status = (int32_t*)((double*)h->spline_scratch.p + 12 * Np);
     const double* foff = h->have_fil_offsets ? (const double*)h->fil_off.p : nullptr;
     StageScope st(h, ST_GEOMETRY);
-    if ((rc = check_cuda(h, cudaMemsetAsync(status, 0, sizeof(int32_t), h->stream), "memset"))) return rc;
     spline_solve_kernel<<<grid_for(nfil, kSolveWarps), 32 * kSolveWarps, smem_bytes, h->stream>>>(
         nfil, d_offsets, d_nodes, knots, periods, (int32_t*)h->fil_of_node.p, (double*)h->coefs.p,
         (double*)h->dcoef1.p, (double*)h->dcoef2.p, (double*)h->spline_scratch.p, status, smem_n, keep_knots ? 1 : 0,
@@ -783,14 +782,16 @@ int geometry_from_filaments(vpbs_handle* h, int64_t nfil, const int64_t* d_offse
         (const double*)h->dcoef1.p, (const double*)h->dcoef2.p, (double*)h->nodes.p, (int32_t*)h->idx_prev.p,
         (double*)h->d1.p, (double*)h->d2.p, (double*)h->dm.p, (double*)h->dp.p, (double*)h->points.p,
         (double*)h->charges.p, (double*)h->li_vel.p, (double*)h->li_psi.p, want_li ? 1 : 0, fuse ? 1 : 0, foff);
-    if (fuse)
+    // the cell count of the evaluation copies delta^- from the previous node's delta^+ where there is one
+    h->dm_pending = fuse && !h->K.open_domain;
+    if (fuse && !h->dm_pending)
         dm_from_prev_kernel<<<grid_for(Np, 256), 256, 0, h->stream>>>(Np, (const int32_t*)h->idx_prev.p,
                                                                        (const double*)h->dp.p, (double*)h->dm.p);
-    else
+    else if (!fuse)
         quad_points_kernel<<<grid_for(Np * h->K.nquad, 128), 128, 0, h->stream>>>(
             h->K, Np, d_offsets, (const int32_t*)h->fil_of_node.p, knots, periods, (const double*)h->coefs.p,
             (const double*)h->dcoef1.p, (double*)h->points.p, (double*)h->charges.p, foff);
-    h->launches += 2;
+    h->launches += h->dm_pending ? 1 : 2;
     return check_cuda(h, cudaGetLastError(), "geometry kernels");
 }
 

@@ -52,10 +52,11 @@ __device__ __forceinline__ int64_t cell_of(const CellGrid& cg, const KParams& K,
 
 // Cell of every quadrature point and node and its rank within the cell (atomic counters).  The nodes'
 // entries follow the points' in every array; their threads start at a whole warp, so that no warp counts
-// both.
+// both.  dm (if given): delta^- of the nodes, the delta^+ of the previous node.
 __global__ void cell_count_kernel(KParams K, CellGrid cg, int64_t Nq, int64_t Np, const double* __restrict__ points,
                                   const double* __restrict__ nodes, int32_t* __restrict__ cell, int32_t* __restrict__ rank,
-                                  int32_t* __restrict__ counts) {
+                                  int32_t* __restrict__ counts, const int32_t* __restrict__ idx_prev,
+                                  const double* __restrict__ dp, double* __restrict__ dm) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, j0 = (Nq + 31) & ~(int64_t)31;
     if ((j >= Nq && j < j0) || j >= j0 + Np) return;
     const bool node = j >= j0;
@@ -63,6 +64,7 @@ __global__ void cell_count_kernel(KParams K, CellGrid cg, int64_t Nq, int64_t Np
     const double* xyz = node ? nodes : points;
     const int32_t c = (int32_t)cell_of(cg, K, xyz[k], xyz[n + k], xyz[2 * n + k]);
     cell[e] = c;
+    if (node && dm) dm[k] = dp[idx_prev[k]];
     rank[e] = warp_aggregated_rank(node ? counts + cg.ncell + 1 : counts, c);
 }
 
@@ -1087,8 +1089,10 @@ __global__ void __launch_bounds__(128) local_self_kernel(
     const double* __restrict__ nodes, const int32_t* __restrict__ idx_prev, const double* __restrict__ d1,
     const double* __restrict__ d2, const double* __restrict__ dm, const double* __restrict__ dp,
     const double* __restrict__ points, const double* __restrict__ charges, const double* __restrict__ li_vel,
-    const double* __restrict__ li_psi, double* __restrict__ vel, double* __restrict__ psi, double3 psi_bg) {
+    const double* __restrict__ li_psi, double* __restrict__ vel, double* __restrict__ psi, double3 psi_bg,
+    unsigned long long* __restrict__ counters) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 2 && do_self) counters[i] = 0ull;  // of the pair kernel that follows
     if (i >= Np) return;
     const bool want_v = fields & VPBS_VELOCITY, want_p = fields & VPBS_STREAMFUNCTION;
     const double pref = K.Gamma / (4.0 * kPi);
@@ -1181,8 +1185,9 @@ int build_cell_lists(vpbs_handle* h) {
     if (h->K.open_domain) return 0;
     // Cell size (internal: the pair set does not depend on it).  Where cells r_cut/2 wide would
     // hold fewer than 8 nodes, cells r_cut wide (M = 1) are used instead: the pair search is
-    // then bound by per-node overhead, which grows with the (2M+1)^2 rows a node walks (1M-node
-    // tangle at r_cut = L/40: 6.3 ms with M = 1 against 9.9 ms with M = 2).
+    // then bound by per-node overhead, which grows with the (2M+1)^2 rows a node walks (FP32,
+    // 1M-node tangle at r_cut = L/45: 1.82 ms with M = 1 against 2.82 with M = 2; FP64, 100k nodes: 0.32 against
+    // 0.41; FP32, 20k nodes: even).
     {
         const int Mu = h->P.nsubdiv;
         int M = Mu;
@@ -1217,7 +1222,10 @@ int build_cell_lists(vpbs_handle* h) {
     StageScope st(h, ST_CELL_LISTS);
     if ((rc = check_cuda(h, cudaMemsetAsync(counts, 0, sizeof(int32_t) * nscan, h->stream), "memset"))) return rc;
     cell_count_kernel<<<grid_for(n + 32, 256), 256, 0, h->stream>>>(h->K, h->cg, Nq, Np, (const double*)h->points.p,
-                                                               (const double*)h->nodes.p, cell, rank, counts);
+                                                               (const double*)h->nodes.p, cell, rank, counts,
+                                                               (const int32_t*)h->idx_prev.p, (const double*)h->dp.p,
+                                                               h->dm_pending ? (double*)h->dm.p : nullptr);
+    h->dm_pending = false;
     if ((rc = exclusive_scan(h, counts, h->src_start, nscan, h->scan_tmp, ncell + 1, (int32_t)Nq))) return rc;
     scatter_kernel<<<grid_for(n, 256), 256, 0, h->stream>>>(
         Nq, Np, h->K.nquad, (const double*)h->points.p, (const double*)h->charges.p, cell, rank, h->src_start,
@@ -1385,13 +1393,10 @@ static bool use_f32_pairs(const vpbs_handle* h) {
            h->cg.M > 0 && h->K.ntab_c > 0 && h->K.ntab_c <= kF32TabMax;
 }
 
+// Adds the pair sums to the outputs; the counters were zeroed by local_and_self.
 int pair_interactions(vpbs_handle* h, int fields) {
     const int64_t Np = h->Np, Nq = h->Nq;
     const bool open = h->K.open_domain;
-    int rc;
-    if ((rc = ensure(h, h->counters, sizeof(unsigned long long) * 2, "counters"))) return rc;
-    if ((rc = check_cuda(h, cudaMemsetAsync(h->counters.p, 0, sizeof(unsigned long long) * 2, h->stream), "memset")))
-        return rc;
     const int skip_local = (!h->K.avoid_explicit_erf && h->K.alpha > 0) ? 1 : 0;
     if (skip_local && open) return set_error(h, VPBS_ERR_PARAMS, "avoid_explicit_erf=false requires Ewald splitting");
     StageScope st(h, ST_PAIRS);
@@ -1515,12 +1520,15 @@ int local_and_self(vpbs_handle* h, int fields, int lia_mode, int with_pairs_self
             bg = make_double3(f * p[0], f * p[1], f * p[2]);
         }
     }
+    int rc;
+    if (do_self && (rc = ensure(h, h->counters, sizeof(unsigned long long) * 2, "counters"))) return rc;
     StageScope st(h, ST_LOCAL_SELF);
     local_self_kernel<<<grid_for(h->Np, 128), 128, 0, h->stream>>>(
         K, h->Np, fields, do_local, do_self, do_li, rv, rpsi, (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p,
         (const double*)h->d1.p, (const double*)h->d2.p, (const double*)h->dm.p, (const double*)h->dp.p,
         (const double*)h->points.p, (const double*)h->charges.p, (const double*)h->li_vel.p,
-        (const double*)h->li_psi.p, (double*)h->vel.p, (double*)h->psi.p, bg);
+        (const double*)h->li_psi.p, (double*)h->vel.p, (double*)h->psi.p, bg,
+        (unsigned long long*)h->counters.p);
     h->launches++;
     return check_cuda(h, cudaGetLastError(), "local term kernel");
 }

@@ -181,6 +181,7 @@ struct vpbs_handle {
 
     // point data (SoA; 3 consecutive blocks of Np or Nq doubles for vectors)
     vpbs::DevBuf nodes, idx_prev, d1, d2, dm, dp, points, charges;
+    bool dm_pending = false;  // dm still to be copied from the previous nodes' dp (build_cell_lists)
     vpbs::DevBuf li_vel, li_psi;  // lia_segment_fraction local integrals (per node)
 
     // cell lists
