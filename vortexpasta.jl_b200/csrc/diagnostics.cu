@@ -181,16 +181,18 @@ extern "C" int vpbs_spectrum(vpbs_handle* h, int32_t kind, double dk, double* ou
                          "spectrum kind must be 0 (energy, vorticity state), 1 (helicity) or 2 (energy, velocity state)");
     if (!h->have_uhat)
         return set_error(h, VPBS_ERR_STATE, "no vorticity coefficients: run a long-range computation first");
-    if (nk > 16384) return set_error(h, VPBS_ERR_ARG, "at most 16384 spectrum bins (shared-memory partial sums)");
+    constexpr int kMostBins = 16384;
+    if (nk > kMostBins) return set_error(h, VPBS_ERR_ARG, "at most 16384 spectrum bins (shared-memory partial sums)");
     int rc = check_cuda(h, cudaSetDevice(h->device), "cudaSetDevice");
     if (rc) return rc;
     const LRSizes& S = h->lr;
     DevBuf acc;
     if ((rc = ensure(h, acc, sizeof(double) * nk, "spectrum bins"))) return rc;
     const size_t smem = sizeof(double) * nk;
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(spectrum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    rc = check_cuda(h, cudaMemsetAsync(acc.p, 0, sizeof(double) * nk, h->stream), "memset");
+    if (smem >= 48 * 1024)  // for the most bins, not these: the attribute belongs to the function, not to the call
+        rc = check_cuda(h, cudaFuncSetAttribute(spectrum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)(kMostBins * sizeof(double))), "spectrum kernel shared memory");
+    if (!rc) rc = check_cuda(h, cudaMemsetAsync(acc.p, 0, sizeof(double) * nk, h->stream), "memset");
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
     const int64_t want = (S.nmodes + 255) / 256;

@@ -734,10 +734,11 @@ __global__ void __launch_bounds__(128) quad_points_kernel(
 // lets 5 blocks (10 warps) share an SM; with 4, 2 blocks (8 warps) fit (1M nodes: 0.61 vs 0.66 ms for
 // the geometry).
 constexpr int kSolveWarps = 2;
+constexpr size_t kSolveSmemMost = 200 * 1024;
 
 static int solve_smem_n(int64_t nmax, size_t* bytes) {
     const size_t b = (size_t)kSolveWarps * 12 * nmax * sizeof(double);
-    if (nmax > 0 && b <= 200 * 1024) {
+    if (nmax > 0 && b <= kSolveSmemMost) {
         *bytes = b;
         return (int)nmax;
     }
@@ -751,11 +752,11 @@ int geometry_from_filaments(vpbs_handle* h, int64_t nfil, const int64_t* d_offse
     int rc;
     size_t smem_bytes = 0;
     const int smem_n = solve_smem_n(nmax, &smem_bytes);
-    // opt in to the exact size every time (a launch at exactly 48 KB also needs it, and the
-    // attribute is per function, not per handle)
+    // the most any call needs, not this one's: the attribute belongs to the function, and another thread's
+    // handle may launch between this line and the launch below (a launch at exactly 48 KB also needs it)
     if (smem_bytes > 0 &&
         (rc = check_cuda(h, cudaFuncSetAttribute(spline_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem_bytes), "spline kernel shared memory")))
+                                                 (int)kSolveSmemMost), "spline kernel shared memory")))
         return rc;
     if ((rc = ensure(h, h->knots, sizeof(double) * (Np + nfil), "knots"))) return rc;
     if ((rc = ensure(h, h->fil_of_node, sizeof(int32_t) * Np, "fil_of_node"))) return rc;
