@@ -134,6 +134,20 @@ def test_open_domain_sizes(vp, oracle, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n,names", [(90, ("velocity",)), (700, ("velocity", "streamfunction")), (4014, ("velocity",)),
+                                     (4014, ("streamfunction",))])
+def test_open_domain_repeats_itself(vp, n, names):
+    """The same call gives the same bits, although the sources are shared out over groups of threads and over CTAs."""
+    p = vp.ParamsBiotSavart(Gamma=1.0, a=1e-8, splitting=vp.NoSplitting())
+    fs = [wobbly(vp, n, n, 0.5)]
+    first, _ = fields(vp, p, fs, names)
+    for _ in range(20):
+        again, _ = fields(vp, p, fs, names)
+        for name in names:
+            assert np.array_equal(again[name], first[name])
+
+
+@pytest.mark.gpu
 def test_open_domain_skips_nan_sources(vp):
     """A filament with a NaN node does not reach the nodes of the others."""
     p = vp.ParamsBiotSavart(Gamma=1.0, a=1e-8, splitting=vp.NoSplitting())

@@ -763,7 +763,8 @@ int geometry_from_filaments(vpbs_handle* h, int64_t nfil, const int64_t* d_offse
     if ((rc = ensure(h, h->coefs, sizeof(double) * 3 * Np, "coefs"))) return rc;
     if ((rc = ensure(h, h->dcoef1, sizeof(double) * 3 * Np, "dcoef1"))) return rc;
     if ((rc = ensure(h, h->dcoef2, sizeof(double) * 3 * Np, "dcoef2"))) return rc;
-    if ((rc = ensure(h, h->spline_scratch, sizeof(double) * 12 * Np + 64, "spline scratch"))) return rc;
+    const size_t scratch = sizeof(double) * 12 * Np + 64, part = h->K.open_domain ? open_part_bytes(h) : 0;
+    if ((rc = ensure(h, h->spline_scratch, scratch > part ? scratch : part, "spline scratch"))) return rc;
     double* knots = (double*)h->knots.p;
     double* periods = knots + Np;
     int32_t* status = (int32_t*)((double*)h->spline_scratch.p + 12 * Np);

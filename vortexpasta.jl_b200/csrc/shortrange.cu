@@ -324,22 +324,31 @@ __device__ __forceinline__ unsigned long long warp_sum_u(unsigned long long v) {
     return v;
 }
 
-// All pairs of an open domain (no splitting: the full Biot-Savart integrand, no cut-off).  A thread
-// per node, sources broadcast from shared memory in tiles; blockIdx.y takes its share of the sources
-// and adds its sums to the output with one atomic per component, so that few nodes still fill the
-// device.  Bound: the FP64 pipe (about 30 instructions per pair).
-constexpr int kOpenThreads = 128;
-constexpr int kOpenTile = 128;
+// All pairs of an open domain (no splitting: the full Biot-Savart integrand, no cut-off).  A CTA takes 128
+// nodes and four groups of threads, a thread per node in each, that deal the sources of a tile in shared memory
+// out among them (a source is broadcast to a warp).  blockIdx.y takes its share of the sources, so that few nodes
+// still fill the device.  The groups' sums are added in their order; the shares' sums go to `part` and the last
+// CTA of a block of nodes to arrive (arrive[blockIdx.x], zeroed by the local term's kernel) adds them in the order
+// of the shares: the same call gives the same bits each time.  Bound: the FP64 pipe (about 30 instructions per pair).  Against one
+// group per CTA and atomic sums, whose order varied: 30,000 nodes 4.74 -> 4.50 ms, 4,014 nodes 0.164 -> 0.168.
+constexpr int kOpenNodes = 128;
+constexpr int kOpenGroups = 4;
+constexpr int kOpenThreads = kOpenNodes * kOpenGroups;
+constexpr int kOpenTile = 512;
+constexpr int kOpenBlocks = 2;  // CTAs per SM
+constexpr int kArrive = 4;      // words of vpbs_handle::counters before the arrivals per block of nodes
 
 template <bool VEL, bool PSI>
-__global__ void __launch_bounds__(kOpenThreads) pair_open_kernel(int64_t Np, int64_t Ns, int per, double pref,
-                                                                 const double* __restrict__ nodes,
-                                                                 const double* __restrict__ points,
-                                                                 const double* __restrict__ charges, double* __restrict__ vel,
-                                                                 double* __restrict__ psi,
-                                                                 unsigned long long* __restrict__ counters) {
+__global__ void __launch_bounds__(kOpenThreads, kOpenBlocks) pair_open_kernel(
+    int64_t Np, int64_t Ns, int per, double pref, const double* __restrict__ nodes, const double* __restrict__ points,
+    const double* __restrict__ charges, double* __restrict__ vel, double* __restrict__ psi, double* __restrict__ part,
+    unsigned* __restrict__ arrive, unsigned long long* __restrict__ counters) {
+    constexpr int NC = (VEL ? 3 : 0) + (PSI ? 3 : 0);
     __shared__ double2 pxy[kOpenTile], pzq[kOpenTile], qyz[kOpenTile];
-    const int64_t i = (int64_t)blockIdx.x * kOpenThreads + threadIdx.x;
+    __shared__ double sums[kOpenGroups - 1][NC][kOpenNodes];
+    __shared__ bool last;
+    const int local = threadIdx.x % kOpenNodes, group = threadIdx.x / kOpenNodes;
+    const int64_t i = (int64_t)blockIdx.x * kOpenNodes + local;
     const int64_t ic = i < Np ? i : Np - 1;
     const double x0 = nodes[ic], x1 = nodes[Np + ic], x2 = nodes[2 * Np + ic];
     const int64_t j0 = (int64_t)blockIdx.y * per, j1 = j0 + per < Ns ? j0 + per : Ns;
@@ -361,7 +370,7 @@ __global__ void __launch_bounds__(kOpenThreads) pair_open_kernel(int64_t Np, int
         }
         __syncthreads();
 #pragma unroll 4
-        for (int t = 0; t < n; ++t) {
+        for (int t = group; t < n; t += kOpenGroups) {
             const double2 a = pxy[t], b = pzq[t], c = qyz[t];
             const double r0 = x0 - a.x, r1 = x1 - a.y, r2 = x2 - b.x;
             const double rinv = rsqrt(r0 * r0 + r1 * r1 + r2 * r2);
@@ -378,19 +387,46 @@ __global__ void __launch_bounds__(kOpenThreads) pair_open_kernel(int64_t Np, int
             }
         }
     }
-    if (i < Np && j0 < j1) {
-        if (VEL) {
-            atomicAdd(&vel[i], pref * v0);
-            atomicAdd(&vel[Np + i], pref * v1);
-            atomicAdd(&vel[2 * Np + i], pref * v2);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) counters[threadIdx.x] = (unsigned long long)Np * (unsigned long long)Ns;
+    double f[6] = {VEL ? v0 : p0, VEL ? v1 : p1, VEL ? v2 : p2, p0, p1, p2};
+    if (group > 0)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) sums[group - 1][c][local] = f[c];
+    __syncthreads();
+    if (group == 0)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+#pragma unroll
+            for (int g = 0; g < kOpenGroups - 1; ++g) f[c] += sums[g][c][local];
+            f[c] *= pref;
         }
-        if (PSI) {
-            atomicAdd(&psi[i], pref * p0);
-            atomicAdd(&psi[Np + i], pref * p1);
-            atomicAdd(&psi[2 * Np + i], pref * p2);
+    if (gridDim.y > 1) {
+        if (group == 0) {
+            if (i < Np)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) part[((int64_t)blockIdx.y * NC + c) * Np + i] = f[c];
+            __threadfence();
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) last = atomicAdd(&arrive[blockIdx.x], 1u) == gridDim.y - 1;
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+#pragma unroll
+        for (int c = 0; c < NC; ++c) f[c] = 0.0;
+        if (group == 0)
+#pragma unroll 4
+            for (unsigned y = 0; y < gridDim.y; ++y)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) f[c] += __ldcg(&part[((int64_t)y * NC + c) * Np + ic]);
+    }
+    if (group == 0 && i < Np) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (VEL) vel[c * Np + i] += f[c];
+            if (PSI) psi[c * Np + i] += f[VEL ? 3 + c : c];
         }
     }
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) counters[threadIdx.x] = (unsigned long long)Np * (unsigned long long)Ns;
 }
 
 // One warp per destination node (visited in cell order when cell lists are used).  R = double
@@ -1090,9 +1126,9 @@ __global__ void __launch_bounds__(128) local_self_kernel(
     const double* __restrict__ d2, const double* __restrict__ dm, const double* __restrict__ dp,
     const double* __restrict__ points, const double* __restrict__ charges, const double* __restrict__ li_vel,
     const double* __restrict__ li_psi, double* __restrict__ vel, double* __restrict__ psi, double3 psi_bg,
-    unsigned long long* __restrict__ counters) {
+    unsigned* __restrict__ counters, int ncount) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < 2 && do_self) counters[i] = 0ull;  // of the pair kernel that follows
+    if (i < ncount) counters[i] = 0u;  // of the pair kernel that follows
     if (i >= Np) return;
     const bool want_v = fields & VPBS_VELOCITY, want_p = fields & VPBS_STREAMFUNCTION;
     const double pref = K.Gamma / (4.0 * kPi);
@@ -1393,6 +1429,31 @@ static bool use_f32_pairs(const vpbs_handle* h) {
            h->cg.M > 0 && h->K.ntab_c > 0 && h->K.ntab_c <= kF32TabMax;
 }
 
+// Blocks of nodes and shares of the sources of pair_open_kernel: the fewest shares of at least 128 sources whose CTAs
+// fill the last round of those the device holds at a time to 95 % (30,000 nodes: 5 shares, 4.50 ms; one share
+// leaves a third of the device idle: 5.76), else those that fill it best.
+static unsigned open_blocks(int64_t Np) { return grid_for(Np, kOpenNodes); }
+static int64_t open_parts(const vpbs_handle* h) {
+    int nsm = 148;
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
+    const int64_t gx = open_blocks(h->Np), held = kOpenBlocks * (int64_t)nsm;
+    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(h->Nq / 128, std::max<int64_t>(held / gx, 16)));
+    int64_t best = 1;
+    double fill = 0.0;
+    for (int64_t parts = 1; parts <= most && fill < 0.95; ++parts) {
+        const double f = (double)(gx * parts) / (double)((gx * parts + held - 1) / held * held);
+        if (f > fill) {
+            fill = f;
+            best = parts;
+        }
+    }
+    return best;
+}
+size_t open_part_bytes(const vpbs_handle* h) {
+    const int64_t parts = open_parts(h);
+    return parts > 1 ? sizeof(double) * 6 * parts * h->Np : 0;
+}
+
 // Adds the pair sums to the outputs; the counters were zeroed by local_and_self.
 int pair_interactions(vpbs_handle* h, int fields) {
     const int64_t Np = h->Np, Nq = h->Nq;
@@ -1403,17 +1464,16 @@ int pair_interactions(vpbs_handle* h, int fields) {
     const unsigned grid = grid_for(Np, 8);
     const bool v = fields & VPBS_VELOCITY, p = fields & VPBS_STREAMFUNCTION;
     if (open) {
-        // about eight CTAs per SM, each with at least one tile of sources
-        const unsigned gx = grid_for(Np, kOpenThreads);
-        int nsm = 148;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-        const int64_t want = std::min<int64_t>((8 * (int64_t)nsm + gx - 1) / gx, (Nq + kOpenTile - 1) / kOpenTile);
-        const int64_t parts = std::max<int64_t>(1, std::min<int64_t>(want, 65535));
+        const unsigned gx = open_blocks(Np);
+        const int64_t parts = open_parts(h);
         const int per = (int)((Nq + parts - 1) / parts);
+        int rc;  // as large already, after vpbs_set_filaments
+        if ((rc = ensure(h, h->spline_scratch, open_part_bytes(h), "partial sums"))) return rc;
         auto launch_open = [&](auto kern) {
             kern<<<dim3(gx, (unsigned)parts), kOpenThreads, 0, h->stream>>>(
                 Np, Nq, per, h->K.Gamma / (4.0 * kPi), (const double*)h->nodes.p, (const double*)h->points.p,
-                (const double*)h->charges.p, (double*)h->vel.p, (double*)h->psi.p, (unsigned long long*)h->counters.p);
+                (const double*)h->charges.p, (double*)h->vel.p, (double*)h->psi.p, (double*)h->spline_scratch.p,
+                (unsigned*)h->counters.p + kArrive, (unsigned long long*)h->counters.p);
         };
         if (v && p) launch_open(pair_open_kernel<true, true>);
         else if (v) launch_open(pair_open_kernel<true, false>);
@@ -1521,14 +1581,15 @@ int local_and_self(vpbs_handle* h, int fields, int lia_mode, int with_pairs_self
         }
     }
     int rc;
-    if (do_self && (rc = ensure(h, h->counters, sizeof(unsigned long long) * 2, "counters"))) return rc;
+    const int ncount = !do_self ? 0 : kArrive + (K.open_domain ? (int)open_blocks(h->Np) : 0);  // fewer than threads
+    if (do_self && (rc = ensure(h, h->counters, sizeof(unsigned) * ncount, "counters"))) return rc;
     StageScope st(h, ST_LOCAL_SELF);
     local_self_kernel<<<grid_for(h->Np, 128), 128, 0, h->stream>>>(
         K, h->Np, fields, do_local, do_self, do_li, rv, rpsi, (const double*)h->nodes.p, (const int32_t*)h->idx_prev.p,
         (const double*)h->d1.p, (const double*)h->d2.p, (const double*)h->dm.p, (const double*)h->dp.p,
         (const double*)h->points.p, (const double*)h->charges.p, (const double*)h->li_vel.p,
         (const double*)h->li_psi.p, (double*)h->vel.p, (double*)h->psi.p, bg,
-        (unsigned long long*)h->counters.p);
+        (unsigned*)h->counters.p, ncount);
     h->launches++;
     return check_cuda(h, cudaGetLastError(), "local term kernel");
 }

@@ -188,7 +188,8 @@ struct vpbs_handle {
     vpbs::CellGrid cg{};
     vpbs::DevBuf src_cell, cell_start, cell_counts, src_sorted, src_seg, src_f32, dst_order;
     int32_t *src_start = nullptr, *dst_start = nullptr;  // of the points' and the nodes' cells, in cell_start
-    vpbs::DevBuf counters;  // [0] in-range pairs, [1] candidates (unsigned long long)
+    // [0] in-range pairs, [1] candidates (unsigned long long); in an open domain then the arrivals per block of nodes
+    vpbs::DevBuf counters;
     vpbs::DevBuf scan_tmp, scan_tmp_lr;  // multi-CTA scan scratch (cell lists; spreading bins)
     vpbs::DevBuf ewald_tab;  // Taylor tables of the Ewald weights (KParams::ewald_tab)
 
@@ -269,6 +270,7 @@ int exclusive_scan(vpbs_handle* h, const int32_t* counts, int32_t* start, int64_
                    int64_t split = INT64_MAX, int32_t sub = 0);
 int local_and_self(vpbs_handle* h, int fields, int lia_mode, int with_pairs_self, double integration_cutoff);
 int pair_interactions(vpbs_handle* h, int fields);
+size_t open_part_bytes(const vpbs_handle* h);  // partial sums of the open-domain pairs, in spline_scratch
 int add_local_integrals(vpbs_handle* h, int fields);
 
 // longrange.cu
