@@ -149,13 +149,14 @@ def test_open_domain_repeats_itself(vp, n, names):
 
 @pytest.mark.gpu
 def test_open_domain_skips_nan_sources(vp):
-    """A filament with a NaN node does not reach the nodes of the others."""
+    """A filament with a NaN node does not reach the nodes of the others, and its pairs are not counted."""
     p = vp.ParamsBiotSavart(Gamma=1.0, a=1e-8, splitting=vp.NoSplitting())
     good, bad = wobbly(vp, 40, 1), wobbly(vp, 30, 2)
     alone, _ = fields(vp, p, [good], ("velocity",))
     bad[7] = np.nan
-    both, _ = fields(vp, p, [good, bad], ("velocity",))
+    both, counts = fields(vp, p, [good, bad], ("velocity",))
     assert rel(both["velocity"][:40], alone["velocity"]) <= 1e-13
+    assert counts == (69 * 3 * 40, 70 * 3 * 70)  # every source of the bad filament is NaN, one of its nodes
 
 
 @pytest.mark.gpu

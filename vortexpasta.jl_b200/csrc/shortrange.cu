@@ -347,12 +347,15 @@ __global__ void __launch_bounds__(kOpenThreads, kOpenBlocks) pair_open_kernel(
     __shared__ double2 pxy[kOpenTile], pzq[kOpenTile], qyz[kOpenTile];
     __shared__ double sums[kOpenGroups - 1][NC][kOpenNodes];
     __shared__ bool last;
+    __shared__ unsigned sources;  // of this share, those that take part in pairs
     const int local = threadIdx.x % kOpenNodes, group = threadIdx.x / kOpenNodes;
     const int64_t i = (int64_t)blockIdx.x * kOpenNodes + local;
     const int64_t ic = i < Np ? i : Np - 1;
     const double x0 = nodes[ic], x1 = nodes[Np + ic], x2 = nodes[2 * Np + ic];
     const int64_t j0 = (int64_t)blockIdx.y * per, j1 = j0 + per < Ns ? j0 + per : Ns;
     double v0 = 0, v1 = 0, v2 = 0, p0 = 0, p1 = 0, p2 = 0;
+    unsigned mine = 0;
+    if (threadIdx.x == 0) sources = 0;
     for (int64_t jt = j0; jt < j1; jt += kOpenTile) {
         const int n = j1 - jt < kOpenTile ? (int)(j1 - jt) : kOpenTile;
         __syncthreads();
@@ -363,6 +366,8 @@ __global__ void __launch_bounds__(kOpenThreads, kOpenBlocks) pair_open_kernel(
             if (!(s0 == s0 && s1 == s1 && s2 == s2)) {  // a NaN position takes part in no pair
                 s0 = s1 = s2 = 1e100;
                 q0 = q1 = q2 = 0.0;
+            } else {
+                ++mine;
             }
             pxy[t] = make_double2(s0, s1);
             pzq[t] = make_double2(s2, q0);
@@ -387,12 +392,17 @@ __global__ void __launch_bounds__(kOpenThreads, kOpenBlocks) pair_open_kernel(
             }
         }
     }
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) counters[threadIdx.x] = (unsigned long long)Np * (unsigned long long)Ns;
+    const int takers = __syncthreads_count(group == 0 && i < Np && x0 == x0 && x1 == x1 && x2 == x2);
+    if (mine) atomicAdd(&sources, mine);
     double f[6] = {VEL ? v0 : p0, VEL ? v1 : p1, VEL ? v2 : p2, p0, p1, p2};
     if (group > 0)
 #pragma unroll
         for (int c = 0; c < NC; ++c) sums[group - 1][c][local] = f[c];
     __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicAdd(&counters[0], (unsigned long long)takers * sources);
+        if (blockIdx.x == 0 && blockIdx.y == 0) counters[1] = (unsigned long long)Np * (unsigned long long)Ns;
+    }
     if (group == 0)
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
