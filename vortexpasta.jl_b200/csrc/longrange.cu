@@ -879,10 +879,10 @@ __device__ __forceinline__ void col_bins(int s0, int b, int w, int n, int nb, in
     }
 }
 
-template <typename T>
+template <typename T, typename G>  // T: kernel rows and sums, G: grid
 __global__ void __launch_bounds__(kColThreads) spread_column_kernel(
     LRSizes S, int nb0, int nb1, int nb2, const int32_t* __restrict__ bin_start, const T* __restrict__ binned,
-    const int32_t* __restrict__ foot, T* __restrict__ grid) {
+    const int32_t* __restrict__ foot, G* __restrict__ grid) {
     __shared__ __align__(16) ColSlot<T> slot[kColBatch];
     __shared__ int yrows[kColBatch];    // bit y: the footprint meets row y of the brick
     __shared__ int32_t pend[kColThreads];
@@ -1009,14 +1009,14 @@ __global__ void __launch_bounds__(kColThreads) spread_column_kernel(
     if (bs[0] + tx >= S.n[0] || bs[1] + ty >= S.n[1]) return;
     const int64_t ng = S.ngrid;
     const int64_t plane = (int64_t)S.n[1] * S.n[0];
-    T* g = grid + ((int64_t)bs[2] * S.n[1] + bs[1] + ty) * S.n[0] + bs[0] + tx;
+    G* g = grid + ((int64_t)bs[2] * S.n[1] + bs[1] + ty) * S.n[0] + bs[0] + tx;
     const int nz = min(kColB, S.n[2] - bs[2]);
 #pragma unroll
     for (int z = 0; z < kColB; ++z)
         if (z < nz) {
-            g[z * plane] = acc0.get(z);
-            g[ng + z * plane] = acc1.get(z);
-            g[2 * ng + z * plane] = acc2.get(z);
+            g[z * plane] = (G)acc0.get(z);
+            g[ng + z * plane] = (G)acc1.get(z);
+            g[2 * ng + z * plane] = (G)acc2.get(z);
         }
 }
 
@@ -1179,6 +1179,14 @@ int longrange_init(vpbs_handle* h) {
     for (int d = 0; d < 3; ++d)
         if (S.n[d] % 16 != 0 || S.n[d] < 32) h->brick = kColB;
     for (int d = 0; d < 3; ++d) h->nbrick[d] = (S.n[d] + h->brick - 1) / h->brick;
+    // FP32 grids of sizes that no whole bricks of 16, 12, 10 or 8 points, as wide as the kernel, tile keep kernel rows,
+    // products and sums in FP64 up to the grid value
+    h->rows64 = P.precision == VPBS_PRECISION_MIXED;
+    for (int B : {16, 12, 10, 8}) {
+        bool tiles = B >= 2 * S.m;
+        for (int d = 0; d < 3; ++d) tiles = tiles && S.n[d] % B == 0 && S.n[d] >= 2 * B;
+        if (tiles) h->rows64 = false;
+    }
     int rc;
     const bool mixed = P.precision == VPBS_PRECISION_MIXED;
     const size_t rsz = mixed ? sizeof(float) : sizeof(double);  // grid precision
@@ -1306,32 +1314,43 @@ int longrange_compute_t(vpbs_handle* h, int fields) {
             if ((rc = ensure(h, h->spread_bin, sizeof(int32_t) * 2 * Nq, "spread bins"))) return rc;
             if ((rc = ensure(h, h->spread_counts, sizeof(int32_t) * nbins, "spread bin counts"))) return rc;
             if ((rc = ensure(h, h->spread_start, sizeof(int32_t) * (nbins + 1), "spread bin starts"))) return rc;
-            if ((rc = ensure(h, h->binned, sizeof(T) * stride * Nq, "binned points"))) return rc;
+            const size_t rsz = h->rows64 ? sizeof(double) : sizeof(T);  // kernel rows
+            if ((rc = ensure(h, h->binned, rsz * stride * Nq, "binned points"))) return rc;
             if ((rc = ensure(h, h->spread_foot, sizeof(int32_t) * 3 * Nq, "footprints"))) return rc;
             int32_t* bin = (int32_t*)h->spread_bin.p;
             int32_t* rank = bin + Nq;
             int32_t* counts = (int32_t*)h->spread_counts.p;
             int32_t* start = (int32_t*)h->spread_start.p;
             int32_t* foot = (int32_t*)h->spread_foot.p;
-            const T* bsrc = (const T*)h->binned.p;
             if ((rc = check_cuda(h, cudaMemsetAsync(counts, 0, sizeof(int32_t) * nbins, h->stream), "memset"))) return rc;
             spread_bin_count_kernel<<<grid_for(Nq, 256), 256, 0, h->stream>>>(S, h->brick, nb0, nb1, nb2, Nq, src, sx[0],
                                                                                sx[1], sx[2], bin, rank, counts);
             if ((rc = exclusive_scan(h, counts, start, nbins, h->scan_tmp_lr))) return rc;
-            spread_bin_scatter_kernel<T><<<grid_for(Nq, 128), 128, 0, h->stream>>>(S, Nq, src, sx[0], sx[1], sx[2], bin, rank,
-                                                                                    start, (T*)h->binned.p, foot);
+            auto scatter = [&](auto* rows) {
+                using R = std::remove_pointer_t<decltype(rows)>;
+                spread_bin_scatter_kernel<R><<<grid_for(Nq, 128), 128, 0, h->stream>>>(S, Nq, src, sx[0], sx[1], sx[2], bin,
+                                                                                        rank, start, rows, foot);
+            };
+            auto columns = [&](auto* rows) {
+                scatter(rows);
+                spread_column_kernel<std::remove_pointer_t<decltype(rows)>, T><<<nblk, kColThreads, 0, h->stream>>>(
+                    S, nb0, nb1, nb2, start, rows, foot, grid);
+            };
             if (h->brick == 16) {
                 // plane-owner kernel (FP32 grids only)
+                scatter((T*)h->binned.p);
                 auto launch_plane = [&](void (*kern)(LRSizes, int, int, int, const int32_t*, const float*, const int32_t*,
                                                      float*), int P) {
                     const size_t psmem = sizeof(float) * 3 * kPlaneB * kPlaneB * (P == 8 ? PlaneLayout<8>::RX : PlaneLayout<4>::RX);
                     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem);
-                    kern<<<nblk, kPlaneThreads, psmem, h->stream>>>(S, nb0, nb1, nb2, start, (const float*)bsrc, foot,
+                    kern<<<nblk, kPlaneThreads, psmem, h->stream>>>(S, nb0, nb1, nb2, start, (const float*)h->binned.p, foot,
                                                                    (float*)grid);
                 };
                 launch_plane(S.m <= 2 ? spread_plane_kernel<4> : spread_plane_kernel<8>, S.m <= 2 ? 4 : 8);
+            } else if (h->rows64) {
+                columns((double*)h->binned.p);
             } else {
-                spread_column_kernel<T><<<nblk, kColThreads, 0, h->stream>>>(S, nb0, nb1, nb2, start, bsrc, foot, grid);
+                columns((T*)h->binned.p);
             }
             h->launches += 3;
         }

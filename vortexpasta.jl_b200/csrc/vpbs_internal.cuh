@@ -201,6 +201,7 @@ struct vpbs_handle {
     vpbs::DevBuf peer_in;                       // vpbs_add_field: a field copied from another GPU
     cudaEvent_t xfer_done = nullptr;            // vpbs_add_field: this handle's fields are complete
     int brick = 0;     // brick edge of the spreading (longrange_init)
+    bool rows64 = false;  // FP32 grid, spread with FP64 kernel rows and sums
     int spread_mode = 0;  // 0: tensor-core spreading where it applies; 1: CUDA-core kernels only
     int* status_host = nullptr;  // mapped pinned word: device-side faults of bounded waits (0: none)
     int* status_dev = nullptr;
