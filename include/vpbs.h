@@ -368,9 +368,10 @@ int vpbs_autotune(vpbs_handle* h, int32_t* chosen);
  * the handle's output fields.  Synchronous. */
 int vpbs_autotune_spread(vpbs_handle* h, int32_t* chosen);
 
-/* Spreading kernels of the FP32 (mixed) form for NUFFT half-supports m <= 4 on grids of 16^3 bricks:
- * mode 0 (default) multiplies each brick on the tensor cores (tcgen05, 3xTF32); mode 1 uses the CUDA
- * cores only (plane-owner kernel).  Tuning and testing support; no counterpart in the reference. */
+/* Spreading kernels.  Mode 0 (default): FP32 (mixed) grids of 16^3 bricks with half-support m <= 4 multiply each
+ * brick on the tensor cores (tcgen05, 3xTF32); elsewhere few points are added by atomics and many by bricks.
+ * Mode 1: bricks on the CUDA cores only (plane-owner and column kernels).  Tuning and testing support; no
+ * counterpart in the reference. */
 int vpbs_spread_mode(vpbs_handle* h, int32_t mode);
 
 /* A block edge for the pair kernel (0: the built-in rule).  Accepted and without effect, as in

@@ -27,9 +27,10 @@ def wobbly(vp, n, seed, spread=0.0):
     return np.stack([3 + r * np.cos(t), 2 + r * np.sin(t), 1 + 0.2 * np.sin(2 * t)], axis=1)
 
 
-def fields(vp, p, fs, names=("velocity", "streamfunction"), **kw):
+def fields(vp, p, fs, names=("velocity", "streamfunction"), spread_mode=0, **kw):
     cache = vp.init_cache(p)
     try:
+        assert cache._lib.vpbs_spread_mode(cache.handle, spread_mode) == 0
         out = {n: [np.zeros((len(f), 3)) for f in fs] for n in names}
         vp.compute_on_nodes_(out, cache, fs, **kw)
         counts = cache.pair_counts() if kw.get("shortrange", True) else None
@@ -89,13 +90,15 @@ def test_spline_solve_extreme_spacings(vp, oracle):
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("m", [1, 2, 3, 5, 6, 8])
-def test_window_widths_on_ragged_grids(vp, oracle, m, precision):
-    """FFT sizes 18, 30, 36 (bricks of 8 leave 2, 6 and 4 cells over): widths 2 .. 16, wider than a brick too."""
+@pytest.mark.parametrize("mode", [0, 1])
+def test_window_widths_on_ragged_grids(vp, oracle, m, precision, mode):
+    """FFT sizes 18, 30, 36 (bricks of 8 leave 2, 6 and 4 cells over): widths 2 .. 16, wider than a brick too; atomics
+    (which so few points take by themselves) and bricks."""
     sp = vp.GaussianSplitting(Ls=(L, L, L), alpha=5.0, rcut=L / 4, Ns=(12, 20, 24))
     p = vp.ParamsBiotSavart(Gamma=1.0, a=1e-8, splitting=sp, backend_long=vp.NonuniformFFTsBackend(1.5, m), precision=precision)
     fs = [wobbly(vp, n, n, 0.5) + np.array([dx, 0.0, dx]) for n, dx in ((40, 0.0), (64, 2.0), (23, 4.5))]
     v, s, _ = oracle.compute_on_nodes(p, fs, velocity=True, streamfunction=True, LIA=False, shortrange=False)
-    got, _ = fields(vp, p, fs, LIA=False, shortrange=False)
+    got, _ = fields(vp, p, fs, LIA=False, shortrange=False, spread_mode=mode)
     # mixed: 32-bit rounding of the transforms, 6e-8 times about four, which the deconvolution multiplies, once per
     # transform, by psi_hat(0) / psi_hat(k): 2.0 (m = 2) to 7 (m = 8) per dimension at the edge of the kept modes,
     # weighted by a filter that leaves e^{-k^2 / 4 alpha^2} = 0.7 there in one dimension (m = 8: 2.2e-6)
@@ -115,9 +118,34 @@ def test_mixed_sums_on_grids_without_whole_bricks(vp, m):
     for precision in ("fp64", "mixed"):
         sp = vp.GaussianSplitting(Ls=(L, L, L), alpha=1.7, rcut=L / 5, Ns=(12, 20, 24))
         p = vp.ParamsBiotSavart(Gamma=1.0, a=1e-8, splitting=sp, backend_long=vp.NonuniformFFTsBackend(1.5, m), precision=precision)
-        got[precision], _ = fields(vp, p, fs, LIA=False, shortrange=False)
+        got[precision], _ = fields(vp, p, fs, LIA=False, shortrange=False, spread_mode=1)
     for name in ("velocity", "streamfunction"):
         assert rel(got["mixed"][name], got["fp64"][name]) <= 1.5e-7, name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("Ns,m,nodes", [(12, 3, 4000), (36, 1, 20000), (36, 4, 1000)])
+def test_spreading_of_few_bricks_or_points_takes_atomics(vp, Ns, m, nodes):
+    """Grids of few bricks (18^3) or points (54^3), where a CTA per brick is slower by 1.4 to 20 times: the stage's
+    time by the default mode is well below that of the bricks."""
+    rng = np.random.default_rng(2)
+    fs = [vp.curves.ring(200, 0.6 + 0.6 * rng.random(), L * rng.random(3), vp.curves.random_rotation(rng)) for _ in range(nodes // 200)]
+    sp = vp.GaussianSplitting(Ls=L, alpha=2.0, rcut=L / 5, Ns=Ns)
+    cache = vp.init_cache(vp.ParamsBiotSavart(Gamma=1.0, a=1e-8, splitting=sp, backend_long=vp.NonuniformFFTsBackend(1.5, m)))
+    best = []
+    try:
+        cache.set_filaments(fs)
+        cache.stage_timing(True)
+        for mode in (0, 1):
+            assert cache._lib.vpbs_spread_mode(cache.handle, mode) == 0
+            times = []
+            for _ in range(8):
+                cache.compute(1, shortrange=False)
+                times.append(cache.stage_times()["spread"])
+            best.append(min(times[2:]))
+    finally:
+        cache.close()
+    assert best[0] < 0.85 * best[1]
 
 
 @pytest.mark.gpu

@@ -365,7 +365,7 @@ int vpbs_destroy(vpbs_handle* h) {
                       &h->grid_r, &h->grid_c, &h->grid_c2, &h->uhat, &h->decx, &h->decy, &h->decz, &h->nodes_lr,
                       &h->vel, &h->psi, &h->spread_bin, &h->spread_counts, &h->spread_start, &h->binned,
                       &h->spread_foot, &h->tc_counts, &h->tc_start, &h->tc_rec, &h->peer_in, &h->ewald_tab, &h->scan_tmp, &h->scan_tmp_lr, &h->rk_vs, &h->rk_tmp,
-                      &h->aos_out, &h->fil_off, &h->fft_tw};
+                      &h->aos_out, &h->fil_off, &h->fft_tw, &h->grid64};
     for (DevBuf* b : bufs) free_buf(*b);
     if (h->pin_in) cudaFreeHost(h->pin_in);
     if (h->status_host) cudaFreeHost(h->status_host);

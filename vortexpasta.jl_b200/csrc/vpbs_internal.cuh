@@ -195,6 +195,7 @@ struct vpbs_handle {
 
     // long range
     vpbs::LRSizes lr{};
+    vpbs::DevBuf grid64;  // sums of the atomic spreading of an FP32 grid
     vpbs::DevBuf grid_r, grid_c, grid_c2, uhat, decx, decy, decz, nodes_lr;
     vpbs::DevBuf spread_bin, spread_counts, spread_start, binned, spread_foot;  // brick spreading
     vpbs::DevBuf tc_counts, tc_start, tc_rec;  // tensor-core spreading: per-brick (point, brick) records
@@ -202,7 +203,7 @@ struct vpbs_handle {
     cudaEvent_t xfer_done = nullptr;            // vpbs_add_field: this handle's fields are complete
     int brick = 0;     // brick edge of the spreading (longrange_init)
     bool rows64 = false;  // FP32 grid, spread with FP64 kernel rows and sums
-    int spread_mode = 0;  // 0: tensor-core spreading where it applies; 1: CUDA-core kernels only
+    int spread_mode = 0;  // 0: tensor cores or atomics where they are faster; 1: bricks on the CUDA cores only
     int* status_host = nullptr;  // mapped pinned word: device-side faults of bounded waits (0: none)
     int* status_dev = nullptr;
     int nbrick[3] = {0, 0, 0};
