@@ -168,6 +168,20 @@ def test_pair_kernels(vp, oracle, nsubdiv, rcut, explicit, precision):
 
 
 @pytest.mark.gpu
+def test_mixed_pair_sums_of_many_pairs(vp):
+    """20,000 pairs a node, 600 a lane: the rounding of the 32-bit sums does not grow with them.  One sum per lane leaves
+    1.3e-7 (streamfunction) and 2.4e-7 (velocity); the weights and separations by themselves, 0.4e-7 and 1.0e-7."""
+    rng = np.random.default_rng(4)
+    fs = [vp.curves.ring(200, 0.8 + 0.7 * rng.random(), L * rng.random(3), vp.curves.random_rotation(rng)) for _ in range(500)]
+    got = {}
+    for precision in ("fp64", "mixed"):
+        p = params(vp, precision, L / 4, Ns=32)
+        got[precision], _ = fields(vp, p, fs, LIA=False, longrange=False)
+    assert rel(got["mixed"]["streamfunction"], got["fp64"]["streamfunction"]) <= 8e-8
+    assert rel(got["mixed"]["velocity"], got["fp64"]["velocity"]) <= 1.9e-7
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [5, 42, 43, 127, 128, 129, 700])
 def test_open_domain_sizes(vp, oracle, n):
     """One node block and its neighbours in size; 15 .. 2100 sources (tiles of 128, shared out over blocks)."""

@@ -576,8 +576,10 @@ __device__ __forceinline__ double tab_s_poly(const double* c, double t) {
 //    left out (the mixed form always takes their long-range part out explicitly).
 //  * Weights from cubic tables on 1/32-wide intervals in x = alpha r (FP32, ~3e-8 absolute),
 //    interval index without a conversion instruction.
-//  * Per-lane FP32 sums, FP32 warp reduction (the D x 3 sums halved from lane half to lane half), FP64
-//    output sums.
+//  * Per-lane FP32 sums over the rows of some kF32Flush evaluations per node, FP32 warp reduction (the D x 3 sums
+//    halved from lane half to lane half), FP64 output sums, so that the rounding does not grow with a node's
+//    pairs (20,000 a node: streamfunction error 1.3e-7 with one sum per lane, 0.5e-7 so, at the same time;
+//    asking after every 32 sources instead of every row costs 3 %).
 // blockIdx.y: the rows are dealt to gridDim.y warps where a system has too few nodes to fill the device.
 // Bound: issue slots (81 % busy, 10 warp instructions per pair in range; 1M nodes, 155 M pairs: 1.76 ms).
 // CTAs that stage tiles of a block's neighbourhood and take a node per warp at a time: 14 instructions per
@@ -586,6 +588,7 @@ __device__ __forceinline__ double tab_s_poly(const double* c, double t) {
 constexpr int kF32TabMax = 192;   // intervals per weight table (x = alpha r_cut <= 5.9)
 constexpr float kF32Band = 4e-6f; // relative band around r_cut^2 decided in FP64
 constexpr float kF32Far = 1e18f;  // coordinate of an absent node or source (its square is finite)
+constexpr int kF32Flush = 16;
 constexpr int kF32Warps = 4;
 constexpr int kF32Blocks = 8;  // CTAs per SM (64 registers)
 // A queue entry: the source's cell-sorted index and above it 2 bits each for its image in x, y and z (0, 1,
@@ -816,6 +819,29 @@ __global__ void __launch_bounds__(32 * kF32Warps, sizeof(E) == 4 ? kF32Blocks : 
 #pragma unroll
         for (int c = 0; c < 3; ++c) v[d][c] = w[d][c] = 0.0f;
     }
+    // the lanes' FP32 sums to the FP64 outputs
+    const double pref = K.Gamma / (4.0 * kPi);
+    const int slot = lane / (32 / D);
+    const int is = __shfl_sync(0xffffffffu, i, slot);
+    int nev = 0;  // evaluations since the last flush (warp-uniform)
+    auto flush = [&]() {
+        float out[3];
+        if (VEL) {
+            group_reduce<D>(v, lane, out);
+            if (lane % (32 / D) == 0 && is >= 0)
+                for (int c = 0; c < 3; ++c) atomicAdd(&vel[c * Np + is], pref * (double)out[c]);
+        }
+        if (PSI) {
+            group_reduce<D>(w, lane, out);
+            if (lane % (32 / D) == 0 && is >= 0)
+                for (int c = 0; c < 3; ++c) atomicAdd(&psi[c * Np + is], pref * (double)out[c]);
+        }
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[d][c] = w[d][c] = 0.0f;
+        nev = 0;
+    };
     int turn = 0;  // rows seen so far: dealt to the gridDim.y warps of the group in turn
     // the nodes of one (y, z) row of cells within r_cut in x at a time (nearly always all of them)
     for (unsigned todo = __ballot_sync(0xffffffffu, lane < nd); todo;) {
@@ -878,6 +904,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, sizeof(E) == 4 ? kF32Blocks : 
                                 __syncwarp();
                                 f32_eval<VEL, PSI, E>(S, d, lane, true, srcP, srcQ, srcR, tab, rc2lo, rc2hi, K.rcut2, alpha, nf, v[d],
                                                    w[d], ninr);
+                                ++nev;
                                 cnt[d] -= 32;
                                 __syncwarp();
                                 if (lane < cnt[d]) S.queue[d][lane] = S.queue[d][32 + lane];
@@ -886,6 +913,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, sizeof(E) == 4 ? kF32Blocks : 
                         }
                     }
                 }
+                if (nev >= kF32Flush * D) flush();
             }
         }
         }
@@ -896,20 +924,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, sizeof(E) == 4 ? kF32Blocks : 
         if (cnt[d] > 0)  // warp-uniform
             f32_eval<VEL, PSI, E>(S, d, lane < cnt[d] ? lane : 0, lane < cnt[d], srcP, srcQ, srcR, tab, rc2lo, rc2hi, K.rcut2, alpha, nf,
                                v[d], w[d], ninr);
-    const double pref = K.Gamma / (4.0 * kPi);
-    const int slot = lane / (32 / D);
-    const int is = __shfl_sync(0xffffffffu, i, slot);
-    float out[3];
-    if (VEL) {
-        group_reduce<D>(v, lane, out);
-        if (lane % (32 / D) == 0 && is >= 0)
-            for (int c = 0; c < 3; ++c) atomicAdd(&vel[c * Np + is], pref * (double)out[c]);
-    }
-    if (PSI) {
-        group_reduce<D>(w, lane, out);
-        if (lane % (32 / D) == 0 && is >= 0)
-            for (int c = 0; c < 3; ++c) atomicAdd(&psi[c * Np + is], pref * (double)out[c]);
-    }
+    flush();
     const unsigned long long total = warp_sum_u((unsigned long long)ninr);
     if (lane == 0) {
         atomicAdd(&counters[0], total);
