@@ -283,6 +283,10 @@ int vpbs_kb_weights(double beta, double rcut, double rtol, const double* r, int6
 int vpbs_f32_weights_eval(int32_t splitting, double alpha, double rcut, double kb_beta, double kb_rtol, const double* r,
                           int64_t n, float* a, float* g);
 
+/* The same for the FP64 pair kernel's weights (degree-5 tables on 1/128-wide intervals). */
+int vpbs_f64_weights_eval(int32_t splitting, double alpha, double rcut, double kb_beta, double kb_rtol, const double* r,
+                          int64_t n, double* a, double* g);
+
 /* Host evaluation of the device's periodic helpers (the same inline code, periodic.cuh): x folded
  * into [0, L) (min_distance.jl:5-20; O(1) for any x, NaN for a non-finite x) and the cell index
  * trunc(folded / L * nc) clamped to [0, nc) (CellLists.jl:194-204, 0-based), or the sentinel nc for

@@ -206,6 +206,41 @@ def test_f32_pair_weights(vp, built_lib, case):
     assert np.abs(g - eg).max() < 2e-7
 
 
+@pytest.mark.parametrize("beta", [2.5, 4.0, 6.0])
+def test_f64_pair_weights(vp, built_lib, beta):
+    """The FP64 pair kernel's weights (degree-5 tables on 1/128-wide intervals) against extended precision: no further
+    off than the degree-9 tables of the other kernels, 1.1e-16 (erfc) and 1.9e-16 (velocity weight, gaussian.jl:273-279):
+    half a unit in the last place of 1 and the rounding of x, whose factor in the weight is at most 0.83."""
+    from vortexpasta_b200 import _lib
+    lib = _lib.load()
+    erfcl = ct.CDLL("libm.so.6").erfcl
+    erfcl.argtypes, erfcl.restype = [ct.c_longdouble], ct.c_longdouble
+    r = np.concatenate([np.linspace(0.0, 1.0, 5001), np.random.default_rng(1).random(30000)])
+    x = (beta * r).astype(np.longdouble)
+    ea = np.array([erfcl(v) for v in x], dtype=np.longdouble)
+    eg = ea + 2 / np.sqrt(np.longdouble(np.pi) + np.longdouble(1.2246467991473532e-16)) * x * np.exp(-x * x)
+    a, g = np.zeros(len(r)), np.zeros(len(r))
+    assert lib.vpbs_f64_weights_eval(0, beta, 1.0, 0.0, 0.0, _lib.dptr(r), len(r), _lib.dptr(a), _lib.dptr(g)) == 0
+    assert np.abs(a - ea).max() <= 1.25e-16
+    assert np.abs(g - eg).max() <= 2.1e-16
+
+
+@pytest.mark.parametrize("beta", [12.44, 30.0])
+def test_f64_pair_weights_kaiser_bessel(vp, built_lib, beta):
+    """The same for the Kaiser-Bessel splitting, against its truncated Chebyshev series (kaiser_bessel.jl:139-147) summed
+    in FP64, which by itself is off by some units in the last place of 1."""
+    from vortexpasta_b200 import _lib
+    lib = _lib.load()
+    rtol = 10 ** (-0.2) * math.exp(-beta)
+    rcut = 0.3
+    r = np.sort(np.random.default_rng(2).random(20000)) * rcut
+    a, g, sa, sg = (np.zeros(len(r)) for _ in range(4))
+    args = (_lib.dptr(r), len(r))
+    assert lib.vpbs_f64_weights_eval(1, 0.0, rcut, beta, rtol, *args, _lib.dptr(a), _lib.dptr(g)) == 0
+    assert lib.vpbs_kb_weights(beta, rcut, rtol, *args, None, None, _lib.dptr(sa), _lib.dptr(sg)) == 0
+    assert np.abs(a - sa).max() <= 2e-15 and np.abs(g - sg).max() <= 2e-15
+
+
 def _host_copies(lib, dsts, srcs):
     from vortexpasta_b200 import _lib  # noqa: F401
     n = len(dsts)

@@ -154,6 +154,13 @@ int process_point_charges(vpbs_handle* h) {
 
 using namespace vpbs;
 
+// Both pair weights at x in extended precision: of the Kaiser-Bessel series S over x = (xmax / rcut) r, or the
+// Gaussian ones where there is none.
+static WeightsL pair_weights_l(const KBSeries& S, double xmax) {
+    if (S.f.empty()) return gaussian_weights_l;
+    return [&S, xmax](long double x, long double* a, long double* g) { kb_weights_series_l(S, x * S.rcut / xmax, a, g); };
+}
+
 extern "C" {
 
 const char* vpbs_last_error(const vpbs_handle* h) { return h ? h->err.c_str() : g_create_error.c_str(); }
@@ -267,8 +274,9 @@ int vpbs_create(const vpbs_params* params, vpbs_handle** out) {
         // fitted to the truncated Chebyshev series for the Kaiser-Bessel kernel
         int ntab = 0;
         std::vector<double> tab;
+        KBSeries S;
         if (kb) {
-            const KBSeries S = kb_series(P.kb_beta, P.rcut, P.kb_rtol);
+            S = kb_series(P.kb_beta, P.rcut, P.kb_rtol);
             if (S.f.empty()) rc = set_error(h, VPBS_ERR_PARAMS, "KaiserBesselSplitting: Chebyshev series did not converge");
             kb_table_host(S, &ntab, nullptr);
             tab.resize((size_t)2 * ntab * kEwaldNC);
@@ -297,13 +305,15 @@ int vpbs_create(const vpbs_params* params, vpbs_handle** out) {
         f32_table_host(tab.data(), ntab, xmax_c, tabc.data());
         const size_t bytes_d = sizeof(double) * tab.size(), bytes_f = sizeof(float) * tabf.size();
         const size_t off_c = (2 * bytes_d + bytes_f + 15) / 16 * 16, bytes_c = sizeof(float4) * tabc.size();
-        // FP64 tables of the cell-tiled pair kernel, stored after the FP32 cubic ones (16-byte multiples)
-        const int ntab_s = tab_s_size(xmax_c);
+        // FP64 tables of the FP64 pair kernel, stored after the FP32 cubic ones (16-byte multiples)
+        // unless the FP32 one serves this handle
+        const bool f32_pairs = P.precision == VPBS_PRECISION_MIXED && P.nsubdiv > 0 && ntab_c <= kF32TabMax;
+        const int ntab_s = f32_pairs ? 0 : tab_s_size(xmax_c);
         std::vector<double> tabs((size_t)2 * ntab_s * kTabSNC);
-        tab_s_host(tab.data(), ntab, xmax_c, tabs.data());
+        if (ntab_s) tab_s_host(pair_weights_l(S, xmax_c), xmax_c, tabs.data());
         const size_t off_s = off_c + bytes_c, bytes_s = sizeof(double) * tabs.size();
         if (!rc) rc = ensure(h, h->ewald_tab, off_s + bytes_s, "Ewald tables");
-        if (!rc)
+        if (!rc && ntab_s)
             rc = check_cuda(h, cudaMemcpy((char*)h->ewald_tab.p + off_s, tabs.data(), bytes_s, cudaMemcpyHostToDevice),
                             "copy Ewald tables");
         if (!rc)
@@ -1159,6 +1169,28 @@ extern "C" int vpbs_f32_weights_eval(int32_t splitting, double alpha, double rcu
         if (!(r[i] >= 0.0 && r[i] <= rcut)) return set_error(nullptr, VPBS_ERR_ARG, "vpbs_f32_weights_eval: r outside [0, rcut]");
         // the kernel forms x = (r^2 rsqrt(r^2)) alpha in FP32; here x = alpha r rounded to FP32
         f32_table_eval_host(tabc.data(), nf, (float)(s * r[i]), &a[i], &g[i]);
+    }
+    return 0;
+}
+
+extern "C" int vpbs_f64_weights_eval(int32_t splitting, double alpha, double rcut, double kb_beta, double kb_rtol,
+                                     const double* r, int64_t n, double* a, double* g) {
+    using namespace vpbs;
+    if (!r || !a || !g || n < 0 || !(rcut > 0)) return set_error(nullptr, VPBS_ERR_ARG, "vpbs_f64_weights_eval: bad arguments");
+    const bool kb = splitting == VPBS_SPLITTING_KAISER_BESSEL;
+    if (!kb && !(alpha > 0)) return set_error(nullptr, VPBS_ERR_ARG, "vpbs_f64_weights_eval: alpha must be positive");
+    KBSeries S;
+    if (kb) {
+        S = kb_series(kb_beta, rcut, kb_rtol);
+        if (S.f.empty()) return set_error(nullptr, VPBS_ERR_PARAMS, "Kaiser-Bessel series did not converge");
+    }
+    const double xmax = kb ? kb_table_xmax(kb_beta) : alpha * rcut, s = xmax / rcut;
+    const int nf = tab_s_size(xmax);
+    std::vector<double2> tab((size_t)nf * kTabSNC);  // both tables (16-byte aligned)
+    tab_s_host(pair_weights_l(S, xmax), xmax, (double*)tab.data());
+    for (int64_t i = 0; i < n; ++i) {
+        if (!(r[i] >= 0.0 && r[i] <= rcut)) return set_error(nullptr, VPBS_ERR_ARG, "vpbs_f64_weights_eval: r outside [0, rcut]");
+        tab_s_eval_host((const double*)tab.data(), nf, s * r[i], &a[i], &g[i]);
     }
     return 0;
 }

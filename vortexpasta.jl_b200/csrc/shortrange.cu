@@ -546,16 +546,23 @@ __device__ __forceinline__ void ewald_weights2(const KParams& K, double x, doubl
     }
 }
 
-// Interval and local coordinate of x in the shared-memory tables (intervals centred at k / 96):
-// k = round(96 x) by the 1.5 * 2^52 trick, t = 96 x - k in [-1/2, 1/2].
-__device__ __forceinline__ double tab_s_pos(double x, int ntab, int* k) {
+// Interval and local coordinate of x in the shared-memory tables (intervals centred at k / 128):
+// k = round(128 x) by the 1.5 * 2^52 trick, t = 128 x - k in [-1/2, 1/2].
+__host__ __device__ __forceinline__ double tab_s_pos(double x, int ntab, int* k) {
     const double y = fma(x, kTabSInvH, 6755399441055744.0);
-    const unsigned kk = (unsigned)__double2loint(y), top = (unsigned)(ntab - 1);
+#if defined(__CUDA_ARCH__)
+    const unsigned kk = (unsigned)__double2loint(y);
+#else
+    uint64_t bits;
+    std::memcpy(&bits, &y, sizeof bits);
+    const unsigned kk = (unsigned)bits;
+#endif
+    const unsigned top = (unsigned)(ntab - 1);
     *k = (int)(kk < top ? kk : top);
     return fma(x, kTabSInvH, -(y - 6755399441055744.0));
 }
 
-__device__ __forceinline__ double tab_s_poly(const double* c, double t) {
+__host__ __device__ __forceinline__ double tab_s_poly(const double* c, double t) {
     const double2* v = reinterpret_cast<const double2*>(c);
     const double2 c0 = v[0], c1 = v[1], c2 = v[2];
     return fma(fma(fma(fma(fma(c2.y, t, c2.x), t, c1.y), t, c1.x), t, c0.y), t, c0.x);
@@ -585,7 +592,6 @@ __device__ __forceinline__ double tab_s_poly(const double* c, double t) {
 // CTAs that stage tiles of a block's neighbourhood and take a node per warp at a time: 14 instructions per
 // pair, a fifth of the time at barriers, 2.89 ms.  D = 4 at 64 registers (32 warps per SM) against D = 8 at
 // 80: 2.09 ms, at 128: 2.48, D = 2: 2.18; evaluating a chunk as soon as one lane is in range, unqueued: 2.89.
-constexpr int kF32TabMax = 192;   // intervals per weight table (x = alpha r_cut <= 5.9)
 constexpr float kF32Band = 4e-6f; // relative band around r_cut^2 decided in FP64
 constexpr float kF32Far = 1e18f;  // coordinate of an absent node or source (its square is finite)
 constexpr int kF32Flush = 16;
@@ -937,8 +943,9 @@ __global__ void __launch_bounds__(32 * kF32Warps, sizeof(E) == 4 ? kF32Blocks : 
 // (cell-sorted arrays), decides r^2 <= r_cut^2 and evaluates in FP64 (Newton-refined reciprocal square root,
 // weights from degree-5 tables in shared memory, one copy per CTA).  SKIP: the node's own two segments left
 // out.  Bound: shared-memory and L1 wavefronts of the gathers (per 32 pairs about 30 for the weights' three
-// 16-byte loads and 30 for the sources), then the FP64 pipe (17 cycles).  1M nodes, 3.13 G pairs: 26.8 ms (CTAs
-// that stage tiles of a block's neighbourhood: 39.5); 20k nodes, both fields: 0.205 (0.517).  Three CTAs per SM of
+// 16-byte loads and 30 for the sources), then the FP64 pipe (17 cycles).  1M nodes, 3.13 G pairs: 27.6 ms (CTAs
+// that stage tiles of a block's neighbourhood: 39.5; weight tables a quarter shorter, of 1/96, which leave more L1:
+// 26.8); 20k nodes, both fields: 0.205 (0.517).  With those tables, three CTAs per SM of
 // 80 registers: 28.7, two of 128: 30.6; both fields in four of 64: 0.217.
 constexpr int kF64Warps = 8;
 // CTAs per SM: 64 registers for one field (some spilled outside the loops), 80 for both
@@ -1344,10 +1351,18 @@ void table_eval_host(const double* tab, int ntab, double x, double* a, double* g
 
 int tab_s_size(double xmax) { return (int)std::floor(xmax * kTabSInvH) + 2; }
 
-// Degree-5 interpolants of both weights on every interval centred at k / 96, through the values of the
-// FP64 table at the 6 Chebyshev points of the interval, in powers of t = 96 x - k (error below 2e-16 for
-// the Gaussian weights).
-void tab_s_host(const double* tab, int ntab, double xmax, double* out) {
+// Both weights of the Gaussian splitting in extended precision (gaussian.jl:273-279).
+void gaussian_weights_l(long double x, long double* a, long double* g) {
+    const long double two_over_sqrt_pi = 1.12837916709551257390L;
+    *a = std::erfc(x);
+    *g = *a + two_over_sqrt_pi * x * std::exp(-x * x);
+}
+
+// Degree-5 interpolants of both weights on every interval centred at k / 128, through their values at the 6
+// Chebyshev points of the interval, in powers of t = 128 x - k.  Largest error over [0, 4],
+// Gaussian weights: 1.1e-16 (erfc) and 1.9e-16 (velocity weight), as of the degree-9 tables, root mean squares 2.1e-17
+// and 2.9e-17 (2.2e-17, 3.7e-17).  Intervals of 1/96 fitted to values rounded to FP64: 2.2e-16 and 3.7e-16.
+void tab_s_host(const WeightsL& weights, double xmax, double* out) {
     constexpr int NC = kTabSNC;
     const int nf = tab_s_size(xmax);
     long double T[NC], A[NC][NC];
@@ -1367,8 +1382,8 @@ void tab_s_host(const double* tab, int ntab, double xmax, double* out) {
     for (int k = 0; k < nf; ++k) {
         long double cf[2][NC] = {};
         for (int j = 0; j < NC; ++j) {
-            double a, g;
-            table_eval_host(tab, ntab, (double)((k + T[j]) / (long double)kTabSInvH), &a, &g);
+            long double a, g;
+            weights((k + T[j]) / (long double)kTabSInvH, &a, &g);
             for (int n = 0; n < NC; ++n) {
                 cf[0][n] += A[j][n] * a;
                 cf[1][n] += A[j][n] * g;
@@ -1377,6 +1392,13 @@ void tab_s_host(const double* tab, int ntab, double xmax, double* out) {
         for (int w = 0; w < 2; ++w)
             for (int n = 0; n < NC; ++n) out[((size_t)w * nf + k) * NC + n] = (double)cf[w][n];
     }
+}
+
+void tab_s_eval_host(const double* tab, int nf, double x, double* a, double* g) {
+    int k;
+    const double t = tab_s_pos(x, nf, &k);
+    *a = tab_s_poly(tab + (size_t)k * kTabSNC, t);
+    *g = tab_s_poly(tab + (size_t)(nf + k) * kTabSNC, t);
 }
 
 int f32_table_size(double xmax) { return (int)std::floor(xmax * kTabCInvH) + 2; }

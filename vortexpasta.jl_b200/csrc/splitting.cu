@@ -21,11 +21,12 @@ namespace vpbs {
 namespace {
 
 // Clenshaw evaluation of sum_k c_k T_k(u).
-double cheb_eval(const std::vector<double>& c, double u) {
+template <typename R>
+R cheb_eval(const std::vector<double>& c, R u) {
     if (c.empty()) return 0.0;
-    double b1 = 0.0, b2 = 0.0;
+    R b1 = 0.0, b2 = 0.0;
     for (int k = (int)c.size() - 1; k >= 1; --k) {
-        const double b = 2.0 * u * b1 + c[k] - b2;
+        const R b = 2.0 * u * b1 + c[k] - b2;
         b2 = b1;
         b1 = b;
     }
@@ -100,6 +101,12 @@ KBSeries kb_series(double beta, double rcut, double rtol) {
 void kb_weights_series(const KBSeries& S, double r, double* a, double* g) {
     const double u = r / S.rcut;
     const double A = 1.0 - cheb_eval(S.F, u);
+    *a = A;
+    *g = A + r * cheb_eval(S.f, u);
+}
+
+void kb_weights_series_l(const KBSeries& S, long double r, long double* a, long double* g) {
+    const long double u = r / S.rcut, A = 1.0L - cheb_eval(S.F, u);
     *a = A;
     *g = A + r * cheb_eval(S.f, u);
 }

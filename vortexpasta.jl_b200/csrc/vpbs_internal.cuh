@@ -5,6 +5,7 @@
 #include <cufft.h>
 
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -37,8 +38,8 @@ struct KParams {
     // (c0, c1, c2, c3) in powers of t = 32 x - k per interval k; weight a then weight g
     const float4* tab_c;
     int ntab_c;
-    // FP64 tables of the cell-tiled pair kernel, read from shared memory: intervals centred at k / 96 in
-    // x, kTabSNC coefficients in powers of t = 96 x - k; weight a then weight g
+    // FP64 tables of pair_f64_kernel, read from shared memory: intervals centred at k / 128 in x, kTabSNC
+    // coefficients in powers of t = 128 x - k; weight a then weight g
     const double* tab_s;
     int ntab_s;
 };
@@ -55,16 +56,21 @@ int ewald_table_size(double xmax);
 void table_eval_host(const double* tab, int ntab, double x, double* a, double* g);
 // FP32 cubic tables fitted to an FP64 table over [0, xmax] (layout of KParams::tab_c): nf intervals.
 constexpr float kTabCInvH = 32.0f;
+constexpr int kF32TabMax = 192;  // intervals that the FP32 pair kernel takes (x = alpha r_cut <= 5.9)
 int f32_table_size(double xmax);
 void f32_table_host(const double* tab, int ntab, double xmax, float4* out);  // out: 2 * f32_table_size(xmax)
 // Device-identical host evaluation of the FP32 cubic tables (same float operations).
 void f32_table_eval_host(const float4* tabc, int nf, float x, float* a, float* g);
 
-// FP64 tables of KParams::tab_s fitted to an FP64 table over [0, xmax]: 2 tab_s_size(xmax) kTabSNC values.
-constexpr double kTabSInvH = 96.0;
+// FP64 tables of KParams::tab_s over [0, xmax], fitted to weights given in extended precision (a and g at x):
+// 2 tab_s_size(xmax) kTabSNC values.
+constexpr double kTabSInvH = 128.0;
 constexpr int kTabSNC = 6;
+using WeightsL = std::function<void(long double x, long double* a, long double* g)>;
+void gaussian_weights_l(long double x, long double* a, long double* g);
 int tab_s_size(double xmax);
-void tab_s_host(const double* tab, int ntab, double xmax, double* out);
+void tab_s_host(const WeightsL& weights, double xmax, double* out);
+void tab_s_eval_host(const double* tab, int nf, double x, double* a, double* g);  // as the kernel does
 
 // Gauss-Legendre rule on [-1, 1] (host; longrange.cu).
 void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w);
@@ -78,6 +84,7 @@ struct KBSeries {
 };
 KBSeries kb_series(double beta, double rcut, double rtol);
 void kb_weights_series(const KBSeries& S, double r, double* a, double* g);
+void kb_weights_series_l(const KBSeries& S, long double r, long double* a, long double* g);
 double kb_table_xmax(double beta);
 void kb_table_host(const KBSeries& S, int* ntab, double* tab);
 
