@@ -211,7 +211,8 @@ int vpbs_get_uhat(vpbs_handle* h, double* out, int64_t n_doubles);
 int vpbs_get_pointdata(vpbs_handle* h, int32_t which, void* out, int64_t n_elems);
 
 /* Short-range counters of the last computation: in-range pairs (r^2 <= r_cut^2) and
- * examined candidate pairs.  Synchronises the handle's stream. */
+ * candidate pairs, those of a node and a source whose distance was formed (how many depends on which nodes share
+ * a warp of the pair kernel).  Synchronises the handle's stream. */
 int vpbs_pair_counts(vpbs_handle* h, int64_t* in_range, int64_t* candidates);
 
 /* Oversampled FFT grid size chosen for Ns modes at oversampling sigma (smallest even

@@ -168,6 +168,18 @@ def test_pair_kernels(vp, oracle, nsubdiv, rcut, explicit, precision):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("names", [("velocity",), ("velocity", "streamfunction")])
+def test_candidates_are_pairs(vp, precision, names):
+    """Node counts that do not fill the groups of 4 or 2 nodes a warp takes, and nodes apart from one another in a group:
+    only pairs of nodes that are there are counted as candidates, so never more than there are."""
+    for fs in ([wobbly(vp, 5, 1)], [wobbly(vp, 5, k) + np.array([0.0, 0.3 * k, 2.0 * k]) for k in range(3)]):
+        _, (pairs, candidates) = fields(vp, params(vp, precision, 0.39 * L), fs, names, LIA=False, longrange=False)
+        n = sum(map(len, fs))
+        assert pairs <= candidates <= n * 3 * n
+
+
+@pytest.mark.gpu
 def test_mixed_pair_sums_of_many_pairs(vp):
     """20,000 pairs a node, 600 a lane: the rounding of the 32-bit sums does not grow with them.  One sum per lane leaves
     1.3e-7 (streamfunction) and 2.4e-7 (velocity); the weights and separations by themselves, 0.4e-7 and 1.0e-7."""

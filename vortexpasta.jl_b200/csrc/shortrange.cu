@@ -855,7 +855,8 @@ __global__ void __launch_bounds__(32 * kF32Warps, sizeof(E) == 4 ? kF32Blocks : 
         const int gy_ = __shfl_sync(0xffffffffu, cy, lead), gz_ = __shfl_sync(0xffffffffu, cz, lead);
         const double xlead = __shfl_sync(0xffffffffu, x[0], lead);
         const bool mine = (todo >> lane & 1) && cy == gy_ && cz == gz_ && fabs(x[0] - xlead) <= K.rcut;
-        todo &= ~__ballot_sync(0xffffffffu, mine);
+        const unsigned members = __ballot_sync(0xffffffffu, mine);
+        todo &= ~members;
         float lo[3], hi[3];
         group_box<D>(mine, x, slack, lo, hi);
         for (int r0 = 0; r0 < W * W; r0 += 32) {  // a lane per row of cells around the nodes' own
@@ -883,7 +884,7 @@ __global__ void __launch_bounds__(32 * kF32Warps, sizeof(E) == 4 ? kF32Blocks : 
                     reinterpret_cast<float*>(S.z2)[lane] = mine ? S.x[lane][2][mz].x : kF32Far;
                 }
                 __syncwarp();
-                ncand += (unsigned)(rb - ra) * D;
+                ncand += (unsigned)(rb - ra) * __popc(members);
                 const E code = (E)(mx | my << 2 | mz << 4) << kIndexBits<E>;
                 float4 pn = __ldg(srcP + min(ra + lane, rb - 1));
                 for (int base = ra; base < rb; base += 32) {
@@ -1058,7 +1059,8 @@ __global__ void __launch_bounds__(32 * kF64Warps, f64_blocks(VEL && PSI)) pair_f
         const int gy_ = __shfl_sync(0xffffffffu, cy, lead), gz_ = __shfl_sync(0xffffffffu, cz, lead);
         const double xlead = __shfl_sync(0xffffffffu, x[0], lead);
         const bool mine = (todo >> lane & 1) && cy == gy_ && cz == gz_ && fabs(x[0] - xlead) <= K.rcut;
-        todo &= ~__ballot_sync(0xffffffffu, mine);
+        const unsigned members = __ballot_sync(0xffffffffu, mine);
+        todo &= ~members;
         float lo[3], hi[3];
         group_box<D>(mine, x, slack, lo, hi);
         for (int r0 = 0; r0 < W * W; r0 += 32) {  // a lane per row of cells around the nodes' own
@@ -1086,7 +1088,7 @@ __global__ void __launch_bounds__(32 * kF64Warps, f64_blocks(VEL && PSI)) pair_f
                     reinterpret_cast<float*>(S.z2)[lane] = mine ? (float)S.x[lane][2][mz] : kF32Far;
                 }
                 __syncwarp();
-                ncand += (unsigned)(rb - ra) * D;
+                ncand += (unsigned)(rb - ra) * __popc(members);
                 const E code = (E)(mx | my << 2 | mz << 4) << kIndexBits<E>;
                 float4 pn = __ldg(srcP + min(ra + lane, rb - 1));
                 for (int base = ra; base < rb; base += 32) {
