@@ -379,6 +379,10 @@ int vpbs_autotune_spread(vpbs_handle* h, int32_t* chosen);
  * counterpart in the reference. */
 int vpbs_spread_mode(vpbs_handle* h, int32_t mode);
 
+/* Width of the pair kernels' queue entries in bits: 0 by the number of sources (32 below 2^26), 64 always.  Testing
+ * support; no counterpart in the reference. */
+int vpbs_pair_entries(vpbs_handle* h, int32_t bits);
+
 /* A block edge for the pair kernel (0: the built-in rule).  Accepted and without effect, as in
  * vpbs_autotune.  Tuning support; no counterpart in the reference. */
 int vpbs_pair_block(vpbs_handle* h, int32_t cells);

@@ -16,7 +16,9 @@ SIZES = [((6, 6, 6), 1.3), ((12, 17, 31), 1.5), ((32, 20, 18), 1.5), ((50, 30, 3
          ((54, 100, 25), 1.25), ((120, 16, 12), 2.0), ((16, 160, 14), 1.5), ((14, 12, 192), 1.5), ((256, 12, 10), 1.5),
          ((12, 256, 12), 1.5), ((10, 14, 256), 1.5), ((20, 12, 512), 1.5), ((400, 10, 12), 1.25), ((12, 10, 500), 1.25),
          # tiles of one line; lines too long for a block and a packed length of one factor (cuFFT)
-         ((12, 10, 1360), 1.5), ((12, 10, 1500), 1.5), ((6, 12, 10), 1.5)]
+         ((12, 10, 1360), 1.5), ((12, 10, 1500), 1.5), ((6, 12, 10), 1.5),
+         # z lines of 1024 (two passes in FP32) and 1620 (too many threads for three components: cuFFT)
+         ((12, 10, 682), 1.5), ((12, 10, 1080), 1.5)]
 
 
 def system(vp):

@@ -27,9 +27,10 @@ def wobbly(vp, n, seed, spread=0.0):
     return np.stack([3 + r * np.cos(t), 2 + r * np.sin(t), 1 + 0.2 * np.sin(2 * t)], axis=1)
 
 
-def fields(vp, p, fs, names=("velocity", "streamfunction"), spread_mode=0, **kw):
+def fields(vp, p, fs, names=("velocity", "streamfunction"), spread_mode=0, entry_bits=0, **kw):
     cache = vp.init_cache(p)
     try:
+        assert cache._lib.vpbs_pair_entries(cache.handle, entry_bits) == 0
         assert cache._lib.vpbs_spread_mode(cache.handle, spread_mode) == 0
         out = {n: [np.zeros((len(f), 3)) for f in fs] for n in names}
         vp.compute_on_nodes_(out, cache, fs, **kw)
@@ -165,6 +166,56 @@ def test_pair_kernels(vp, oracle, nsubdiv, rcut, explicit, precision):
                 assert rel(got[n], want) <= TOL[precision], (n, names)
         if precision == "fp64":
             assert counts[0] == st["pairs_in_range"]
+
+
+def pairs_in_range(oracle, p, fs):
+    """The pair count of the CPU restatement; the mixed form always leaves a node's own two segments out."""
+    from copy import copy
+    q = copy(p)
+    if p.precision == "mixed":
+        q.avoid_explicit_erf = False
+    return oracle.compute_on_nodes(q, fs, velocity=True, streamfunction=True, LIA=False, longrange=False)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("Ls,rcut", [((L, L, L), L / 3), ((L, 0.7 * L, 1.6 * L), 0.2 * L), ((L, L, 2.5 * L), L / 12),
+                                     ((L, L, L), L / 60), ((0.3 * L, L, L), L / 40)])
+@pytest.mark.parametrize("entry_bits", [0, 64])
+def test_pair_counts(vp, oracle, Ls, rcut, precision, entry_bits):
+    """The same pairs as the CPU restatement, also in the mixed form, whose screen and decision are in 32 bits: periods of
+    different lengths, and cut-offs so short that the 32-bit places are coarse beside them (L / 60: margin 8e-5 of
+    r_cut^2).  The queue entries of systems above 2^26 sources too."""
+    rng = np.random.default_rng(5)
+    fs = [vp.curves.ring(n, 0.2 + 0.7 * rng.random(), np.array(Ls) * rng.random(3), vp.curves.random_rotation(rng))
+          for n in (64, 150, 33, 400, 7, 250, 250)]
+    sp = vp.GaussianSplitting(Ls=Ls, alpha=3.4 / rcut, rcut=rcut, Ns=(16, 16, 16))
+    p = vp.ParamsBiotSavart(Gamma=1.1, a=1e-8, splitting=sp, backend_long=vp.NonuniformFFTsBackend(1.5, 4), precision=precision)
+    v, s, st = pairs_in_range(oracle, p, fs)
+    for names in (("velocity", "streamfunction"), ("velocity",), ("streamfunction",)):
+        got, counts = fields(vp, p, fs, names, entry_bits=entry_bits, LIA=False, longrange=False)
+        assert counts[0] == st["pairs_in_range"]
+        for n, want in (("velocity", v), ("streamfunction", s)):
+            if n in names:
+                assert rel(got[n], want) <= TOL[precision], (n, names)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("beta,names", [(12.0, ("velocity", "streamfunction")), (18.0, ("velocity", "streamfunction")),
+                                        (18.0, ("streamfunction",)), (35.0, ("velocity",))])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_pairs_with_long_weight_tables(vp, oracle, beta, names, precision):
+    """alpha r_cut beyond what the kernels keep in shared memory: 5.9 for the FP32 one (the mixed form takes the FP64
+    one), 16.6 for both fields and 33.3 for one in the FP64 one (a warp per node with tables in global memory)."""
+    fs = [wobbly(vp, n, n, 1.0) + np.array(o) for n, o in ((64, (-3, -2, -1)), (37, (3.2, 4.2, 5.2)), (150, (0, 0, 0)))]
+    sp = vp.GaussianSplitting(Ls=L, alpha=beta / (L / 4), rcut=L / 4, Ns=16)
+    p = vp.ParamsBiotSavart(Gamma=1.1, a=1e-8, splitting=sp, backend_long=vp.NonuniformFFTsBackend(1.5, 4), precision=precision)
+    v, s, st = pairs_in_range(oracle, p, fs)
+    got, counts = fields(vp, p, fs, names, LIA=False, longrange=False)
+    assert counts[0] == st["pairs_in_range"]
+    for n, want in (("velocity", v), ("streamfunction", s)):
+        if n in names:
+            assert rel(got[n], want) <= TOL[precision], n
 
 
 @pytest.mark.gpu

@@ -1534,7 +1534,7 @@ int pair_interactions(vpbs_handle* h, int fields) {
     if (h->cg.M > 0 && (use_f32_pairs(h) || tab_bytes <= kPairSmemMost)) {
         int nsm = 148;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-        const bool f32 = use_f32_pairs(h), big = Nq >= (int64_t)1 << kIndexBits<uint32_t>;
+        const bool f32 = use_f32_pairs(h), big = h->wide_entries || Nq >= (int64_t)1 << kIndexBits<uint32_t>;
         const int Wc = 2 * h->cg.M + 1, D = v && p ? 2 : 4, warps = f32 ? kF32Warps : kF64Warps;
         const unsigned nblk = grid_for(Np, D * warps);
         // a group's rows are shared out where the groups are fewer than the 32 warps an SM holds (1400 nodes,

@@ -235,6 +235,12 @@ int vpbs_autotune_spread(vpbs_handle* h, int32_t* chosen) {
     return rc;
 }
 
+int vpbs_pair_entries(vpbs_handle* h, int32_t bits) {
+    if (!h || (bits != 0 && bits != 64)) return VPBS_ERR_ARG;
+    h->wide_entries = bits == 64;
+    return 0;
+}
+
 int vpbs_pair_block(vpbs_handle* h, int32_t cells) {
     return !h || cells < 0 || cells > 8 ? VPBS_ERR_ARG : 0;
 }

@@ -197,6 +197,7 @@ struct vpbs_handle {
     int32_t *src_start = nullptr, *dst_start = nullptr;  // of the points' and the nodes' cells, in cell_start
     // [0] in-range pairs, [1] candidates (unsigned long long); in an open domain then the arrivals per block of nodes
     vpbs::DevBuf counters;
+    bool wide_entries = false;  // 64-bit queue entries of the pair kernels whatever the size (vpbs_pair_entries)
     vpbs::DevBuf scan_tmp, scan_tmp_lr;  // multi-CTA scan scratch (cell lists; spreading bins)
     vpbs::DevBuf ewald_tab;  // Taylor tables of the Ewald weights (KParams::ewald_tab)
 
