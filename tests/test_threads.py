@@ -44,6 +44,15 @@ def test_shared_memory_limits_are_fixed():
     assert all(s.startswith("k") or s in ("tsmem", "psmem") for s in sizes), sizes
 
 
+def test_no_lazily_filled_statics():
+    """A static container of a function that is filled on first use would be filled by several threads at once: statics
+    are const (initialised under the compiler's guard), or guarded by a mutex as the copy pool."""
+    csrc = Path(__file__).resolve().parents[1] / "vortexpasta.jl_b200" / "csrc"
+    found = [(f.name, line.strip()) for f in csrc.glob("*.cu*") for line in f.read_text().splitlines()
+             if re.match(r"\s+static (?!const|assert)[\w:<>,\s*&]+;", line)]
+    assert found == [("api.cu", "static std::mutex mu;")], found
+
+
 @pytest.mark.gpu
 def test_filaments_of_different_lengths_in_two_threads(vp):
     """Spline solves of 1000- and 30-node filaments (188 KB and 6 KB of shared memory a block) from two threads."""

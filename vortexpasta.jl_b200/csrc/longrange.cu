@@ -60,8 +60,12 @@ namespace {
 // With u = m sin t (r = cos t) the transform is m int_{-pi/2}^{pi/2} psi(m sin t) cos(xi m sin t) cos t dt,
 // a smooth integrand, evaluated with a 128-point Gauss-Legendre rule.
 double es_hat(double xi, int m, double beta, int kind) {
-    static std::vector<double> gx, gw;
-    if (gx.empty()) gauss_legendre(128, gx, gw);
+    struct Rule {
+        std::vector<double> x, w;
+        Rule() { gauss_legendre(128, x, w); }
+    };
+    static const Rule rule;  // filled once, whichever thread comes first
+    const std::vector<double>&gx = rule.x, &gw = rule.w;
     double s = 0.0;
     for (size_t i = 0; i < gx.size(); ++i) {
         const double th = 0.5 * kPi * gx[i], c = std::cos(th);
