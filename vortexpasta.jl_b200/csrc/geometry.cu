@@ -486,6 +486,7 @@ __device__ __noinline__ void solve_serial(const FilView& f, const double* t, dou
 // dynamic shared memory (smem_n doubles x 12 per warp) when smem_n > 0, else in `scratch`.
 // keep_knots: reuse the knots and periods already in `knots` / `periods` (the knots frozen
 // inside a time step, RK4.jl with update_coefficients!(f; knots = ts_base)).
+// status: set where a filament is too short or too long and left out (null: the host has checked the lengths).
 __global__ void __launch_bounds__(128) spline_solve_kernel(
     int64_t nfil, const int64_t* __restrict__ offsets, const double* __restrict__ X,
     double* __restrict__ knots, double* __restrict__ periods, int32_t* __restrict__ fil_of_node,
@@ -499,7 +500,7 @@ __global__ void __launch_bounds__(128) spline_solve_kernel(
     const int64_t off = offsets[fidx];
     const int n = (int)(offsets[fidx + 1] - off);
     if (n < 5 || (smem_n > 0 && n > smem_n)) {
-        if (lane == 0) atomicExch(status, 1);
+        if (lane == 0 && status) atomicExch(status, 1);
         return;
     }
     const double* Xf = X + 3 * off;
@@ -763,16 +764,15 @@ int geometry_from_filaments(vpbs_handle* h, int64_t nfil, const int64_t* d_offse
     if ((rc = ensure(h, h->coefs, sizeof(double) * 3 * Np, "coefs"))) return rc;
     if ((rc = ensure(h, h->dcoef1, sizeof(double) * 3 * Np, "dcoef1"))) return rc;
     if ((rc = ensure(h, h->dcoef2, sizeof(double) * 3 * Np, "dcoef2"))) return rc;
-    const size_t scratch = sizeof(double) * 12 * Np + 64, part = h->K.open_domain ? open_part_bytes(h) : 0;
+    const size_t scratch = sizeof(double) * 12 * Np, part = h->K.open_domain ? open_part_bytes(h) : 0;
     if ((rc = ensure(h, h->spline_scratch, scratch > part ? scratch : part, "spline scratch"))) return rc;
     double* knots = (double*)h->knots.p;
     double* periods = knots + Np;
-    int32_t* status = (int32_t*)((double*)h->spline_scratch.p + 12 * Np);
     const double* foff = h->have_fil_offsets ? (const double*)h->fil_off.p : nullptr;
     StageScope st(h, ST_GEOMETRY);
     spline_solve_kernel<<<grid_for(nfil, kSolveWarps), 32 * kSolveWarps, smem_bytes, h->stream>>>(
         nfil, d_offsets, d_nodes, knots, periods, (int32_t*)h->fil_of_node.p, (double*)h->coefs.p,
-        (double*)h->dcoef1.p, (double*)h->dcoef2.p, (double*)h->spline_scratch.p, status, smem_n, keep_knots ? 1 : 0,
+        (double*)h->dcoef1.p, (double*)h->dcoef2.p, (double*)h->spline_scratch.p, nullptr, smem_n, keep_knots ? 1 : 0,
         foff);
     h->launches++;
     const bool want_li = h->K.lia_fraction > 0;
