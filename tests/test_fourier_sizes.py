@@ -53,3 +53,19 @@ def test_long_range_over_grid_sizes(vp, oracle, Ns, sigma, precision, tol):
                     assert rel(np.concatenate(out[n]), want) <= tol, (n, names)
     finally:
         cache.close()
+
+
+@pytest.mark.gpu
+def test_memory_of_grids_without_a_plan(vp):
+    """Grids that take cuFFT hold three real values a point, not the four of the interleaved layout, which they never
+    use: 36 bytes a point with the two complex grids, and cuFFT's work space of 24."""
+    import torch
+    p = params(vp, (256, 256, 1080), 1.5, precision="mixed")
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    cache = vp.init_cache(p)
+    used = before - torch.cuda.mem_get_info()[0]
+    cache.close()
+    points = 384 * 384 * 1620
+    modes = 3 * 16 * 129 * 256 * 1080
+    assert used - modes < 62 * points

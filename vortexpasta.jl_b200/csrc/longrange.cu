@@ -1252,9 +1252,6 @@ int longrange_init(vpbs_handle* h) {
     int rc;
     const bool mixed = P.precision == VPBS_PRECISION_MIXED;
     const size_t rsz = mixed ? sizeof(float) : sizeof(double);  // grid precision
-    // room for the interleaved layout (longrange_compute_t) where a later evaluation may take it
-    const size_t per_point = mixed && S.m <= 4 ? sizeof(float4) : 3 * rsz;
-    if ((rc = ensure(h, h->grid_r, per_point * S.ngrid, "real grid"))) return rc;
     if ((rc = ensure(h, h->uhat, sizeof(double2) * 3 * S.nmodes, "uhat"))) return rc;
     // separable deconvolution factors 1/psi_hat and 1/psi_hat * exp(-k^2 / 4 alpha^2) (the
     // Kaiser-Bessel filter is not separable: the Fourier kernel applies it per mode)
@@ -1283,6 +1280,9 @@ int longrange_init(vpbs_handle* h) {
     if ((rc = check_cuda(h, cudaMemcpy(h->decx.p, all.data(), sizeof(double) * tot, cudaMemcpyHostToDevice), "copy tables")))
         return rc;
     if ((rc = fourier_init(h))) return rc;
+    // room for the interleaved layout (longrange_compute_t) where a later evaluation may take it
+    const size_t per_point = mixed && S.m <= 4 && h->fplan ? sizeof(float4) : 3 * rsz;
+    if ((rc = ensure(h, h->grid_r, per_point * S.ngrid, "real grid"))) return rc;
     if (h->fplan) return 0;
     // sizes the pruned transforms do not take (lines longer than a block can hold, or of one factor)
     if ((rc = ensure(h, h->grid_c, 2 * rsz * 3 * S.ncgrid, "complex grid"))) return rc;
