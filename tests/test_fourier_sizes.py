@@ -56,6 +56,26 @@ def test_long_range_over_grid_sizes(vp, oracle, Ns, sigma, precision, tol):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("Ns", [72, 170, 288])
+def test_mixed_transforms_do_not_shrink(vp, Ns):
+    """FFT sizes 108, 256, 432 = 2^a 3^b.  With the transforms' constants rounded to FP32 every pass takes 1e-8 to 2e-8 of
+    the amplitude, and the smooth streamfunction is off by 1.5e-7 to 1.8e-7; rounding that averages out leaves 0.5e-7
+    to 0.9e-7."""
+    rng = np.random.default_rng(6)
+    fs = [vp.curves.ring(200, 0.8 + 0.7 * rng.random(), L * rng.random(3), vp.curves.random_rotation(rng)) for _ in range(100)]
+    got = {}
+    for precision in ("fp64", "mixed"):
+        sp = vp.GaussianSplitting(Ls=L, alpha=Ns / 7.0, rcut=L / 5, Ns=Ns)
+        p = vp.ParamsBiotSavart(Gamma=1.0, a=1e-8, splitting=sp, backend_long=vp.NonuniformFFTsBackend(1.5, 5), precision=precision)
+        cache = vp.init_cache(p)
+        out = [np.zeros((200, 3)) for _ in fs]
+        vp.compute_on_nodes_({"streamfunction": out}, cache, fs, LIA=False, shortrange=False)
+        cache.close()
+        got[precision] = np.concatenate(out)
+    assert rel(got["mixed"], got["fp64"]) <= 1.2e-7
+
+
+@pytest.mark.gpu
 def test_memory_of_grids_without_a_plan(vp):
     """Grids that take cuFFT hold three real values a point, not the four of the interleaved layout, which they never
     use: 36 bytes a point with the two complex grids, and cuFFT's work space of 24."""
