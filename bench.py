@@ -168,7 +168,9 @@ def run_reference(args):
 def stage_model(stage, S):
     """Algorithmic work per launch of each stage: (bound, amount, unit).  S["gsz"] is the grid
     element size (8 bytes in the plain form, 4 in the FP32 forms)."""
-    Np, Nq, n3, nc3, g = S["Np"], S["Nq"], S["n3"], S["nc3"], S["gsz"]
+    Np, Nq, n3, g = S["Np"], S["Nq"], S["n3"], S["gsz"]
+    # complex values that the pruned transforms pass between the dimensions: after x, and after y
+    cx, cy = 3 * S["kept_x"] * 2 * g, 3 * S["kept_xy"] * 2 * g
     if stage == "pairs":
         return S["pair_bound"], S["pairs"] * F_PAIR_VEL, "flop"
     if stage == "spread":
@@ -176,11 +178,12 @@ def stage_model(stage, S):
     if stage == "interp":
         return "hbm", 3 * n3 * g + Np * 3 * 8 + Np * 3 * 8, "byte"
     if stage == "fourier":
-        # reads the retained modes of the forward transform, writes the whole (zero-padded) grid
-        # for the inverse transform and the FP64 vorticity coefficients
-        return "hbm", 3 * S["nm"] * 2 * g + 3 * nc3 * 2 * g + 3 * S["nm"] * 16, "byte"
+        # the z transforms with the operators between them: the kept modes in and out, and the FP64 vorticity
+        # coefficients
+        return "hbm", 2 * cy + 3 * S["nm"] * 16, "byte"
     if stage in ("fft_forward", "fft_inverse"):
-        return "hbm", 2 * 2 * 3 * n3 * g, "byte"
+        # x: the real grid and the kept modes of every line; y: those in, the kept rows out (or the other way)
+        return "hbm", 3 * n3 * g + 2 * cx + cy, "byte"
     if stage == "local_self":
         # per node: position, previous index, s', s'', delta^-, delta^+, output read + write; each
         # quadrature point (position + charge) is gathered by the two nodes of its segment but
@@ -318,8 +321,8 @@ def form_summary(p, m, Np, Nq, world, args, peaks):
     n = [_lib.load().vpbs_fft_size(N, p.backend_long.sigma) for N in p.splitting.Ns]
     fp32 = p.precision == "mixed"
     Ns = p.splitting.Ns
-    S = {"Np": Np, "Nq": Nq, "n3": n[0] * n[1] * n[2], "nc3": (n[0] // 2 + 1) * n[1] * n[2],
-         "nm": (Ns[0] // 2 + 1) * Ns[1] * Ns[2],
+    S = {"Np": Np, "Nq": Nq, "n3": n[0] * n[1] * n[2], "kept_x": Ns[0] // 2 * n[1] * n[2],
+         "kept_xy": Ns[0] // 2 * Ns[1] * n[2], "nm": (Ns[0] // 2 + 1) * Ns[1] * Ns[2],
          "pairs": m["pairs_in_range"], "nq": len(p.quadrature), "gsz": 4 if fp32 else 8,
          "pair_bound": "fp32" if fp32 else "fp64"}
     avg = {k: statistics.mean(v) for k, v in m["stage_ms"].items()}
@@ -467,9 +470,7 @@ def time_ensemble(vp, all_systems, args, local_rank, rank, world, autotune):
            "dt_kelvin_wave_limited_systems": kw_limited,
            "setup_s": t_setup, "finite": nonfinite == 0.0}
     if autotune:
-        out["autotuned"] = {"pair_block_systems_off_rule": sum(1 for t in ens.tuned if t),
-                            "pair_block_edges": sorted(set(ens.tuned)),
-                            "spread_mode_systems_cuda_cores": sum(1 for m in ens.spread_modes if m)}
+        out["autotuned"] = {"spread_mode_systems_cuda_cores": sum(1 for m in ens.spread_modes if m)}
     return out
 
 
@@ -698,8 +699,6 @@ def run_kernel_case(args):
     for name, p in cases:
         c = vp.init_cache(p)
         try:
-            if args.pair_block:
-                _lib.check(_lib.load().vpbs_pair_block(c.handle, args.pair_block), c.handle, "pair_block")
             c.set_filaments(fs)
             c.stage_timing(True)
             for _ in range(3):
@@ -730,8 +729,6 @@ def main():
                     help="RK4 steps of the batching-form ensemble reported under 'ensemble' (0: skip)")
     ap.add_argument("--kernel-case", choices=sorted(KERNEL_CASES), default=None,
                     help="run a small fixed workload for kernel profiling instead of the benchmark")
-    ap.add_argument("--pair-block", type=int, default=0,
-                    help="with --kernel-case: the pair kernel's cells per CTA edge (0: the built-in rule)")
     args = ap.parse_args()
     if args.warmup < 3 and args.impl == "ours":
         print("warning: fewer than 3 warm-up steps", file=sys.stderr)

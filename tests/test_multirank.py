@@ -100,6 +100,9 @@ def test_form_summary_stage_model():
     fs1, p1 = vp.configs.tangle1m()
     out = bench.form_summary(p1, m, 1_000_000, 3_000_000, 1, args, peaks)
     assert out["stages"]["interp"]["frac"] > 0 and out["stages"]["fourier"]["frac"] > 0
+    # the pruned transforms of 768^3 at sigma = 1.5 move 1 + 2 / sigma + 1 / sigma^2 grids each way (2.78 of 10.9 GB)
+    assert out["stages"]["fft_forward"]["achieved"] == pytest.approx((1 + 2 / 1.5 + 1 / 2.25) * 3 * 768 ** 3 * 8 / 1e6)
+    assert out["stages"]["fft_inverse"]["achieved"] == out["stages"]["fft_forward"]["achieved"]
 
 
 def test_bench_world_size_checks(monkeypatch):

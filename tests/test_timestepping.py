@@ -1,5 +1,5 @@
 """Batching form: the on-device RK4 step against a host-driven RK4 built from public velocity
-evaluations, the CUDA-graph ensemble against step-by-step RK4, and the autotuner."""
+evaluations, the CUDA-graph ensemble against step-by-step RK4, and the autotuners."""
 
 import math
 
@@ -92,6 +92,7 @@ def test_ensemble_graph_matches_stepwise_rk4():
 
 @pytest.mark.gpu
 def test_autotune_keeps_results():
+    """The pair kernels have no block size left to choose: the call is accepted and answers with the built-in rule."""
     fs = configs.tangle(40, 100, seed=7)
     p = configs.params_for(L / 8, 3.5, 64, 4)
     c = vp.init_cache(p)
@@ -100,7 +101,7 @@ def test_autotune_keeps_results():
         c.compute(_lib.VELOCITY)
         v0 = c.get(_lib.VELOCITY)
         b = timestepping.autotune(c)
-        assert b in (0, 1, 2, 3, 4)
+        assert b == 0
         c.compute(_lib.VELOCITY)
         v1 = c.get(_lib.VELOCITY)
     finally:

@@ -5,8 +5,8 @@
   (vpbs_rk4_step; knots frozen inside the step as the reference's RK4 does).
 * ``Ensemble``: independent systems (any sizes and grids) advanced together; one RK4 step of all
   of them is captured in one CUDA graph and replayed with one launch per step
-  (vpbs_ensemble_*).  ``autotune_pairs=True`` first runs the pair-kernel and spreading autotuners
-  on every system.
+  (vpbs_ensemble_*).  ``autotune_pairs=True`` first runs the spreading autotuner on every system (the
+  pair kernels, which the name is from, have no choice left to tune).
 
 Device memory for the node arrays comes from torch (plumbing only); every kernel is the
 library's.
@@ -60,8 +60,8 @@ def autotune(cache: BiotSavartCache) -> int:
 
 
 def autotune_spread(cache: BiotSavartCache) -> int:
-    """Pick the spreading mode for the loaded point data (vpbs_spread_mode: 0 tensor cores where they
-    apply, 1 CUDA cores only)."""
+    """Pick the spreading mode for the loaded point data (vpbs_spread_mode: 0 tensor cores or atomics where
+    they apply, 1 bricks on the CUDA cores only)."""
     m = ct.c_int32()
     _lib.check(cache._lib.vpbs_autotune_spread(cache.handle, ct.byref(m)), cache.handle, "autotune_spread")
     return int(m.value)
