@@ -4,7 +4,7 @@
 // memory), multiplies by the twiddles, transforms in registers and writes R values.  Passes within
 // shared memory are in place: every thread keeps its butterflies (32 or 16 values at most) in registers
 // across one barrier, so a line takes no second buffer.  The radices are as large as the registers
-// allow: two passes (one trip through shared memory) up to n = 24 * 32 in FP32 and 256 in FP64.
+// allow: two passes (one trip through shared memory) up to n = 32 * 32 in FP32 and 16 * 16 in FP64.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -16,7 +16,7 @@ namespace fft {
 
 constexpr int kMaxPasses = 6;
 // Complex values a thread keeps across the barrier of a pass.  The wide form (radices up to 32, FP32
-// only) takes 64 registers for them and saves a pass for n = 288 .. 768; else 16 values are kept.
+// only) takes 64 registers for them and saves a pass for most n between 256 and 1024; else 16 values are kept.
 __host__ __device__ constexpr int pass_values(bool wide) { return wide ? 32 : 16; }
 
 // Butterflies of radix R a thread holds in one in-place pass.

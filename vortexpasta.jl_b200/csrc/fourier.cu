@@ -13,8 +13,9 @@
 // every kernel reads all of a line before it writes any of it, so the passes are in place.
 // k_x = Ns0/2 (always zeroed) is never transformed.
 //
-// Bound: HBM traffic of the passes (sigma = 1.5: 4.3 grids of real values in all, against 8 for the
-// unpruned transforms plus 1.3 for a separate operator pass), then shared-memory and issue rate.
+// Bound: HBM traffic of the passes (2 + 4 / sigma + 4 / sigma^2 grids of real values for one field, 6.4 at sigma =
+// 1.5, and the FP64 coefficients; 12 and more for unpruned transforms and an operator pass), then shared-memory
+// and issue rate.
 // Against cuFFT and the separate operator kernel: 768^3 FP64 59.0 -> 29.3 ms when first measured, 25 since;
 // 384^3 FP32, four evaluations, 13.1 -> 5.8 ms; 288^3 FP32 1.39 -> 0.73 ms.
 #include <algorithm>
@@ -516,7 +517,8 @@ bool make_plans(const LRSizes& S, FourierPlan& F, std::vector<unsigned char>& ta
 }  // namespace
 
 // The pruned transforms for the sizes in h->lr, or no plan (h->fplan null) where a line has fewer than
-// two factors or its tile does not fit a block: those sizes use cuFFT.
+// two factors, is longer than 2048, or its tile does not fit a block (z lines of three components above 512 threads:
+// 1620, in FP64 also 1944): those sizes use cuFFT.
 int fourier_init(vpbs_handle* h) {
     const LRSizes& S = h->lr;
     const bool mixed = h->P.precision == VPBS_PRECISION_MIXED;

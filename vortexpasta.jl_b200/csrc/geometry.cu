@@ -195,8 +195,10 @@ __device__ void solve4(double H[4][4], double r[4][3]) {
 //     y_l + A_l b_{l-1} + C_l t_{l+1} = g_l,   y_l = (t_l, b_l): first two and last two unknowns of block l.
 // log2 P steps of cyclic reduction double the distance of the coupling (shuffles between lanes l and l +- s,
 // a 4 x 4 system each) until every block is coupled to itself alone.  Solution in Y[.][0..2].
-// Elimination goes without pivoting: false if a pivot is below 1/16 of the unit diagonal (node spacings that
-// differ by orders of magnitude from one to the next), and the caller solves serially.
+// Nothing is pivoted.  The blocks need it as little as the whole system does (collocation matrices of B-splines are
+// totally positive, and so are their diagonal blocks); the 4 x 4 systems of the reduction are no such matrices:
+// false if a pivot of theirs is below 1/16 of the unit diagonal (node spacings that differ by orders of magnitude
+// from one to the next), and the caller solves serially.
 // Bound: a chain of about n / P + 5 * 4 dependent divisions instead of n (200 nodes: 75 us serially).
 __device__ __noinline__ bool solve_partitioned(const FilView& f, const double* t, double T, const double* Xf, int n,
                                                double o0, double o1, double o2, double* band, double* Y, int lane) {

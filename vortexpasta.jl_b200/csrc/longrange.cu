@@ -208,10 +208,10 @@ __global__ void __launch_bounds__(256) fourier_kernel(
 }
 
 // ---- brick spreading (no global atomics) ----
-// The oversampled grid is tiled into bricks of B^3 points.  Points are binned by the brick
-// holding the first grid point of their footprint; a footprint of w <= B points can then only
-// reach the brick of its bin and the next one in each direction, so brick b collects the points
-// of bins b and b-1 (per dimension, periodic).  Every grid value is written exactly once, with
+// The oversampled grid is tiled into bricks of B^3 points (B = 16 or 8).  Points are binned by the brick
+// holding the first grid point of their footprint.  Bricks of 16 are used for w <= 8 only: a footprint can then
+// only reach the brick of its bin and the next one in each direction, so brick b collects the points of bins b
+// and b-1 (per dimension, periodic); bricks of 8 (w up to 16) collect up to four bins (col_bins).  Every grid value is written exactly once, with
 // plain stores, by the CTA that owns its brick.
 
 __device__ __forceinline__ int footprint_start(double x, double scale, int n, int m) {
@@ -855,7 +855,8 @@ bool spread_by_atomics(const LRSizes& S, int64_t Nq, bool convert) {
 // kernel rows phi_x[8], phi_y[8], phi_z[8], so every point is one unconditional rank-1 update:
 //     acc_c[z] += q_c phi_x[x] phi_y[y] * phi_z[z].
 // A warp covers four y rows and skips the points whose footprint misses them.
-// Bound: the FP64 pipe (28 instructions per point, warp and brick met).  Bricks of 8 instead of 16
+// Bound: shared-memory reads (LSU 71 % busy: a point's eight z values, row factors and charges serve 24 multiply-adds
+// of a thread), then the FP64 pipe (28 instructions per point, warp and brick met).  Bricks of 8 instead of 16
 // give 6.6 (m = 4) or 9.6 (m = 5) bricks met per point instead of 3.0 or 3.8, each of an eighth of the
 // cells: 2.5 to 3.2 times fewer updates with zero.  1M nodes, FP64, 768^3, m = 5: 7.25 ms (16^3 bricks: 13.96);
 // 100k nodes, 288^3, m = 4: 0.43 ms (1.18).  A warp per brick, without barriers, waits for every staging load in
