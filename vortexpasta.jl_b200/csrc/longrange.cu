@@ -10,6 +10,7 @@
 //     times the Ewald Gaussian exp(-k^2/4 alpha^2) (cache_common.jl:64-76) and the type-2
 //     deconvolution, left where the inverse transforms read them;
 //  3. complex-to-real transforms and ES-kernel interpolation at the nodes (type 2).
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 #include <vector>
@@ -789,20 +790,21 @@ __global__ void __launch_bounds__(kTcThreads, 2) spread_tc_kernel(LRSizes S, int
     if (warp == 0) tc::tmem_dealloc(tmem, 128);
 }
 
-// Spreading with global atomics into a zeroed grid, for few points: 32 points per CTA, their kernel values in
-// shared memory, then a thread per x-line of the footprints.  FP32 grids take the sums from an FP64 one (added in
+// Spreading with global atomics into a zeroed grid, for few points: `batch` points per CTA (32; fewer where the
+// points are too few for two CTAs per SM so), their kernel values in shared memory, then a thread per x-line of the
+// footprints.  FP32 grids take the sums from an FP64 one (added in
 // FP32 in this way they would be 1.5 times less accurate than the columns' sums in registers).  Bound: the atomics,
 // 2e11 a second on grids of 54^3 and more, a third of that where a small grid's footprints collide.
 constexpr int kAtomicBatch = 32;
 
-__global__ void __launch_bounds__(256) spread_atomic_kernel(LRSizes S, int64_t Nq, const double* __restrict__ src, double sx0,
-                                                            double sx1, double sx2, double* __restrict__ grid) {
+__global__ void __launch_bounds__(256) spread_atomic_kernel(LRSizes S, int64_t Nq, int batch, const double* __restrict__ src,
+                                                            double sx0, double sx1, double sx2, double* __restrict__ grid) {
     __shared__ double phi[kAtomicBatch][3][2 * kMaxHalfSupport];
     __shared__ int start[kAtomicBatch][3];
     __shared__ double qs[kAtomicBatch][3];
     const int w = 2 * S.m;
-    const int64_t base = (int64_t)blockIdx.x * kAtomicBatch;
-    const int np = (int)(Nq - base < kAtomicBatch ? Nq - base : kAtomicBatch);
+    const int64_t base = (int64_t)blockIdx.x * batch;
+    const int np = (int)(Nq - base < batch ? Nq - base : batch);
     for (int e = threadIdx.x; e < 3 * np; e += blockDim.x) {
         const int p = e / 3, d = e % 3;
         const int64_t j = base + p;
@@ -834,8 +836,8 @@ __global__ void __launch_bounds__(256) grid_to_float_kernel(int64_t n, const dou
 }
 
 // Whether spread_atomic_kernel takes less time than the columns below: 5 ps an update against 40 us (five
-// launches, an empty brick's work) and 0.1 us per point that an average brick meets; 10 ps a grid point where
-// an FP32 grid is converted.  FP64, m = 4: 3,000 points on 54^3 58 us against 84, 60,000 points 546 against 402;
+// launches, an empty brick's work; 30 in FP32) and 0.1 us per point that an average brick meets; 10 ps a grid point
+// where an FP32 grid is converted.  FP64, m = 4: 3,000 points on 54^3 58 us against 84, 60,000 points 546 against 402;
 // 12,000 points on 18^3 (27 bricks for 148 SMs) 0.20 ms against 1.04.
 bool spread_by_atomics(const LRSizes& S, int64_t Nq, bool convert) {
     const double w = 2.0 * S.m;
@@ -844,7 +846,7 @@ bool spread_by_atomics(const LRSizes& S, int64_t Nq, bool convert) {
         const double nb = (S.n[d] + 7) / 8;
         met *= std::fmin(nb, 1.0 + (w - 1.0) / 8.0) / nb;
     }
-    return 5e-6 * 3.0 * w * w * w * (double)Nq + (convert ? 1e-5 * (double)S.ngrid : 0.0) < 40.0 + 0.1 * met;
+    return 5e-6 * 3.0 * w * w * w * (double)Nq + (convert ? 1e-5 * (double)S.ngrid : 0.0) < (convert ? 30.0 : 40.0) + 0.1 * met;
 }
 
 // Register-column spreading for FP64 grids and wide kernels, any grid size, no atomics: one CTA of two
@@ -1253,6 +1255,8 @@ int longrange_init(vpbs_handle* h) {
     int rc;
     const bool mixed = P.precision == VPBS_PRECISION_MIXED;
     const size_t rsz = mixed ? sizeof(float) : sizeof(double);  // grid precision
+    const bool may_interleave = mixed && S.m <= 4;  // longrange_compute_t
+    if (!may_interleave && (rc = ensure(h, h->grid_r, 3 * rsz * S.ngrid, "real grid"))) return rc;
     if ((rc = ensure(h, h->uhat, sizeof(double2) * 3 * S.nmodes, "uhat"))) return rc;
     // separable deconvolution factors 1/psi_hat and 1/psi_hat * exp(-k^2 / 4 alpha^2) (the
     // Kaiser-Bessel filter is not separable: the Fourier kernel applies it per mode)
@@ -1281,9 +1285,8 @@ int longrange_init(vpbs_handle* h) {
     if ((rc = check_cuda(h, cudaMemcpy(h->decx.p, all.data(), sizeof(double) * tot, cudaMemcpyHostToDevice), "copy tables")))
         return rc;
     if ((rc = fourier_init(h))) return rc;
-    // room for the interleaved layout (longrange_compute_t) where a later evaluation may take it
-    const size_t per_point = mixed && S.m <= 4 && h->fplan ? sizeof(float4) : 3 * rsz;
-    if ((rc = ensure(h, h->grid_r, per_point * S.ngrid, "real grid"))) return rc;
+    // room for the interleaved layout where a later evaluation may take it
+    if ((rc = ensure(h, h->grid_r, (may_interleave && h->fplan ? sizeof(float4) : 3 * rsz) * S.ngrid, "real grid"))) return rc;
     if (h->fplan) return 0;
     // sizes the pruned transforms do not take (lines longer than a block can hold, or of one factor)
     if ((rc = ensure(h, h->grid_c, 2 * rsz * 3 * S.ncgrid, "complex grid"))) return rc;
@@ -1379,7 +1382,10 @@ int longrange_compute_t(vpbs_handle* h, int fields) {
                 sums = (double*)h->grid64.p;
             }
             if ((rc = check_cuda(h, cudaMemsetAsync(sums, 0, sizeof(double) * 3 * S.ngrid, h->stream), "memset grid"))) return rc;
-            spread_atomic_kernel<<<grid_for(Nq, kAtomicBatch), 256, 0, h->stream>>>(S, Nq, src, sx[0], sx[1], sx[2], sums);
+            int nsm = 148;
+            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
+            const int batch = (int)std::min<int64_t>(kAtomicBatch, (Nq + 2 * nsm - 1) / (2 * nsm));
+            spread_atomic_kernel<<<grid_for(Nq, batch), 256, 0, h->stream>>>(S, Nq, batch, src, sx[0], sx[1], sx[2], sums);
             h->launches++;
             if constexpr (sizeof(T) == 4) {
                 grid_to_float_kernel<<<grid_for(3 * S.ngrid, 256), 256, 0, h->stream>>>(3 * S.ngrid, sums, grid);
