@@ -17,7 +17,8 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 OUT_DIR = PKG / "lib"
 LIB = OUT_DIR / "libvpbs.so"
-SOURCES = ["api.cu", "geometry.cu", "shortrange.cu", "longrange.cu", "fourier.cu", "features.cu", "mlp.cu", "timestep.cu", "diagnostics.cu", "splitting.cu"]
+SOURCES = ["api.cu", "geometry.cu", "shortrange.cu", "longrange.cu", "fourier.cu", "fourier_f32.cu", "fourier_f64.cu",
+           "features.cu", "mlp.cu", "timestep.cu", "diagnostics.cu", "splitting.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

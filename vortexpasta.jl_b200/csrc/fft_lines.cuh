@@ -145,18 +145,18 @@ __device__ __forceinline__ C rotate(C a, int e, double c, double s) {
     using T = decltype(a.x);
     e %= R;
     if (e == 0) return a;
-    if (4 * e % R == 0) return 4 * e / R == 2 ? mk(-a.x, -a.y) : 4 * e / R == 1 ? mul_i<SIGN>(a) : mul_i<-SIGN>(a);
-    if (8 * e % R == 0) {  // c = +-s
-        const double f = c < 0 ? -c : c;
-        const T u = c < 0 ? -a.x : a.x, v = c < 0 ? -a.y : a.y;
-        return (c > 0) == (SIGN * s > 0) ? mk(times(u - v, f), times(u + v, f)) : mk(times(u + v, f), times(v - u, f));
-    }
-    const T ch = (T)c, sh = (T)(SIGN * s);
-    if constexpr (sizeof(T) == 4) {
-        const T cl = (T)(c - (double)ch), sl = (T)(SIGN * s - (double)sh);
+    if constexpr (sizeof(T) == 8) {
+        return mul(a, mk((T)c, (T)(SIGN * s)));  // (the cases below cost FP64 registers: 6 % of the inverse)
+    } else {
+        if (4 * e % R == 0) return 4 * e / R == 2 ? mk(-a.x, -a.y) : 4 * e / R == 1 ? mul_i<SIGN>(a) : mul_i<-SIGN>(a);
+        if (8 * e % R == 0) {  // c = +-s
+            const double f = c < 0 ? -c : c;
+            const T u = c < 0 ? -a.x : a.x, v = c < 0 ? -a.y : a.y;
+            return (c > 0) == (SIGN * s > 0) ? mk(times(u - v, f), times(u + v, f)) : mk(times(u + v, f), times(v - u, f));
+        }
+        const T ch = (T)c, sh = (T)(SIGN * s), cl = (T)(c - (double)ch), sl = (T)(SIGN * s - (double)sh);
         return mk(fmaf(a.x, ch, fmaf(-a.y, sh, fmaf(a.x, cl, -a.y * sl))), fmaf(a.x, sh, fmaf(a.y, ch, fmaf(a.x, sl, a.y * cl))));
     }
-    return mul(a, mk(ch, sh));
 }
 
 // v <- DFT of v with kernel exp(SIGN 2 pi i n k / R), natural order.
