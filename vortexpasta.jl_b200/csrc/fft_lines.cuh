@@ -133,30 +133,22 @@ struct Units {
 // sqrt(1/2), sqrt(3)/2, cos and sin(pi/8) are all too small, and every value that passes a transform shrinks by
 // 2e-8 to 5e-8 (sizes 2^a 3^b; the streamfunction of a 432^3 grid was off by 1.8e-7, with this 0.5e-7).  The
 // extra instructions cost the FP32 transforms 2 %.
-template <typename T>
-__device__ __forceinline__ T times(T a, double c) {
-    const T hi = (T)c;
-    if constexpr (sizeof(T) == 4) return fmaf(a, hi, a * (T)(c - (double)hi));
-    return a * hi;
+__device__ __forceinline__ float times(float a, double c) {
+    const float hi = (float)c;
+    return fmaf(a, hi, a * (float)(c - (double)hi));
 }
-// a e^{SIGN 2 pi i e / R}, e and R known at compile time
+// a e^{SIGN 2 pi i e / R} in FP32, e (0 < e < R) and R known at compile time
 template <int R, int SIGN, typename C>
 __device__ __forceinline__ C rotate(C a, int e, double c, double s) {
     using T = decltype(a.x);
-    e %= R;
-    if (e == 0) return a;
-    if constexpr (sizeof(T) == 8) {
-        return mul(a, mk((T)c, (T)(SIGN * s)));  // (the cases below cost FP64 registers: 6 % of the inverse)
-    } else {
-        if (4 * e % R == 0) return 4 * e / R == 2 ? mk(-a.x, -a.y) : 4 * e / R == 1 ? mul_i<SIGN>(a) : mul_i<-SIGN>(a);
-        if (8 * e % R == 0) {  // c = +-s
-            const double f = c < 0 ? -c : c;
-            const T u = c < 0 ? -a.x : a.x, v = c < 0 ? -a.y : a.y;
-            return (c > 0) == (SIGN * s > 0) ? mk(times(u - v, f), times(u + v, f)) : mk(times(u + v, f), times(v - u, f));
-        }
-        const T ch = (T)c, sh = (T)(SIGN * s), cl = (T)(c - (double)ch), sl = (T)(SIGN * s - (double)sh);
-        return mk(fmaf(a.x, ch, fmaf(-a.y, sh, fmaf(a.x, cl, -a.y * sl))), fmaf(a.x, sh, fmaf(a.y, ch, fmaf(a.x, sl, a.y * cl))));
+    if (4 * e % R == 0) return 4 * e / R == 2 ? mk(-a.x, -a.y) : 4 * e / R == 1 ? mul_i<SIGN>(a) : mul_i<-SIGN>(a);
+    if (8 * e % R == 0) {  // c = +-s
+        const double f = c < 0 ? -c : c;
+        const T u = c < 0 ? -a.x : a.x, v = c < 0 ? -a.y : a.y;
+        return (c > 0) == (SIGN * s > 0) ? mk(times(u - v, f), times(u + v, f)) : mk(times(u + v, f), times(v - u, f));
     }
+    const T ch = (T)c, sh = (T)(SIGN * s), cl = (T)(c - (double)ch), sl = (T)(SIGN * s - (double)sh);
+    return mk(fmaf(a.x, ch, fmaf(-a.y, sh, fmaf(a.x, cl, -a.y * sl))), fmaf(a.x, sh, fmaf(a.y, ch, fmaf(a.x, sl, a.y * cl))));
 }
 
 // v <- DFT of v with kernel exp(SIGN 2 pi i n k / R), natural order.
@@ -181,7 +173,13 @@ struct Dft<3, SIGN> {
         constexpr double h3 = unit_sin(1, 3);
         const C a = add(v[1], v[2]), d = sub(v[1], v[2]);
         const C m = mk(v[0].x - (T)0.5 * a.x, v[0].y - (T)0.5 * a.y);
-        const C q = mul_i<SIGN>(mk(times(d.x, h3), times(d.y, h3)));
+        C q;
+        if constexpr (sizeof(T) == 8) {
+            const T f = (T)h3;
+            q = mul_i<SIGN>(mk(f * d.x, f * d.y));
+        } else {
+            q = mul_i<SIGN>(mk(times(d.x, h3), times(d.y, h3)));
+        }
         v[0] = add(v[0], a);
         v[1] = add(m, q);
         v[2] = sub(m, q);
@@ -226,6 +224,7 @@ template <int A, int B, int SIGN>
 struct DftAB {
     template <typename C>
     __device__ __forceinline__ static void run(C (&v)[A * B]) {
+        using T = decltype(v[0].x);
         constexpr Units<A * B> U;
         C y[B][A];
 #pragma unroll
@@ -236,7 +235,12 @@ struct DftAB {
             Dft<A, SIGN>::run(t);
 #pragma unroll
             for (int k1 = 0; k1 < A; ++k1) {
-                y[n2][k1] = rotate<A * B, SIGN>(t[k1], n2 * k1, U.c[n2 * k1], U.s[n2 * k1]);
+                if (n2 * k1 == 0)
+                    y[n2][k1] = t[k1];
+                else if constexpr (sizeof(T) == 8)  // plain products: FP64 has no registers for more cases (6 % of the inverse)
+                    y[n2][k1] = mul(t[k1], mk((T)U.c[n2 * k1], (T)(SIGN * U.s[n2 * k1])));
+                else
+                    y[n2][k1] = rotate<A * B, SIGN>(t[k1], n2 * k1, U.c[n2 * k1], U.s[n2 * k1]);
             }
         }
 #pragma unroll
