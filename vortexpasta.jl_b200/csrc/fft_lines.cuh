@@ -1,5 +1,5 @@
 // One-dimensional FFTs of lines held in shared memory, for the pruned 3-D transforms of the long
-// range (fourier.cu): Stockham passes of radix 2..32 (FP64: 2..16), any length 2^a 3^b 5^c with at least
+// range (fourier_kernels.cuh): Stockham passes of radix 2..32 (FP64: 2..16), any length 2^a 3^b 5^c with at least
 // two factors.  A pass reads R values per butterfly (from memory in the first pass, else from shared
 // memory), multiplies by the twiddles, transforms in registers and writes R values.  Passes within
 // shared memory are in place: every thread keeps its butterflies (32 or 16 values at most) in registers

@@ -142,7 +142,7 @@ struct LRSizes {
     int kernel;      // VPBS_NUFFT_*
 };
 
-// What the Fourier-space pass does between the forward and the inverse z transforms (fourier.cu).
+// What the Fourier-space pass does between the forward and the inverse z transforms (fourier_kernels.cuh).
 struct FourierOp {
     enum Source { GRID, COEFFICIENTS };  // the spread grid's transform, or the held coefficients
     enum Quantity { VORTICITY = 1, STREAMFUNCTION = 2, VELOCITY = 3 };
