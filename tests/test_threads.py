@@ -37,7 +37,7 @@ def test_shared_memory_limits_are_fixed():
     """cudaFuncSetAttribute changes the function, for every handle of the process: its sizes are constants (or sizes of
     types), never what one call needs, or a call with less could fail a concurrent launch that needs more."""
     csrc = Path(__file__).resolve().parents[1] / "vortexpasta.jl_b200" / "csrc"
-    sizes = [m for f in csrc.glob("*.cu") for m in
+    sizes = [m for f in csrc.glob("*.cu*") for m in
              re.findall(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*\(int\)\s*\(?(\w+)", f.read_text())]
     assert len(sizes) >= 6
     # k...: constants; tsmem, psmem: the size of a type and of the plane kernel's tile, one per template instance
