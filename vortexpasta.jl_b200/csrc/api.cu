@@ -154,11 +154,13 @@ int process_point_charges(vpbs_handle* h) {
 
 using namespace vpbs;
 
-// Both pair weights at x in extended precision: of the Kaiser-Bessel series S over x = (xmax / rcut) r, or the
-// Gaussian ones where there is none.
+// Both pair weights in extended precision: of the Kaiser-Bessel series S over x = (xmax / rcut) r, or the Gaussian ones
+// where there is none.
 static WeightsL pair_weights_l(const KBSeries& S, double xmax) {
     if (S.f.empty()) return gaussian_weights_l;
-    return [&S, xmax](long double x, long double* a, long double* g) { kb_weights_series_l(S, x * S.rcut / xmax, a, g); };
+    return [&S, xmax](long double x, const long double* h, int n, long double* a, long double* g) {
+        for (int i = 0; i < n; ++i) kb_weights_series_l(S, (x + h[i]) * S.rcut / xmax, &a[i], &g[i]);
+    };
 }
 
 extern "C" {

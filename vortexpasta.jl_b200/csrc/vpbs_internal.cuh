@@ -62,12 +62,12 @@ void f32_table_host(const double* tab, int ntab, double xmax, float4* out);  // 
 // Device-identical host evaluation of the FP32 cubic tables (same float operations).
 void f32_table_eval_host(const float4* tabc, int nf, float x, float* a, float* g);
 
-// FP64 tables of KParams::tab_s over [0, xmax], fitted to weights given in extended precision (a and g at x):
-// 2 tab_s_size(xmax) kTabSNC values.
+// FP64 tables of KParams::tab_s over [0, xmax], fitted to weights given in extended precision (a and g at the n
+// places x + h[i], |h[i]| <= 1/256): 2 tab_s_size(xmax) kTabSNC values.
 constexpr double kTabSInvH = 128.0;
 constexpr int kTabSNC = 6;
-using WeightsL = std::function<void(long double x, long double* a, long double* g)>;
-void gaussian_weights_l(long double x, long double* a, long double* g);
+using WeightsL = std::function<void(long double x, const long double* h, int n, long double* a, long double* g)>;
+void gaussian_weights_l(long double x, const long double* h, int n, long double* a, long double* g);
 int tab_s_size(double xmax);
 void tab_s_host(const WeightsL& weights, double xmax, double* out);
 void tab_s_eval_host(const double* tab, int nf, double x, double* a, double* g);  // as the kernel does
